@@ -47,22 +47,22 @@ def listed():
         # a batch of requests through layers without a fused chain: many small products a step
         dict(name="fotulix sixteen requests", kind="engine", family="fotulix", requests=16, prompt=300, tokens=16),
         # the prompt of the headline benchmark, attention layer of the 8B sizes
-        dict(name="attention, prompt 2048", kind="gqa", size="8b", dtype="bfloat16", requests=1, tokens=2048, past=0),
+        dict(name="attention prompt 2048", kind="gqa", size="8b", dtype="bfloat16", requests=1, tokens=2048, past=0),
         # the headline decode: eight requests at 4,096 keys, 1B sizes
-        dict(name="attention, 8 tokens", kind="gqa", size="1b", dtype="bfloat16", requests=8, tokens=1, past=4095),
+        dict(name="attention 8 tokens", kind="gqa", size="1b", dtype="bfloat16", requests=8, tokens=1, past=4095),
         # the 32-bit engine, which logits are checked against
-        dict(name="attention fp32, prompt 300", kind="gqa", size="1b", dtype="float32", requests=1, tokens=300, past=0),
+        dict(name="attention fp32 prompt 300", kind="gqa", size="1b", dtype="float32", requests=1, tokens=300, past=0),
         # a feed-forward over a prompt
-        dict(name="mlp, prompt 2048", kind="mlp", size="1b", dtype="bfloat16", requests=1, tokens=2048, past=0),
+        dict(name="mlp prompt 2048", kind="mlp", size="1b", dtype="bfloat16", requests=1, tokens=2048, past=0),
         # experts in a decode step
-        dict(name="experts, 8 tokens", kind="experts", size="w1024", dtype="bfloat16", requests=8, tokens=1, past=0),
+        dict(name="experts 8 tokens", kind="experts", size="w1024", dtype="bfloat16", requests=8, tokens=1, past=0),
         # a family's attention over a prompt, with the bias by distance
-        dict(name="biased attention, prompt 2048", kind="bias", size="w2048", dtype="bfloat16", requests=1, tokens=2048, past=0),
+        dict(name="biased attention prompt 2048", kind="bias", size="w2048", dtype="bfloat16", requests=1, tokens=2048, past=0),
         # recurrences over prompts: one long one, ragged ones side by side, two, one
-        dict(name="gated linear, prompt 2048", kind="gla", size="w2048", dtype="bfloat16", requests=1, tokens=2048, past=0),
-        dict(name="delta rule, ragged prompts", kind="delta", size="w2048", dtype="bfloat16", requests=4, tokens=611, past=0),
-        dict(name="retention, two prompts", kind="retention", size="w2048", dtype="bfloat16", requests=2, tokens=1000, past=0),
-        dict(name="state space, prompt 2048", kind="mamba2", size="w1024", dtype="bfloat16", requests=1, tokens=2048, past=0),
+        dict(name="gated linear prompt 2048", kind="gla", size="w2048", dtype="bfloat16", requests=1, tokens=2048, past=0),
+        dict(name="delta rule ragged prompts", kind="delta", size="w2048", dtype="bfloat16", requests=4, tokens=611, past=0),
+        dict(name="retention two prompts", kind="retention", size="w2048", dtype="bfloat16", requests=2, tokens=1000, past=0),
+        dict(name="state space prompt 2048", kind="mamba2", size="w1024", dtype="bfloat16", requests=1, tokens=2048, past=0),
     ]
 
 
