@@ -255,7 +255,7 @@ gated_scan_kernel(const TA* __restrict__ q, int q_stride, const TA* __restrict__
                   const TA* __restrict__ v, int v_stride, const float* __restrict__ alpha, int a_stride,
                   float q_scale, float* __restrict__ out,
                   float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
-                  int H, int dv, int vec) {
+                  int H, int dv, int vec, int below) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -266,6 +266,7 @@ gated_scan_kernel(const TA* __restrict__ q, int q_stride, const TA* __restrict__
     const int lt = tid - WORKERS;
     const int cg = tid / R, rg = tid % R;                    // of the computing threads: column group, lane in it
     const int t_begin = cu_q[b], t_end = cu_q[b + 1];
+    if (below > 0 && t_end - t_begin >= below) return;       // this entry goes in chunks
     const int rounds = (t_end - t_begin + TC - 1) / TC;
     if (DKP != DK) {                                         // rows beyond DK stay zero
         for (int e = tid; e < 2 * HALF; e += THREADS) smem[e] = 0.f;
@@ -439,7 +440,7 @@ delta_scan_kernel(const TA* __restrict__ r, int r_stride, const TA* __restrict__
                   const TA* __restrict__ v, int v_stride, const float* __restrict__ w, const float* __restrict__ u,
                   const float* __restrict__ au, int f_stride, float* __restrict__ out,
                   float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
-                  int H, int dv, int vec) {
+                  int H, int dv, int vec, int below) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -450,6 +451,7 @@ delta_scan_kernel(const TA* __restrict__ r, int r_stride, const TA* __restrict__
     const int lt = tid - WORKERS;
     const int cg = tid / R, rg = tid % R;
     const int t_begin = cu_q[b], t_end = cu_q[b + 1];
+    if (below > 0 && t_end - t_begin >= below) return;       // this entry goes in chunks
     const int rounds = (t_end - t_begin + TC - 1) / TC;
     if (DKP != DK) {
         for (int e = tid; e < 2 * HALF; e += THREADS) smem[e] = 0.f;
@@ -689,7 +691,7 @@ __global__ void __launch_bounds__(THREADS, DK <= 128 ? 2 : 1)
 head_scan_kernel(const TA* __restrict__ q, int q_stride, const TA* __restrict__ k, int k_stride, const TA* __restrict__ v,
                  int v_stride, const float* __restrict__ decay, int a_stride, const float* __restrict__ gain, int g_stride,
                  float q_scale, float* __restrict__ out, float* __restrict__ state, const int* __restrict__ cu_q,
-                 const int* __restrict__ state_slots, int H, int dv, int share, int vec) {
+                 const int* __restrict__ state_slots, int H, int dv, int share, int vec, int below) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -701,6 +703,7 @@ head_scan_kernel(const TA* __restrict__ q, int q_stride, const TA* __restrict__ 
     const int lt = tid - WORKERS;
     const int cg = tid / R, rg = tid % R;
     const int t_begin = cu_q[b], t_end = cu_q[b + 1];
+    if (below > 0 && t_end - t_begin >= below) return;       // this entry goes in chunks
     const int rounds = (t_end - t_begin + TC - 1) / TC;
     if (DKP != DK) {                                         // rows beyond DK stay zero
         for (int e = tid; e < 2 * HALF; e += THREADS) smem[e] = 0.f;
@@ -850,7 +853,7 @@ head_scan_async_kernel(const float* __restrict__ q, int q_stride, const float* _
                        const float* __restrict__ v, int v_stride, const float* __restrict__ decay, int a_stride,
                        const float* __restrict__ gain, int g_stride, float q_scale, float* __restrict__ out,
                        float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
-                       int H, int dv, int share) {
+                       int H, int dv, int share, int below) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -862,6 +865,7 @@ head_scan_async_kernel(const float* __restrict__ q, int q_stride, const float* _
     const int lt = tid - WORKERS;
     const int cg = tid / R, rg = tid % R;
     const int t_begin = cu_q[b], t_end = cu_q[b + 1];
+    if (below > 0 && t_end - t_begin >= below) return;       // this entry goes in chunks
     const int rounds = (t_end - t_begin + TC - 1) / TC;
     if (DKP != DK || !gain) {                                // rows beyond DK stay zero; without gains they stay one
         for (int e = tid; e < HEAD_STAGES * HALF; e += THREADS) smem[e] = e % HALF >= HALF - TC ? 1.f : 0.f;
@@ -1155,10 +1159,11 @@ int allow_shared(Kernel kernel, size_t bytes) {
 RI_API int ri_recurrent_key_dim() { return DK; }
 RI_API int ri_recurrent_state_rows() { return DKP; }
 
-// `single` != 0: every entry brings exactly one token (the kernel without staging takes the step)
-RI_API int ri_gated_scan(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
+// `single` != 0: every entry brings exactly one token (the kernel without staging takes the step).  `below` > 0: only the
+// entries of fewer tokens (the others go in chunks, recurrent_chunks.cu).
+RI_API int ri_gated_scan_short(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
                          const float* alpha, int a_stride, int act_dtype, float q_scale, float* out, float* state,
-                         const int* cu_q, const int* state_slots, int entries, int H, int dv, int single,
+                         const int* cu_q, const int* state_slots, int entries, int H, int dv, int single, int below,
                          void* stream) {
     if (entries <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
@@ -1177,17 +1182,24 @@ RI_API int ri_gated_scan(const void* q, int q_stride, const void* k, int k_strid
     if (!allowed) { RI_CHECKED(allow_shared(gated_scan_kernel<TA>, smem)); allowed = true; } \
     RI_CHECKED(ri_launch(gated_scan_kernel<TA>, grid, dim3(THREADS), smem, s, (const TA*)q, q_stride, \
         (const TA*)k, k_stride, (const TA*)v, v_stride, alpha, a_stride, q_scale, out, state, \
-        cu_q, state_slots, H, dv, vec)); } while (0)
+        cu_q, state_slots, H, dv, vec, below)); } while (0)
     if (act_dtype == RI_BF16) RI_GS(bf16);
     else RI_GS(float);
 #undef RI_GS
     return ri_launch_status();
 }
 
-RI_API int ri_delta_scan(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride,
+RI_API int ri_gated_scan(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
+                         const float* alpha, int a_stride, int act_dtype, float q_scale, float* out, float* state,
+                         const int* cu_q, const int* state_slots, int entries, int H, int dv, int single, void* stream) {
+    return ri_gated_scan_short(q, q_stride, k, k_stride, v, v_stride, alpha, a_stride, act_dtype, q_scale, out, state, cu_q,
+                               state_slots, entries, H, dv, single, 0, stream);
+}
+
+RI_API int ri_delta_scan_short(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride,
                          const float* w, const float* u, const float* au, int f_stride, int act_dtype,
                          float* out, float* state, const int* cu_q, const int* state_slots, int entries, int H,
-                         int dv, int single, void* stream) {
+                         int dv, int single, int below, void* stream) {
     if (entries <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const dim3 grid((dv + COLS - 1) / COLS, H, entries);
@@ -1204,7 +1216,7 @@ RI_API int ri_delta_scan(const void* r, int r_stride, const void* k, int k_strid
     static bool allowed = false; \
     if (!allowed) { RI_CHECKED(allow_shared(delta_scan_kernel<TA>, smem)); allowed = true; } \
     RI_CHECKED(ri_launch(delta_scan_kernel<TA>, grid, dim3(THREADS), smem, s, (const TA*)r, r_stride, \
-        (const TA*)k, k_stride, (const TA*)v, v_stride, w, u, au, f_stride, out, state, cu_q, state_slots, H, dv, vec)); \
+        (const TA*)k, k_stride, (const TA*)v, v_stride, w, u, au, f_stride, out, state, cu_q, state_slots, H, dv, vec, below)); \
     } while (0)
     if (act_dtype == RI_BF16) RI_DS(bf16);
     else RI_DS(float);
@@ -1212,13 +1224,20 @@ RI_API int ri_delta_scan(const void* r, int r_stride, const void* k, int k_strid
     return ri_launch_status();
 }
 
+RI_API int ri_delta_scan(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride,
+                         const float* w, const float* u, const float* au, int f_stride, int act_dtype, float* out, float* state,
+                         const int* cu_q, const int* state_slots, int entries, int H, int dv, int single, void* stream) {
+    return ri_delta_scan_short(r, r_stride, k, k_stride, v, v_stride, w, u, au, f_stride, act_dtype, out, state, cu_q, state_slots,
+                               entries, H, dv, single, 0, stream);
+}
+
 // The head form: see head_scan_kernel.  share: heads that read one key head.  cos_t / sin_t with positions (with `single`
 // only; else null): keys and queries are rotated on the way in (see StepRotation).
-RI_API int ri_head_scan(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
+RI_API int ri_head_scan_short(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
                         const float* decay, int a_stride, const float* gain, int g_stride, int act_dtype, float q_scale,
                         float* out, float* state, const int* cu_q, const int* state_slots, int entries, int H, int dv,
                         int share, const int* positions, const float* cos_t, const float* sin_t, int rot, int interleaved,
-                        int single, void* stream) {
+                        int single, int below, void* stream) {
     if (entries <= 0) return 0;
     if (share <= 0 || H % share || (cos_t && (!single || !positions || !sin_t || rot < 2 || rot > DK || (rot & 1))))
         return (int)cudaErrorInvalidValue;
@@ -1241,7 +1260,7 @@ RI_API int ri_head_scan(const void* q, int q_stride, const void* k, int k_stride
     const size_t smem = 2 * (size_t)HeadShape<C>::HALF * sizeof(float); \
     if (!allowed) { RI_CHECKED(allow_shared(head_scan_kernel<TA>, smem)); allowed = true; } \
     RI_CHECKED(ri_launch(head_scan_kernel<TA>, grid, dim3(THREADS), smem, s, (const TA*)q, q_stride, (const TA*)k, k_stride, \
-        (const TA*)v, v_stride, decay, a_stride, gain, g_stride, q_scale, out, state, cu_q, state_slots, H, dv, share, vec)); \
+        (const TA*)v, v_stride, decay, a_stride, gain, g_stride, q_scale, out, state, cu_q, state_slots, H, dv, share, vec, below)); \
     } while (0)
 #define RI_HSA(CC) do { \
     static bool allowed = false; \
@@ -1249,7 +1268,7 @@ RI_API int ri_head_scan(const void* q, int q_stride, const void* k, int k_stride
     if (!allowed) { RI_CHECKED(allow_shared(head_scan_async_kernel<CC>, smem)); allowed = true; } \
     const dim3 g((dv + HeadShape<CC>::COLS - 1) / HeadShape<CC>::COLS, H, entries); \
     RI_CHECKED(ri_launch(head_scan_async_kernel<CC>, g, dim3(THREADS), smem, s, (const float*)q, q_stride, (const float*)k, k_stride, \
-        (const float*)v, v_stride, decay, a_stride, gain, g_stride, q_scale, out, state, cu_q, state_slots, H, dv, share)); \
+        (const float*)v, v_stride, decay, a_stride, gain, g_stride, q_scale, out, state, cu_q, state_slots, H, dv, share, below)); \
     return ri_launch_status(); } while (0)
     if (!single && act_dtype == RI_F32 && vec && dv % 4 == 0 && v_stride % 4 == 0 && aligned4(v, 4)) {
         if (narrow) RI_HSA(C / 2);
@@ -1260,6 +1279,15 @@ RI_API int ri_head_scan(const void* q, int q_stride, const void* k, int k_stride
 #undef RI_HS
 #undef RI_HSA
     return ri_launch_status();
+}
+
+RI_API int ri_head_scan(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
+                        const float* decay, int a_stride, const float* gain, int g_stride, int act_dtype, float q_scale,
+                        float* out, float* state, const int* cu_q, const int* state_slots, int entries, int H, int dv,
+                        int share, const int* positions, const float* cos_t, const float* sin_t, int rot, int interleaved,
+                        int single, void* stream) {
+    return ri_head_scan_short(q, q_stride, k, k_stride, v, v_stride, decay, a_stride, gain, g_stride, act_dtype, q_scale, out, state,
+                              cu_q, state_slots, entries, H, dv, share, positions, cos_t, sin_t, rot, interleaved, single, 0, stream);
 }
 
 RI_API void ri_set_pdl(int on) { ri_pdl_flag() = on ? 1 : 0; }

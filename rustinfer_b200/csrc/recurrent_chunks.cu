@@ -1,0 +1,940 @@
+// The recurrences with decays over long portions of a prompt, in chunks of 64 tokens as matrix products (compiled with
+// recurrent.cu for one key size; key sizes 64 and 128, value sizes that are multiples of 64):
+//
+//   head    S_t = a_t S_{t-1} + k_t (g_t v_t)^T         o_t = S_t^T q_t      a, g one number a head
+//   gated   S_t = diag(alpha_t) S_{t-1} + k_t v_t^T     o_t = S_t^T q_t
+//
+// The walk of recurrent.cu takes a prompt token by token: one request offers heads x value channels of columns, and every
+// column's state waits for the last token's.  With D_ij the product of the decays of the tokens j + 1 .. i, a chunk that starts
+// from the state S is
+//
+//   O = (Q * D_i0) S + (Q K^T * D) V                    (D_ij = 0 for j > i)
+//   S' = D_end,0 S + (K * D_end,j)^T V
+//
+// so the chunks' own contributions (K * D)^T V need no state (`chunk_states`, all chunks at once), the state in front of every
+// chunk is a sum over chunks, element by element (`chunk_scan`), and the outputs are products again (`chunk_outputs`).
+//
+// Everything stays 32-bit: a factor is cut into three bf16 pieces whose sum it is, and the six products of pieces above 2^-24
+// are added up in fp32 on the tensor cores, the small ones first.  bf16 inputs are one piece.  The products of decays are formed
+// by multiplication, never as quotients or through logarithms, so they stay below one and a decay of zero is a zero.  A value
+// that is no number keeps out of the products (zero times infinity in a masked place would reach earlier tokens) and makes its
+// column's later outputs NaN by itself.
+#include "common.cuh"
+
+#ifndef RI_KDIM
+#error "compile with -DRI_KDIM=<key size>"
+#endif
+
+namespace {
+constexpr int CK = 64;                          // tokens of a chunk
+constexpr bool BUILT = RI_KDIM == 64 || RI_KDIM == 128;
+}
+
+#if RI_KDIM == 64 || RI_KDIM == 128
+namespace {
+constexpr int DK = RI_KDIM;
+constexpr int KP = DK + 8;                      // bf16 of a padded row: an odd count of 16-byte pieces, ldmatrix meets no conflict
+constexpr int QUARTERS = CK / 16;
+
+// The entry and tokens of chunk `index` among the entries that bring at least `least` tokens.
+struct Chunk { int entry, t0, n; };
+__device__ __forceinline__ int chunks_of(int tokens, int least) { return tokens >= least ? (tokens + CK - 1) / CK : 0; }
+
+// every lane of a warp calls; entry -1: no such chunk
+__device__ __forceinline__ Chunk find_chunk(const int* cu_q, int entries, int least, int index) {
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    for (int e0 = 0; e0 < entries; e0 += 32) {
+        const int e = e0 + lane;
+        const int begin = e < entries ? cu_q[e] : 0, len = e < entries ? cu_q[e + 1] - begin : 0;
+        const int own = chunks_of(len, least);
+        int sum = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += up;
+        }
+        const int at = index - base - (sum - own);           // the chunk's number in this lane's entry
+        const unsigned hit = __ballot_sync(0xffffffffu, at >= 0 && at < own);
+        if (hit) {
+            const int src = __ffs(hit) - 1, a = __shfl_sync(0xffffffffu, at, src);
+            Chunk c;
+            c.entry = e0 + src;
+            c.t0 = __shfl_sync(0xffffffffu, begin, src) + a * CK;
+            c.n = min(CK, __shfl_sync(0xffffffffu, len, src) - a * CK);
+            return c;
+        }
+        base += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    return Chunk{-1, 0, 0};
+}
+// number of the first chunk of entry `e` (every lane of a warp calls)
+__device__ __forceinline__ int first_chunk(const int* cu_q, int e, int least) {
+    int sum = 0;
+    for (int i = threadIdx.x & 31; i < e; i += 32) sum += chunks_of(cu_q[i + 1] - cu_q[i], least);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return sum;
+}
+
+// ---- pieces
+__device__ __forceinline__ uint32_t pair_bf16(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ float low_of(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float high_of(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+// x, y -> their pieces as bf16 pairs, each the rounded rest of the one before: their sum is the number, and what the products
+// left out add up to has either sign
+__device__ __forceinline__ void cut(float x, float y, uint32_t (&p)[3]) {
+    p[0] = pair_bf16(x, y);
+    x -= low_of(p[0]); y -= high_of(p[0]);
+    p[1] = pair_bf16(x, y);
+    p[2] = pair_bf16(x - low_of(p[1]), y - high_of(p[1]));
+}
+// four neighbours into a tile of P pieces: `tile` points at the first one's place in piece 0, pieces lie `stride` bf16 apart
+template <int P>
+__device__ __forceinline__ void put4(bf16* tile, size_t stride, float4 x) {
+    if constexpr (P == 1) {
+        *reinterpret_cast<uint2*>(tile) = make_uint2(pair_bf16(x.x, x.y), pair_bf16(x.z, x.w));
+    } else {
+        uint32_t lo[3], hi[3];
+        cut(x.x, x.y, lo);
+        cut(x.z, x.w, hi);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(tile + p * stride) = make_uint2(lo[p], hi[p]);
+    }
+}
+// one number into three tiles
+__device__ __forceinline__ void put1(bf16* tile, int stride, float x) {
+    uint32_t p[3];
+    cut(x, 0.f, p);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<unsigned short*>(tile + i * stride) = (unsigned short)p[i];
+}
+
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    return make_float4(low_of(raw.x), high_of(raw.x), low_of(raw.y), high_of(raw.y));
+}
+__device__ __forceinline__ float4 times(float4 v, float s) { return make_float4(v.x * s, v.y * s, v.z * s, v.w * s); }
+__device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+
+// ---- fragments of m16n8k16
+__device__ __forceinline__ void ldsm(uint32_t (&r)[4], const bf16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm_t(uint32_t (&r)[4], const bf16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// where a lane's ldmatrix row lies in a 16 x 16 block of rows of `ld` bf16
+__device__ __forceinline__ int at_a(int lane, int ld) { return (lane & 15) * ld + (lane >> 4) * 8; }                          // A of [m][k]
+__device__ __forceinline__ int at_at(int lane, int ld) { return ((lane & 7) + (lane >> 4) * 8) * ld + ((lane >> 3) & 1) * 8; } // A of [k][m], trans
+__device__ __forceinline__ int at_b(int lane, int ld) { return ((lane & 7) + (lane >> 4) * 8) * ld + ((lane >> 3) & 1) * 8; }  // B of [n][k]
+__device__ __forceinline__ int at_bt(int lane, int ld) { return ((lane & 7) + ((lane >> 3) & 1) * 8) * ld + (lane >> 4) * 8; } // B of [k][n], trans
+
+// d[m][n] += A B over one step of 16: the products of pieces that matter, the small ones first.  The tensor core cuts off what
+// its accumulator has no bits for, half a unit of the last place a product on average and always downwards: a chain of them
+// into one accumulator was ten times further from the 64-bit sum than the token-by-token walk.  So a step's products start
+// from zero and join the sum by one rounded addition.
+template <int MT, int NT, int PA, int PB>
+__device__ __forceinline__ void products(float (&d)[MT][2 * NT][4], const uint32_t (&a)[PA][MT][4], const uint32_t (&b)[PB][NT][4]) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+        float x[2 * NT][4] = {};
+#pragma unroll
+        for (int s = PA + PB - 2; s >= 0; --s) {
+            if (s > 2) continue;                             // below 2^-24 of the product
+#pragma unroll
+            for (int pa = 0; pa < PA; ++pa) {
+                const int pb = s - pa;
+                if (pb < 0 || pb >= PB) continue;
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    mma(x[2 * n], a[pa][m], b[pb][n][0], b[pb][n][1]);
+                    mma(x[2 * n + 1], a[pa][m], b[pb][n][2], b[pb][n][3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < 2 * NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d[m][n][e] += x[n][e];
+    }
+}
+
+// Products of a head's decays inside a chunk, by one warp: pre[i] = a_0 .. a_i, suf[j] = a_{j+1} .. a_last; tokens behind the
+// chunk's end have decay 1.  Returns the product of all.  In 64 bits: with one fixed decay the roundings of 32-bit products
+// all fall the same way, and the next chunk's again.
+__device__ __forceinline__ double chunk_products(const float* a, float* pre, float* suf) {
+    const int lane = threadIdx.x & 31;
+    const double x = a[2 * lane], y = a[2 * lane + 1], xy = x * y;
+    double up = xy, down = xy;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, up, o), d = __shfl_down_sync(0xffffffffu, down, o);
+        if (lane >= o) up *= u;
+        if (lane + o < 32) down *= d;
+    }
+    double before = __shfl_up_sync(0xffffffffu, up, 1), after = __shfl_down_sync(0xffffffffu, down, 1);
+    if (lane == 0) before = 1.0;
+    if (lane == 31) after = 1.0;
+    if (pre) { pre[2 * lane] = (float)(before * x); pre[2 * lane + 1] = (float)up; }
+    if (suf) { suf[2 * lane] = (float)(y * after); suf[2 * lane + 1] = (float)after; }
+    return __shfl_sync(0xffffffffu, down, 0);
+}
+
+// ------------------------------------------------------------------------------------------------- the chunks' own contributions
+// dS[value channel][key channel] of one chunk and a tile of VT value channels of one key head (several heads' where they share
+// their keys).  Eight warps, 2 x 4 over 64 value channels at a time.  GATED: a decay a key channel, on the keys; else one a
+// head, on the values.  Totals: the products of a chunk's decays, as two floats whose sum is the 64-bit product (head form),
+// one a key channel (gated form).
+constexpr int ST_THREADS = 256;
+template <typename TA, int VT, bool GATED>
+constexpr int states_bytes() {
+    return ((sizeof(TA) == 2 && !GATED ? 1 : 3) * CK * KP + (GATED ? 1 : 3) * CK * (VT + 8)) * 2 + (GATED ? QUARTERS * DK : 4 * CK) * 4;
+}
+
+template <typename TA, int VT, bool GATED>
+__global__ void __launch_bounds__(ST_THREADS, 2)
+chunk_states_kernel(const TA* __restrict__ k, int k_stride, const TA* __restrict__ v, int v_stride,
+                    const float* __restrict__ decay, int a_stride, const float* __restrict__ gain, int g_stride,
+                    float* __restrict__ states, float* __restrict__ totals, const int* __restrict__ cu_q, int entries,
+                    int least, int H, int dv, int share) {
+    constexpr int PK = sizeof(TA) == 2 && !GATED ? 1 : 3, PV = GATED ? 1 : 3, VP = VT + 8;
+    static_assert(!GATED || sizeof(TA) == 2, "the gated form takes bf16 values as they come");
+    extern __shared__ __align__(16) unsigned char raw[];
+    bf16* ks = reinterpret_cast<bf16*>(raw);                 // [PK][CK][KP]
+    bf16* vs = ks + PK * CK * KP;                            // [PV][CK][VP]
+    float* fs = reinterpret_cast<float*>(vs + PV * CK * VP); // a[2][CK], suf[2][CK], or the quarters' products [4][DK]
+    pdl_trigger();
+    pdl_wait();
+    const Chunk c = find_chunk(cu_q, entries, least, blockIdx.x);
+    if (c.entry < 0) return;
+    const int kh = blockIdx.y, c0 = blockIdx.z * VT, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col0 = kh * share * dv + c0;                   // the tile's first column of v
+    constexpr int VN = CK * VT / 4 / ST_THREADS;
+    if constexpr (!GATED) {
+        constexpr int KN = CK * DK / 4 / ST_THREADS;
+        float4 kv[KN], vv[VN];
+#pragma unroll
+        for (int j = 0; j < KN; ++j) {
+            const int e = tid + j * ST_THREADS, t = e / (DK / 4), i = (e % (DK / 4)) * 4;
+            kv[j] = t < c.n ? load4(k + (size_t)(c.t0 + t) * k_stride + (size_t)kh * DK + i) : zero4();
+        }
+#pragma unroll
+        for (int j = 0; j < VN; ++j) {
+            const int e = tid + j * ST_THREADS, t = e / (VT / 4), i = (e % (VT / 4)) * 4;
+            vv[j] = t < c.n ? load4(v + (size_t)(c.t0 + t) * v_stride + col0 + i) : zero4();
+        }
+        const int first_head = kh * share + c0 / dv, heads = VT > dv ? VT / dv : 1;      // at most two
+        float* a = fs + (warp & 1) * CK;
+        if (warp < heads) {
+            for (int t = lane; t < CK; t += 32) a[t] = t < c.n ? decay[(size_t)(c.t0 + t) * a_stride + first_head + warp] : 1.f;
+            __syncwarp();
+            float* suf = fs + 2 * CK + warp * CK;
+            const double total = chunk_products(a, nullptr, suf);
+            if (lane == 0 && c0 % dv == 0) {
+                float* to = totals + ((size_t)blockIdx.x * H + first_head + warp) * 2;
+                const float hi = (float)total;
+                to[0] = hi;
+                to[1] = (float)(total - (double)hi);
+            }
+            __syncwarp();
+            if (gain)
+                for (int t = lane; t < c.n; t += 32) suf[t] *= gain[(size_t)(c.t0 + t) * g_stride + first_head + warp];
+        }
+#pragma unroll
+        for (int j = 0; j < KN; ++j) {
+            const int e = tid + j * ST_THREADS, t = e / (DK / 4), i = (e % (DK / 4)) * 4;
+            put4<PK>(ks + t * KP + i, CK * KP, kv[j]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < VN; ++j) {
+            const int e = tid + j * ST_THREADS, t = e / (VT / 4), i = (e % (VT / 4)) * 4, which = heads > 1 ? i / dv : 0;
+            put4<PV>(vs + t * VP + i, CK * VP, times(vv[j], fs[2 * CK + which * CK + t]));
+        }
+    } else {
+        uint2 vv[VN];                                        // bf16 values as they come
+#pragma unroll
+        for (int j = 0; j < VN; ++j) {
+            const int e = tid + j * ST_THREADS, t = e / (VT / 4), i = (e % (VT / 4)) * 4;
+            vv[j] = t < c.n ? *reinterpret_cast<const uint2*>(v + (size_t)(c.t0 + t) * v_stride + col0 + i) : make_uint2(0u, 0u);
+        }
+        // a key channel of a quarter (16 tokens) a thread: the keys times the decays behind them inside the quarter
+        constexpr int PASSES = QUARTERS * DK / ST_THREADS;
+        float kk[PASSES][16];
+#pragma unroll
+        for (int p = 0; p < PASSES; ++p) {
+            const int unit = tid + p * ST_THREADS, ch = unit % DK, r = unit / DK;
+            float a[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const bool in = r * 16 + t < c.n;
+                const size_t at = (size_t)(c.t0 + r * 16 + t);
+                a[t] = in ? decay[at * a_stride + (size_t)kh * DK + ch] : 1.f;
+                kk[p][t] = in ? to_f32<TA>(k[at * k_stride + (size_t)kh * DK + ch]) : 0.f;
+            }
+            float f = 1.f;
+#pragma unroll
+            for (int t = 15; t >= 0; --t) { kk[p][t] *= f; f *= a[t]; }
+            fs[r * DK + ch] = f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int p = 0; p < PASSES; ++p) {
+            const int unit = tid + p * ST_THREADS, ch = unit % DK, r = unit / DK;
+            float f = 1.f;
+            for (int m = r + 1; m < QUARTERS; ++m) f *= fs[m * DK + ch];
+            if (r == 0 && c0 == 0) totals[((size_t)blockIdx.x * H + kh) * DK + ch] = f * fs[ch];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) put1(ks + (r * 16 + t) * KP + ch, CK * KP, kk[p][t] * f);
+        }
+#pragma unroll
+        for (int j = 0; j < VN; ++j) {
+            const int e = tid + j * ST_THREADS, t = e / (VT / 4), i = (e % (VT / 4)) * 4;
+            *reinterpret_cast<uint2*>(vs + t * VP + i) = vv[j];
+        }
+    }
+    __syncthreads();
+    constexpr int NT = DK / 64;                              // blocks of 16 key channels a warp
+    const int n0 = (warp & 3) * (16 * NT);
+    float* to = states + ((size_t)blockIdx.x * H * dv + col0) * DK;
+#pragma unroll 1
+    for (int half = 0; half < VT / 64; ++half) {
+        const int m0 = half * 64 + (warp >> 2) * 32;
+        float d[2][2 * NT][4] = {};
+#pragma unroll
+        for (int t0 = 0; t0 < CK; t0 += 16) {
+            uint32_t fa[PV][2][4], fb[PK][NT][4];
+#pragma unroll
+            for (int p = 0; p < PV; ++p)
+#pragma unroll
+                for (int m = 0; m < 2; ++m) ldsm_t(fa[p][m], vs + p * CK * VP + t0 * VP + m0 + m * 16 + at_at(lane, VP));
+#pragma unroll
+            for (int p = 0; p < PK; ++p)
+#pragma unroll
+                for (int n = 0; n < NT; ++n) ldsm_t(fb[p][n], ks + p * CK * KP + t0 * KP + n0 + n * 16 + at_bt(lane, KP));
+            products<2, NT, PV, PK>(d, fa, fb);
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < 2 * NT; ++n) {
+                float* x = to + (size_t)(m0 + m * 16 + (lane >> 2)) * DK + n0 + n * 8 + (lane & 3) * 2;
+                *reinterpret_cast<float2*>(x) = make_float2(d[m][n][0], d[m][n][1]);
+                *reinterpret_cast<float2*>(x + 8 * DK) = make_float2(d[m][n][2], d[m][n][3]);
+            }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------- the state in front of every chunk
+// Four neighbouring key channels a thread, the chunks of its entry in order: cuts[chunk] becomes the state the chunk starts
+// from, in pieces ([chunk][head][piece][value][key]), the entry's slot the state behind the last.
+constexpr int SCAN_AHEAD = 8;                   // chunks whose loads are in flight together
+template <bool GATED>
+__global__ void __launch_bounds__(256)
+chunk_scan_kernel(const float* __restrict__ states, const float* __restrict__ totals, bf16* __restrict__ cuts,
+                  float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ state_slots, int least,
+                  int H, int dv) {
+    pdl_trigger();
+    pdl_wait();
+    const int b = blockIdx.y;
+    const int count = chunks_of(cu_q[b + 1] - cu_q[b], least);
+    if (count == 0) return;
+    const int base = first_chunk(cu_q, b, least);
+    const size_t one = (size_t)dv * DK, per = H * one, at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (at >= per) return;
+    const int h = (int)(at / one), i = (int)(at % DK);
+    float* own = state + (size_t)state_slots[b] * per + at;
+    float4 S = load4(own);
+    for (int c0 = 0; c0 < count; c0 += SCAN_AHEAD) {
+        float4 x[SCAN_AHEAD], a[GATED ? SCAN_AHEAD : 1];
+        float2 t[GATED ? 1 : SCAN_AHEAD];
+#pragma unroll
+        for (int j = 0; j < SCAN_AHEAD; ++j) {
+            const size_t chunk = base + min(c0 + j, count - 1);
+            x[j] = load4(states + chunk * per + at);
+            if constexpr (GATED) a[j] = load4(totals + (chunk * H + h) * DK + i);
+            else t[j] = *reinterpret_cast<const float2*>(totals + (chunk * H + h) * 2);
+        }
+#pragma unroll
+        for (int j = 0; j < SCAN_AHEAD; ++j)
+            if (c0 + j < count) {
+                put4<3>(cuts + ((size_t)(base + c0 + j) * H + h) * 3 * one + at % one, one, S);
+                if constexpr (GATED) {
+                    S = make_float4(fmaf(a[j].x, S.x, x[j].x), fmaf(a[j].y, S.y, x[j].y), fmaf(a[j].z, S.z, x[j].z), fmaf(a[j].w, S.w, x[j].w));
+                } else {
+                    const float hi = t[j].x, lo = t[j].y;
+                    S = make_float4(fmaf(hi, S.x, fmaf(lo, S.x, x[j].x)), fmaf(hi, S.y, fmaf(lo, S.y, x[j].y)),
+                                    fmaf(hi, S.z, fmaf(lo, S.z, x[j].z)), fmaf(hi, S.w, fmaf(lo, S.w, x[j].w)));
+                }
+            }
+    }
+    *reinterpret_cast<float4*>(own) = S;
+}
+
+// ------------------------------------------------------------------------------------------------- outputs
+// The outputs of one chunk for `heads` heads of one key head, two CTAs an SM.  Eight warps: a quarter of the tokens x half of
+// the keys (scores) or of a tile of 32 value channels (outputs).  The queries stay cut up in shared memory, the scores lie
+// where the keys lay; the state's pieces come by cp.async, a tile's while the last one's values are multiplied; the values are
+// read and cut by the lanes that need them.
+constexpr int OUT_THREADS = 256;
+constexpr int OT = 32;                          // value channels of a tile
+constexpr int AP = CK + 8;
+struct OutLayout {                              // offsets in bf16, then floats
+    static constexpr int q = 0, a = q + 3 * CK * KP, s = a + 3 * CK * AP, end = s + 3 * OT * KP;
+    static constexpr int k = a;                 // keys, before the scores (gated: up to 48 rows)
+    static constexpr int floats = 5 * CK + 4 * 16 * 16;
+    static constexpr int bytes = end * 2 + floats * 4;
+    static_assert(k + 3 * CK * KP <= end && k + 3 * 48 * KP <= end && 16 * 144 * 2 <= end - k, "what lies where scores and tiles lie later");
+};
+
+__device__ __forceinline__ void cp16(bf16* smem, const bf16* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+// a tile of the state's pieces on its way into shared memory
+__device__ __forceinline__ void fetch_state(bf16* st, const bf16* cuts, int c0, int dv) {
+    constexpr int SN = 3 * OT * DK / 8 / OUT_THREADS;
+#pragma unroll
+    for (int j = 0; j < SN; ++j) {
+        const int e = threadIdx.x + j * OUT_THREADS, p = e / (OT * DK / 8), r = e / (DK / 8) % OT, i = (e % (DK / 8)) * 8;
+        cp16(st + (p * OT + r) * KP + i, cuts + ((size_t)p * dv + c0 + r) * DK + i);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+}
+
+// The tiles of one head's value channels from the chunk's scores, the queries and the state in front of it; the first tile of
+// the state is on its way, and everything else becomes visible with the first barrier.  pre: the decays from the chunk's start,
+// null where the queries carry them; gain null: none.
+template <typename TA, int PQ, int PV>
+__device__ __forceinline__ void value_tiles(bf16* sm, const float* pre, const float* gain, const Chunk& c, const bf16* cuts, const TA* v,
+                                            int v_stride, float q_scale, float* out, int out_stride, int dv, int first, int last) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wm = warp >> 1, wn = warp & 1, g = lane >> 2, t4 = lane & 3;
+    const bf16 *qs = sm + OutLayout::q, *as = sm + OutLayout::a;
+    bf16* st = sm + OutLayout::s;
+    for (int c0 = first; c0 < last; c0 += OT) {
+        // values of this lane's columns at the tokens of its fragments, up to its quarter: a step's are 2t, 2t + 1, 2t + 8, 2t + 9
+        float vx[QUARTERS][2][4];
+#pragma unroll
+        for (int m = 0; m < QUARTERS; ++m)
+            if (m <= wm) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = m * 16 + 2 * t4 + (e & 1) + (e >> 1) * 8;
+                    const TA* p = v + (size_t)(c.t0 + t) * v_stride + c0 + wn * 16 + g;
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) vx[m][n][e] = t < c.n ? to_f32<TA>(p[n * 8]) : 0.f;
+                }
+            }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        float o[1][2][4] = {};
+#pragma unroll
+        for (int k0 = 0; k0 < DK; k0 += 16) {                // from the state in front of the chunk
+            uint32_t fa[PQ][1][4], fb[3][1][4];
+#pragma unroll
+            for (int p = 0; p < PQ; ++p) ldsm(fa[p][0], qs + p * CK * KP + wm * 16 * KP + k0 + at_a(lane, KP));
+#pragma unroll
+            for (int p = 0; p < 3; ++p) ldsm(fb[p][0], st + p * OT * KP + wn * 16 * KP + k0 + at_b(lane, KP));
+            products<1, 1, PQ, 3>(o, fa, fb);
+        }
+        __syncthreads();                                     // the state's tile is read
+        if (c0 + OT < last) fetch_state(st, cuts, c0 + OT, dv);
+        if (pre) {
+            const float p0 = pre[wm * 16 + g], p1 = pre[wm * 16 + g + 8];
+#pragma unroll
+            for (int n = 0; n < 2; ++n) { o[0][n][0] *= p0; o[0][n][1] *= p0; o[0][n][2] *= p1; o[0][n][3] *= p1; }
+        }
+        int bad[2] = {CK, CK};                               // first token whose value in the lane's column is no number
+#pragma unroll
+        for (int m = 0; m < QUARTERS; ++m)
+            if (m <= wm) {                                   // from the chunk's own tokens up to this quarter
+                uint32_t fa[3][1][4], fb[PV][1][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) ldsm(fa[p][0], as + p * CK * AP + wm * 16 * AP + m * 16 + at_a(lane, AP));
+                float gx[4] = {1.f, 1.f, 1.f, 1.f};
+                if (gain) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) gx[e] = gain[m * 16 + 2 * t4 + (e & 1) + (e >> 1) * 8];
+                }
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    float x[4];
+#pragma unroll
+                    for (int e = 3; e >= 0; --e) {
+                        x[e] = gain ? vx[m][n][e] * gx[e] : vx[m][n][e];
+                        if (!(fabsf(x[e]) <= 3.402823466e38f)) { bad[n] = min(bad[n], m * 16 + 2 * t4 + (e & 1) + (e >> 1) * 8); x[e] = 0.f; }
+                    }
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        if constexpr (PV == 1) {
+                            fb[0][0][2 * n + half] = pair_bf16(x[2 * half], x[2 * half + 1]);
+                        } else {
+                            uint32_t p[3];
+                            cut(x[2 * half], x[2 * half + 1], p);
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) fb[i][0][2 * n + half] = p[i];
+                        }
+                    }
+                }
+                products<1, 1, 3, PV>(o, fa, fb);
+            }
+        const bool any_bad = __any_sync(0xffffffffu, min(bad[0], bad[1]) < CK);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const int col = wn * 16 + n * 8 + t4 * 2;
+            if (any_bad) {                                   // later outputs of such a column are NaN
+                int b = min(bad[n], __shfl_xor_sync(0xffffffffu, bad[n], 1));
+                b = min(b, __shfl_xor_sync(0xffffffffu, b, 2));
+                const int b0 = __shfl_sync(0xffffffffu, b, 8 * t4), b1 = __shfl_sync(0xffffffffu, b, 8 * t4 + 4);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    if (wm * 16 + g + 8 * r >= b0) o[0][n][2 * r] = __int_as_float(0x7fc00000);
+                    if (wm * 16 + g + 8 * r >= b1) o[0][n][2 * r + 1] = __int_as_float(0x7fc00000);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int t = wm * 16 + g + 8 * r;
+                if (t < c.n)
+                    *reinterpret_cast<float2*>(out + (size_t)(c.t0 + t) * out_stride + c0 + col) =
+                        make_float2(o[0][n][2 * r] * q_scale, o[0][n][2 * r + 1] * q_scale);
+            }
+        }
+    }
+}
+
+template <typename TA>
+__global__ void __launch_bounds__(OUT_THREADS, 2)
+head_chunk_outputs_kernel(const TA* __restrict__ q, int q_stride, const TA* __restrict__ k, int k_stride,
+                          const TA* __restrict__ v, int v_stride, const float* __restrict__ decay, int a_stride,
+                          const float* __restrict__ gain, int g_stride, float q_scale, const bf16* __restrict__ cuts,
+                          float* __restrict__ out, const int* __restrict__ cu_q, int entries, int least, int H, int dv,
+                          int share, int heads) {
+    constexpr int PQ = sizeof(TA) == 2 ? 1 : 3;              // pieces of queries and keys
+    extern __shared__ __align__(16) unsigned char raw[];
+    bf16* sm = reinterpret_cast<bf16*>(raw);
+    bf16 *qs = sm + OutLayout::q, *ks = sm + OutLayout::k, *as = sm + OutLayout::a;
+    float* a = reinterpret_cast<float*>(sm + OutLayout::end);
+    float *pre = a + CK, *pre_in = pre + CK, *suf_in = pre_in + CK;      // from the chunk's start; inside a quarter: from its start, to its end
+    float* gains = suf_in + CK;
+    float* dq = gains + CK;                                  // [4][16][16] decays inside a quarter
+    pdl_trigger();
+    pdl_wait();
+    const Chunk c = find_chunk(cu_q, entries, least, blockIdx.x);
+    if (c.entry < 0) return;
+    const int h0 = blockIdx.y * heads, kh = h0 / share;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 1, wn = warp & 1;
+    const int g = lane >> 2, t4 = lane & 3;
+    // a head's decays and gains, a token a thread, one head ahead
+    float next_a = 1.f, next_g = 1.f;
+    auto ask = [&](int h) {
+        if (tid < c.n) {
+            next_a = decay[(size_t)(c.t0 + tid) * a_stride + h];
+            if (gain) next_g = gain[(size_t)(c.t0 + tid) * g_stride + h];
+        }
+    };
+    {
+        constexpr int KN = CK * DK / 4 / OUT_THREADS;
+        float4 x[KN], y[KN];
+#pragma unroll
+        for (int j = 0; j < KN; ++j) {
+            const int e = tid + j * OUT_THREADS, t = e / (DK / 4), i = (e % (DK / 4)) * 4;
+            x[j] = t < c.n ? load4(q + (size_t)(c.t0 + t) * q_stride + (size_t)kh * DK + i) : zero4();
+            y[j] = t < c.n ? load4(k + (size_t)(c.t0 + t) * k_stride + (size_t)kh * DK + i) : zero4();
+        }
+        ask(h0);
+#pragma unroll
+        for (int j = 0; j < KN; ++j) {
+            const int e = tid + j * OUT_THREADS, t = e / (DK / 4), i = (e % (DK / 4)) * 4;
+            put4<PQ>(qs + t * KP + i, CK * KP, x[j]);
+            put4<PQ>(ks + t * KP + i, CK * KP, y[j]);
+        }
+    }
+    __syncthreads();
+    // scores of this warp's 16 tokens against 32 keys (none where every key is later)
+    float s[1][4][4] = {};
+    if (2 * wn <= wm) {
+#pragma unroll
+        for (int k0 = 0; k0 < DK; k0 += 16) {
+            uint32_t fa[PQ][1][4], fb[PQ][2][4];
+#pragma unroll
+            for (int p = 0; p < PQ; ++p) {
+                ldsm(fa[p][0], qs + p * CK * KP + wm * 16 * KP + k0 + at_a(lane, KP));
+#pragma unroll
+                for (int n = 0; n < 2; ++n) ldsm(fb[p][n], ks + p * CK * KP + (wn * 32 + n * 16) * KP + k0 + at_b(lane, KP));
+            }
+            products<1, 2, PQ, PQ>(s, fa, fb);
+        }
+    }
+    for (int hh = 0; hh < heads; ++hh) {
+        const int h = h0 + hh;
+        const bf16* from = cuts + ((size_t)blockIdx.x * H + h) * 3 * dv * DK;
+        if (tid < CK) { a[tid] = tid < c.n ? next_a : 1.f; }
+        __syncthreads();                                     // the last head's (or the keys') readers are done, the decays are there
+        fetch_state(sm + OutLayout::s, from, 0, dv);
+        if (tid < CK) gains[tid] = next_g;
+        if (hh + 1 < heads) ask(h + 1);
+        if (warp == 7) chunk_products(a, pre, nullptr);
+        if (warp >= 2 && warp < 4) {                         // 64 threads: the column of key j inside its quarter
+            const int j = tid - 64, r = j >> 4, jj = j & 15;
+            double f = 1.0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                if (i > jj) f *= a[r * 16 + i];
+                dq[(r * 16 + i) * 16 + jj] = (float)f;
+            }
+            suf_in[j] = (float)f;
+        }
+        if (warp >= 4 && warp < 6) {
+            const int i = tid - 128, r = i >> 4;
+            double f = 1.0;
+            for (int m = r * 16; m <= i; ++m) f *= a[m];
+            pre_in[i] = (float)f;
+        }
+        __syncthreads();
+        // scores times decays, cut up: the quarters on the diagonal by the table, those left of it by their factors; a later
+        // key's weight is zero by choice, not by product
+        if (2 * wn <= wm) {
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const int cq = wn * 2 + (n >> 1);            // the keys' quarter
+                if (cq > wm) continue;
+                float between = 1.f;
+                for (int m = cq + 1; m < wm; ++m) between *= pre_in[m * 16 + 15];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int col = wn * 32 + n * 8 + t4 * 2, row = wm * 16 + g + 8 * r;
+                    float x, y;
+                    if (cq == wm) {
+                        const float* d = dq + row * 16 + (col & 15);
+                        x = col <= row ? s[0][n][2 * r] * d[0] : 0.f;
+                        y = col + 1 <= row ? s[0][n][2 * r + 1] * d[1] : 0.f;
+                    } else {
+                        const float w = pre_in[row] * between;
+                        x = s[0][n][2 * r] * (w * suf_in[col]);
+                        y = s[0][n][2 * r + 1] * (w * suf_in[col + 1]);
+                    }
+                    uint32_t p[3];
+                    cut(x, y, p);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(as + i * CK * AP + row * AP + col) = p[i];
+                }
+            }
+        }
+        value_tiles<TA, PQ, 3>(sm, pre, gain ? gains : nullptr, c, from, v + (size_t)h * dv, v_stride, q_scale, out + (size_t)h * dv, H * dv, dv, 0, dv);
+    }
+}
+
+// Sums of 16 values over a warp's lanes: at every offset a lane hands half of its values to its partner and keeps the other
+// half's sums.  The lane gets value `lane >> 1` (both lanes of a pair).
+__device__ __forceinline__ float sums16(float (&x)[16]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int n = 16, o = 16; n > 1; n /= 2, o /= 2) {
+        const bool upper = lane & o;
+#pragma unroll
+        for (int i = 0; i < n / 2; ++i) {
+            const float send = upper ? x[i] : x[i + n / 2], keep = upper ? x[i + n / 2] : x[i];
+            x[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
+}
+
+// A decay a key channel: the scores cannot be one product.  Inside a quarter (16 tokens) a thread takes a key channel and
+// multiplies its way through the pairs of tokens in fp32, and the channels' parts are summed; between quarters r > s the
+// decays part at quarter r's start, q_i (a_start .. a_i) on one side and (a_{j+1} .. a_{start-1}) k_j on the other, both below
+// one, and the score is a product again, with the keys scaled for each r.
+// The scores and the queries from the chunk's start go out in pieces, [chunk][head]{scores [3][CK][CK], queries [3][CK][DK]}, for
+// the CTAs that take the chunk's value channels (the scores are most of the work where one CTA makes them for itself).
+constexpr int GATED_PARTS = 3 * CK * (CK + DK);
+struct ScoreLayout {                            // queries, keys (48 rows) or the scores, floats
+    static constexpr int q = 0, k = 3 * CK * KP, end = k + (48 * KP > CK * AP ? 3 * 48 * KP : 3 * CK * AP);
+    static constexpr int bytes = end * 2 + QUARTERS * DK * 4;
+    static_assert(3 * CK * AP <= end - k && 16 * 144 * 2 <= end - k, "scores and the warps' parts fit where the keys lie");
+};
+__global__ void __launch_bounds__(OUT_THREADS, 2)
+gated_chunk_scores_kernel(const bf16* __restrict__ q, int q_stride, const bf16* __restrict__ k, int k_stride,
+                          const float* __restrict__ decay, int a_stride, bf16* __restrict__ parts, const int* __restrict__ cu_q,
+                          int entries, int least, int H) {
+    constexpr int UNITS = QUARTERS * DK / OUT_THREADS, WQ = DK / 32;     // (channel, quarter) pairs a thread; warps of channels
+    extern __shared__ __align__(16) unsigned char raw[];
+    bf16* sm = reinterpret_cast<bf16*>(raw);
+    bf16 *qs = sm + ScoreLayout::q, *ks = sm + ScoreLayout::k, *as = ks;
+    float* qt = reinterpret_cast<float*>(sm + ScoreLayout::end);         // [4][DK] products of a quarter's decays
+    float* part = reinterpret_cast<float*>(ks);                          // [4 * WQ][144], before the keys are laid out
+    static_assert(QUARTERS * WQ <= 16, "the warps' parts fit");
+    pdl_trigger();
+    pdl_wait();
+    const Chunk c = find_chunk(cu_q, entries, least, blockIdx.x);
+    if (c.entry < 0) return;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float kk[UNITS][16];
+#pragma unroll
+    for (int u = 0; u < UNITS; ++u) {
+        const int unit = tid + u * OUT_THREADS, ch = unit % DK, r = unit / DK;
+        float a[16], qq[16];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            const bool in = r * 16 + t < c.n;
+            const size_t at = (size_t)(c.t0 + r * 16 + t);
+            a[t] = in ? decay[at * a_stride + (size_t)h * DK + ch] : 1.f;
+            qq[t] = in ? to_f32<bf16>(q[at * q_stride + (size_t)h * DK + ch]) : 0.f;
+            kk[u][t] = in ? to_f32<bf16>(k[at * k_stride + (size_t)h * DK + ch]) : 0.f;
+        }
+        // pairs i >= j of the quarter: keys j and 16 - j have 16 queries between them
+#pragma unroll
+        for (int set = 0; set <= 8; ++set) {
+            float x[16];
+            float f = kk[u][set];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                if (i < set) continue;
+                if (i > set) f *= a[i];
+                x[i - set] = qq[i] * f;
+            }
+            if (set > 0) {
+                const int j = 16 - set;
+                float e = set == 8 ? 0.f : kk[u][j];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    if (i < j) continue;
+                    if (i > j) e *= a[i];
+                    x[i] = qq[i] * e;
+                }
+            }
+            const float sum = sums16(x);
+            if ((lane & 1) == 0) part[(unit >> 5) * 144 + set * 16 + (lane >> 1)] = sum;
+        }
+        float f = 1.f;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) { f *= a[t]; put1(qs + (r * 16 + t) * KP + ch, CK * KP, qq[t] * f); }   // from the quarter's start
+        qt[r * DK + ch] = f;
+        f = 1.f;
+#pragma unroll
+        for (int t = 15; t >= 0; --t) { kk[u][t] *= f; f *= a[t]; }      // to the quarter's end
+    }
+    __syncthreads();
+    // the quarters on the diagonal: the channels' warps in order
+    float diag[QUARTERS * 256 / OUT_THREADS];
+#pragma unroll
+    for (int n = 0; n < QUARTERS * 256 / OUT_THREADS; ++n) {
+        const int e = tid + n * OUT_THREADS, b = e >> 8, i = e >> 4 & 15, j = e & 15;
+        diag[n] = 0.f;
+        if (j <= i) {
+            const int at = j <= 8 ? j * 16 + i - j : (16 - j) * 16 + i;
+            for (int w = 0; w < WQ; ++w) diag[n] += part[(b * WQ + w) * 144 + at];
+        }
+    }
+    // quarters right of the first: 16 x 8 scores a warp, quarter `to` against the keys of those before it, kept till all are read
+    float s[QUARTERS - 1][4];
+#pragma unroll
+    for (int to = 1; to < QUARTERS; ++to) {
+        __syncthreads();                                     // the parts, or the last quarter's keys, are read
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            const int unit = tid + u * OUT_THREADS, ch = unit % DK, r = unit / DK;
+            if (r < to) {
+                float f = 1.f;
+                for (int m = r + 1; m < to; ++m) f *= qt[m * DK + ch];
+#pragma unroll
+                for (int t = 0; t < 16; ++t) put1(ks + (r * 16 + t) * KP + ch, 48 * KP, kk[u][t] * f);
+            }
+        }
+        __syncthreads();
+        if (warp < 2 * to) {
+            float d[1][2][4] = {};                           // the second half is not used
+            const int n0 = warp * 8;
+#pragma unroll
+            for (int k0 = 0; k0 < DK; k0 += 16) {
+                uint32_t fa[3][4], fb[3][2];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    ldsm(fa[p], qs + p * CK * KP + to * 16 * KP + k0 + at_a(lane, KP));
+                    const bf16* b = ks + p * 48 * KP + (n0 + (lane >> 2)) * KP + k0 + (lane & 3) * 2;
+                    fb[p][0] = *reinterpret_cast<const uint32_t*>(b);
+                    fb[p][1] = *reinterpret_cast<const uint32_t*>(b + 8);
+                }
+                float x[4] = {};
+                mma(x, fa[0], fb[2][0], fb[2][1]);
+                mma(x, fa[1], fb[1][0], fb[1][1]);
+                mma(x, fa[2], fb[0][0], fb[0][1]);
+                mma(x, fa[0], fb[1][0], fb[1][1]);
+                mma(x, fa[1], fb[0][0], fb[0][1]);
+                mma(x, fa[0], fb[0][0], fb[0][1]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) d[0][0][e] += x[e];
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[to - 1][e] = d[0][0][e];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int to = 1; to < QUARTERS; ++to)
+        if (warp < 2 * to) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                uint32_t p[3];
+                cut(s[to - 1][2 * e], s[to - 1][2 * e + 1], p);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    *reinterpret_cast<uint32_t*>(as + i * CK * AP + (to * 16 + (lane >> 2) + 8 * e) * AP + warp * 8 + (lane & 3) * 2) = p[i];
+            }
+        }
+#pragma unroll
+    for (int n = 0; n < QUARTERS * 256 / OUT_THREADS; ++n) {
+        const int e = tid + n * OUT_THREADS, b = e >> 8, i = e >> 4 & 15, j = e & 15;
+        put1(as + (b * 16 + i) * AP + b * 16 + j, CK * AP, diag[n]);
+    }
+#pragma unroll
+    for (int u = 0; u < UNITS; ++u) {                        // queries from the chunk's start: the pieces' sum is the number
+        const int unit = tid + u * OUT_THREADS, ch = unit % DK, r = unit / DK;
+        if (r == 0) continue;
+        float f = 1.f;
+        for (int m = 0; m < r; ++m) f *= qt[m * DK + ch];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            bf16* x = qs + (r * 16 + t) * KP + ch;
+            const float sum = __bfloat162float(x[0]) + (__bfloat162float(x[CK * KP]) + __bfloat162float(x[2 * CK * KP]));
+            put1(x, CK * KP, sum * f);
+        }
+    }
+    __syncthreads();
+    bf16* to = parts + ((size_t)blockIdx.x * H + h) * GATED_PARTS;
+    for (int e = tid; e < 3 * CK * CK / 8; e += OUT_THREADS)             // [piece][row]
+        *reinterpret_cast<uint4*>(to + e * 8) = *reinterpret_cast<const uint4*>(as + (e / (CK / 8)) * AP + (e % (CK / 8)) * 8);
+    to += 3 * CK * CK;
+    for (int e = tid; e < 3 * CK * DK / 8; e += OUT_THREADS)
+        *reinterpret_cast<uint4*>(to + e * 8) = *reinterpret_cast<const uint4*>(qs + (e / (DK / 8)) * KP + (e % (DK / 8)) * 8);
+}
+
+// dv / gridDim.z value channels of one chunk and head
+__global__ void __launch_bounds__(OUT_THREADS, 2)
+gated_chunk_outputs_kernel(const bf16* __restrict__ parts, const bf16* __restrict__ v, int v_stride, float q_scale,
+                           const bf16* __restrict__ cuts, float* __restrict__ out, const int* __restrict__ cu_q, int entries,
+                           int least, int H, int dv) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    bf16* sm = reinterpret_cast<bf16*>(raw);
+    pdl_trigger();
+    pdl_wait();
+    const Chunk c = find_chunk(cu_q, entries, least, blockIdx.x);
+    if (c.entry < 0) return;
+    const int h = blockIdx.y, first = (int)blockIdx.z * (dv / (int)gridDim.z), last = first + dv / (int)gridDim.z;
+    const bf16* from = cuts + ((size_t)blockIdx.x * H + h) * 3 * dv * DK;
+    const bf16* own = parts + ((size_t)blockIdx.x * H + h) * GATED_PARTS;
+    for (int e = threadIdx.x; e < 3 * CK * CK / 8; e += OUT_THREADS)
+        cp16(sm + OutLayout::a + (e / (CK / 8)) * AP + (e % (CK / 8)) * 8, own + e * 8);
+    own += 3 * CK * CK;
+    for (int e = threadIdx.x; e < 3 * CK * DK / 8; e += OUT_THREADS)
+        cp16(sm + OutLayout::q + (e / (DK / 8)) * KP + (e % (DK / 8)) * 8, own + e * 8);
+    fetch_state(sm + OutLayout::s, from, first, dv);
+    value_tiles<bf16, 3, 1>(sm, nullptr, nullptr, c, from, v + (size_t)h * dv, v_stride, q_scale, out + (size_t)h * dv, H * dv, dv, first, last);
+}
+
+inline bool aligned4(const void* p, int esize) { return (reinterpret_cast<uintptr_t>(p) % (4 * (size_t)esize)) == 0; }
+template <typename Kernel>
+int allow(Kernel kernel, int bytes) { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); }
+}  // namespace
+
+// Whether the head form (`gated` 0) or the gated one takes these arrays; what they do not take walks.
+RI_API int ri_chunks_ok(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, int act_dtype, int dv, int gated) {
+    const int esize = act_dtype == RI_BF16 ? 2 : 4;
+    return dv > 0 && dv % 64 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 && aligned4(q, esize) &&
+           aligned4(k, esize) && aligned4(v, esize) && (!gated || act_dtype == RI_BF16);
+}
+
+// The entries of at least `least` tokens in chunks; `chunks`: the number the grids are made for, at least that of all those
+// entries.  Scratch: states fp32 [chunks][H][dv][DK], totals fp32 [chunks][H][2], cuts bf16 [chunks][H][3][dv][DK].
+RI_API int ri_head_chunks(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
+                          const float* decay, int a_stride, const float* gain, int g_stride, int act_dtype, float q_scale,
+                          float* out, float* state, const int* cu_q, const int* state_slots, int entries, int least, int chunks,
+                          int H, int dv, int share, float* states, float* totals, void* cuts, void* stream) {
+    if (entries <= 0 || chunks <= 0) return 0;
+    if (share <= 0 || H % share || !ri_chunks_ok(q, q_stride, k, k_stride, v, v_stride, act_dtype, dv, 0)) return (int)cudaErrorInvalidValue;
+    cudaStream_t s = (cudaStream_t)stream;
+    // heads a CTA of the outputs serves: their scores' products are shared; fewer where the CTAs would not fill the SMs twice
+    int heads = share;
+    while (heads % 2 == 0 && (long long)chunks * (H / heads) < 4LL * ri_device_sms()) heads /= 2;
+    const int scan_blocks = (int)(((size_t)H * dv * DK / 4 + 255) / 256);
+#define RI_STATES(TA, VT) do { \
+    static bool allowed = false; \
+    if (!allowed) { RI_CHECKED(allow(chunk_states_kernel<TA, VT, false>, states_bytes<TA, VT, false>())); allowed = true; } \
+    RI_CHECKED(ri_launch(chunk_states_kernel<TA, VT, false>, dim3(chunks, H / share, share * dv / VT), dim3(ST_THREADS), \
+        states_bytes<TA, VT, false>(), s, (const TA*)k, k_stride, (const TA*)v, v_stride, decay, a_stride, gain, g_stride, states, totals, \
+        cu_q, entries, least, H, dv, share)); } while (0)
+#define RI_HC(TA) do { \
+    static bool allowed = false; \
+    if (!allowed) { RI_CHECKED(allow(head_chunk_outputs_kernel<TA>, OutLayout::bytes)); allowed = true; } \
+    if (dv % 128 == 0 || (dv == 64 && share % 2 == 0)) RI_STATES(TA, 128); else RI_STATES(TA, 64); \
+    RI_CHECKED(ri_launch(chunk_scan_kernel<false>, dim3(scan_blocks, entries), dim3(256), 0, s, states, totals, (bf16*)cuts, state, cu_q, \
+        state_slots, least, H, dv)); \
+    RI_CHECKED(ri_launch(head_chunk_outputs_kernel<TA>, dim3(chunks, H / heads), dim3(OUT_THREADS), OutLayout::bytes, s, (const TA*)q, q_stride, \
+        (const TA*)k, k_stride, (const TA*)v, v_stride, decay, a_stride, gain, g_stride, q_scale, (const bf16*)cuts, out, cu_q, entries, least, \
+        H, dv, share, heads)); } while (0)
+    if (act_dtype == RI_BF16) RI_HC(bf16);
+    else RI_HC(float);
+#undef RI_HC
+#undef RI_STATES
+    return ri_launch_status();
+}
+
+// The gated form (bf16 q, k, v; fp32 decays [T][a_stride], a_stride 0: one row for all tokens); totals fp32 [chunks][H][DK],
+// parts bf16 [chunks][H][ri_gated_chunk_parts()].
+RI_API int ri_gated_chunk_parts() { return GATED_PARTS; }
+RI_API int ri_gated_chunks(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
+                           const float* alpha, int a_stride, int act_dtype, float q_scale, float* out, float* state, const int* cu_q,
+                           const int* state_slots, int entries, int least, int chunks, int H, int dv, float* states, float* totals,
+                           void* cuts, void* parts, void* stream) {
+    if (entries <= 0 || chunks <= 0) return 0;
+    if (!ri_chunks_ok(q, q_stride, k, k_stride, v, v_stride, act_dtype, dv, 1)) return (int)cudaErrorInvalidValue;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int scan_blocks = (int)(((size_t)H * dv * DK / 4 + 255) / 256);
+    static bool allowed = false;
+    if (!allowed) {
+        RI_CHECKED(allow(gated_chunk_scores_kernel, ScoreLayout::bytes));
+        RI_CHECKED(allow(gated_chunk_outputs_kernel, OutLayout::bytes));
+        RI_CHECKED(allow(chunk_states_kernel<bf16, 128, true>, states_bytes<bf16, 128, true>()));
+        RI_CHECKED(allow(chunk_states_kernel<bf16, 64, true>, states_bytes<bf16, 64, true>()));
+        allowed = true;
+    }
+#define RI_STATES(VT) RI_CHECKED(ri_launch(chunk_states_kernel<bf16, VT, true>, dim3(chunks, H, dv / VT), dim3(ST_THREADS), \
+        states_bytes<bf16, VT, true>(), s, (const bf16*)k, k_stride, (const bf16*)v, v_stride, alpha, a_stride, (const float*)nullptr, 0, states, \
+        totals, cu_q, entries, least, H, dv, 1))
+    if (dv % 128 == 0) RI_STATES(128);
+    else RI_STATES(64);
+#undef RI_STATES
+    RI_CHECKED(ri_launch(chunk_scan_kernel<true>, dim3(scan_blocks, entries), dim3(256), 0, s, states, totals, (bf16*)cuts, state, cu_q, state_slots,
+                         least, H, dv));
+    RI_CHECKED(ri_launch(gated_chunk_scores_kernel, dim3(chunks, H), dim3(OUT_THREADS), ScoreLayout::bytes, s, (const bf16*)q, q_stride,
+                         (const bf16*)k, k_stride, alpha, a_stride, (bf16*)parts, cu_q, entries, least, H));
+    RI_CHECKED(ri_launch(gated_chunk_outputs_kernel, dim3(chunks, H, dv % 128 == 0 ? dv / 128 : 1), dim3(OUT_THREADS), OutLayout::bytes, s,
+                         (const bf16*)parts, (const bf16*)v, v_stride, q_scale, (const bf16*)cuts, out, cu_q, entries, least, H, dv));
+    return ri_launch_status();
+}
+#else
+RI_API int ri_chunks_ok(const void*, int, const void*, int, const void*, int, int, int, int) { return 0; }
+RI_API int ri_head_chunks(const void*, int, const void*, int, const void*, int, const float*, int, const float*, int, int, float, float*,
+                          float*, const int*, const int*, int, int, int, int, int, int, float*, float*, void*, void*) {
+    return (int)cudaErrorInvalidValue;
+}
+RI_API int ri_gated_chunks(const void*, int, const void*, int, const void*, int, const float*, int, int, float, float*, float*, const int*,
+                           const int*, int, int, int, int, int, float*, float*, void*, void*, void*) {
+    return (int)cudaErrorInvalidValue;
+}
+RI_API int ri_gated_chunk_parts() { return 0; }
+#endif
+
+RI_API int ri_recurrent_chunk_tokens() { return BUILT ? CK : 0; }

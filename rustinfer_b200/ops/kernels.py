@@ -1226,6 +1226,31 @@ def recurrent_state_rows(key_dim: int) -> int:
     return lanes * per_lane
 
 
+CHUNK_TOKENS = 64               # tokens of a chunk (recurrent_chunks.cu)
+# tokens from which an entry goes in chunks: 16 heads of 128 x 128 take 38.8 us either way at 256 tokens with one decay a head (270
+# against 107 us at 2,048); 8 heads of 128 x 256 with one a channel 43 against 63 us at 256, 81 against 65 at 512, 312 against 154 at 2,048
+CHUNK_MIN_TOKENS, GATED_CHUNK_MIN_TOKENS = 256, 384
+CHUNK_STATE_FLOATS = 1 << 27    # the most a call keeps of chunks' states (with their pieces 1.25 GiB); beyond it the entries walk
+
+
+def _scan_chunks(T: int, entries: int, longest: int, state: int, least: int) -> int:
+    """Chunks a call with `longest` tokens in its longest entry is laid out for (an upper bound), 0: every entry walks."""
+    if longest < least or entries < 1 or longest > T:
+        return 0
+    chunks = T // CHUNK_TOKENS + min(entries, T // least)
+    return chunks if chunks * state <= CHUNK_STATE_FLOATS else 0
+
+
+def _chunk_scratch(chunks: int, device: torch.device, *sizes: int):
+    """A block of memory, to be held until the launches are made, and in it the addresses of arrays of so many bytes a chunk (the chunks' own states, the products of their decays, the states in front
+    of them in three bf16 pieces and so on), each on a 256-byte boundary of one block."""
+    at = [0]
+    for n in sizes:
+        at.append(at[-1] + (chunks * n + 255) // 256 * 256)
+    buf = torch.empty(at[-1], dtype=torch.uint8, device=device)
+    return buf, [buf.data_ptr() + a for a in at[:-1]]
+
+
 def _scan_common(state: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor,
                  T: int, H: int, dk: int, dv: int, what: str) -> None:
     _i32(cu_q, "cu_q"); _i32(state_slots, "state_slots")
@@ -1249,12 +1274,13 @@ def _cols(t: torch.Tensor, T: int, n: int, dtype: torch.dtype, what: str) -> Non
 
 def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, z_bias: Optional[torch.Tensor],
                q_scale: float, tau: float, out: torch.Tensor, state: torch.Tensor, cu_q: torch.Tensor,
-               state_slots: torch.Tensor, entries: int, num_heads: int, key_dim: int, value_dim: int) -> None:
+               state_slots: torch.Tensor, entries: int, num_heads: int, key_dim: int, value_dim: int, longest: int = 0) -> None:
     """Gated linear attention over every entry's tokens in order, from and into state[slot]:
     S = diag(sigmoid(z + z_bias)^(1/tau)) S + k v^T, out = S^T (q * q_scale).  q, k [T, H*dk], v [T, H*dv]
     (column views allowed), z fp32 [T, H*dk]; state [slots, H, dv, recurrent_state_rows(dk)].  Two
     launches: the decays of all tokens at once (z is overwritten with them), then the walk (a step in
-    which every entry brings one token, T == entries, goes to the kernel without staging)."""
+    which every entry brings one token, T == entries, goes to the kernel without staging).  `longest`: as `head_scan`'s
+    (bf16 q, k, v)."""
     require_cuda(q, k, v, z, z_bias, out, state, cu_q, state_slots)
     T, H, dk, dv = q.shape[0], num_heads, key_dim, value_dim
     _scan_common(state, out, cu_q, state_slots, T, H, dk, dv, "gated_scan")
@@ -1265,10 +1291,19 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
         raise KernelError("gated_scan: z_bias has H*dk elements")
     check(L.core().ri_gated_decay(_p(z), _p(z_bias), dtype_code(z_bias.dtype) if z_bias is not None else 0,
                                   1.0 / float(tau), T, H * dk, stream_ptr()), "gated_decay")
-    check(L.recurrent(dk).ri_gated_scan(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(z), z.stride(0),
-                                        dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q),
-                                        _p(state_slots), int(entries), H, dv, 1 if T == int(entries) else 0,
-                                        stream_ptr()), "gated_scan")
+    lib = L.recurrent(dk)
+    qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
+    row = (_p(z), z.stride(0), dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries))
+    below = 0
+    if lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 1):
+        chunks = _scan_chunks(T, int(entries), longest, H * dv * dk, GATED_CHUNK_MIN_TOKENS)
+        if chunks:
+            held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 4 * H * dk, 6 * H * dv * dk, 2 * H * lib.ri_gated_chunk_parts())
+            check(lib.ri_gated_chunks(*qkv, *row, GATED_CHUNK_MIN_TOKENS, chunks, H, dv, *scratch, stream_ptr()), "gated_chunks")
+            if T == longest * int(entries):                   # every entry is as long
+                return
+            below = GATED_CHUNK_MIN_TOKENS
+    check(lib.ri_gated_scan_short(*qkv, *row, H, dv, 1 if T == int(entries) else 0, below, stream_ptr()), "gated_scan")
 
 
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, q_scale: float,
@@ -1294,12 +1329,14 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
 def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, q_scale: float, out: torch.Tensor,
               state: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, entries: int, num_heads: int, key_dim: int,
               value_dim: int, gain: Optional[torch.Tensor] = None, key_heads: Optional[int] = None,
-              rotation: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int, bool]] = None) -> None:
+              rotation: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int, bool]] = None, longest: int = 0) -> None:
     """Linear attention with one decay a head, over every entry's tokens in order, from and into state[slot]:
     S = decay_h S + k (gain_h v)^T, out = S^T (q * q_scale).  `decay` fp32 [H] (fixed) or [T, H]; `gain` fp32 [T, H] or
     None (1); head h reads key and query head h // (H / key_heads) of q, k [T, key_heads*dk]; v [T, H*dv]; column views
     allowed.  State as `gated_scan`.  `rotation` (positions int32 [T], cos, sin fp32 [positions, rot/2], rot, interleaved):
-    keys and queries are rotated on the way in; only for a step in which every entry brings one token (T == entries)."""
+    keys and queries are rotated on the way in; only for a step in which every entry brings one token (T == entries).
+    `longest`: the most tokens an entry brings, from a caller that does not need a token's sums to be the same however its
+    prompt was cut: entries of CHUNK_MIN_TOKENS or more then go in chunks (recurrent_chunks.cu)."""
     require_cuda(q, k, v, decay, out, state, cu_q, state_slots, gain, *(rotation[:3] if rotation else ()))
     T, H, dk, dv = q.shape[0], num_heads, key_dim, value_dim
     G = key_heads or H
@@ -1320,11 +1357,22 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
         if T != int(entries) or cos.dtype != torch.float32 or cos.shape[1] != rot // 2 or sin.shape != cos.shape \
                 or not cos.is_contiguous() or not sin.is_contiguous():
             raise KernelError("head_scan: rotation goes with single tokens; cos/sin are fp32 [positions, rot/2]")
-    check(L.recurrent(dk).ri_head_scan(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
-                                       H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0,
-                                       dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots),
-                                       int(entries), H, dv, H // G, _p(pos), _p(cos), _p(sin), int(rot), 1 if inter else 0,
-                                       1 if T == int(entries) else 0, stream_ptr()), "head_scan")
+    lib = L.recurrent(dk)
+    qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
+    row = (_p(decay), H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0, dtype_code(q.dtype), float(q_scale),
+           _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries))
+    below = 0
+    if rotation is None and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 0):
+        chunks = _scan_chunks(T, int(entries), longest, H * dv * dk, CHUNK_MIN_TOKENS)
+        if chunks:
+            held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 8 * H, 6 * H * dv * dk)
+            check(lib.ri_head_chunks(*qkv, *row, CHUNK_MIN_TOKENS, chunks, H, dv, H // G, *scratch, stream_ptr()),
+                  "head_chunks")
+            if T == longest * int(entries):                   # every entry is as long
+                return
+            below = CHUNK_MIN_TOKENS
+    check(lib.ri_head_scan_short(*qkv, *row, H, dv, H // G, _p(pos), _p(cos), _p(sin), int(rot), 1 if inter else 0,
+                                 1 if T == int(entries) else 0, below, stream_ptr()), "head_scan")
 
 
 def delta_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, za: torch.Tensor, za_bias: Optional[torch.Tensor],

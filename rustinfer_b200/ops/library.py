@@ -71,6 +71,13 @@ _SIGNATURES = {
     "ri_gated_head_norm": [_P, _P, _I, _P, _I, _I, _I, _F, _P, _I, _I, _I, _I, _P],
     "ri_activation": [_P, _P, _I, _L, _I, _P],
     "ri_scaled_sum": [_P, _P, _F, _F, _P, _I, _L, _P],
+    "ri_gated_scan_short": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "ri_delta_scan_short": [_P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "ri_head_scan_short": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _P],
+    "ri_chunks_ok": [_P, _I, _P, _I, _P, _I, _I, _I, _I],
+    "ri_head_chunks": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P],
+    "ri_gated_chunks": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
+    "ri_gated_chunk_parts": [],
     "ri_gated_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "ri_delta_scan": [_P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "ri_rms_sandwich": [_P, _I, _P, _I, _I, _P, _P, _P, _L, _I, _P, _P, _P, _P, _I, _P, _I, _I, _F, _P, _P, _P, _I, _P],
@@ -173,7 +180,7 @@ def recurrent(key_dim: int) -> ctypes.CDLL:
     """The linear-attention recurrences (gated and delta rule) for one key size."""
     if not 1 <= key_dim <= 512:
         raise KernelError(f"the recurrence kernels take key sizes up to 512, got {key_dim}")
-    lib = _load(f"ri_recurrent_k{key_dim}", ["recurrent.cu"], [f"RI_KDIM={key_dim}"])
+    lib = _load(f"ri_recurrent_k{key_dim}", ["recurrent.cu", "recurrent_chunks.cu"], [f"RI_KDIM={key_dim}"])
     lib.ri_recurrent_state_rows.restype = _I
     return lib
 

@@ -120,7 +120,8 @@ class GatedLinearAttention(_StateMixer):
         z = self.a2(self.a1(x, out_dtype=dt), out_dtype=torch.float32)
         o = torch.empty((T, self.H * self.dv), dtype=torch.float32, device=x.device)
         K.gated_scan(p["q"], p["k"], p["v"], z, self.a_bias, self.dk ** -0.5, self.tau, o, cache.state,
-                     step.cu_q, step.state_slots, step.num_entries, self.H, self.dk, self.dv)
+                     step.cu_q, step.state_slots, step.num_entries, self.H, self.dk, self.dv,
+                     longest=step.max_q_len if dt == torch.bfloat16 else 0)
         y = torch.empty((T, self.H * self.dv), dtype=dt, device=x.device)
         K.gated_head_norm(o, p["g"], self.norm_w, False, K.GATE_SILU, self.norm_eps, y, self.H, self.dv)
         return self.o(y, out_dtype=dt)
@@ -316,7 +317,8 @@ class Retention(Mixer):
                 K.rotate_cols(p[:, : 2 * qk], step.positions, pos.cos, pos.sin, 2 * self.H, self.dk, pos.rotary_dim, inter)
         o = torch.empty((T, vg), dtype=torch.float32, device=x.device)
         K.head_scan(p[:, :qk], p[:, qk: 2 * qk], p[:, 2 * qk: 2 * qk + vg], self.decay_row, self.k_scale, o, cache.state,
-                    step.cu_q, step.state_slots, step.num_entries, self.H, self.dk, self.dv, rotation=rotation)
+                    step.cu_q, step.state_slots, step.num_entries, self.H, self.dk, self.dv, rotation=rotation,
+                    longest=step.max_q_len if self.ctx.dtype == torch.bfloat16 else 0)
         y = torch.empty((T, vg), dtype=self.ctx.dtype, device=x.device)
         K.part_norm_gate(o, p[:, 2 * qk + vg:], None, self.H, self.norm_eps, False, y)
         return self.o(y, out_dtype=torch.float32)

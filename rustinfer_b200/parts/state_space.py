@@ -79,7 +79,8 @@ class Mamba2(Mixer):
         x = xbc[:, :I]
         y = torch.empty((T, I), dtype=torch.float32, device=dev)
         K.head_scan(xbc[:, I + GN:], xbc[:, I: I + GN], x, sizes[1], 1.0, y, state_cache.state, step.cu_q, step.state_slots,
-                    step.num_entries, self.H, self.N, self.vd, gain=sizes[0], key_heads=self.G)
+                    step.num_entries, self.H, self.N, self.vd, gain=sizes[0], key_heads=self.G,
+                    longest=step.max_q_len if self.ctx.dtype == torch.bfloat16 else 0)
         out = torch.empty((T, I), dtype=self.ctx.dtype, device=dev)
         K.part_norm_gate(y, proj[:, :I], self.norm_w, self.norm_groups, self.norm_eps, True, out, skip=(self.skip, x))
         return self.o(out, out_dtype=torch.float32)
