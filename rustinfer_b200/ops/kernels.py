@@ -193,7 +193,8 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int =
     """out = x[M,K] @ w[N,K]^T on the tcgen05 tensor cores, bf16 inputs, fp32 accumulation.
     epilogue: EPI_BF16 / EPI_F32 store into out [M,N]; EPI_SILU stores silu(gate)*up into
     out [M,N/2] for a weight whose rows alternate gate_j, up_j; EPI_RESIDUAL adds into the
-    fp32 out [M,N]; EPI_RELU2 stores max(x, 0)^2 as bf16; EPI_GELU is EPI_SILU with gelu_tanh(gate)*up."""
+    fp32 out [M,N]; EPI_RELU2 stores max(x, 0)^2 as bf16; EPI_GELU is EPI_SILU with gelu_tanh(gate)*up.  Without a `plan`, up
+    to 32 rows against weights of a few megabytes go to the kernel without tensor memory (gemm_few.cu)."""
     require_cuda(x, w, out)
     if not gemm_tc_supports(x, w):
         raise KernelError("gemm_tc: contiguous, 16-byte aligned bfloat16 x [M,K] and w [N,K] with K a multiple of 8")
@@ -206,6 +207,11 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int =
     want = torch.bfloat16 if pairs or epilogue in (EPI_BF16, EPI_RELU2) else torch.float32
     if out.dtype != want or out.shape != (M, cols) or (pairs and N % 2):
         raise KernelError(f"gemm_tc: out must be {want} [{M}, {cols}] for epilogue {epilogue}")
+    if plan is None and M <= 32:                              # a decode step's small products
+        shape = int(L.gemm_tc().ri_gemm_few_shape(M, N, Kd))
+        if shape >= 0:
+            check(L.gemm_tc().ri_gemm_few(_p(x), _p(w), M, N, Kd, _p(out), out.stride(0), epilogue, shape, stream_ptr()), "gemm_few")
+            return
     plan = plan or gemm_tc_plan(M, N, Kd, num_sms, epilogue)
     swap, bn, splits = plan[:3]
     a_box = plan[3] if len(plan) > 3 else 128

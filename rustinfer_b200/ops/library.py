@@ -71,6 +71,8 @@ _SIGNATURES = {
     "ri_gated_head_norm": [_P, _P, _I, _P, _I, _I, _I, _F, _P, _I, _I, _I, _I, _P],
     "ri_activation": [_P, _P, _I, _L, _I, _P],
     "ri_scaled_sum": [_P, _P, _F, _F, _P, _I, _L, _P],
+    "ri_gemm_few": [_P, _P, _I, _I, _I, _P, _I, _I, _I, _P],
+    "ri_gemm_few_shape": [_I, _I, _I],
     "ri_gated_scan_short": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "ri_delta_scan_short": [_P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "ri_head_scan_short": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _P],
@@ -186,7 +188,7 @@ def recurrent(key_dim: int) -> ctypes.CDLL:
 
 
 def gemm_tc() -> ctypes.CDLL:
-    lib = _load("ri_gemm_tc", ["gemm_tc.cu", "decode_chain.cu", "decode_chain_wide.cu"])
+    lib = _load("ri_gemm_tc", ["gemm_tc.cu", "gemm_few.cu", "decode_chain.cu", "decode_chain_wide.cu"])
     kb = os.environ.get("RUSTINFER_B200_STREAM_KB")
     if kb and not getattr(lib, "_budget_set", False):
         lib.ri_gemm_tc_set_stream_budget.argtypes = [_I]
