@@ -132,6 +132,27 @@ __global__ void rotate_cols_kernel(float* __restrict__ x, int stride, const int*
     }
 }
 
+__device__ __forceinline__ float4 four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// The same for halves that come in aligned fours: four pairs a thread, a token a row of CTAs (no division of 64-bit numbers).
+// 2,000 tokens of 32 rotated heads of 128: 18.7 -> 8.2 us (65 MB there and back; they lie in L2).
+__global__ void __launch_bounds__(256)
+rotate_fours_kernel(float* __restrict__ x, int stride, const int* __restrict__ positions, const float* __restrict__ cos_t,
+                    const float* __restrict__ sin_t, int heads, int dk, int half) {
+    pdl_trigger();
+    pdl_wait();
+    const int per = half >> 2, n = heads * per, t = blockIdx.x;
+    const size_t at = (size_t)positions[t] * half;
+    float* row = x + (size_t)t * stride;
+    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < n; e += gridDim.y * blockDim.x) {
+        const int h = e / per, i = (e - h * per) * 4;
+        float* p = row + h * dk + i;
+        const float4 u = four(p), v = four(p + half), c = four(cos_t + at + i), s = four(sin_t + at + i);
+        *reinterpret_cast<float4*>(p) = make_float4(u.x * c.x - v.x * s.x, u.y * c.y - v.y * s.y, u.z * c.z - v.z * s.z, u.w * c.w - v.w * s.w);
+        *reinterpret_cast<float4*>(p + half) = make_float4(v.x * c.x + u.x * s.x, v.y * c.y + u.y * s.y, v.z * c.z + u.z * s.z, v.w * c.w + u.w * s.w);
+    }
+}
+
 // A row of o [T][n_parts * n] in n_parts parts, each normed by its own root mean square.  With y = o (+ skip[channel / skip_group] * x):
 //   gate_first:  g = y * silu(z);  out = g / rms(g) * w        else:  out = y / rms(y) * w * silu(z)
 // (w null: 1; w has a number for every channel of the row).  GROUP threads a part, the part's values in shared memory.
@@ -178,6 +199,70 @@ part_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ x, 
     }
 }
 
+// The same for parts of up to 1,024 channels that come in aligned fours: a warp a part, NV fours a lane, every load asked for
+// before the first is used and the part kept in registers.  2,048 rows of 4 parts of 512 channels: 31.1 -> 13.2 us (59 MB, 8.9 us at
+// the copy bandwidth); 2,000 rows of 16 parts of 128: 18.1 -> 10.5 us (41 MB, 6.2 us).
+template <typename TO> __device__ __forceinline__ void put_four(TO* p, float4 v);
+template <> __device__ __forceinline__ void put_four<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+template <> __device__ __forceinline__ void put_four<bf16>(bf16* p, float4 v) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+__device__ __forceinline__ float silu_of(float g) { return g / (1.0f + expf(-g)); }
+
+template <typename TO, int NV>
+__global__ void __launch_bounds__(256)
+part_norm_gate_fours_kernel(const float* __restrict__ o, const float* __restrict__ x, int x_stride, const float* __restrict__ skip,
+                            int skip_group, const float* __restrict__ z, int z_stride, const float* __restrict__ w, float eps,
+                            int gate_first, TO* __restrict__ out, long long items, int parts, int n) {
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (item >= items) return;
+    const long long t = item / parts;
+    const int c0 = (int)(item - t * parts) * n;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 y[NV], g[NV], xs[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = (j * 32 + lane) * 4;
+        y[j] = g[j] = xs[j] = zero;
+        if (i < n) {
+            y[j] = four(o + (size_t)t * parts * n + c0 + i);
+            g[j] = four(z + (size_t)t * z_stride + c0 + i);
+            if (skip) xs[j] = four(x + (size_t)t * x_stride + c0 + i);
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = (j * 32 + lane) * 4;
+        if (i >= n) continue;
+        if (skip) {                                          // a group of the skip's numbers holds whole fours
+            const float d = skip[(c0 + i) / skip_group];
+            y[j] = make_float4(fmaf(d, xs[j].x, y[j].x), fmaf(d, xs[j].y, y[j].y), fmaf(d, xs[j].z, y[j].z), fmaf(d, xs[j].w, y[j].w));
+        }
+        g[j] = make_float4(silu_of(g[j].x), silu_of(g[j].y), silu_of(g[j].z), silu_of(g[j].w));
+        if (gate_first) y[j] = make_float4(y[j].x * g[j].x, y[j].y * g[j].y, y[j].z * g[j].z, y[j].w * g[j].w);
+        ss += (y[j].x * y[j].x + y[j].y * y[j].y) + (y[j].z * y[j].z + y[j].w * y[j].w);
+    }
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)n + eps);
+    TO* dst = out + (size_t)t * parts * n + c0;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = (j * 32 + lane) * 4;
+        if (i >= n) continue;
+        float4 r = make_float4(y[j].x * inv, y[j].y * inv, y[j].z * inv, y[j].w * inv);
+        if (w) {
+            const float4 ww = four(w + c0 + i);
+            r = make_float4(r.x * ww.x, r.y * ww.y, r.z * ww.z, r.w * ww.w);
+        }
+        if (!gate_first) r = make_float4(r.x * g[j].x, r.y * g[j].y, r.z * g[j].z, r.w * g[j].w);
+        put_four<TO>(dst + i, r);
+    }
+}
+
 }  // namespace
 
 // h fp32 [rows][d] += rms(y) * w in place; act (may be null) gets the new h rounded to act_dtype.  w fp32: one number
@@ -216,6 +301,13 @@ RI_API int ri_rotate_cols(float* x, int stride, const int* positions, const floa
                           int heads, int dk, int rot, int interleaved, void* stream) {
     if (tokens <= 0 || rot <= 0) return 0;
     if (rot > dk || (rot & 1) || !cos_t || !sin_t) return (int)cudaErrorInvalidValue;
+    auto at16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+    if (!interleaved && rot % 8 == 0 && dk % 4 == 0 && stride % 4 == 0 && at16(x) && at16(cos_t) && at16(sin_t)) {
+        const int rows = (heads * (rot / 8) + 255) / 256;
+        RI_CHECKED(ri_launch(rotate_fours_kernel, dim3((unsigned)tokens, (unsigned)(rows < 65535 ? rows : 65535)), dim3(256), 0, (cudaStream_t)stream, x,
+                             stride, positions, cos_t, sin_t, heads, dk, rot / 2));
+        return ri_launch_status();
+    }
     const long long total = (long long)tokens * heads * (rot / 2), nb = (total + 255) / 256;
     const long long most = (long long)ri_device_sms() * 16;
     RI_CHECKED(ri_launch(rotate_cols_kernel, dim3((unsigned)(nb < most ? nb : most)), dim3(256), 0, (cudaStream_t)stream, x, stride,
@@ -232,6 +324,19 @@ RI_API int ri_part_norm_gate(const float* o, const float* x, int x_stride, const
     if (parts <= 0 || n <= 0 || (skip && (!x || skip_group <= 0)) || !z) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
     const long long items = (long long)rows * parts;
+    auto at16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+    if (n % 4 == 0 && n <= 1024 && z_stride % 4 == 0 && at16(o) && at16(z) && at16(w) && at16(out) &&
+        (!skip || (x_stride % 4 == 0 && skip_group % 4 == 0 && at16(x)))) {
+        const dim3 grid((unsigned)((items + 7) / 8));
+#define RI_PF(TO, NV) RI_CHECKED(ri_launch(part_norm_gate_fours_kernel<TO, NV>, grid, dim3(256), 0, s, o, x, x_stride, skip, skip_group, z, z_stride, w, \
+            eps, gate_first, (TO*)out, items, parts, n))
+#define RI_PF2(TO) do { if (n <= 128) RI_PF(TO, 1); else if (n <= 256) RI_PF(TO, 2); else if (n <= 512) RI_PF(TO, 4); else RI_PF(TO, 8); } while (0)
+        if (out_dtype == RI_BF16) RI_PF2(bf16);
+        else RI_PF2(float);
+#undef RI_PF2
+#undef RI_PF
+        return ri_launch_status();
+    }
     const bool warp = n <= 256;
     const size_t smem = (size_t)(warp ? 8 : 1) * n * sizeof(float);
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;

@@ -372,6 +372,106 @@ __global__ void delta_prepare_kernel(const TA* __restrict__ k, int k_stride, con
     }
 }
 
+// Rows that come in aligned fours: a lane holds its fours in registers, every load asked for before the first is used.
+__device__ __forceinline__ float4 take4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 take4(const bf16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                       __uint_as_float(raw.y & 0xffff0000u));
+}
+__device__ __forceinline__ void give4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void give4(bf16* p, float4 v) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+
+// gated_head_norm for heads of up to 512 channels, NV fours a lane.  2,048 tokens of 8 heads of 256: 16.7 -> 9.4 us (33 MB, 5.0 us
+// at the copy bandwidth).
+template <typename TA, typename TW, int NV>
+__global__ void __launch_bounds__(128)
+gated_head_norm_fours_kernel(const float* __restrict__ o, const TA* __restrict__ gate, int gate_stride, const TW* __restrict__ w,
+                             int w_per_head, int act, float eps, TA* __restrict__ out, int tokens, int H, int dv) {
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (item >= (long long)tokens * H) return;
+    const int t = (int)(item / H), hh = (int)(item % H);
+    const float* x = o + ((size_t)t * H + hh) * dv;
+    const TA* gp = gate + (size_t)t * gate_stride + (size_t)hh * dv;
+    const TW* wp = w + (w_per_head ? (size_t)hh * dv : 0);
+    float4 y[NV], g[NV], ww[NV];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = (j * 32 + lane) * 4;
+        y[j] = i < dv ? take4(x + i) : zero;
+        g[j] = i < dv ? take4(gp + i) : zero;
+        ww[j] = i < dv ? take4(wp + i) : zero;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) ss += (y[j].x * y[j].x + y[j].y * y[j].y) + (y[j].z * y[j].z + y[j].w * y[j].w);
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)dv + eps);
+    TA* op = out + ((size_t)t * H + hh) * dv;
+    auto one = [&](float v, float gg, float we) {
+        const float sg = sigmoid_f(gg);
+        return v * inv * we * (act == 0 ? gg * sg : sg);
+    };
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = (j * 32 + lane) * 4;
+        if (i < dv)
+            give4(op + i, make_float4(one(y[j].x, g[j].x, ww[j].x), one(y[j].y, g[j].y, ww[j].y), one(y[j].z, g[j].z, ww[j].z), one(y[j].w, g[j].w, ww[j].w)));
+    }
+}
+
+// delta_prepare for heads of up to 512 channels.  2,444 tokens of 16 heads of 128: 28.7 -> 18.4 us (100 MB, 15 us at the copy bandwidth).
+template <typename TA, typename TW, int NV>
+__global__ void __launch_bounds__(128)
+delta_prepare_fours_kernel(const TA* __restrict__ k, int k_stride, const TA* __restrict__ za, int za_stride,
+                           const TW* __restrict__ za_bias, float* __restrict__ zw, const TW* __restrict__ zw_bias, float decay_rate,
+                           float unit_eps, float* __restrict__ u, float* __restrict__ au, int tokens, int H, int dk) {
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (item >= (long long)tokens * H) return;
+    const int t = (int)(item / H), hh = (int)(item % H);
+    const TA* kp = k + (size_t)t * k_stride + (size_t)hh * dk;
+    const TA* ap = za + (size_t)t * za_stride + (size_t)hh * dk;
+    const size_t base = ((size_t)t * H + hh) * dk;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 kk[NV], a[NV], w[NV], ba[NV], bw[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = (j * 32 + lane) * 4;
+        const bool in = i < dk;
+        kk[j] = in ? take4(kp + i) : zero;
+        a[j] = in ? take4(ap + i) : zero;
+        w[j] = in ? take4(zw + base + i) : zero;
+        ba[j] = in && za_bias ? take4(za_bias + hh * dk + i) : zero;
+        bw[j] = in && zw_bias ? take4(zw_bias + hh * dk + i) : zero;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) ss += (kk[j].x * kk[j].x + kk[j].y * kk[j].y) + (kk[j].z * kk[j].z + kk[j].w * kk[j].w);
+    const float inv = 1.0f / sqrtf(warp_sum(ss) + unit_eps);
+    auto decay = [&](float z) { return expf(-decay_rate * sigmoid_f(z)); };
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = (j * 32 + lane) * 4;
+        if (i >= dk) continue;
+        const float4 e = make_float4(kk[j].x * inv, kk[j].y * inv, kk[j].z * inv, kk[j].w * inv);
+        give4(u + base + i, e);
+        give4(au + base + i, make_float4(sigmoid_f(a[j].x + ba[j].x) * e.x, sigmoid_f(a[j].y + ba[j].y) * e.y, sigmoid_f(a[j].z + ba[j].z) * e.z,
+                                         sigmoid_f(a[j].w + ba[j].w) * e.w));
+        give4(zw + base + i, make_float4(decay(w[j].x + bw[j].x), decay(w[j].y + bw[j].y), decay(w[j].z + bw[j].z), decay(w[j].w + bw[j].w)));
+    }
+}
+inline bool in_fours(const void* p, int size) { return (uintptr_t)p % (4 * (uintptr_t)size) == 0; }
+inline int size_of(int dtype) { return dtype == RI_BF16 ? 2 : 4; }
+
 inline int ew_blocks(long long n) { return (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8); }
 }  // namespace
 
@@ -464,6 +564,19 @@ RI_API int ri_gated_head_norm(const float* o, const void* gate, int gate_stride,
     const long long items = (long long)tokens * H;
     const int warps = 4;
     const dim3 grid((unsigned)((items + warps - 1) / warps));
+    if (dv % 4 == 0 && dv <= 512 && gate_stride % 4 == 0 && in_fours(o, 4) && in_fours(gate, size_of(act_dtype)) && in_fours(w, size_of(w_dtype)) &&
+        in_fours(out, size_of(act_dtype))) {
+#define RI_GF(TA, TW, NV) RI_CHECKED(ri_launch(gated_head_norm_fours_kernel<TA, TW, NV>, grid, dim3(128), 0, s, o, (const TA*)gate, gate_stride, \
+        (const TW*)w, w_per_head, act, eps, (TA*)out, tokens, H, dv))
+#define RI_GF2(TA, TW) do { if (dv <= 128) RI_GF(TA, TW, 1); else if (dv <= 256) RI_GF(TA, TW, 2); else RI_GF(TA, TW, 4); } while (0)
+        if (act_dtype == RI_BF16 && w_dtype == RI_BF16) RI_GF2(bf16, bf16);
+        else if (act_dtype == RI_BF16) RI_GF2(bf16, float);
+        else if (w_dtype == RI_BF16) RI_GF2(float, bf16);
+        else RI_GF2(float, float);
+#undef RI_GF2
+#undef RI_GF
+        return ri_launch_status();
+    }
 #define RI_GHN(TA, TW) RI_CHECKED(ri_launch(gated_head_norm_kernel<TA, TW>, grid, dim3(32 * warps), 0, s, o, \
         (const TA*)gate, gate_stride, (const TW*)w, w_per_head, act, eps, (TA*)out, tokens, H, dv))
     if (act_dtype == RI_BF16 && w_dtype == RI_BF16) RI_GHN(bf16, bf16);
@@ -527,6 +640,19 @@ RI_API int ri_delta_prepare(const void* k, int k_stride, const void* za, int za_
     const long long items = (long long)tokens * H;
     const int warps = 4;
     const dim3 grid((unsigned)((items + warps - 1) / warps));
+    if (dk % 4 == 0 && dk <= 512 && k_stride % 4 == 0 && za_stride % 4 == 0 && in_fours(k, size_of(act_dtype)) && in_fours(za, size_of(act_dtype)) &&
+        in_fours(za_bias, size_of(w_dtype)) && in_fours(zw_bias, size_of(w_dtype)) && in_fours(zw, 4) && in_fours(u, 4) && in_fours(au, 4)) {
+#define RI_DF(TA, TW, NV) RI_CHECKED(ri_launch(delta_prepare_fours_kernel<TA, TW, NV>, grid, dim3(128), 0, s, (const TA*)k, k_stride, (const TA*)za, \
+        za_stride, (const TW*)za_bias, zw, (const TW*)zw_bias, decay_rate, unit_eps, u, au, tokens, H, dk))
+#define RI_DF2(TA, TW) do { if (dk <= 128) RI_DF(TA, TW, 1); else if (dk <= 256) RI_DF(TA, TW, 2); else RI_DF(TA, TW, 4); } while (0)
+        if (act_dtype == RI_BF16 && w_dtype == RI_BF16) RI_DF2(bf16, bf16);
+        else if (act_dtype == RI_BF16) RI_DF2(bf16, float);
+        else if (w_dtype == RI_BF16) RI_DF2(float, bf16);
+        else RI_DF2(float, float);
+#undef RI_DF2
+#undef RI_DF
+        return ri_launch_status();
+    }
 #define RI_DP(TA, TW) RI_CHECKED(ri_launch(delta_prepare_kernel<TA, TW>, grid, dim3(32 * warps), 0, s, (const TA*)k, k_stride, \
         (const TA*)za, za_stride, (const TW*)za_bias, zw, (const TW*)zw_bias, decay_rate, unit_eps, u, au, tokens, H, dk))
     if (act_dtype == RI_BF16 && w_dtype == RI_BF16) RI_DP(bf16, bf16);

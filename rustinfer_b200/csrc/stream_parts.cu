@@ -284,6 +284,76 @@ __global__ void __launch_bounds__(1024) qkv_prepare_kernel(const TI* __restrict_
     }
 }
 
+// The same without norms and convolution, for rows and heads that come in aligned fours: four channels a thread straight from the
+// projection to q or the cache, no row in shared memory.  A rotated four fetches its partner from the projection.  2,048 tokens of
+// 32 + 2 x 8 heads of 64: 19.9 -> 10.0 us (38 MB, 5.7 us at the copy bandwidth).
+__device__ __forceinline__ float4 take4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 take4(const bf16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                       __uint_as_float(raw.y & 0xffff0000u));
+}
+__device__ __forceinline__ void give4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void give4(bf16* p, float4 v) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+
+template <typename TI, typename TA>
+__global__ void __launch_bounds__(256)
+qkv_fours_kernel(const TI* __restrict__ qkv, int row_stride, const float* __restrict__ bias, const int* __restrict__ positions,
+                 const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot, int interleaved,
+                 const int* __restrict__ slot_of_token, TA* __restrict__ cache, TA* __restrict__ q_out, int Hq, int Hkv, int Hv, int dk,
+                 int dv, int has_kv, int page_size, const float* __restrict__ q_scale) {
+    pdl_trigger();
+    pdl_wait();
+    const int t = blockIdx.x, nq = Hq * dk, nk = has_kv ? Hkv * dk : 0, nv = has_kv ? Hv * dv : 0;
+    const int i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    const int slot = has_kv && cache && slot_of_token ? slot_of_token[t] : -1;
+    if (i >= nq + nk + nv || (i >= nq && slot < 0)) return;
+    const TI* row = qkv + (size_t)t * row_stride;
+    auto get = [&](int at) {
+        float4 v = take4(row + at);
+        if (bias) {
+            const float4 b = take4(bias + at);
+            v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+        }
+        return v;
+    };
+    float4 v = get(i);
+    if (i < nq + nk) {
+        const int c = i % dk;
+        if (c < rot) {
+            const int half = rot >> 1;
+            const size_t base = (size_t)positions[t] * half;
+            if (interleaved) {
+                const float2 cs = *reinterpret_cast<const float2*>(cos_t + base + (c >> 1)), sn = *reinterpret_cast<const float2*>(sin_t + base + (c >> 1));
+                v = make_float4(v.x * cs.x - v.y * sn.x, v.y * cs.x + v.x * sn.x, v.z * cs.y - v.w * sn.y, v.w * cs.y + v.z * sn.y);
+            } else {
+                const bool first = c < half;
+                const float4 w = get(first ? i + half : i - half);
+                const float4 cs = take4(cos_t + base + (first ? c : c - half)), sn = take4(sin_t + base + (first ? c : c - half));
+                if (first) v = make_float4(v.x * cs.x - w.x * sn.x, v.y * cs.y - w.y * sn.y, v.z * cs.z - w.z * sn.z, v.w * cs.w - w.w * sn.w);
+                else v = make_float4(v.x * cs.x + w.x * sn.x, v.y * cs.y + w.y * sn.y, v.z * cs.z + w.z * sn.z, v.w * cs.w + w.w * sn.w);
+            }
+        }
+        if (i < nq) {
+            const float qf = q_scale ? q_scale[positions[t]] : 1.f;
+            give4(q_out + (size_t)t * nq + i, make_float4(v.x * qf, v.y * qf, v.z * qf, v.w * qf));
+            return;
+        }
+    }
+    TA* page = cache + (size_t)(slot / page_size) * ((size_t)page_size * ((size_t)Hkv * dk + (size_t)Hv * dv));
+    const int off = slot % page_size;
+    if (i < nq + nk) {
+        const int g = (i - nq) / dk;
+        give4(page + ((size_t)g * page_size + off) * dk + (i - nq - g * dk), v);
+    } else {
+        const int at = i - nq - nk, g = at / dv;
+        give4(page + (size_t)Hkv * page_size * dk + ((size_t)g * page_size + off) * dv + (at - g * dv), v);
+    }
+}
+
 }  // namespace
 
 RI_API int ri_embed_rmsnorm(const int* ids, const void* table, int table_dtype, const void* w, int w_dtype, float eps,
@@ -350,6 +420,20 @@ RI_API int ri_qkv_prepare(const void* qkv, int in_dtype, int row_stride, const f
     cudaStream_t s = (cudaStream_t)stream;
     const size_t smem = (size_t)(Hq * dk + (has_kv ? Hkv * dk : 0) + 33) * sizeof(float);
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
+    auto fours = [](const void* p, int size) { return (uintptr_t)p % (4 * (uintptr_t)size) == 0; };
+    const int in_size = in_dtype == RI_BF16 ? 2 : 4, act_size = act_dtype == RI_BF16 ? 2 : 4;
+    if (!conv_w && norm_mode == 0 && (act_dtype == RI_BF16 || in_dtype == RI_F32) && row_stride % 4 == 0 && dk % 4 == 0 && (!has_kv || dv % 4 == 0) &&
+        (interleaved ? rot % 4 == 0 : rot % 8 == 0) && fours(qkv, in_size) && fours(bias, 4) && fours(cos_t, 4) && fours(sin_t, 4) &&
+        fours(cache, act_size) && fours(q_out, act_size)) {
+        const int n = Hq * dk + (has_kv ? Hkv * dk + Hv * dv : 0);
+        const dim3 grid((unsigned)tokens, (unsigned)((n / 4 + 255) / 256));
+#define RI_QF(TI, TA) RI_CHECKED(ri_launch(qkv_fours_kernel<TI, TA>, grid, dim3(256), 0, s, (const TI*)qkv, row_stride, bias, positions, cos_t, sin_t, \
+            rot, interleaved, slot_of_token, (TA*)cache, (TA*)q_out, Hq, Hkv, Hv, dk, dv, has_kv, page_size, q_scale))
+        if (act_dtype == RI_BF16) { if (in_dtype == RI_BF16) RI_QF(bf16, bf16); else RI_QF(float, bf16); }
+        else RI_QF(float, float);
+#undef RI_QF
+        return ri_launch_status();
+    }
 #define RI_QP(TI, TA, TW) do { \
         static bool configured = false; \
         if (!configured && smem > 48 * 1024) { \

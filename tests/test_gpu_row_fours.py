@@ -1,0 +1,98 @@
+"""Kernels that take rows in aligned fours against the general ones, which the same rows reach when they start one element later."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+BF = torch.bfloat16
+
+
+def K():
+    from rustinfer_b200.ops import kernels
+    return kernels
+
+
+def both(x):
+    """x [rows, n] as a view whose rows come in aligned fours, and as one whose rows do not."""
+    n = x.shape[1]
+    a = torch.zeros(x.shape[0], (n + 7) // 4 * 4, dtype=x.dtype, device=DEV)
+    b = torch.zeros(x.shape[0], n + 3 - (n % 2), dtype=x.dtype, device=DEV)
+    a[:, :n], b[:, 1: n + 1] = x, x
+    return a[:, :n], b[:, 1: n + 1]
+
+
+def close(a, b, dtype):
+    # the sums of a row are added in another order: a few roundings of 32 bits, which may tip one of bf16
+    return ((a.float() - b.float()).norm() / b.float().norm()).item() < (2e-6 if dtype == torch.float32 else 1e-3)
+
+
+@pytest.mark.parametrize("parts,n", [(1, 4), (3, 124), (2, 128), (4, 132), (1, 512), (2, 516), (1, 1024)])
+@pytest.mark.parametrize("gate_first", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_norm_by_parts(parts, n, gate_first, dtype):
+    torch.manual_seed(n)
+    T, C = 9, parts * n
+    o, w = torch.randn(T, C, device=DEV), torch.randn(C, device=DEV)
+    skip, got = torch.randn(C // 4, device=DEV), []
+    for z, x in zip(both(torch.randn(T, C, device=DEV)), both(torch.randn(T, C, device=DEV))):
+        out = torch.empty(T, C, dtype=dtype, device=DEV)
+        K().part_norm_gate(o, z, w, parts, 1e-5, gate_first, out, skip=(skip, x))
+        got.append(out)
+    assert close(*got, dtype)
+
+
+@pytest.mark.parametrize("heads,dk,rot", [(1, 8, 8), (5, 24, 16), (33, 128, 128)])
+def test_rotation(heads, dk, rot):
+    T = 7
+    cos, sin = torch.randn(50, rot // 2, device=DEV), torch.randn(50, rot // 2, device=DEV)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV) * 7
+    a, b = both(torch.randn(T, heads * dk, device=DEV))
+    for x in (a, b):
+        K().rotate_cols(x, pos, cos, sin, heads, dk, rot, False)
+    assert close(a, b, torch.float32)
+
+
+@pytest.mark.parametrize("H,dv", [(1, 4), (3, 100), (2, 128), (3, 132), (1, 256), (2, 512)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_norm_of_a_head_with_its_gate(H, dv, dtype, per_head):
+    T = 11
+    o, w, got = torch.randn(T, H * dv, device=DEV), torch.randn(H * dv if per_head else dv, device=DEV).to(dtype), []
+    for gate in both(torch.randn(T, H * dv, device=DEV).to(dtype)):
+        out = torch.empty(T, H * dv, dtype=dtype, device=DEV)
+        K().gated_head_norm(o, gate, w, per_head, K().GATE_SILU, 1e-5, out, H, dv)
+        got.append(out)
+    assert close(*got, dtype)
+
+
+@pytest.mark.parametrize("H,d", [(2, 64), (1, 128)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_vectors_of_the_delta_rule(H, d, dtype):
+    T, got = 5, []
+    r, v, zw, ab = (torch.randn(T, H * d, device=DEV).to(dtype) for _ in range(4))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    a = torch.randn(T, H * d, device=DEV).to(dtype)
+    for k in both(torch.randn(T, H * d, device=DEV).to(dtype)):
+        out, state = torch.empty(T, H * d, device=DEV), torch.zeros(1, H, d, K().recurrent_state_rows(d), device=DEV)
+        z = zw.float().clone()
+        K().delta_scan(r, k, v, a, ab[0].contiguous(), z, None, 0.6, 1e-6, out, state, i32([0, T]), i32([0]), 1, H, d, d)
+        got += [out, z]
+    assert close(got[0], got[2], torch.float32) and close(got[1], got[3], torch.float32)
+
+
+@pytest.mark.parametrize("Hq,Hkv,dk,dv,rot,inter", [(4, 2, 24, 40, 0, False), (3, 3, 16, 8, 16, False), (4, 1, 32, 32, 24, True), (2, 1, 8, 4, 8, False)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_queries_keys_and_values(Hq, Hkv, dk, dv, rot, inter, dtype):
+    T, page, n = 6, 4, Hq * dk + Hkv * (dk + dv)
+    cos, sin = (torch.randn(40, rot // 2, device=DEV) for _ in range(2)) if rot else (None, None)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV) * 5
+    slots = torch.tensor([3, -1, 0, 9, 4, 7], dtype=torch.int32, device=DEV)
+    bias, scale, got = torch.randn(n, device=DEV), torch.rand(40, device=DEV), []
+    for qkv in both(torch.randn(T, n, device=DEV)):
+        cache = torch.full((3, page * Hkv * (dk + dv)), 9.0, dtype=dtype, device=DEV)
+        q = torch.empty(T, Hq * dk, dtype=dtype, device=DEV)
+        K().qkv_prepare(qkv, bias, None, None, 0, 0.0, pos, cos, sin, rot, inter, slots, cache, q, Hq, Hkv, dk, dv, True, q_scale=scale)
+        got += [q, cache]
+    assert close(got[0], got[2], dtype) and close(got[1], got[3], dtype)
