@@ -81,7 +81,10 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, TO* __restrict__ o
                        int table_stride, const int* __restrict__ cu_q, const int* __restrict__ kv_len,
                        const int* __restrict__ tile_entry, const int* __restrict__ tile_q0,
                        int Hq, int Hkv, int page_size, float scale, int window, int block, int sink, Extra ex) {
-    pdl_trigger();
+    // A successor that starts early lands on whatever SMs this kernel's last wave leaves free, several CTAs to one, and stays there:
+    // the fp32 product behind a prompt of 300 tokens took three times as long.  Short kernels let it start at once.
+    const bool late = gridDim.x > 8;
+    if (!late) pdl_trigger();
     pdl_wait();
     extern __shared__ float smem[];
     float* Qs = smem;
@@ -206,6 +209,7 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, TO* __restrict__ o
                 if (VD % 8 == 0 || l8 + 8 * i < VD) acc[i] = fmaf(p, vr[8 * i], acc[i]);
         }
     }
+    if (late) pdl_trigger();
     if (row_valid) {
         const float inv = l > 0.f ? 1.0f / l : 0.f;
         const float den = ex.gate ? 1.0f + expf(-ex.gate[(size_t)(q_begin + j0 + row) * ex.gate_stride + h]) : 1.f;

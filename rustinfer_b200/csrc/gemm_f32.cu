@@ -125,14 +125,16 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
                      float* __restrict__ C, int ldc, int M, int N, int K) {
     constexpr int AP = WM + 4, WP = WN + 4;
     __shared__ __align__(16) float sm[WSTAGES][BK * (AP + WP)];
-    pdl_trigger();
-    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tr = warp / 2 * 4 + lane / 8, tc = warp % 2 * 8 + lane % 8;
     const int m0 = blockIdx.y * WM, n0 = blockIdx.x * WN;
     // a thread copies one k of every block: rows tid / BK, + WTHREADS / BK, ...
     const int ck = tid % BK, cr = tid / BK;
     constexpr int STEP = WTHREADS / BK;
+    // weights on their way into L2 a few blocks before they are copied, a line a row (128 rows, 128 threads)
+    auto ask = [&](int k) {
+        if (n0 + tid < N && k < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)(n0 + tid) * ldw + k));
+    };
     auto stage = [&](int block) {
         float* to = sm[block % WSTAGES] + ck * AP;
         const int k = block * BK + ck;
@@ -149,6 +151,9 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
         }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;\n" ::); };
+    constexpr int LINE = 32, AHEAD = 8 * LINE;               // floats of a line, and how far ahead it is asked for
+    for (int k = 0; k < AHEAD; k += LINE) ask(k);
+    pdl_wait();
     f32x2 acc[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -165,6 +170,7 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
         __syncthreads();
         if (b + WSTAGES - 1 < blocks) stage(b + WSTAGES - 1);
         commit();
+        if (b % (LINE / BK) == 0) ask(b * BK + AHEAD);
         const float* as = sm[b % WSTAGES] + tr * 4;
         const float* ws = sm[b % WSTAGES] + BK * AP + tc * 4;
 #pragma unroll
@@ -182,6 +188,7 @@ gemm_f32_wide_kernel(const float* __restrict__ A, int lda, const float* __restri
             }
         }
     }
+    pdl_trigger();                                           // not before: a successor's CTAs would crowd the SMs this grid leaves free
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int gm = m0 + tr * 4 + (i & 3) + (i >> 2) * (WM / 2);
