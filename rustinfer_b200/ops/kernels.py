@@ -1233,23 +1233,39 @@ def recurrent_state_rows(key_dim: int) -> int:
 
 
 CHUNK_TOKENS = 64               # tokens of a chunk (recurrent_chunks.cu)
-# tokens from which an entry goes in chunks: 16 heads of 128 x 128 take 38.8 us either way at 256 tokens with one decay a head (270
+# tokens from which an entry can go in chunks: 16 heads of 128 x 128 take 38.8 us either way at 256 tokens with one decay a head (270
 # against 107 us at 2,048); 8 heads of 128 x 256 with one a channel 43 against 63 us at 256, 81 against 65 at 512, 312 against 154 at 2,048
 CHUNK_MIN_TOKENS, GATED_CHUNK_MIN_TOKENS = 256, 384
+# what the two ways take, in us: a walk so much a token of its longest entry, or of all while its CTAs fill the GPU; chunks a fixed part
+# and so much a token and element of the state (fitted to 1 to 8 entries of 128 to 8,192 tokens, 4 to 64 heads)
+_WALK_US, _CHUNK_FIXED_US, _CHUNK_US = {False: 0.133, True: 0.152}, {False: 25.0, True: 40.0}, {False: 1.7e-7, True: 1.9e-7}
 CHUNK_STATE_FLOATS = 1 << 27    # the most a call keeps of chunks' states (with their pieces 1.25 GiB); beyond it the entries walk
 
 
-def _scan_chunks(T: int, entries: int, longest: int, state: int, least: int) -> int:
-    """Chunks a call with `longest` tokens in its longest entry is laid out for (an upper bound), 0: every entry walks."""
+def _scan_chunks(T: int, entries: int, longest: int, heads: int, key_dim: int, value_dim: int, gated: bool, num_sms: int) -> int:
+    """Chunks a call with `longest` tokens in its longest entry is laid out for (an upper bound), 0: every entry walks.  In chunks
+    when that is a tenth faster, the other entries taken to be equally long: those too short for chunks walk all the same."""
+    least = GATED_CHUNK_MIN_TOKENS if gated else CHUNK_MIN_TOKENS
     if longest < least or entries < 1 or longest > T:
         return 0
+    state = heads * key_dim * value_dim
     chunks = T // CHUNK_TOKENS + min(entries, T // least)
-    return chunks if chunks * state <= CHUNK_STATE_FLOATS else 0
+    if chunks * state > CHUNK_STATE_FLOATS:
+        return 0
+    filled = heads * value_dim / (16 if key_dim > 64 else 32) / (2 * num_sms)   # of the GPU by one entry's walk: CTAs over places for them
+    walk = lambda most, all_tokens: _WALK_US[gated] * max(most, all_tokens * filled)
+    rest = T - longest
+    short = rest > 0 and rest < least * (entries - 1)
+    cost = _CHUNK_FIXED_US[gated] + _CHUNK_US[gated] * state * (longest if short else T)
+    if short:
+        cost += 3.0 + walk(rest / (entries - 1), rest)
+    return chunks if cost < 0.9 * walk(longest, T) else 0
 
 
 def _chunk_scratch(chunks: int, device: torch.device, *sizes: int):
-    """A block of memory, to be held until the launches are made, and in it the addresses of arrays of so many bytes a chunk (the chunks' own states, the products of their decays, the states in front
-    of them in three bf16 pieces and so on), each on a 256-byte boundary of one block."""
+    """A block of memory, to be held until the launches are made, and in it the addresses of arrays of so many bytes a chunk (the
+    chunks' own states, the products of their decays, the states in front of them in three bf16 pieces and so on), each on a
+    256-byte boundary."""
     at = [0]
     for n in sizes:
         at.append(at[-1] + (chunks * n + 255) // 256 * 256)
@@ -1302,7 +1318,7 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
     row = (_p(z), z.stride(0), dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries))
     below = 0
     if lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 1):
-        chunks = _scan_chunks(T, int(entries), longest, H * dv * dk, GATED_CHUNK_MIN_TOKENS)
+        chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, True, L.num_sms())
         if chunks:
             held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 4 * H * dk, 6 * H * dv * dk, 2 * H * lib.ri_gated_chunk_parts())
             check(lib.ri_gated_chunks(*qkv, *row, GATED_CHUNK_MIN_TOKENS, chunks, H, dv, *scratch, stream_ptr()), "gated_chunks")
@@ -1342,7 +1358,7 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
     allowed.  State as `gated_scan`.  `rotation` (positions int32 [T], cos, sin fp32 [positions, rot/2], rot, interleaved):
     keys and queries are rotated on the way in; only for a step in which every entry brings one token (T == entries).
     `longest`: the most tokens an entry brings, from a caller that does not need a token's sums to be the same however its
-    prompt was cut: entries of CHUNK_MIN_TOKENS or more then go in chunks (recurrent_chunks.cu)."""
+    prompt was cut: entries of CHUNK_MIN_TOKENS or more may then go in chunks (recurrent_chunks.cu)."""
     require_cuda(q, k, v, decay, out, state, cu_q, state_slots, gain, *(rotation[:3] if rotation else ()))
     T, H, dk, dv = q.shape[0], num_heads, key_dim, value_dim
     G = key_heads or H
@@ -1369,7 +1385,7 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
            _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries))
     below = 0
     if rotation is None and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 0):
-        chunks = _scan_chunks(T, int(entries), longest, H * dv * dk, CHUNK_MIN_TOKENS)
+        chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, False, L.num_sms())
         if chunks:
             held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 8 * H, 6 * H * dv * dk)
             check(lib.ri_head_chunks(*qkv, *row, CHUNK_MIN_TOKENS, chunks, H, dv, H // G, *scratch, stream_ptr()),

@@ -14,6 +14,13 @@ def K():
     return kernels
 
 
+@pytest.fixture(autouse=True)
+def chunks_whatever_they_cost(monkeypatch, request):
+    """Portions of a few hundred tokens go in chunks, so that their edges are met without long prompts."""
+    if "walk" not in request.node.name:
+        monkeypatch.setattr(K(), "_CHUNK_FIXED_US", {False: -1e9, True: -1e9})
+
+
 def i32(x):
     return torch.tensor(x, dtype=torch.int32, device=DEV)
 
@@ -114,11 +121,14 @@ def test_a_value_that_is_no_number_reaches_later_tokens_only(gated, value):
 
 
 def test_calls_that_keep_the_walk():
-    """Short entries, sizes the chunks are not made for, rows that are not aligned and callers that do not ask for chunks."""
-    k = K()
-    assert k._scan_chunks(255, 1, 255, 1 << 14, 256) == 0 and k._scan_chunks(4096, 16, 0, 1 << 14, 256) == 0
-    assert k._scan_chunks(8192, 1, 8192, 1 << 24, 256) == 0                # more scratch than a call takes
-    assert k._scan_chunks(600, 3, 400, 1 << 14, 256) >= 7
+    """Short entries, batches that walk as fast, sizes the chunks are not made for, rows that are not aligned and callers that do not
+    ask for chunks."""
+    chunks = lambda T, n, longest, H=16, dk=128, dv=128, gated=False: K()._scan_chunks(T, n, longest, H, dk, dv, gated, 148)
+    assert chunks(255, 1, 255) == 0 and chunks(4096, 16, 0) == 0
+    assert chunks(8192, 1, 8192, H=1024) == 0                             # more scratch than a call takes
+    assert chunks(1138, 5, 272, H=64, dv=64) == 0                         # one entry that could, four that walk beside it
+    assert chunks(2048, 1, 2048) >= 32 and chunks(1749, 2, 999) >= 28 and chunks(2056, 9, 2048) >= 33
+    assert chunks(384, 1, 384, H=8, dv=256, gated=True) == 0 and chunks(2048, 1, 2048, H=8, dv=256, gated=True) >= 32
     lib = __import__("rustinfer_b200.ops.library", fromlist=["recurrent"]).recurrent(64)
     ok = lambda stride, dv: lib.ri_chunks_ok(256, stride, 256, stride, 256, stride, 0, dv, 0)
     assert ok(128, 64) and not ok(129, 64) and not ok(128, 48)
