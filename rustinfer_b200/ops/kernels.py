@@ -171,7 +171,19 @@ def gemm_tc_plan(M: int, N: int, K: int, num_sms: Optional[int] = None, epilogue
         tiles = -(-M // 128) * -(-N // bn)
     kblocks = -(-K // 64)
     splits, a_box = 1, 128
-    if tiles * 2 <= num_sms:
+    if not swap and N > 64 and tiles * 2 <= num_sms:
+        # few tiles of many tokens: a k-block costs a CTA 0.35 us whether its tile is 64 or 256 wide, so narrow tiles fill the SMs for
+        # nothing, where K slices of wide ones had to meet (through the workspace, or as adds of every slice into the stream): 300 x
+        # 1,024 x 2,048 35 -> 16 us (68 -> 16 added into the stream), 1,024 x 2,048 x 2,048 26 -> 16 (72 -> 16), 2,048 x 1,024 x 2,048
+        # 26 -> 17 (72 -> 16), of which some 13 us are the eager launch.  Slices only of a long K (300 x 1,024 x 4,096: 24 us
+        # whole, 18 in two; 52 before), and none where they would add into the stream (28 against 24).
+        bn = 64 if -(-M // 128) * -(-N // 64) <= num_sms else 128
+        tiles = -(-M // 128) * -(-N // bn)
+        if epilogue != EPI_RESIDUAL:
+            splits = max(1, min(num_sms // tiles, kblocks // 32))
+            while splits > 1 and tiles * splits * bn * 128 > _TC_WORKSPACE_FLOATS:
+                splits -= 1
+    elif tiles * 2 <= num_sms:
         splits = max(1, min(num_sms // tiles, kblocks // 4, 32))
         if epilogue != EPI_RESIDUAL:                       # slices meet in the workspace
             while splits > 1 and tiles * splits * bn * 128 > _TC_WORKSPACE_FLOATS:
