@@ -1329,7 +1329,7 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
     qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
     row = (_p(z), z.stride(0), dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries))
     below = 0
-    if lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 1):
+    if longest >= GATED_CHUNK_MIN_TOKENS and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 1):
         chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, True, L.num_sms())
         if chunks:
             held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 4 * H * dk, 6 * H * dv * dk, 2 * H * lib.ri_gated_chunk_parts())
@@ -1396,7 +1396,7 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
     row = (_p(decay), H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0, dtype_code(q.dtype), float(q_scale),
            _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries))
     below = 0
-    if rotation is None and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 0):
+    if longest >= CHUNK_MIN_TOKENS and rotation is None and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 0):
         chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, False, L.num_sms())
         if chunks:
             held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 8 * H, 6 * H * dv * dk)
