@@ -193,7 +193,7 @@ class LightningAttention(Mixer):
     H*dv].  The four projections are one product whose result stays fp32: the activations are formed from
     it in fp32 and the recurrence reads them unrounded, so the decays, the state and everything that
     enters it are 32-bit in both engine precisions.  The walk is the gated recurrence's with the same row
-    of decays for every token."""
+    of decays for every token; long portions in the bfloat16 engine go through the form with one decay a head."""
     graph_safe = True
     joined = ["q", "k", "v", "g"]
 
@@ -228,6 +228,7 @@ class LightningAttention(Mixer):
         super().prepare(ctx)
         per_channel = [d for d in self.decay for _ in range(self.dk)]
         self.decay_row = torch.tensor(per_channel, dtype=torch.float64).to(torch.float32).to(ctx.device)
+        self.decay_heads = torch.tensor(self.decay, dtype=torch.float64).to(torch.float32).to(ctx.device)
 
     def load(self, tensors: Dict[str, torch.Tensor]) -> None:
         n = self._name
@@ -242,8 +243,12 @@ class LightningAttention(Mixer):
         p = self.proj(x, out_dtype=torch.float32)
         K.activation_cols(p[:, : 2 * qk + vg], K.ACT_SILU)
         o = torch.empty((T, vg), dtype=torch.float32, device=x.device)
-        K.decay_scan(p[:, :qk], p[:, qk: 2 * qk], p[:, 2 * qk: 2 * qk + vg], self.decay_row, self.q_scale, o,
-                     cache.state, step.cu_q, step.state_slots, step.num_entries, self.H, self.dk, self.dv)
+        qkv = p[:, :qk], p[:, qk: 2 * qk], p[:, 2 * qk: 2 * qk + vg]
+        rest = self.q_scale, o, cache.state, step.cu_q, step.state_slots, step.num_entries, self.H, self.dk, self.dv
+        if self.ctx.dtype == torch.bfloat16 and step.max_q_len >= K.CHUNK_MIN_TOKENS:    # prompts: the form that can go in chunks
+            K.head_scan(*qkv, self.decay_heads, *rest, longest=step.max_q_len)
+        else:
+            K.decay_scan(*qkv, self.decay_row, *rest)
         y = torch.empty((T, vg), dtype=self.ctx.dtype, device=x.device)
         K.row_norm_gate(o, p[:, 2 * qk + vg:], self.norm_w, self.norm_eps, y)
         return self.o(y, out_dtype=torch.float32)
