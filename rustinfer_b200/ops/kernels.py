@@ -1325,19 +1325,23 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
         raise KernelError("gated_scan: z_bias has H*dk elements")
     check(L.core().ri_gated_decay(_p(z), _p(z_bias), dtype_code(z_bias.dtype) if z_bias is not None else 0,
                                   1.0 / float(tau), T, H * dk, stream_ptr()), "gated_decay")
-    lib = L.recurrent(dk)
-    qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
-    row = (_p(z), z.stride(0), dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries))
     below = 0
-    if longest >= GATED_CHUNK_MIN_TOKENS and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 1):
+    if longest >= GATED_CHUNK_MIN_TOKENS:
+        lib = L.recurrent(dk)
+        qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
         chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, True, L.num_sms())
-        if chunks:
+        if chunks and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 1):
             held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 4 * H * dk, 6 * H * dv * dk, 2 * H * lib.ri_gated_chunk_parts())
-            check(lib.ri_gated_chunks(*qkv, *row, GATED_CHUNK_MIN_TOKENS, chunks, H, dv, *scratch, stream_ptr()), "gated_chunks")
+            check(lib.ri_gated_chunks(*qkv, _p(z), z.stride(0), dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q),
+                                      _p(state_slots), int(entries), GATED_CHUNK_MIN_TOKENS, chunks, H, dv, *scratch, stream_ptr()),
+                  "gated_chunks")
             if T == longest * int(entries):                   # every entry is as long
                 return
             below = GATED_CHUNK_MIN_TOKENS
-    check(lib.ri_gated_scan_short(*qkv, *row, H, dv, 1 if T == int(entries) else 0, below, stream_ptr()), "gated_scan")
+    check(L.recurrent(dk).ri_gated_scan_short(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(z), z.stride(0),
+                                              dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q),
+                                              _p(state_slots), int(entries), H, dv, 1 if T == int(entries) else 0, below,
+                                              stream_ptr()), "gated_scan")
 
 
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, q_scale: float,
@@ -1391,22 +1395,24 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
         if T != int(entries) or cos.dtype != torch.float32 or cos.shape[1] != rot // 2 or sin.shape != cos.shape \
                 or not cos.is_contiguous() or not sin.is_contiguous():
             raise KernelError("head_scan: rotation goes with single tokens; cos/sin are fp32 [positions, rot/2]")
-    lib = L.recurrent(dk)
-    qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
-    row = (_p(decay), H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0, dtype_code(q.dtype), float(q_scale),
-           _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries))
     below = 0
-    if longest >= CHUNK_MIN_TOKENS and rotation is None and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 0):
+    if longest >= CHUNK_MIN_TOKENS and rotation is None:
+        lib = L.recurrent(dk)
+        qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
         chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, False, L.num_sms())
-        if chunks:
+        if chunks and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 0):
             held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 8 * H, 6 * H * dv * dk)
-            check(lib.ri_head_chunks(*qkv, *row, CHUNK_MIN_TOKENS, chunks, H, dv, H // G, *scratch, stream_ptr()),
-                  "head_chunks")
+            check(lib.ri_head_chunks(*qkv, _p(decay), H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0,
+                                     dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries),
+                                     CHUNK_MIN_TOKENS, chunks, H, dv, H // G, *scratch, stream_ptr()), "head_chunks")
             if T == longest * int(entries):                   # every entry is as long
                 return
             below = CHUNK_MIN_TOKENS
-    check(lib.ri_head_scan_short(*qkv, *row, H, dv, H // G, _p(pos), _p(cos), _p(sin), int(rot), 1 if inter else 0,
-                                 1 if T == int(entries) else 0, below, stream_ptr()), "head_scan")
+    check(L.recurrent(dk).ri_head_scan_short(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
+                                             H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0,
+                                             dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots),
+                                             int(entries), H, dv, H // G, _p(pos), _p(cos), _p(sin), int(rot), 1 if inter else 0,
+                                             1 if T == int(entries) else 0, below, stream_ptr()), "head_scan")
 
 
 def delta_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, za: torch.Tensor, za_bias: Optional[torch.Tensor],
