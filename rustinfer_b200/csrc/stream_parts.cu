@@ -422,7 +422,12 @@ RI_API int ri_qkv_prepare(const void* qkv, int in_dtype, int row_stride, const f
     if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
     auto fours = [](const void* p, int size) { return (uintptr_t)p % (4 * (uintptr_t)size) == 0; };
     const int in_size = in_dtype == RI_BF16 ? 2 : 4, act_size = act_dtype == RI_BF16 ? 2 : 4;
-    if (!conv_w && norm_mode == 0 && (act_dtype == RI_BF16 || in_dtype == RI_F32) && row_stride % 4 == 0 && dk % 4 == 0 && (!has_kv || dv % 4 == 0) &&
+    // queries stored over their projection: a rotated four would read a partner that another thread has already stored; the general
+    // kernel reads a token's whole row first
+    const uintptr_t from = (uintptr_t)qkv, from_end = from + ((size_t)(tokens - 1) * row_stride + (size_t)Hq * dk + (has_kv ? Hkv * dk + Hv * dv : 0)) * in_size;
+    const uintptr_t to = (uintptr_t)q_out, to_end = to + (size_t)tokens * Hq * dk * act_size;
+    const bool apart = to_end <= from || from_end <= to;
+    if (apart && !conv_w && norm_mode == 0 && (act_dtype == RI_BF16 || in_dtype == RI_F32) && row_stride % 4 == 0 && dk % 4 == 0 && (!has_kv || dv % 4 == 0) &&
         (interleaved ? rot % 4 == 0 : rot % 8 == 0) && fours(qkv, in_size) && fours(bias, 4) && fours(cos_t, 4) && fours(sin_t, 4) &&
         fours(cache, act_size) && fours(q_out, act_size)) {
         const int n = Hq * dk + (has_kv ? Hkv * dk + Hv * dv : 0);

@@ -96,3 +96,15 @@ def test_queries_keys_and_values(Hq, Hkv, dk, dv, rot, inter, dtype):
         K().qkv_prepare(qkv, bias, None, None, 0, 0.0, pos, cos, sin, rot, inter, slots, cache, q, Hq, Hkv, dk, dv, True, q_scale=scale)
         got += [q, cache]
     assert close(got[0], got[2], dtype) and close(got[1], got[3], dtype)
+
+
+@pytest.mark.parametrize("rot,inter", [(64, False), (24, True), (0, False)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_queries_stored_over_their_projection(rot, inter, dtype):
+    T, Hq, dk = 300, 16, 64
+    cos, sin = (torch.randn(T, rot // 2, device=DEV) for _ in range(2)) if rot else (None, None)
+    pos, x = torch.arange(T, dtype=torch.int32, device=DEV), torch.randn(T, Hq * dk, device=DEV).to(dtype)
+    apart, over = torch.empty_like(x), x.clone()
+    for src, dst in ((x, apart), (over, over)):
+        K().qkv_prepare(src, None, None, None, 0, 0.0, pos, cos, sin, rot, inter, None, None, dst, Hq, 1, dk, dk, False)
+    assert close(over, apart, dtype)
