@@ -1251,7 +1251,16 @@ CHUNK_MIN_TOKENS, GATED_CHUNK_MIN_TOKENS = 256, 384
 # what the two ways take, in us: a walk so much a token of its longest entry, or of all while its CTAs fill the GPU; chunks a fixed part
 # and so much a token and element of the state (fitted to 1 to 8 entries of 128 to 8,192 tokens, 4 to 64 heads)
 _WALK_US, _CHUNK_FIXED_US, _CHUNK_US = {False: 0.133, True: 0.152}, {False: 25.0, True: 40.0}, {False: 1.7e-7, True: 1.9e-7}
-CHUNK_STATE_FLOATS = 1 << 27    # the most a call keeps of chunks' states (with their pieces 1.25 GiB); beyond it the entries walk
+CHUNK_SCRATCH_BYTES = 1288 << 20    # the most scratch a call in chunks takes (1.26 GiB); a call that would take more walks, which takes none
+
+
+def _chunk_sizes(heads: int, key_dim: int, value_dim: int, gated: bool) -> Tuple[int, ...]:
+    """Bytes a chunk takes of every scratch array: the chunk's own state, the products of its decays, the state in front of it in three
+    bf16 pieces and, in the gated form, its scores and queries in three pieces each."""
+    state = heads * key_dim * value_dim
+    if not gated:
+        return 4 * state, 8 * heads, 6 * state
+    return 4 * state, 4 * heads * key_dim, 6 * state, 6 * heads * CHUNK_TOKENS * (CHUNK_TOKENS + key_dim)
 
 
 def _scan_chunks(T: int, entries: int, longest: int, heads: int, key_dim: int, value_dim: int, gated: bool, num_sms: int) -> int:
@@ -1262,7 +1271,7 @@ def _scan_chunks(T: int, entries: int, longest: int, heads: int, key_dim: int, v
         return 0
     state = heads * key_dim * value_dim
     chunks = T // CHUNK_TOKENS + min(entries, T // least)
-    if chunks * state > CHUNK_STATE_FLOATS:
+    if chunks * sum(_chunk_sizes(heads, key_dim, value_dim, gated)) > CHUNK_SCRATCH_BYTES:
         return 0
     filled = heads * value_dim / (16 if key_dim > 64 else 32) / (2 * num_sms)   # of the GPU by one entry's walk: CTAs over places for them
     walk = lambda most, all_tokens: _WALK_US[gated] * max(most, all_tokens * filled)
@@ -1274,14 +1283,16 @@ def _scan_chunks(T: int, entries: int, longest: int, heads: int, key_dim: int, v
     return chunks if cost < 0.9 * walk(longest, T) else 0
 
 
-def _chunk_scratch(chunks: int, device: torch.device, *sizes: int):
-    """A block of memory, to be held until the launches are made, and in it the addresses of arrays of so many bytes a chunk (the
-    chunks' own states, the products of their decays, the states in front of them in three bf16 pieces and so on), each on a
-    256-byte boundary."""
+def _chunk_scratch(chunks: int, device: torch.device, sizes: Tuple[int, ...]):
+    """A block of memory, to be held until the launches are made, and in it the addresses of arrays of so many bytes a chunk, each on
+    a 256-byte boundary.  None where the GPU has no room left: the walk needs no scratch, so such a call walks."""
     at = [0]
     for n in sizes:
         at.append(at[-1] + (chunks * n + 255) // 256 * 256)
-    buf = torch.empty(at[-1], dtype=torch.uint8, device=device)
+    try:
+        buf = torch.empty(at[-1], dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
     return buf, [buf.data_ptr() + a for a in at[:-1]]
 
 
@@ -1330,8 +1341,11 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
         lib = L.recurrent(dk)
         qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
         chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, True, L.num_sms())
+        held = None
         if chunks and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 1):
-            held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 4 * H * dk, 6 * H * dv * dk, 2 * H * lib.ri_gated_chunk_parts())
+            held = _chunk_scratch(chunks, q.device, _chunk_sizes(H, dk, dv, True))
+        if held is not None:
+            scratch = held[1]
             check(lib.ri_gated_chunks(*qkv, _p(z), z.stride(0), dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q),
                                       _p(state_slots), int(entries), GATED_CHUNK_MIN_TOKENS, chunks, H, dv, *scratch, stream_ptr()),
                   "gated_chunks")
@@ -1400,8 +1414,11 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
         lib = L.recurrent(dk)
         qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
         chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, False, L.num_sms())
+        held = None
         if chunks and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 0):
-            held, scratch = _chunk_scratch(chunks, q.device, 4 * H * dv * dk, 8 * H, 6 * H * dv * dk)
+            held = _chunk_scratch(chunks, q.device, _chunk_sizes(H, dk, dv, False))
+        if held is not None:
+            scratch = held[1]
             check(lib.ri_head_chunks(*qkv, _p(decay), H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0,
                                      dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots), int(entries),
                                      CHUNK_MIN_TOKENS, chunks, H, dv, H // G, *scratch, stream_ptr()), "head_chunks")

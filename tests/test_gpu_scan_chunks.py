@@ -165,3 +165,30 @@ def test_calls_that_keep_the_walk():
     ok = lambda stride, dv: lib.ri_chunks_ok(256, stride, 256, stride, 256, stride, 0, dv, 0)
     assert ok(128, 64) and not ok(129, 64) and not ok(128, 48)
     assert not lib.ri_chunks_ok(256, 128, 256, 128, 256, 128, 0, 64, 1)    # the gated form takes bf16
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_a_call_without_room_for_scratch_walks(gated, monkeypatch):
+    torch.manual_seed(1)
+    T, H, dk, dv = 450, 2, 64, 64
+    x = torch.randn(T, 2 * H * dk + H * dv, device=DEV).bfloat16()
+    q, k, v = x[:, : H * dk], x[:, H * dk: 2 * H * dk], x[:, 2 * H * dk:]
+
+    def run(longest):
+        out, state = torch.empty(T, H * dv, device=DEV), torch.ones(1, H, dv, K().recurrent_state_rows(dk), device=DEV)
+        args = (out, state, i32([0, T]), i32([0]), 1, H, dk, dv)
+        if gated:
+            K().gated_scan(q, k, v, torch.ones(T, H * dk, device=DEV), None, 1.0, 4.0, *args, longest=longest)
+        else:
+            K().head_scan(q, k, v, torch.full((H,), 0.9, device=DEV), 1.0, *args, longest=longest)
+        return out, state
+    walked, empty = run(0), torch.empty
+    in_chunks = run(T)
+
+    def full(*size, **kw):
+        if kw.get("dtype") == torch.uint8:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    got = run(T)
+    assert all(torch.equal(a, b) for a, b in zip(got, walked)) and not torch.equal(in_chunks[0], walked[0])
