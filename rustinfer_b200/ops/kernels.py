@@ -1296,15 +1296,25 @@ def _chunk_scratch(chunks: int, device: torch.device, sizes: Tuple[int, ...]):
     return buf, [buf.data_ptr() + a for a in at[:-1]]
 
 
+def _recurrent_sizes_agree(lib, dk: int, what: str) -> None:
+    """The library lays out states and, where it has them, chunks as this module counts them: a shorter chunk there would find no
+    place in the scratch and the grids made here."""
+    kept, rows = int(lib.ri_recurrent_state_rows()), recurrent_state_rows(dk)
+    if kept != rows:
+        raise KernelError(f"{what}: the kernel stores {kept} rows a column, the host counts {rows}")
+    tokens, parts = int(lib.ri_recurrent_chunk_tokens()), int(lib.ri_gated_chunk_parts())
+    if tokens not in (0, CHUNK_TOKENS) or (tokens and 2 * parts != _chunk_sizes(1, dk, 64, True)[3]):
+        raise KernelError(f"{what}: the kernel's chunks are {tokens} tokens and {parts} parts, the host counts {CHUNK_TOKENS} and "
+                          f"{_chunk_sizes(1, dk, 64, True)[3] // 2}")
+
+
 def _scan_common(state: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor,
                  T: int, H: int, dk: int, dv: int, what: str) -> None:
     _i32(cu_q, "cu_q"); _i32(state_slots, "state_slots")
     _contig(state, "state"); _contig(out, "out")
     rows = recurrent_state_rows(dk)
     if dk not in _rows_checked:                       # once per key size: host and kernel count alike
-        kept = int(L.recurrent(dk).ri_recurrent_state_rows())
-        if kept != rows:
-            raise KernelError(f"{what}: the kernel stores {kept} rows a column, the host counts {rows}")
+        _recurrent_sizes_agree(L.recurrent(dk), dk, what)
         _rows_checked.add(dk)
     if state.dtype != torch.float32 or state.dim() != 4 or tuple(state.shape[1:]) != (H, dv, rows):
         raise KernelError(f"{what}: state is fp32 [slots, {H}, {dv}, {rows}] (recurrent_state_rows({dk}) rows a column)")

@@ -19,3 +19,15 @@ def test_scratch_stays_below_its_bound(H, dk, dv, gated):
         assert chunks * a_chunk <= 1.26 * 2 ** 30
         most = max(most, chunks)
     assert (H == 1) or most > 0                              # the bound leaves ordinary prompts their chunks
+
+
+@pytest.mark.parametrize("rows,tokens,parts,fits", [(128, 64, 36864, True), (128, 0, 0, True), (128, 32, 36864, False), (128, 64, 18432, False),
+                                                    (132, 64, 36864, False)])
+def test_a_library_that_counts_otherwise_is_refused(rows, tokens, parts, fits):
+    lib = type("Library", (), dict(ri_recurrent_state_rows=lambda self: rows, ri_recurrent_chunk_tokens=lambda self: tokens,
+                                   ri_gated_chunk_parts=lambda self: parts))()
+    if fits:
+        K._recurrent_sizes_agree(lib, 128, "scan")
+    else:
+        with pytest.raises(K.KernelError):
+            K._recurrent_sizes_agree(lib, 128, "scan")
