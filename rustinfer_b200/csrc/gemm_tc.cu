@@ -15,7 +15,9 @@
 // flight (decode: the weights stream through once, tokens are the narrow N of the MMA) and
 // the activations otherwise (prefill).  Split-K: grid.z CTAs take slices of K, park fp32
 // partial tiles in a workspace, and the CTA whose ticket is last adds them in slice order
-// (so the result does not depend on which CTA came last) and runs the epilogue.
+// (so the result does not depend on which CTA came last) and runs the epilogue.  Slices of a
+// product that is added into the stream add their own parts there instead when the weight is
+// on the 128-row side, or when they are not given a workspace.
 //
 // Epilogues: store bf16 / store fp32 / SiLU(gate)*up for a weight whose rows alternate
 // gate_j, up_j / add into the fp32 residual stream.
@@ -263,9 +265,58 @@ __device__ __forceinline__ void store_row64(const Params& p, int tok, int feat0,
     }
 }
 
-// Persistent over tiles: CTA x takes tiles x, x + gridDim.x, ...; blockIdx.z is the K slice.
+// A warp's 32 rows of a finished tile (or K slice of one) from registers: slices meet in the workspace as they do below, or, where
+// there is none, add their parts into the stream.
 template <int BN>
-__global__ void __launch_bounds__(THREADS, 2)
+__device__ __forceinline__ void finish_sums(const Params& p, int tile, int tok, int b0, int quarter, int lane, int* ticket_slot, float (&sum)[BN]) {
+    if (p.splits > 1 && p.workspace) {
+        float* mine = p.workspace + ((size_t)tile * p.splits + blockIdx.z) * (BN * 128) + quarter * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < BN; ++j) mine[(size_t)j * 128] = sum[j];
+        __threadfence();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (threadIdx.x == 64) *ticket_slot = atomicAdd(&p.counters[tile], 1);
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (*ticket_slot != p.splits - 1) return;
+        __threadfence();
+        if (threadIdx.x == 64) p.counters[tile] = 0;
+        const float* base = p.workspace + (size_t)tile * p.splits * (BN * 128) + quarter * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < BN; ++j) sum[j] = 0.f;
+        for (int s = 0; s < p.splits; ++s)
+#pragma unroll
+            for (int j = 0; j < BN; ++j) sum[j] += __ldcg(base + (size_t)s * (BN * 128) + (size_t)j * 128);
+    }
+    if (p.vec && b0 + BN <= p.b_rows) {
+#pragma unroll
+        for (int c0 = 0; c0 < BN; c0 += 64) {
+            float v[64];
+#pragma unroll
+            for (int j = 0; j < 64; ++j) v[j] = sum[c0 + j];
+            store_row64(p, tok, b0 + c0, v);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < BN; ++j) store_one(p, p.a_rows, p.b_rows, tok, b0 + j, sum[j], j + 1 < BN ? sum[j + 1] : 0.f);
+    }
+}
+
+// k-blocks of one chain of products in a SUMS kernel, of a slice of `n_kb` of `all_kb`: four at most, as even as they come.  A K of
+// fewer than eight k-blocks is one chain under every plan, so that a token's sums have the same bits whatever step it is in.
+__device__ __forceinline__ int chain_kblocks(int n_kb, int all_kb) {
+    const int chains = all_kb < 8 ? 1 : (n_kb + 3) / 4;
+    return chains > 0 && n_kb > 0 ? (n_kb + chains - 1) / chains : 1;
+}
+
+// Persistent over tiles: CTA x takes tiles x, x + gridDim.x, ...; blockIdx.z is the K slice.
+//
+// SUMS: the tensor core cuts off what its accumulator has no bits for, always downwards, so a chain over all of K drifts from the
+// sum with its length (300 x 1,024 x 2,048: 2.1e-6 of it in one chain, 2.4e-7 in chains of four k-blocks; x 8,192: 9.1e-6, 2.5e-7).  Here
+// every four k-blocks start a chain of their own in the other accumulator, and the epilogue warps add the last one to a running sum in
+// registers, by rounded additions, while the next is computed.  A k-block then takes 0.36 us instead of 0.32 (the issuing thread waits and
+// commits once more a chain).  For tiles of 64 and 128 columns with an SM each: the sum of a tile fills a thread's registers.
+template <int BN, bool SUMS>
+__global__ void __launch_bounds__(THREADS, SUMS ? 1 : 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const Params p) {
     using C = Cfg<BN>;
@@ -286,6 +337,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int kb_begin = blockIdx.z * per;
     const int kb_end = min(kb_begin + per, kblocks);
     const int n_kb = max(kb_end - kb_begin, 0);
+    const int chain = SUMS ? chain_kblocks(n_kb, kblocks) : max(n_kb, 1);          // k-blocks of a chain of products
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -365,27 +417,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // a grouped product's tiles are found in offsets that the kernels before wrote: this thread reads them too
         // (otherwise it touches only shared and tensor memory and needs no wait)
         if (p.grp_offsets) pdl_wait();
-        for (int tile = blockIdx.x; tile < p.n_tiles && ok; tile += gridDim.x, ++t) {
+        for (int tile = blockIdx.x; tile < p.n_tiles && ok; tile += gridDim.x) {
             if (p.grp_offsets) {
                 int ga0, ga_end, gb0, gfeat0;
-                if (!grouped_tile<BN>(p, tile, ga0, ga_end, gb0, gfeat0)) { --t; continue; }    // no accumulator is used
+                if (!grouped_tile<BN>(p, tile, ga0, ga_end, gb0, gfeat0)) continue;             // no accumulator is used
             }
-            const int buf = t & 1, use = t >> 1;
-            // the epilogue has emptied this accumulator (first use of a buffer passes at once)
-            if (!mbar_wait(&acc_empty[buf], (use & 1) ^ 1, p.error, ERR_MMA_WAIT)) { ok = false; break; }
-            tc_fence_after();
-            const unsigned tmem_d = tmem_base + buf * C::ACC_COLS;
-            for (int i = 0; i < n_kb; ++i) {
-                if (!mbar_try_wait(&full[s], par) && !mbar_wait(&full[s], par, p.error, ERR_MMA_WAIT)) { ok = false; break; }
+            // a tile without k-blocks (a slice behind the last) is a chain without products: its accumulator is passed on
+            for (int first = 0; ok && (first < n_kb || first == 0); first += chain, ++t) {
+                const int buf = t & 1, use = t >> 1, end = SUMS ? min(first + chain, n_kb) : n_kb;
+                // the epilogue has emptied this accumulator (first use of a buffer passes at once)
+                if (!mbar_wait(&acc_empty[buf], (use & 1) ^ 1, p.error, ERR_MMA_WAIT)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t da = desc0 + (uint64_t)(s * stage_step), db = da + (uint64_t)b_step;
+                const unsigned tmem_d = tmem_base + buf * C::ACC_COLS;
+                for (int i = first; i < end; ++i) {
+                    if (!mbar_try_wait(&full[s], par) && !mbar_wait(&full[s], par, p.error, ERR_MMA_WAIT)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t da = desc0 + (uint64_t)(s * stage_step), db = da + (uint64_t)b_step;
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k)
-                    mma_bf16_ss(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
-                if (s & 1) tc_commit(&empty[s >> 1]);     // the pair is free once these MMAs have read it
-                if (++s == STAGES) { s = 0; par ^= 1u; }
+                    for (int k = 0; k < BK / 16; ++k)
+                        mma_bf16_ss(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > first || k > 0) ? 1u : 0u);
+                    if (s & 1) tc_commit(&empty[s >> 1]); // the pair is free once these MMAs have read it
+                    if (++s == STAGES) { s = 0; par ^= 1u; }
+                }
+                tc_commit(&acc_full[buf]);                // the accumulator is complete
             }
-            tc_commit(&acc_full[buf]);                    // the accumulator is complete
         }
         if (!ok) {
             // whatever was loaded last must have landed before shared memory is given up
@@ -401,16 +456,38 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         bool ok = true;
         int t = 0;
         pdl_wait();                                       // out, workspace and counters belong to earlier kernels till now
-        const bool atomic_out = p.splits > 1 && p.epilogue == EPI_RESIDUAL;
-        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x, ++t) {
+        const bool atomic_out = p.splits > 1 && p.epilogue == EPI_RESIDUAL && (p.swap || !p.workspace);
+        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
             int a0 = (tile % p.tiles_a) * p.a_box, b0 = (tile / p.tiles_a) * BN;
             int a_end = 0x3fffffff;
             if (p.grp_offsets) {
                 int bw0;
-                if (!grouped_tile<BN>(p, tile, a0, a_end, bw0, b0)) { --t; continue; }
+                if (!grouped_tile<BN>(p, tile, a0, a_end, bw0, b0)) continue;
             }
             // lanes beyond the rows this tile loaded (or, grouped, beyond its group's rows) hold nothing of this tile
             const int ra = (quarter * 32 + lane < p.a_box && a0 + quarter * 32 + lane < a_end) ? a0 + quarter * 32 + lane : 0x3fffffff;
+            if constexpr (SUMS) {
+                float sum[BN];
+                for (int first = 0; first < n_kb || first == 0; first += chain, ++t) {
+                    const int buf = t & 1, use = t >> 1;
+                    if (ok) ok = mbar_wait(&acc_full[buf], use & 1, p.error, ERR_EPILOGUE_WAIT);
+                    tc_fence_after();
+                    const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + buf * C::ACC_COLS;
+                    const bool have = ok && n_kb > 0;
+#pragma unroll
+                    for (int c0 = 0; c0 < BN; c0 += 32) {
+                        float v[32];
+                        if (have) tmem_ld_row<32>(taddr + c0, v);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) sum[c0 + j] = (first > 0 ? sum[c0 + j] : 0.f) + (have ? v[j] : 0.f);
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[buf]);
+                }
+                finish_sums<BN>(p, tile, ra, b0, quarter, lane, ticket_slot, sum);
+                continue;
+            }
             const int buf = t & 1, use = t >> 1;
             // (also for a K slice that got no k-block: the MMA thread commits at once, but it must
             // have passed its own wait on `acc_empty` before these warps arrive there, or it would
@@ -421,8 +498,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const bool have = ok && n_kb > 0;
             bool last = true;
             if (atomic_out) {
-                // K slices of a product that is added into the fp32 stream: every slice adds
-                // its own part, no meeting point needed (the order of the adds is not fixed)
+                // K slices of a product that is added into the fp32 stream without a meeting point:
+                // every slice adds its own part (the order of the adds is not fixed)
                 last = false;
                 float* h = reinterpret_cast<float*>(p.out);
                 for (int c0 = 0; c0 < BN; c0 += 16) {
@@ -495,6 +572,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            ++t;
         }
     }
     tc_fence_before();
@@ -948,11 +1026,11 @@ int ri_tc_weight_map(const void* ptr, int rows, int cols, int box_rows, CUtensor
 }
 
 namespace {
-template <int BN>
+template <int BN, bool SUMS = false>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, int tiles, cudaStream_t s) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)SMEM_TOTAL);
         if (e != cudaSuccess) return (int)e;
         configured = true;
@@ -960,7 +1038,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, int ti
     const int sms = device_sms();
     // one CTA per SM walks the tiles; with K slices every CTA has exactly one tile
     const int ctas = (p.splits > 1 || tiles < sms) ? tiles : sms;
-    RI_CHECKED(ri_launch(gemm_tc_kernel<BN>, dim3(ctas, 1, p.splits), dim3(THREADS), (size_t)p.budget + SMEM_EXTRA, s, ma, mb, p));
+    RI_CHECKED(ri_launch(gemm_tc_kernel<BN, SUMS>, dim3(ctas, 1, p.splits), dim3(THREADS), (size_t)p.budget + SMEM_EXTRA, s, ma, mb, p));
     return ri_launch_status();
 }
 }  // namespace
@@ -997,7 +1075,7 @@ int gemm_tc_impl(const void* X, const void* W, int M, int N, int K, void* out, i
                  int swap, int bn, int splits, int a_box, float* workspace, int* counters, int* error,
                  float* sk_acc, const Params* rope, void* stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || K % 8 != 0 || splits < 1 || (splits > 1 && (!workspace || !counters)) || !error ||
+    if (K <= 0 || K % 8 != 0 || splits < 1 || (splits > 1 && (!counters || (!workspace && epilogue != EPI_RESIDUAL))) || !error ||
         a_box < 8 || a_box > BM || a_box % 8 != 0)
         return (int)cudaErrorInvalidValue;
     const void* A = swap ? W : X;
@@ -1103,6 +1181,11 @@ int gemm_tc_impl(const void* X, const void* W, int M, int N, int K, void* out, i
     if (st != 0) return st;
     cudaStream_t s = (cudaStream_t)stream;
     const int tiles = p.n_tiles;
+    // tiles with an SM each; where a CTA walks several, the store of one hides behind the products of the next, and stays there
+    if (!swap && tiles <= device_sms()) {
+        if (bn == 64) return launch<64, true>(ma, mb, p, tiles, s);
+        if (bn == 128) return launch<128, true>(ma, mb, p, tiles, s);
+    }
     switch (bn) {
         case 16: return launch<16>(ma, mb, p, tiles, s);
         case 32: return launch<32>(ma, mb, p, tiles, s);

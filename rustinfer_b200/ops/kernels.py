@@ -3,6 +3,7 @@
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Dict, Optional, Sequence, Tuple
 
 import torch
@@ -158,6 +159,37 @@ def gemm_tc_error(device: torch.device) -> int:
     return code
 
 
+@functools.lru_cache(maxsize=4096)
+def _mid_tiles(row_tiles: int, N: int, kblocks: int, num_sms: int) -> Tuple[int, int]:
+    """Width of the tiles and number of K slices for many tokens whose 256-wide tiles leave half of the SMs idle.
+
+    Narrow tiles fill the SMs for nothing: a k-block costs a CTA about the same time whether its tile is 64 or 128 columns wide (0.36
+    us).  K slices meet through the workspace, the dearer the wider the tile and the more of them.  So what each choice would take is
+    put together from its k-blocks and its meeting, as fitted to 66 to 2,048 rows x 256 to 4,096 features x K of 512 to 14,336, and the
+    least is taken; measured, chosen against the others (us, in a graph): 300 x 1,024 x 1,024 whole 9.4, in two 9.6; 300 x 1,024 x 2,048
+    in three 11.2, whole 15.2; 300 x 2,048 x 8,192 128 wide in three 27.9, in two 35.2, whole 51.4.  Tiles of 256 columns in slices stay
+    where neither narrow kind leaves room for slices of a long K (300 x 4,096 x 14,336: 67 in three, 95 whole at 128 columns)."""
+    best = None
+    for bn in (64, 128, 256):
+        tiles = row_tiles * -(-N // bn)
+        if tiles > num_sms or (bn == 256 and N < 256):
+            continue
+        most = max(1, min(num_sms // tiles, kblocks // 4, 32 if bn == 256 else 8))
+        while most > 1 and tiles * most * bn * 128 > _TC_WORKSPACE_FLOATS:
+            most -= 1
+        for splits in ((most,) if bn == 256 else range(1, most + 1)):
+            slice_kb = -(-kblocks // splits)
+            if bn == 256:
+                us = 12.0 + 3.6 * splits + 0.5 * slice_kb
+            elif bn == 128:
+                us = (3.5 if splits == 1 else 6.0 + 1.1 * splits) + 0.38 * slice_kb
+            else:
+                us = (3.0 if splits == 1 else 5.2 + 0.55 * splits) + 0.36 * slice_kb
+            if best is None or us < best[0]:
+                best = us, bn, splits
+    return best[1], best[2]
+
+
 def gemm_tc_plan(M: int, N: int, K: int, num_sms: Optional[int] = None, epilogue: int = EPI_BF16):
     """(swap, bn, splits, a_box): which operand sits on the 128-row side of the MMA, the
     tile of the other one, how many K slices, and how many rows of the 128 a tile really
@@ -172,17 +204,7 @@ def gemm_tc_plan(M: int, N: int, K: int, num_sms: Optional[int] = None, epilogue
     kblocks = -(-K // 64)
     splits, a_box = 1, 128
     if not swap and N > 64 and tiles * 2 <= num_sms:
-        # few tiles of many tokens: a k-block costs a CTA 0.35 us whether its tile is 64 or 256 wide, so narrow tiles fill the SMs for
-        # nothing, where K slices of wide ones had to meet (through the workspace, or as adds of every slice into the stream): 300 x
-        # 1,024 x 2,048 35 -> 16 us (68 -> 16 added into the stream), 1,024 x 2,048 x 2,048 26 -> 16 (72 -> 16), 2,048 x 1,024 x 2,048
-        # 26 -> 17 (72 -> 16), of which some 13 us are the eager launch.  Slices only of a long K (300 x 1,024 x 4,096: 24 us
-        # whole, 18 in two; 52 before), and none where they would add into the stream (28 against 24).
-        bn = 64 if -(-M // 128) * -(-N // 64) <= num_sms else 128
-        tiles = -(-M // 128) * -(-N // bn)
-        if epilogue != EPI_RESIDUAL:
-            splits = max(1, min(num_sms // tiles, kblocks // 32))
-            while splits > 1 and tiles * splits * bn * 128 > _TC_WORKSPACE_FLOATS:
-                splits -= 1
+        bn, splits = _mid_tiles(-(-M // 128), N, kblocks, num_sms)
     elif tiles * 2 <= num_sms:
         splits = max(1, min(num_sms // tiles, kblocks // 4, 32))
         if epilogue != EPI_RESIDUAL:                       # slices meet in the workspace
@@ -229,11 +251,11 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int =
     a_box = plan[3] if len(plan) > 3 else 128
     ws, counters, err, meeting = gemm_tc_state(x.device)
     tiles = (-(-N // a_box)) * (-(-M // bn)) if swap else (-(-M // a_box)) * (-(-N // bn))
-    meets = splits > 1 and epilogue != EPI_RESIDUAL
-    if tiles > counters.numel() or (meets and tiles * splits * bn * 128 > ws.numel()):
+    fits = tiles * splits * bn * 128 <= ws.numel()
+    if tiles > counters.numel() or (splits > 1 and epilogue != EPI_RESIDUAL and not fits):
         raise KernelError("gemm_tc: the split-K workspace is too small for this plan")
     check(L.gemm_tc().ri_gemm_tc(_p(x), _p(w), M, N, Kd, _p(out), out.stride(0), epilogue, swap, bn, splits,
-                                 a_box, _p(ws), _p(counters), _p(err), _p(meeting), stream_ptr()), "gemm_tc")
+                                 a_box, _p(ws) if fits else None, _p(counters), _p(err), _p(meeting), stream_ptr()), "gemm_tc")
 
 
 def gemm_tc_rope(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, positions: torch.Tensor,

@@ -16,7 +16,9 @@ def test_mid_sizes(M, N, K):
     torch.manual_seed(N)
     x, w = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
     want = x.double() @ w.double().T
-    tol = 1e-6 + K / 16 * 6e-8                               # a chain of K / 16 additions that cut off
+    # bf16 products are exact in 32 bits.  A chain of 16 additions cuts off half a unit of 2^-23 each of a sum that grows to its end:
+    # 16 / 2 * 6e-8 at most where all sums have one sign, measured 2.4e-7 for these of either, however long K (2.1e-6 at 2,048 in one)
+    tol = 4e-7
     rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
     out, half, pair = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV).bfloat16(), torch.empty(M, N // 2, device=DEV).bfloat16()
     k.gemm_tc(x, w, out, k.EPI_F32)
@@ -28,4 +30,26 @@ def test_mid_sizes(M, N, K):
     k.gemm_tc(x, w, half, k.EPI_BF16)
     k.gemm_tc(x, w, pair, k.EPI_SILU)
     assert rel(half, want) < 3e-3 and rel(pair, torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]) < 4e-3
+    assert k.gemm_tc_error(out.device) == 0
+
+
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("M,N,K,splits", [(70, 200, 576, 6), (130, 128, 704, 1), (300, 136, 1160, 4), (128, 64, 512, 1)])
+def test_chains_and_slices(M, N, K, splits, bn):
+    """Tiles that sum short chains: an uneven last chain, slices that get no k-block, rows of the stream with and without vector adds."""
+    from rustinfer_b200.ops import kernels as k
+    torch.manual_seed(K)
+    x, w = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn(N, K, device=DEV) / K ** 0.5).bfloat16()
+    want = x.double() @ w.double().T
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+    h = torch.randn(M, N + 3, device=DEV)
+    for out in (h[:, :N].contiguous(), h.clone()[:, :N]):    # rows of whole vectors, rows that are not
+        was = out.double()
+        k.gemm_tc(x, w, out, k.EPI_RESIDUAL, (0, bn, splits, 128))
+        assert rel(out, was + want) < 4e-7
+        k.gemm_tc(x, w, out, k.EPI_F32, (0, bn, splits, 128))
+        assert rel(out, want) < 4e-7
+        again = torch.empty_like(out)
+        k.gemm_tc(x, w, again, k.EPI_F32, (0, bn, splits, 128))
+        assert torch.equal(out, again)                       # slices are added in their order, not in that of their arrival
     assert k.gemm_tc_error(out.device) == 0
