@@ -6,7 +6,9 @@
 // the sums do not depend on arrival.  Weights go from memory straight into the registers of the tensor-core instruction: a
 // sum over k may visit k in any order, so a lane takes 16 consecutive bytes of one weight row and the same 16 of its tokens'
 // rows, and calls them the k its fragment holds.  The weights of a warp's first blocks are asked for before the kernel waits for
-// its predecessor.
+// its predecessor.  The tensor core cuts off what its accumulator has no bits for, so a warp's products are taken in chains of eight
+// that join its sum by rounded additions (8 x 128 x 8,192: 4.7e-7 from the 64-bit sum in one chain of 32 a warp, 1.4e-7 in chains; the
+// tcgen05 kernel's slices 2.5e-7).
 #include "common.cuh"
 
 namespace {
@@ -46,7 +48,19 @@ gemm_few_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, int M, i
     };
     weights(b0);
     pdl_wait();
-    float acc[MT][NT][4] = {};
+    // rounds of a chain of eight products; with four warps K is at most 1,024, sixteen products a warp, which stay one chain
+    constexpr int FOLD = 4 / U;
+    constexpr bool CHAINS = WARPS > 4;
+    float acc[MT][NT][4] = {}, part[MT][NT][4];
+    auto join = [&] {
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[m][n][e] += part[m][n][e];
+    };
+    int round = 0;
     for (int b = b0; b < b1; b += U) {
         uint4 x[U][2 * MT];
 #pragma unroll
@@ -62,6 +76,14 @@ gemm_few_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, int M, i
 #pragma unroll
             for (int n = 0; n < NT; ++n) now[u][n] = w[u][n];
         if (b + U < b1) weights(b + U);
+        if (CHAINS && round == 0) {
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) part[m][n][e] = 0.f;
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -69,10 +91,13 @@ gemm_few_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, int M, i
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
                     const uint4 lo = x[u][2 * m], hi = x[u][2 * m + 1], v = now[u][n];
-                    mma(acc[m][n], lo.x, hi.x, lo.y, hi.y, v.x, v.y);
-                    mma(acc[m][n], lo.z, hi.z, lo.w, hi.w, v.z, v.w);
+                    float (&d)[4] = CHAINS ? part[m][n] : acc[m][n];
+                    mma(d, lo.x, hi.x, lo.y, hi.y, v.x, v.y);
+                    mma(d, lo.z, hi.z, lo.w, hi.w, v.z, v.w);
                 }
+        if (CHAINS && ++round == FOLD) { join(); round = 0; }
     }
+    if (round > 0) join();
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -126,8 +151,7 @@ int launch(const void* X, const void* W, int M, int N, int K, void* out, int ld_
 // 16,384 x 1,024 9.8 / 10.7; 16,384 x 2,048 15.5 / 16.0, but behind a chain kernel, where the other one asks for more of its weights
 // ahead, the whole step was 3 % slower; 28,672 x 4,096 48 against 45 (the stream of weights is the bound, and TMA keeps more of it
 // on the way).  24 rows: 1,024 x 1,024 3.0 / 9.8, 2,048 x 2,048 4.8 / 11.9, 8,192 x 1,024 8.0 / 11.4, 16,384 x 1,024 14.2 / 12.9.
-// Narrow tiles while their CTAs find an SM each, sixteen warps where K is long, so that no warp's chain of products is longer than
-// the slices of the other kernel (their sums are no further from 64 bits).  Under 65,536 weights the other kernel stays (64 x 64 about
+// Narrow tiles while their CTAs find an SM each, sixteen warps where K is long.  Under 65,536 weights the other kernel stays (64 x 64 about
 // 3 against 1.5 us): sums of one or two k-blocks come out of it in the bits a prompt's product has, and models of such sizes, with
 // experts a rounding away from one another, answer the same however their tokens are cut.
 RI_API int ri_gemm_few_shape(int M, int N, int K) {
