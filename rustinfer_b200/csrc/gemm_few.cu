@@ -151,15 +151,15 @@ int launch(const void* X, const void* W, int M, int N, int K, void* out, int ld_
 // 16,384 x 1,024 9.8 / 10.7; 16,384 x 2,048 15.5 / 16.0, but behind a chain kernel, where the other one asks for more of its weights
 // ahead, the whole step was 3 % slower; 28,672 x 4,096 48 against 45 (the stream of weights is the bound, and TMA keeps more of it
 // on the way).  24 rows: 1,024 x 1,024 3.0 / 9.8, 2,048 x 2,048 4.8 / 11.9, 8,192 x 1,024 8.0 / 11.4, 16,384 x 1,024 14.2 / 12.9.
-// Narrow tiles while their CTAs find an SM each, sixteen warps where K is long.  Under 65,536 weights the other kernel stays (64 x 64 about
-// 3 against 1.5 us): sums of one or two k-blocks come out of it in the bits a prompt's product has, and models of such sizes, with
-// experts a rounding away from one another, answer the same however their tokens are cut.
+// Narrow tiles while they are few, 16 features a CTA up to two CTAs an SM, sixteen warps where K is long.
+// Up to seven k-blocks of 64 the other kernel stays, although it takes longer (8 x 1,024 x 128: 4.0 us against 1.7): no plan of it cuts
+// such a K, so a token's sums have the same bits in a step of single tokens, in one of fifty and in a prompt, and models of such sizes,
+// with experts a rounding away from one another, answer the same however their tokens are cut.
 RI_API int ri_gemm_few_shape(int M, int N, int K) {
-    if (M < 1 || M > 32 || N < 1 || K < 8 || K % 8) return -1;
+    if (M < 1 || M > 32 || N < 1 || K <= 7 * 64 || K % 8) return -1;
     const long long weights = (long long)N * K;
-    if (weights < 65536) return -1;
     if (N <= 1024 && K <= 8192) return 0;
-    if (N <= 4736 && weights <= (17 << 20)) return 1;
+    if (N <= 2 * 16 * ri_device_sms() && weights <= (17 << 20)) return 1;
     if (M <= 16) return weights <= (26 << 20) && K <= 4096 ? 2 : -1;
     return weights <= (8 << 20) && K <= 1024 ? 3 : -1;
 }

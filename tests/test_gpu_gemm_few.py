@@ -9,7 +9,7 @@ DEV = "cuda:0"
 
 
 # features on both sides of every change of tile, odd ones; k that is one piece, no multiple of a warp's blocks, several rounds of them
-@pytest.mark.parametrize("N,K", [(9, 8192), (130, 1000), (1024, 1024), (1026, 264), (4736, 96), (4738, 104), (8192, 1000), (600, 8192)])
+@pytest.mark.parametrize("N,K", [(9, 8192), (130, 1000), (1024, 1024), (1026, 520), (4736, 456), (4738, 504), (8192, 1000), (600, 8192)])
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 24, 32])
 def test_every_epilogue(M, N, K):
     from rustinfer_b200.ops import kernels as k, library as L
@@ -43,4 +43,20 @@ def test_every_epilogue(M, N, K):
             k.gemm_tc(x, w, pair, epi)
             assert rel(pair, act * up) < 4e-3
     shape = L.gemm_tc().ri_gemm_few_shape
-    assert shape(33, 1024, 1024) == -1 and shape(8, 255, 256) == -1 and shape(8, 256, 256) >= 0 and shape(8, 28672, 4096) == -1 and shape(24, 16384, 2048) == -1 and shape(8, 1024, 1024) >= 0
+    assert shape(33, 1024, 1024) == -1 and shape(8, 4096, 448) == -1 and shape(8, 9, 456) >= 0 and shape(8, 28672, 4096) == -1 and shape(24, 16384, 2048) == -1 and shape(8, 1024, 1024) >= 0
+    assert shape(M, N, K) >= 0
+    assert [shape(8, 32 * L.num_sms() + d, 1024) for d in (0, 2)] == [1, 2]    # two CTAs of 16 features an SM
+
+
+# K of up to seven k-blocks; features that few tokens would find one, two and four tiles a CTA for
+@pytest.mark.parametrize("N,K", [(9, 8), (1024, 64), (1024, 128), (1026, 264), (4096, 128), (8192, 448)])
+def test_short_sums_have_the_same_bits_in_any_step(N, K):
+    from rustinfer_b200.ops import kernels as k
+    torch.manual_seed(K)
+    x, w = torch.randn(700, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    all_rows = torch.empty(700, N, device=DEV)
+    k.gemm_tc(x, w, all_rows, k.EPI_F32)
+    for m in (1, 8, 16, 17, 32, 33, 64, 65, 130, 300):
+        out = torch.empty(m, N, device=DEV)
+        k.gemm_tc(x[:m], w, out, k.EPI_F32)
+        assert torch.equal(out, all_rows[:m]), m
