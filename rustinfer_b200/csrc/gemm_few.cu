@@ -6,8 +6,8 @@
 // the sums do not depend on arrival.  Weights go from memory straight into the registers of the tensor-core instruction: a
 // sum over k may visit k in any order, so a lane takes 16 consecutive bytes of one weight row and the same 16 of its tokens'
 // rows, and calls them the k its fragment holds.  The weights of a warp's first blocks are asked for before the kernel waits for
-// its predecessor.  The tensor core cuts off what its accumulator has no bits for, so a warp's products are taken in chains of eight
-// that join its sum by rounded additions (8 x 128 x 8,192: 4.7e-7 from the 64-bit sum in one chain of 32 a warp, 1.4e-7 in chains; the
+// its predecessor.  The tensor core cuts off what its accumulator has no bits for, so a warp's products are taken in chains of four
+// or eight that join its sum by rounded additions (8 x 128 x 8,192: 4.7e-7 from the 64-bit sum in one chain of 32 a warp, 1.4e-7 in chains; the
 // tcgen05 kernel's slices 2.5e-7).
 #include "common.cuh"
 
@@ -48,8 +48,10 @@ gemm_few_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, int M, i
     };
     weights(b0);
     pdl_wait();
-    // rounds of a chain of eight products; with four warps K is at most 1,024, sixteen products a warp, which stay one chain
-    constexpr int FOLD = 4 / U;
+    // rounds of a chain: one, but two of four products where the additions of twice the tokens cost more than a round's loads hide (24 x
+    // 2,048 x 8,192: 15.0 us joined every round, 13.8 every second); with four warps K is at most 1,024, sixteen products a warp, which
+    // stay one chain
+    constexpr int FOLD = MT == 2 && U == 2 ? 2 : 1;
     constexpr bool CHAINS = WARPS > 4;
     float acc[MT][NT][4] = {}, part[MT][NT][4];
     auto join = [&] {
@@ -60,7 +62,7 @@ gemm_few_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, int M, i
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[m][n][e] += part[m][n][e];
     };
-    int round = 0;
+    int round = 0;                                           // of the chain under way
     for (int b = b0; b < b1; b += U) {
         uint4 x[U][2 * MT];
 #pragma unroll
@@ -95,9 +97,9 @@ gemm_few_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, int M, i
                     mma(d, lo.x, hi.x, lo.y, hi.y, v.x, v.y);
                     mma(d, lo.z, hi.z, lo.w, hi.w, v.z, v.w);
                 }
-        if (CHAINS && ++round == FOLD) { join(); round = 0; }
+        if (CHAINS && (FOLD == 1 || ++round == FOLD)) { join(); round = 0; }
     }
-    if (round > 0) join();
+    if (FOLD > 1 && round > 0) join();
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
