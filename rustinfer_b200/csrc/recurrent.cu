@@ -440,7 +440,7 @@ delta_scan_kernel(const TA* __restrict__ r, int r_stride, const TA* __restrict__
                   const TA* __restrict__ v, int v_stride, const float* __restrict__ w, const float* __restrict__ u,
                   const float* __restrict__ au, int f_stride, float* __restrict__ out,
                   float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
-                  int H, int dv, int vec, int below) {
+                  int H, int dv, int vec) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -451,7 +451,6 @@ delta_scan_kernel(const TA* __restrict__ r, int r_stride, const TA* __restrict__
     const int lt = tid - WORKERS;
     const int cg = tid / R, rg = tid % R;
     const int t_begin = cu_q[b], t_end = cu_q[b + 1];
-    if (below > 0 && t_end - t_begin >= below) return;       // this entry goes in chunks
     const int rounds = (t_end - t_begin + TC - 1) / TC;
     if (DKP != DK) {
         for (int e = tid; e < 2 * HALF; e += THREADS) smem[e] = 0.f;
@@ -1161,7 +1160,7 @@ RI_API int ri_recurrent_state_rows() { return DKP; }
 
 // `single` != 0: every entry brings exactly one token (the kernel without staging takes the step).  `below` > 0: only the
 // entries of fewer tokens (the others go in chunks, recurrent_chunks.cu).
-RI_API int ri_gated_scan_short(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
+RI_API int ri_gated_scan(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
                          const float* alpha, int a_stride, int act_dtype, float q_scale, float* out, float* state,
                          const int* cu_q, const int* state_slots, int entries, int H, int dv, int single, int below,
                          void* stream) {
@@ -1189,17 +1188,10 @@ RI_API int ri_gated_scan_short(const void* q, int q_stride, const void* k, int k
     return ri_launch_status();
 }
 
-RI_API int ri_gated_scan(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
-                         const float* alpha, int a_stride, int act_dtype, float q_scale, float* out, float* state,
-                         const int* cu_q, const int* state_slots, int entries, int H, int dv, int single, void* stream) {
-    return ri_gated_scan_short(q, q_stride, k, k_stride, v, v_stride, alpha, a_stride, act_dtype, q_scale, out, state, cu_q,
-                               state_slots, entries, H, dv, single, 0, stream);
-}
-
-RI_API int ri_delta_scan_short(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride,
+RI_API int ri_delta_scan(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride,
                          const float* w, const float* u, const float* au, int f_stride, int act_dtype,
                          float* out, float* state, const int* cu_q, const int* state_slots, int entries, int H,
-                         int dv, int single, int below, void* stream) {
+                         int dv, int single, void* stream) {
     if (entries <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const dim3 grid((dv + COLS - 1) / COLS, H, entries);
@@ -1216,7 +1208,7 @@ RI_API int ri_delta_scan_short(const void* r, int r_stride, const void* k, int k
     static bool allowed = false; \
     if (!allowed) { RI_CHECKED(allow_shared(delta_scan_kernel<TA>, smem)); allowed = true; } \
     RI_CHECKED(ri_launch(delta_scan_kernel<TA>, grid, dim3(THREADS), smem, s, (const TA*)r, r_stride, \
-        (const TA*)k, k_stride, (const TA*)v, v_stride, w, u, au, f_stride, out, state, cu_q, state_slots, H, dv, vec, below)); \
+        (const TA*)k, k_stride, (const TA*)v, v_stride, w, u, au, f_stride, out, state, cu_q, state_slots, H, dv, vec)); \
     } while (0)
     if (act_dtype == RI_BF16) RI_DS(bf16);
     else RI_DS(float);
@@ -1224,16 +1216,9 @@ RI_API int ri_delta_scan_short(const void* r, int r_stride, const void* k, int k
     return ri_launch_status();
 }
 
-RI_API int ri_delta_scan(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride,
-                         const float* w, const float* u, const float* au, int f_stride, int act_dtype, float* out, float* state,
-                         const int* cu_q, const int* state_slots, int entries, int H, int dv, int single, void* stream) {
-    return ri_delta_scan_short(r, r_stride, k, k_stride, v, v_stride, w, u, au, f_stride, act_dtype, out, state, cu_q, state_slots,
-                               entries, H, dv, single, 0, stream);
-}
-
 // The head form: see head_scan_kernel.  share: heads that read one key head.  cos_t / sin_t with positions (with `single`
 // only; else null): keys and queries are rotated on the way in (see StepRotation).
-RI_API int ri_head_scan_short(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
+RI_API int ri_head_scan(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
                         const float* decay, int a_stride, const float* gain, int g_stride, int act_dtype, float q_scale,
                         float* out, float* state, const int* cu_q, const int* state_slots, int entries, int H, int dv,
                         int share, const int* positions, const float* cos_t, const float* sin_t, int rot, int interleaved,
@@ -1279,15 +1264,6 @@ RI_API int ri_head_scan_short(const void* q, int q_stride, const void* k, int k_
 #undef RI_HS
 #undef RI_HSA
     return ri_launch_status();
-}
-
-RI_API int ri_head_scan(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
-                        const float* decay, int a_stride, const float* gain, int g_stride, int act_dtype, float q_scale,
-                        float* out, float* state, const int* cu_q, const int* state_slots, int entries, int H, int dv,
-                        int share, const int* positions, const float* cos_t, const float* sin_t, int rot, int interleaved,
-                        int single, void* stream) {
-    return ri_head_scan_short(q, q_stride, k, k_stride, v, v_stride, decay, a_stride, gain, g_stride, act_dtype, q_scale, out, state,
-                              cu_q, state_slots, entries, H, dv, share, positions, cos_t, sin_t, rot, interleaved, single, 0, stream);
 }
 
 RI_API void ri_set_pdl(int on) { ri_pdl_flag() = on ? 1 : 0; }

@@ -1384,10 +1384,10 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
             if T == longest * int(entries):                   # every entry is as long
                 return
             below = GATED_CHUNK_MIN_TOKENS
-    check(L.recurrent(dk).ri_gated_scan_short(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(z), z.stride(0),
-                                              dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q),
-                                              _p(state_slots), int(entries), H, dv, 1 if T == int(entries) else 0, below,
-                                              stream_ptr()), "gated_scan")
+    check(L.recurrent(dk).ri_gated_scan(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(z), z.stride(0),
+                                        dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q),
+                                        _p(state_slots), int(entries), H, dv, 1 if T == int(entries) else 0, below,
+                                        stream_ptr()), "gated_scan")
 
 
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, q_scale: float,
@@ -1406,7 +1406,7 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
         raise KernelError("decay_scan: decay is fp32 [H*dk]")
     check(L.recurrent(dk).ri_gated_scan(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay), 0,
                                         dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q),
-                                        _p(state_slots), int(entries), H, dv, 1 if T == int(entries) else 0,
+                                        _p(state_slots), int(entries), H, dv, 1 if T == int(entries) else 0, 0,
                                         stream_ptr()), "decay_scan")
 
 
@@ -1457,11 +1457,11 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
             if T == longest * int(entries):                   # every entry is as long
                 return
             below = CHUNK_MIN_TOKENS
-    check(L.recurrent(dk).ri_head_scan_short(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
-                                             H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0,
-                                             dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots),
-                                             int(entries), H, dv, H // G, _p(pos), _p(cos), _p(sin), int(rot), 1 if inter else 0,
-                                             1 if T == int(entries) else 0, below, stream_ptr()), "head_scan")
+    check(L.recurrent(dk).ri_head_scan(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(decay),
+                                       H if decay.dim() == 2 else 0, _p(gain), H if gain is not None else 0,
+                                       dtype_code(q.dtype), float(q_scale), _p(out), _p(state), _p(cu_q), _p(state_slots),
+                                       int(entries), H, dv, H // G, _p(pos), _p(cos), _p(sin), int(rot), 1 if inter else 0,
+                                       1 if T == int(entries) else 0, below, stream_ptr()), "head_scan")
 
 
 def delta_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, za: torch.Tensor, za_bias: Optional[torch.Tensor],

@@ -73,15 +73,12 @@ _SIGNATURES = {
     "ri_scaled_sum": [_P, _P, _F, _F, _P, _I, _L, _P],
     "ri_gemm_few": [_P, _P, _I, _I, _I, _P, _I, _I, _I, _P],
     "ri_gemm_few_shape": [_I, _I, _I],
-    "ri_gated_scan_short": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "ri_delta_scan_short": [_P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "ri_head_scan_short": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "ri_chunks_ok": [_P, _I, _P, _I, _P, _I, _I, _I, _I],
     "ri_head_chunks": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P],
     "ri_gated_chunks": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
     "ri_gated_chunk_parts": [],
     "ri_recurrent_chunk_tokens": [],
-    "ri_gated_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P],
+    "ri_gated_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "ri_delta_scan": [_P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "ri_rms_sandwich": [_P, _I, _P, _I, _I, _P, _P, _P, _L, _I, _P, _P, _P, _P, _I, _P, _I, _I, _F, _P, _P, _P, _I, _P],
     "ri_short_conv": [_P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _P, _P, _I, _P],
@@ -91,7 +88,7 @@ _SIGNATURES = {
     "ri_sigmoid_gate": [_P, _I, _I, _P, _I, _I, _P, _I, _I, _I, _F, _P],
     "ri_softcap": [_P, _L, _F, _P],
     "ri_glu_pairs": [_P, _P, _I, _L, _I, _F, _F, _P],
-    "ri_head_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _P],
+    "ri_head_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "ri_norm_add": [_P, _P, _I, _P, _I, _F, _P, _I, _I, _I, _P, _P, _P, _P, _P, _I, _P, _I, _P],
     "ri_rotate_cols": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "ri_part_norm_gate": [_P, _P, _I, _P, _I, _P, _I, _P, _F, _I, _P, _I, _I, _I, _I, _P],
