@@ -18,7 +18,8 @@
 // are added up in fp32 on the tensor cores, the small ones first.  bf16 inputs are one piece.  The products of decays are formed
 // by multiplication, never as quotients or through logarithms, so they stay below one and a decay of zero is a zero.  A value
 // that is no number keeps out of the products (zero times infinity in a masked place would reach earlier tokens) and makes its
-// column's later outputs NaN by itself.
+// column's later outputs NaN by itself.  An infinity in a query, a key, a decay or a state is NaN from its place on too: its pieces are
+// infinity and what is left of it, where the walk carries it until two of either sign meet.
 #include "common.cuh"
 
 #ifndef RI_KDIM

@@ -1420,7 +1420,8 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
     allowed.  State as `gated_scan`.  `rotation` (positions int32 [T], cos, sin fp32 [positions, rot/2], rot, interleaved):
     keys and queries are rotated on the way in; only for a step in which every entry brings one token (T == entries).
     `longest`: the most tokens an entry brings, from a caller that does not need a token's sums to be the same however its
-    prompt was cut: entries of CHUNK_MIN_TOKENS or more may then go in chunks (recurrent_chunks.cu)."""
+    prompt was cut and whichever entries share the call: entries of CHUNK_MIN_TOKENS or more may then go in chunks
+    (recurrent_chunks.cu), which differ from the walk in rounding, and make NaN of an infinity that the walk carries on."""
     require_cuda(q, k, v, decay, out, state, cu_q, state_slots, gain, *(rotation[:3] if rotation else ()))
     T, H, dk, dv = q.shape[0], num_heads, key_dim, value_dim
     G = key_heads or H
