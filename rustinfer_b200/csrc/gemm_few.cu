@@ -24,6 +24,27 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// the sums of one token and two neighbouring features into `out`
+__device__ __forceinline__ void store_pair(void* out, int ld_out, int epilogue, int N, int tok, int feat, float s0, float s1) {
+    const bool two = feat + 1 < N;
+    if (epilogue == EPI_SILU || epilogue == EPI_GELU) {
+        float act;
+        if (epilogue == EPI_SILU) act = __fdividef(s0, 1.f + __expf(-s0));
+        else act = __fdividef(s0, 1.f + __expf(-2.f * (0.7978845608028654f * (s0 + 0.044715f * s0 * s0 * s0))));   // 0.5 (1 + tanh y) = 1 / (1 + e^-2y)
+        reinterpret_cast<bf16*>(out)[(size_t)tok * ld_out + (feat >> 1)] = __float2bfloat16_rn(act * s1);
+    } else if (epilogue == EPI_F32 || epilogue == EPI_RESIDUAL) {
+        float* p = reinterpret_cast<float*>(out) + (size_t)tok * ld_out + feat;
+        const bool add = epilogue == EPI_RESIDUAL;
+        p[0] = add ? p[0] + s0 : s0;
+        if (two) p[1] = add ? p[1] + s1 : s1;
+    } else {
+        if (epilogue == EPI_RELU2) { s0 = fmaxf(s0, 0.f); s1 = fmaxf(s1, 0.f); s0 *= s0; s1 *= s1; }
+        bf16* p = reinterpret_cast<bf16*>(out) + (size_t)tok * ld_out + feat;
+        p[0] = __float2bfloat16_rn(s0);
+        if (two) p[1] = __float2bfloat16_rn(s1);
+    }
+}
+
 // MT: tiles of 16 tokens; NT: tiles of 8 features a CTA; U: blocks of 32 k a warp has on the way
 template <int MT, int NT, int WARPS, int U>
 __global__ void __launch_bounds__(WARPS * 32)
@@ -119,24 +140,58 @@ gemm_few_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, int M, i
             s0 += p.x;
             s1 += p.y;
         }
-        const bool two = feat + 1 < N;
-        if (epilogue == EPI_SILU || epilogue == EPI_GELU) {
-            float act;
-            if (epilogue == EPI_SILU) act = __fdividef(s0, 1.f + __expf(-s0));
-            else act = __fdividef(s0, 1.f + __expf(-2.f * (0.7978845608028654f * (s0 + 0.044715f * s0 * s0 * s0))));   // 0.5 (1 + tanh y) = 1 / (1 + e^-2y)
-            reinterpret_cast<bf16*>(out)[(size_t)tok * ld_out + (feat >> 1)] = __float2bfloat16_rn(act * s1);
-        } else if (epilogue == EPI_F32 || epilogue == EPI_RESIDUAL) {
-            float* p = reinterpret_cast<float*>(out) + (size_t)tok * ld_out + feat;
-            const bool add = epilogue == EPI_RESIDUAL;
-            p[0] = add ? p[0] + s0 : s0;
-            if (two) p[1] = add ? p[1] + s1 : s1;
-        } else {
-            if (epilogue == EPI_RELU2) { s0 = fmaxf(s0, 0.f); s1 = fmaxf(s1, 0.f); s0 *= s0; s1 *= s1; }
-            bf16* p = reinterpret_cast<bf16*>(out) + (size_t)tok * ld_out + feat;
-            p[0] = __float2bfloat16_rn(s0);
-            if (two) p[1] = __float2bfloat16_rn(s1);
-        }
+        store_pair(out, ld_out, epilogue, N, tok, feat, s0, s1);
     }
+}
+
+// K of up to 448: a warp owns 8 features and all of K, its products in one chain of 16 k each in the order of k, which is how one
+// accumulator of the tcgen05 kernel takes them: the sums have the same bits.  Bound by the trip to memory of a round of eight steps; the
+// next round's weights are on the way while one is multiplied, the first round's before the kernel waits for its predecessor.
+constexpr int SHORT_WARPS = 2, SHORT_STEPS = 8;              // warps a CTA; steps of 16 k that are on the way together
+template <int MT>
+__global__ void __launch_bounds__(SHORT_WARPS * 32)
+gemm_short_kernel(const bf16* __restrict__ X, const bf16* __restrict__ W, int M, int N, int K, void* __restrict__ out, int ld_out, int epilogue) {
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int f0 = (blockIdx.x * SHORT_WARPS + (threadIdx.x >> 5)) * 8;
+    auto two = [&](const bf16* row, bool valid, int k) { return valid && k < K ? *reinterpret_cast<const uint32_t*>(row + k) : 0u; };
+    const bf16* wrow = W + (size_t)min(f0 + g, N - 1) * K;
+    uint32_t w[SHORT_STEPS][2], wn[SHORT_STEPS][2];
+    auto weights = [&](uint32_t (&to)[SHORT_STEPS][2], int k0) {
+#pragma unroll
+        for (int s = 0; s < SHORT_STEPS; ++s)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) to[s][h] = two(wrow, f0 + g < N, k0 + s * 16 + h * 8 + 2 * t);
+    };
+    weights(w, 0);
+    pdl_wait();
+    float acc[MT][4] = {};
+    for (int k0 = 0; k0 < K; k0 += SHORT_STEPS * 16) {
+        uint32_t x[SHORT_STEPS][MT][4];
+#pragma unroll
+        for (int s = 0; s < SHORT_STEPS; ++s)
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int row = m * 16 + g + (e & 1) * 8;
+                    x[s][m][e] = two(X + (size_t)min(row, M - 1) * K, row < M, k0 + s * 16 + (e >> 1) * 8 + 2 * t);
+                }
+        weights(wn, k0 + SHORT_STEPS * 16);
+#pragma unroll
+        for (int s = 0; s < SHORT_STEPS; ++s)
+#pragma unroll
+            for (int m = 0; m < MT; ++m) mma(acc[m], x[s][m][0], x[s][m][1], x[s][m][2], x[s][m][3], w[s][0], w[s][1]);
+#pragma unroll
+        for (int s = 0; s < SHORT_STEPS; ++s) { w[s][0] = wn[s][0]; w[s][1] = wn[s][1]; }
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int tok = m * 16 + g + 8 * h, feat = f0 + 2 * t;
+            if (tok < M && feat < N) store_pair(out, ld_out, epilogue, N, tok, feat, acc[m][2 * h], acc[m][2 * h + 1]);
+        }
 }
 
 template <int MT, int NT, int WARPS, int U>
@@ -154,12 +209,14 @@ int launch(const void* X, const void* W, int M, int N, int K, void* out, int ld_
 // ahead, the whole step was 3 % slower; 28,672 x 4,096 48 against 45 (the stream of weights is the bound, and TMA keeps more of it
 // on the way).  24 rows: 1,024 x 1,024 3.0 / 9.8, 2,048 x 2,048 4.8 / 11.9, 8,192 x 1,024 8.0 / 11.4, 16,384 x 1,024 14.2 / 12.9.
 // Narrow tiles while they are few, 16 features a CTA up to two CTAs an SM, sixteen warps where K is long.
-// Up to seven k-blocks of 64 the other kernel stays, although it takes longer (8 x 1,024 x 128: 4.0 us against 1.7): no plan of it cuts
-// such a K, so a token's sums have the same bits in a step of single tokens, in one of fifty and in a prompt, and models of such sizes,
-// with experts a rounding away from one another, answer the same however their tokens are cut.
+// Up to seven k-blocks of 64 no plan of the tcgen05 kernel cuts K, and a token's sums have the same bits in a step of single tokens, in one
+// of fifty and in a prompt: models of such sizes, with experts a rounding away from one another, answer the same however their tokens are
+// cut.  The kernel with one chain a sum keeps those bits, where it is faster: 8 x 1,024 x 128 1.6 against 4.0 us, 16 x 4,096 x 128 3.3 / 4.7,
+// 16 x 1,024 x 448 3.8 / 6.1, 32 x 2,048 x 256 5.9 / 7.2; but 32 x 1,024 x 448 9.5 / 8.0, 8 x 8,192 x 448 14.8 / 6.1.
 RI_API int ri_gemm_few_shape(int M, int N, int K) {
-    if (M < 1 || M > 32 || N < 1 || K <= 7 * 64 || K % 8) return -1;
+    if (M < 1 || M > 32 || N < 1 || K < 8 || K % 8) return -1;
     const long long weights = (long long)N * K;
+    if (K <= 7 * 64) return weights <= (1 << 19) && (M <= 16 || K <= 256) ? 4 : -1;
     if (N <= 1024 && K <= 8192) return 0;
     if (N <= 2 * 16 * ri_device_sms() && weights <= (17 << 20)) return 1;
     if (M <= 16) return weights <= (26 << 20) && K <= 4096 ? 2 : -1;
@@ -177,6 +234,12 @@ RI_API int ri_gemm_few(const void* X, const void* W, int M, int N, int K, void* 
         case 1: RI_FEW(2, 16, 2);
         case 2: if (M > 16) break; return launch<1, 4, 8, 2>(X, W, M, N, K, out, ld_out, epilogue, s);
         case 3: if (M <= 16) break; return launch<2, 4, 4, 4>(X, W, M, N, K, out, ld_out, epilogue, s);
+        case 4: {
+            const dim3 grid((N + 8 * SHORT_WARPS - 1) / (8 * SHORT_WARPS)), block(SHORT_WARPS * 32);
+            if (M <= 16) RI_CHECKED(ri_launch(gemm_short_kernel<1>, grid, block, 0, s, (const bf16*)X, (const bf16*)W, M, N, K, out, ld_out, epilogue));
+            else RI_CHECKED(ri_launch(gemm_short_kernel<2>, grid, block, 0, s, (const bf16*)X, (const bf16*)W, M, N, K, out, ld_out, epilogue));
+            return ri_launch_status();
+        }
     }
 #undef RI_FEW
     return (int)cudaErrorInvalidValue;

@@ -9,7 +9,7 @@ DEV = "cuda:0"
 
 
 # features on both sides of every change of tile, odd ones; k that is one piece, no multiple of a warp's blocks, several rounds of them
-@pytest.mark.parametrize("N,K", [(9, 8192), (130, 1000), (1024, 1024), (1026, 520), (4736, 456), (4738, 504), (8192, 1000), (600, 8192)])
+@pytest.mark.parametrize("N,K", [(66, 8), (130, 200), (2050, 104), (9, 8192), (130, 1000), (1024, 1024), (1026, 520), (4736, 456), (4738, 504), (8192, 1000), (600, 8192)])
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 24, 32])
 def test_every_epilogue(M, N, K):
     from rustinfer_b200.ops import kernels as k, library as L
