@@ -22,6 +22,14 @@
 //               output accumulates in tensor memory across tiles; it is rescaled (load,
 //               multiply, store) only when a row's maximum has grown by more than 2^8 since
 //               the reference it was scaled to, which after the first tiles is rare
+// A second form (EXACT) serves mixers whose softmax weights meet the values unrounded: a weight is cut into three bf16 pieces
+// (their sum is the weight), P V runs once a piece into the same accumulator, the small pieces first; scores may carry a bias by
+// distance, the denominator a sink, the output a gate, each a head.  The biases of the group's heads lie in shared memory; a
+// warp whose rows see a whole tile from the table's last distance on (most tiles of a long prompt) adds one number a row, the
+// others read one a score.  What bounds it is the softmax warps' issue rate (about ten instructions a score, half of them
+// the pieces) before the tensor core (16 MMAs a tile, 2/3 of the cycles reading operands).  Against the mma.sync kernel
+// (attention_rows.cu), 32 heads of 64 over 8, bias of 128 distances: 2 tokens 6.7 -> 6.6 us, 300 tokens 20.8 -> 14.1,
+// 2,048 tokens 226 -> 66, 16 x 300 101 -> 62; 8 heads of 128 over 2: 2 tokens 8.5 -> 6.7, 2,048 tokens 200 -> 51.
 // Every wait on an mbarrier is bounded; a time-out leaves a code in *error and the kernel
 // winds down (tensor memory freed, copies in flight drained).
 #include "common.cuh"
@@ -61,6 +69,10 @@ constexpr int OFF_BAR = OFF_P + P_BYTES;
 // shared memory gets its dynamic part on a 1024-byte boundary; the kernel checks that and refuses
 // to run otherwise.
 constexpr size_t SMEM = (size_t)OFF_BAR + 128;
+// The form with unrounded weights keeps three tiles of pieces, and the biases of the group's heads behind the barriers.
+constexpr int PIECES = 3;
+constexpr int OFF_BAR_EXACT = OFF_P + PIECES * P_BYTES, OFF_BIAS = OFF_BAR_EXACT + 128;
+constexpr int BIAS_BYTES = 14 * 1024;             // of the biases, at most: two CTAs an SM
 
 enum { ERR_PRODUCER = 11, ERR_MMA = 12, ERR_SOFTMAX = 13, ERR_ALIGNMENT = 14 };
 
@@ -156,18 +168,36 @@ struct Params {
     int Hq, Hkv, G, tpt, page_size, box_rows;
     float scale_log2; int window;
     int* error;
+    // the form with unrounded weights only
+    const float* bias;      // bias[h * bias_len + min(distance, bias_len - 1)] is added to head h's scores (null: none)
+    int bias_len, bias_span, bias_stride;             // distances kept in shared memory, floats from one head to the next
+    const float* sink_values;                         // the denominator holds exp(sink_values[h]) too (null: none)
+    const float* gate; int gate_stride; float gate_scale;      // head h's output times gate_scale * sigmoid(gate[t][h]) (null: as it is)
 };
+constexpr float LOG2E = 1.4426950408889634f;
+
+// 2k and 2k + 1 of a thread's weights as three bf16 pairs, each the rounded rest of the one before: their sum is the weight
+__device__ __forceinline__ void cut_pair(float x, float y, unsigned (&w)[PIECES]) {
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+        w[i] = *reinterpret_cast<const unsigned*>(&h);
+        x -= __uint_as_float(w[i] << 16);
+        y -= __uint_as_float(w[i] & 0xffff0000u);
+    }
+}
 
 // three CTAs per SM for heads of 64, two for 128 (tensor memory, shared memory and registers
 // allow it): the other CTAs' softmax fills the issue slots one leaves while it waits on its chain
-__global__ void __launch_bounds__(THREADS, HD == 64 ? 3 : 2)
+template <bool EXACT>
+__global__ void __launch_bounds__(THREADS, EXACT ? (HD == 64 ? 2 : 1) : HD == 64 ? 3 : 2)
 attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params p) {
     extern __shared__ __align__(1024) unsigned char sm[];
     if ((smem_u32(sm) & 1023u) != 0) {                         // the 128-byte swizzle wants 1024-byte tiles
         if (threadIdx.x == 0) atomicCAS(p.error, 0, ERR_ALIGNMENT);
         return;
     }
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + OFF_BAR);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + (EXACT ? OFF_BAR_EXACT : OFF_BAR));
     uint64_t* k_full = bars;              // [NS]
     uint64_t* k_empty = k_full + NS;      // [NS]
     uint64_t* v_full = k_empty + NS;      // [NS]
@@ -305,9 +335,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params 
             const unsigned p_addr = smem_u32(sm + OFF_P);
             const unsigned v_addr = smem_u32(sm + OFF_V + s * KV_STAGE);
 #pragma unroll
-            for (int k = 0; k < BN / 16; ++k)                  // 16 keys per MMA: two 8-key groups of V
-                mma_ss(tmem_base + COL_O, desc_kmajor(p_addr + k * 32), desc_mnmajor(v_addr + k * 2048),
-                       idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+            for (int piece = EXACT ? PIECES - 1 : 0; piece >= 0; --piece)      // the small ones first
+#pragma unroll
+                for (int k = 0; k < BN / 16; ++k)              // 16 keys per MMA: two 8-key groups of V
+                    mma_ss(tmem_base + COL_O, desc_kmajor(p_addr + piece * P_BYTES + k * 32), desc_mnmajor(v_addr + k * 2048),
+                           idesc_o, (j > 0 || k > 0 || piece < (EXACT ? PIECES - 1 : 0)) ? 1u : 0u);
             tc_commit(&v_empty[s]);
             tc_commit(p_empty);
             tc_commit(o_done);
@@ -318,7 +350,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params 
         const int r = quarter * 32 + lane;                     // this thread's row = its TMEM lane
         const int jj = r / p.G, hh = r - jj * p.G;
         const bool row_ok = n_tiles > 0 && jj < ntok;
-        const int p_row = p_first + jj;
+        // (with unrounded weights a row past the portion goes the way of the last one, on queries of zero, and is dropped)
+        const int p_row = p_first + (EXACT ? max(min(jj, ntok - 1), 0) : jj);
         const int lo_row = p.window > 0 ? max(0, p_row - p.window + 1) : 0;
         const unsigned lane_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
         pdl_wait();
@@ -339,6 +372,25 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params 
         }
         float m = -INFINITY, l = 0.f;                          // m: the maximum the output is scaled to
         bool ok = true;
+        float* biases = reinterpret_cast<float*>(sm + OFF_BIAS);       // [G][bias_stride], in units of log2
+        float far = 0.f;                                       // the bias from the table's last distance on
+        // the warp's first row sees its tile's last key no nearer than the last distance: one bias for the whole tile
+        const int p_warp = p_first + quarter * 32 / p.G;
+        if constexpr (EXACT) {
+            if (p.bias && n_tiles > 0) {
+                const int need = min(p.bias_span, max(p_last - lo_tile + 1, p.bias_len));
+                for (int h = 0; h < p.G; ++h)
+                    for (int i = threadIdx.x - 64; i < need; i += THREADS - 64)
+                        biases[h * p.bias_stride + i] = p.bias[(size_t)(g * p.G + h) * p.bias_len + min(i, p.bias_len - 1)] * LOG2E;
+                asm volatile("bar.sync 1, %0;" ::"n"(THREADS - 64) : "memory");       // the softmax warps alone
+                far = biases[hh * p.bias_stride + p.bias_len - 1];
+            }
+            if (p.sink_values && row_ok) {
+                // a term exp(sink_h) without a value: the maximum starts there, and the sum at exp(sink_h - sink_h) = 1
+                m = p.sink_values[g * p.G + hh] * LOG2E;
+                l = 1.f;
+            }
+        }
         for (int j = 0; j < n_tiles && ok; ++j) {
             const int t = t_begin + j;
             if (!mbar_wait(s_full, j & 1, p.error, ERR_SOFTMAX)) { ok = false; break; }
@@ -349,12 +401,33 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params 
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(s_empty);                // the tensor core may write the next tile's scores
-            const bool masked = p.window > 0 || t * BN + BN - 1 > p_row || !row_ok;
+            const bool masked = EXACT ? t * BN + BN - 1 > p_row || t * BN < lo_row : p.window > 0 || t * BN + BN - 1 > p_row || !row_ok;
+            if constexpr (EXACT) {                             // scores in units of log2, biases added
+                if (p.bias && p_warp - (t * BN + BN - 1) < p.bias_len - 1) {
+                    const float* own = biases + hh * p.bias_stride;
+                    const int d0 = p_row - t * BN;             // distance of the tile's first key
+                    if (masked) {
+#pragma unroll
+                        for (int i = 0; i < BN; ++i) s[i] = fmaf(s[i], p.scale_log2, own[min(max(d0 - i, 0), p.bias_span - 1)]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < BN; ++i) s[i] = fmaf(s[i], p.scale_log2, own[d0 - i]);
+                    }
+                } else {
+                    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), far2 = make_float2(far, far);
+#pragma unroll
+                    for (int i = 0; i < BN; i += 2) {
+                        const float2 x = __ffma2_rn(make_float2(s[i], s[i + 1]), sc2, far2);
+                        s[i] = x.x;
+                        s[i + 1] = x.y;
+                    }
+                }
+            }
             if (masked) {
 #pragma unroll
                 for (int i = 0; i < BN; ++i) {
                     const int key = t * BN + i;
-                    s[i] = (row_ok && key <= p_row && key >= lo_row) ? s[i] : -INFINITY;
+                    s[i] = ((EXACT || row_ok) && key <= p_row && key >= lo_row) ? s[i] : -INFINITY;
                 }
             }
             // four independent chains each for the maximum and the sum: one thread owns the whole
@@ -365,7 +438,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params 
                 mx4[0] = max3(mx4[0], s[i], s[i + 1]); mx4[1] = max3(mx4[1], s[i + 2], s[i + 3]);
                 mx4[2] = max3(mx4[2], s[i + 4], s[i + 5]); mx4[3] = max3(mx4[3], s[i + 6], s[i + 7]);
             }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * (EXACT ? 1.f : p.scale_log2);
             // The reference maximum moves only when the row's maximum has outgrown it by 2^8
             // (probabilities up to 256 are exact enough in bf16 and harmless in fp32 sums);
             // then the output in tensor memory and the sum are brought to the new reference.
@@ -403,7 +476,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params 
                 for (int i = 0; i < BN; i += 4) {
 #pragma unroll
                     for (int k = 0; k < 2; ++k) {
-                        const float2 x = __ffma2_rn(make_float2(s[i + 2 * k], s[i + 2 * k + 1]), scale2, shift2);
+                        const float2 own = make_float2(s[i + 2 * k], s[i + 2 * k + 1]);
+                        const float2 x = EXACT ? __fadd2_rn(own, shift2) : __ffma2_rn(own, scale2, shift2);
                         if (decltype(with_poly)::value && POLY_OF > 0 && ((i / 2 + k) % POLY_OF) == POLY_OF - 1) {
                             const float2 e = ex2_poly2(x);
                             s[i + 2 * k] = e.x;
@@ -416,13 +490,25 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params 
                     }
                 }
             };
-            if (__any_sync(0xffffffffu, masked)) exponentials(std::false_type{});
+            if (EXACT || __any_sync(0xffffffffu, masked)) exponentials(std::false_type{});
             else exponentials(std::true_type{});
             l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
             // P row (bf16) into the A operand of P V
             if (!mbar_wait(p_empty, (j & 1) ^ 1, p.error, ERR_SOFTMAX)) { ok = false; break; }
             {
                 unsigned char* prow = sm + OFF_P + r * 128;
+                if constexpr (EXACT) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        unsigned w[4][PIECES];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) cut_pair(s[c * 8 + 2 * i], s[c * 8 + 2 * i + 1], w[i]);
+#pragma unroll
+                        for (int piece = 0; piece < PIECES; ++piece)
+                            *reinterpret_cast<uint4*>(prow + piece * P_BYTES + ((c ^ (r & 7)) << 4)) =
+                                make_uint4(w[0][piece], w[1][piece], w[2][piece], w[3][piece]);
+                    }
+                } else
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     uint4 w;
@@ -455,7 +541,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap cache_map, const Params 
         if (ok && n_tiles > 0) ok = mbar_wait(o_done, (n_tiles - 1) & 1, p.error, ERR_SOFTMAX);
         if (ok && n_tiles > 0) {
             tc_fence_after();
-            const float inv = l > 0.f ? 1.f / l : 0.f;
+            float inv = l > 0.f ? 1.f / l : 0.f;
+            if constexpr (EXACT) {
+                if (p.gate && row_ok)
+                    inv *= p.gate_scale / (1.0f + expf(-p.gate[(size_t)(q_begin + tok0 + jj) * p.gate_stride + g * p.G + hh]));
+            }
             bf16* dst = p.out + (size_t)(q_begin + tok0 + jj) * p.out_stride + (size_t)(g * p.G + hh) * HD;
 #pragma unroll
             for (int c0 = 0; c0 < HD; c0 += 16) {
@@ -547,6 +637,37 @@ RI_API int ri_attention_tc_supports(int Hq, int Hkv, int page_size) {
 }
 RI_API int ri_attention_tc_tokens_per_tile(int Hq, int Hkv) { return BM / (Hq / Hkv); }
 
+namespace {
+int bias_span(int bias_len, int G) { return bias_len + BN + (32 + G - 1) / G + 1; }     // see the table's use in the kernel
+int bias_stride(int span) { return (span + 31) / 32 * 32 + 8; }      // the heads of a group 8 banks apart
+Params params(const void* q, int q_stride, void* out, int out_stride, const int* block_table, int table_stride, const int* cu_q,
+              const int* kv_len, const int* tile_entry, const int* tile_tok0, int Hq, int Hkv, int page_size, float scale, int window, int* error) {
+    Params p{};
+    p.q = (const bf16*)q; p.q_stride = q_stride; p.out = (bf16*)out; p.out_stride = out_stride;
+    p.block_table = block_table; p.table_stride = table_stride;
+    p.cu_q = cu_q; p.kv_len = kv_len; p.tile_entry = tile_entry; p.tile_tok0 = tile_tok0;
+    p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.tpt = BM / p.G; p.page_size = page_size;
+    p.box_rows = page_size < BN ? page_size : BN;
+    p.scale_log2 = scale * LOG2E; p.window = window; p.error = error;
+    return p;
+}
+template <bool EXACT>
+int launch(const Params& p, const void* cache, long long n_pages, int n_tiles, size_t smem, void* stream) {
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             EXACT ? OFF_BIAS + BIAS_BYTES : (int)SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    CUtensorMap map;
+    int st = cache_map(cache, n_pages * 2 * p.Hkv * p.page_size, p.box_rows, &map);
+    if (st != 0) return st;
+    RI_CHECKED(ri_launch(attention_tc_kernel<EXACT>, dim3(p.Hkv, n_tiles), dim3(THREADS), smem, (cudaStream_t)stream, map, p));
+    return ri_launch_status();
+}
+}  // namespace
+
 // Tiles are (entry, first token) pairs of 128 / (Hq/Hkv) tokens.  error: one int that a
 // timed-out wait sets (zero it before use).
 RI_API int ri_attention_prefill_tc(const void* q, int q_stride, void* out, int out_stride, const void* cache,
@@ -556,22 +677,37 @@ RI_API int ri_attention_prefill_tc(const void* q, int q_stride, void* out, int o
                                    void* stream) {
     if (n_tiles <= 0) return 0;
     if (!ri_attention_tc_supports(Hq, Hkv, page_size) || !error) return (int)cudaErrorInvalidValue;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
+    return launch<false>(params(q, q_stride, out, out_stride, block_table, table_stride, cu_q, kv_len, tile_entry, tile_tok0, Hq, Hkv,
+                                page_size, scale, window, error), cache, n_pages, n_tiles, SMEM, stream);
+}
+
+// 1 if the form with unrounded weights takes a bias of `bias_len` distances (0: none) for this grouping and page size.
+RI_API int ri_attention_tc_exact_supports(int Hq, int Hkv, int page_size, int bias_len) {
+    if (!ri_attention_tc_supports(Hq, Hkv, page_size) || bias_len < 0 || bias_len > BIAS_BYTES / 4) return 0;
+    const int G = Hq / Hkv;
+    return !bias_len || (long long)G * bias_stride(bias_span(bias_len, G)) * 4 <= BIAS_BYTES ? 1 : 0;
+}
+
+// As ri_attention_prefill_tc, with the softmax weights unrounded (three bf16 pieces), a bias by distance [Hq][bias_len], a sink
+// a head (a term of the denominator) and a gate a head (fp32 [T][gate_stride]), each null where there is none.
+RI_API int ri_attention_prefill_tc_exact(const void* q, int q_stride, void* out, int out_stride, const void* cache,
+                                         long long n_pages, const int* block_table, int table_stride, const int* cu_q,
+                                         const int* kv_len, const int* tile_entry, const int* tile_tok0, int n_tiles,
+                                         int Hq, int Hkv, int page_size, float scale, int window, const float* bias, int bias_len,
+                                         const float* sink_values, const float* gate, int gate_stride, float gate_scale, int* error,
+                                         void* stream) {
+    if (n_tiles <= 0) return 0;
+    if (!ri_attention_tc_exact_supports(Hq, Hkv, page_size, bias ? bias_len : 0) || (bias && bias_len < 1) || !error)
+        return (int)cudaErrorInvalidValue;
+    Params p = params(q, q_stride, out, out_stride, block_table, table_stride, cu_q, kv_len, tile_entry, tile_tok0, Hq, Hkv, page_size, scale,
+                      window, error);
+    size_t smem = OFF_BIAS;
+    if (bias) {
+        p.bias = bias; p.bias_len = bias_len;
+        p.bias_span = bias_span(bias_len, p.G); p.bias_stride = bias_stride(p.bias_span);
+        smem += (size_t)p.G * p.bias_stride * sizeof(float);
     }
-    Params p;
-    p.q = (const bf16*)q; p.q_stride = q_stride; p.out = (bf16*)out; p.out_stride = out_stride;
-    p.block_table = block_table; p.table_stride = table_stride; p.cu_q = cu_q; p.kv_len = kv_len;
-    p.tile_entry = tile_entry; p.tile_tok0 = tile_tok0;
-    p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.tpt = BM / p.G; p.page_size = page_size;
-    p.box_rows = page_size < BN ? page_size : BN;
-    p.scale_log2 = scale * 1.4426950408889634f; p.window = window; p.error = error;
-    CUtensorMap map;
-    int st = cache_map(cache, n_pages * 2 * Hkv * page_size, p.box_rows, &map);
-    if (st != 0) return st;
-    RI_CHECKED(ri_launch(attention_tc_kernel, dim3(Hkv, n_tiles), dim3(THREADS), SMEM, (cudaStream_t)stream, map, p));
-    return ri_launch_status();
+    p.sink_values = sink_values;
+    p.gate = gate; p.gate_stride = gate_stride; p.gate_scale = gate_scale;
+    return launch<true>(p, cache, n_pages, n_tiles, smem, stream);
 }

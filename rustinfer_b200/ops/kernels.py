@@ -1801,6 +1801,36 @@ def attention_prefill_tc(q, out, cache, block_table, cu_q, kv_len, tile_entry, t
                                       _p(err), stream_ptr()), "attention_prefill_tc")
 
 
+def tc_exact_supports(num_heads: int, num_kv_heads: int, head_dim: int, page_size: int, bias_len: int = 0) -> bool:
+    """Whether `attention_prefill_exact` takes this geometry with a bias of so many distances (0: none)."""
+    return head_dim in (64, 128) and bool(
+        L.attention_tc(head_dim).ri_attention_tc_exact_supports(num_heads, num_kv_heads, page_size, bias_len))
+
+
+def attention_prefill_exact(q, out, cache, block_table, cu_q, kv_len, tile_entry, tile_tok0, num_heads: int, num_kv_heads: int,
+                            head_dim: int, scale: float, window: Optional[int], sink_values: Optional[torch.Tensor] = None,
+                            bias: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, gate_scale: float = 1.0) -> None:
+    """`attention_prefill_tc` with the softmax weights unrounded (three bf16 pieces a weight) and `attention_plain`'s bias by
+    distance, sinks and gate a head.  bf16 out; tiles as `attention_prefill_tc`'s."""
+    _attention_args(q, out, cache, block_table, cu_q, kv_len, num_heads, num_kv_heads, head_dim)
+    require_cuda(tile_entry, tile_tok0, sink_values, bias, gate)
+    _i32(tile_entry, "tile_entry"); _i32(tile_tok0, "tile_tok0")
+    _slopes_ok(None, num_heads, bias)
+    _gate_ok(gate, q, num_heads)
+    if tile_tok0.numel() < tile_entry.numel():
+        raise KernelError("attention_prefill_exact: a first token for every tile")
+    if sink_values is not None and (sink_values.dtype != torch.float32 or sink_values.numel() != num_heads or not sink_values.is_contiguous()):
+        raise KernelError("attention_prefill_exact: sinks are contiguous fp32 [heads]")
+    if out.stride(0) % 8 or out.data_ptr() % 16 or cache.data_ptr() % 16:
+        raise KernelError("attention_prefill_exact: out rows and the cache must be 16-byte aligned")
+    err = gemm_tc_state(q.device)[2]
+    check(L.attention_tc(head_dim).ri_attention_prefill_tc_exact(
+        _p(q), q.stride(0), _p(out), out.stride(0), _p(cache), cache.shape[0], _p(block_table), block_table.stride(0), _p(cu_q),
+        _p(kv_len), _p(tile_entry), _p(tile_tok0), tile_entry.numel(), num_heads, num_kv_heads, cache.shape[3], float(scale),
+        int(window) if window else 0, _p(bias), bias.shape[1] if bias is not None else 0, _p(sink_values),
+        *_gate_args(gate, gate_scale), _p(err), stream_ptr()), "attention_prefill_tc_exact")
+
+
 def decode_scratch_floats(entries: int, num_heads: int, head_dim: int, splits: int):
     return entries * num_heads * splits * head_dim, entries * num_heads * splits
 

@@ -33,7 +33,9 @@ _SIGNATURES = {
     "ri_attention_decode_bf16": [_P, _I, _P, _I, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _I, _I, _P, _P, _L, _P, _I, _P],
     "ri_attention_mma_tokens_per_tile": [_I],
     "ri_attention_prefill_tc": [_P, _I, _P, _I, _P, _L, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P],
+    "ri_attention_prefill_tc_exact": [_P, _I, _P, _I, _P, _L, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _F, _I, _P, _I, _P, _P, _I, _F, _P, _P],
     "ri_attention_tc_supports": [_I, _I, _I],
+    "ri_attention_tc_exact_supports": [_I, _I, _I, _I],
     "ri_gemm_tc": [_P, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
     "ri_gemm_tc_rope": [_P, _P, _I, _I, _I, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P],
     "ri_decode_chain": [_P, _I, _P, _I, _P, _P, _I, _P],
