@@ -36,6 +36,10 @@ namespace {
 constexpr int DK = RI_KDIM;
 constexpr int KP = DK + 8;                      // bf16 of a padded row: an odd count of 16-byte pieces, ldmatrix meets no conflict
 constexpr int QUARTERS = CK / 16;
+// States between the kernels lie in blocks of 16 value x 16 key channels, [value block][key block][lane][8]: what a lane of
+// m16n8k16 holds of a block, (v, k) (v, k + 8) (v + 8, k) (v + 8, k + 8) and each one's neighbour in k, v = lane / 4, k = 2 (lane % 4),
+// is both a lane's accumulators of one product and its operand of the next.
+constexpr int KS = DK / 16;                     // key blocks
 
 // The entry and tokens of chunk `index` among the entries that bring at least `least` tokens.
 struct Chunk { int entry, t0, n; };
@@ -331,20 +335,21 @@ chunk_states_kernel(const TA* __restrict__ k, int k_stride, const TA* __restrict
 #pragma unroll
         for (int m = 0; m < 2; ++m)
 #pragma unroll
-            for (int n = 0; n < 2 * NT; ++n) {
-                float* x = to + (size_t)(m0 + m * 16 + (lane >> 2)) * DK + n0 + n * 8 + (lane & 3) * 2;
-                *reinterpret_cast<float2*>(x) = make_float2(d[m][n][0], d[m][n][1]);
-                *reinterpret_cast<float2*>(x + 8 * DK) = make_float2(d[m][n][2], d[m][n][3]);
+            for (int n = 0; n < NT; ++n) {
+                float* x = to + ((size_t)(m0 / 16 + m) * KS + n0 / 16 + n) * 256 + lane * 8;
+                *reinterpret_cast<float4*>(x) = make_float4(d[m][2 * n][0], d[m][2 * n][1], d[m][2 * n + 1][0], d[m][2 * n + 1][1]);
+                *reinterpret_cast<float4*>(x + 4) = make_float4(d[m][2 * n][2], d[m][2 * n][3], d[m][2 * n + 1][2], d[m][2 * n + 1][3]);
             }
     }
 }
 
 // ------------------------------------------------------------------------------------------------- the state in front of every chunk
-// Four neighbouring key channels a thread, the chunks of its entry in order: cuts[chunk] becomes the state the chunk starts
-// from, in pieces ([chunk][head][piece][value][key]), the entry's slot the state behind the last.
+// A lane's eight numbers of one block a thread, the chunks of its entry in order: cuts[chunk] becomes the state the chunk starts
+// from, in pieces ([chunk][head][piece][block][lane]), the entry's slot the state behind the last.
 constexpr int SCAN_AHEAD = 8;                   // chunks whose loads are in flight together
+constexpr int SCAN_THREADS = 128;
 template <bool GATED>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(SCAN_THREADS)
 chunk_scan_kernel(const float* __restrict__ states, const float* __restrict__ totals, bf16* __restrict__ cuts,
                   float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ state_slots, int least,
                   int H, int dv) {
@@ -354,165 +359,173 @@ chunk_scan_kernel(const float* __restrict__ states, const float* __restrict__ to
     const int count = chunks_of(cu_q[b + 1] - cu_q[b], least);
     if (count == 0) return;
     const int base = first_chunk(cu_q, b, least);
-    const size_t one = (size_t)dv * DK, per = H * one, at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const size_t one = (size_t)dv * DK, per = H * one, at = ((size_t)blockIdx.x * SCAN_THREADS + threadIdx.x) * 8;
     if (at >= per) return;
-    const int h = (int)(at / one), i = (int)(at % DK);
-    float* own = state + (size_t)state_slots[b] * per + at;
-    float4 S = load4(own);
+    const int h = (int)(at / one), lane = threadIdx.x & 31;
+    const int block = (int)(at % one / 256), v0 = block / KS * 16 + (lane >> 2), i = block % KS * 16 + (lane & 3) * 2;
+    float* own = state + (size_t)state_slots[b] * per + ((size_t)h * dv + v0) * DK + i;
+    float2 S[4];                                             // (v0, i), (v0, i + 8), (v0 + 8, i), (v0 + 8, i + 8)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) S[j] = *reinterpret_cast<const float2*>(own + (j >> 1) * 8 * DK + (j & 1) * 8);
     for (int c0 = 0; c0 < count; c0 += SCAN_AHEAD) {
-        float4 x[SCAN_AHEAD], a[GATED ? SCAN_AHEAD : 1];
-        float2 t[GATED ? 1 : SCAN_AHEAD];
+        float4 x[SCAN_AHEAD][2];
+        float2 a[GATED ? SCAN_AHEAD : 1][2], t[GATED ? 1 : SCAN_AHEAD];
 #pragma unroll
         for (int j = 0; j < SCAN_AHEAD; ++j) {
             const size_t chunk = base + min(c0 + j, count - 1);
-            x[j] = load4(states + chunk * per + at);
-            if constexpr (GATED) a[j] = load4(totals + (chunk * H + h) * DK + i);
-            else t[j] = *reinterpret_cast<const float2*>(totals + (chunk * H + h) * 2);
+            x[j][0] = load4(states + chunk * per + at);
+            x[j][1] = load4(states + chunk * per + at + 4);
+            if constexpr (GATED) {
+                const float* p = totals + (chunk * H + h) * DK + i;
+                a[j][0] = *reinterpret_cast<const float2*>(p);
+                a[j][1] = *reinterpret_cast<const float2*>(p + 8);
+            } else {
+                t[j] = *reinterpret_cast<const float2*>(totals + (chunk * H + h) * 2);
+            }
         }
 #pragma unroll
         for (int j = 0; j < SCAN_AHEAD; ++j)
             if (c0 + j < count) {
-                put4<3>(cuts + ((size_t)(base + c0 + j) * H + h) * 3 * one + at % one, one, S);
-                if constexpr (GATED) {
-                    S = make_float4(fmaf(a[j].x, S.x, x[j].x), fmaf(a[j].y, S.y, x[j].y), fmaf(a[j].z, S.z, x[j].z), fmaf(a[j].w, S.w, x[j].w));
-                } else {
-                    const float hi = t[j].x, lo = t[j].y;
-                    S = make_float4(fmaf(hi, S.x, fmaf(lo, S.x, x[j].x)), fmaf(hi, S.y, fmaf(lo, S.y, x[j].y)),
-                                    fmaf(hi, S.z, fmaf(lo, S.z, x[j].z)), fmaf(hi, S.w, fmaf(lo, S.w, x[j].w)));
+                uint32_t p[4][3];
+#pragma unroll
+                for (int n = 0; n < 4; ++n) cut(S[n].x, S[n].y, p[n]);
+                bf16* to = cuts + ((size_t)(base + c0 + j) * H + h) * 3 * one + at % one;
+#pragma unroll
+                for (int n = 0; n < 3; ++n) *reinterpret_cast<uint4*>(to + n * one) = make_uint4(p[0][n], p[1][n], p[2][n], p[3][n]);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const float4 xx = x[j][n >> 1];
+                    const float u = n & 1 ? xx.z : xx.x, w = n & 1 ? xx.w : xx.y;
+                    if constexpr (GATED) {
+                        S[n] = make_float2(fmaf(a[j][n & 1].x, S[n].x, u), fmaf(a[j][n & 1].y, S[n].y, w));
+                    } else {
+                        const float hi = t[j].x, lo = t[j].y;
+                        S[n] = make_float2(fmaf(hi, S[n].x, fmaf(lo, S[n].x, u)), fmaf(hi, S[n].y, fmaf(lo, S[n].y, w)));
+                    }
                 }
             }
     }
-    *reinterpret_cast<float4*>(own) = S;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float2*>(own + (j >> 1) * 8 * DK + (j & 1) * 8) = S[j];
 }
 
 // ------------------------------------------------------------------------------------------------- outputs
-// The outputs of one chunk for `heads` heads of one key head, two CTAs an SM.  Eight warps: a quarter of the tokens x half of
-// the keys (scores) or of a tile of 32 value channels (outputs).  The queries stay cut up in shared memory, the scores lie
-// where the keys lay; the state's pieces come by cp.async, a tile's while the last one's values are multiplied; the values are
-// read and cut by the lanes that need them.
-constexpr int OUT_THREADS = 256;
-constexpr int OT = 32;                          // value channels of a tile
+// The outputs of one chunk for `heads` heads of one key head, two CTAs an SM.  A warp owns a block of 16 value channels for MH
+// quarters of the tokens and works for itself: queries, scores and values, cut up, come from shared memory, the state's pieces
+// straight from memory in the order of the fragments, a step ahead, so that no tile of the state is waited for.
+constexpr int OUT_THREADS = 256, OUT_WARPS = OUT_THREADS / 32;
 constexpr int AP = CK + 8;
+constexpr int OUT_V = 128, VP = OUT_V + 8;      // value channels of a CTA of the gated form
 struct OutLayout {                              // offsets in bf16, then floats
-    static constexpr int q = 0, a = q + 3 * CK * KP, s = a + 3 * CK * AP, end = s + 3 * OT * KP;
-    static constexpr int k = a;                 // keys, before the scores (gated: up to 48 rows)
-    static constexpr int floats = 5 * CK + 4 * 16 * 16;
-    static constexpr int bytes = end * 2 + floats * 4;
-    static_assert(k + 3 * CK * KP <= end && k + 3 * 48 * KP <= end && 16 * 144 * 2 <= end - k, "what lies where scores and tiles lie later");
+    static constexpr int q = 0, a = q + 3 * CK * KP;         // queries; keys, later the scores, and behind them the values
+    static constexpr int k = a, v = a + 3 * CK * AP;
+    static constexpr int end = 3 * CK * KP > 3 * CK * (AP + 64) ? a + 3 * CK * KP : v + 3 * CK * 64;
+    static constexpr int floats = 5 * CK + 4 * 16 * 16 + 64;
+    static constexpr int bytes = end * 2 + floats * 4, gated_bytes = (v + CK * VP) * 2;
 };
 
 __device__ __forceinline__ void cp16(bf16* smem, const bf16* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
 }
-// a tile of the state's pieces on its way into shared memory
-__device__ __forceinline__ void fetch_state(bf16* st, const bf16* cuts, int c0, int dv) {
-    constexpr int SN = 3 * OT * DK / 8 / OUT_THREADS;
-#pragma unroll
-    for (int j = 0; j < SN; ++j) {
-        const int e = threadIdx.x + j * OUT_THREADS, p = e / (OT * DK / 8), r = e / (DK / 8) % OT, i = (e % (DK / 8)) * 8;
-        cp16(st + (p * OT + r) * KP + i, cuts + ((size_t)p * dv + c0 + r) * DK + i);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-}
 
-// The tiles of one head's value channels from the chunk's scores, the queries and the state in front of it; the first tile of
-// the state is on its way, and everything else becomes visible with the first barrier.  pre: the decays from the chunk's start,
-// null where the queries carry them; gain null: none.
-template <typename TA, int PQ, int PV>
-__device__ __forceinline__ void value_tiles(bf16* sm, const float* pre, const float* gain, const Chunk& c, const bf16* cuts, const TA* v,
-                                            int v_stride, float q_scale, float* out, int out_stride, int dv, int first, int last) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wm = warp >> 1, wn = warp & 1, g = lane >> 2, t4 = lane & 3;
-    const bf16 *qs = sm + OutLayout::q, *as = sm + OutLayout::a;
-    bf16* st = sm + OutLayout::s;
-    for (int c0 = first; c0 < last; c0 += OT) {
-        // values of this lane's columns at the tokens of its fragments, up to its quarter: a step's are 2t, 2t + 1, 2t + 8, 2t + 9
-        float vx[QUARTERS][2][4];
+// The values of a warp's 16 channels as fragments of a quarter of the tokens.  A value that is no number is left out and its
+// token noted: `bad` is the first such token of the columns lane / 4 and lane / 4 + 8.
+struct StagedValues {                                        // bf16, in shared memory
+    const bf16* at;                                          // [CK][VP] at the warp's first channel
+    __device__ __forceinline__ void take(int quarter, uint32_t (&b)[1][1][4], int (&bad)[2]) {
+        const int lane = threadIdx.x & 31;
+        ldsm_t(b[0][0], at + quarter * 16 * VP + at_bt(lane, VP));
 #pragma unroll
-        for (int m = 0; m < QUARTERS; ++m)
-            if (m <= wm) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int t = m * 16 + 2 * t4 + (e & 1) + (e >> 1) * 8;
-                    const TA* p = v + (size_t)(c.t0 + t) * v_stride + c0 + wn * 16 + g;
-#pragma unroll
-                    for (int n = 0; n < 2; ++n) vx[m][n][e] = t < c.n ? to_f32<TA>(p[n * 8]) : 0.f;
-                }
-            }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();
-        float o[1][2][4] = {};
-#pragma unroll
-        for (int k0 = 0; k0 < DK; k0 += 16) {                // from the state in front of the chunk
-            uint32_t fa[PQ][1][4], fb[3][1][4];
-#pragma unroll
-            for (int p = 0; p < PQ; ++p) ldsm(fa[p][0], qs + p * CK * KP + wm * 16 * KP + k0 + at_a(lane, KP));
-#pragma unroll
-            for (int p = 0; p < 3; ++p) ldsm(fb[p][0], st + p * OT * KP + wn * 16 * KP + k0 + at_b(lane, KP));
-            products<1, 1, PQ, 3>(o, fa, fb);
+        for (int r = 3; r >= 0; --r) {
+            const int t = quarter * 16 + 2 * (lane & 3) + (r & 1) * 8;
+            if ((b[0][0][r] & 0x7f800000u) == 0x7f800000u) { bad[r >> 1] = min(bad[r >> 1], t + 1); b[0][0][r] &= 0xffffu; }
+            if ((b[0][0][r] & 0x7f80u) == 0x7f80u) { bad[r >> 1] = min(bad[r >> 1], t); b[0][0][r] &= 0xffff0000u; }
         }
-        __syncthreads();                                     // the state's tile is read
-        if (c0 + OT < last) fetch_state(st, cuts, c0 + OT, dv);
-        if (pre) {
-            const float p0 = pre[wm * 16 + g], p1 = pre[wm * 16 + g + 8];
+    }
+};
+struct GainedValues {                                        // three pieces in shared memory, 64 channels a row, 16 bytes at i ^ row % 8
+    const bf16* at;
+    int col;                                                 // the warp's first channel
+    const int* noted;                                        // [64] the first such token of every channel
+    __device__ __forceinline__ void take(int quarter, uint32_t (&b)[3][1][4], int (&bad)[2]) {
+        const int lane = threadIdx.x & 31, t = quarter * 16 + (lane & 15);
 #pragma unroll
-            for (int n = 0; n < 2; ++n) { o[0][n][0] *= p0; o[0][n][1] *= p0; o[0][n][2] *= p1; o[0][n][3] *= p1; }
+        for (int p = 0; p < 3; ++p) ldsm_t(b[p][0], at + p * CK * 64 + t * 64 + (((col >> 3) + (lane >> 4)) ^ (t & 7)) * 8);
+        bad[0] = noted[col + (lane >> 2)];
+        bad[1] = noted[col + (lane >> 2) + 8];
+    }
+};
+
+// The outputs of a warp's 16 value channels, tokens 16 first .. 16 (first + MH) - 1: pre: the decays from the chunk's start, null
+// where the queries carry them; cuts: the channels' blocks of the state in front of the chunk, pieces dv * DK apart; out: the
+// channels of the chunk's first token.
+template <int PQ, int PV, int MH, typename Values>
+__device__ __forceinline__ void value_columns(const bf16* qs, const bf16* as, const float* pre, int tokens, int first, const bf16* cuts,
+                                              size_t one, Values& values, float q_scale, float* out, int out_stride) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    float o[MH][1][2][4] = {};
+    uint4 next[3];
+#pragma unroll
+    for (int p = 0; p < 3; ++p) next[p] = *reinterpret_cast<const uint4*>(cuts + p * one + lane * 8);
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {                           // from the state in front of the chunk
+        uint32_t fb[3][1][4];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            fb[p][0][0] = next[p].x; fb[p][0][1] = next[p].y; fb[p][0][2] = next[p].z; fb[p][0][3] = next[p].w;
+            if (k + 1 < KS) next[p] = *reinterpret_cast<const uint4*>(cuts + p * one + (k + 1) * 256 + lane * 8);
         }
-        int bad[2] = {CK, CK};                               // first token whose value in the lane's column is no number
 #pragma unroll
-        for (int m = 0; m < QUARTERS; ++m)
-            if (m <= wm) {                                   // from the chunk's own tokens up to this quarter
-                uint32_t fa[3][1][4], fb[PV][1][4];
+        for (int m = 0; m < MH; ++m) {
+            uint32_t fa[PQ][1][4];
 #pragma unroll
-                for (int p = 0; p < 3; ++p) ldsm(fa[p][0], as + p * CK * AP + wm * 16 * AP + m * 16 + at_a(lane, AP));
-                float gx[4] = {1.f, 1.f, 1.f, 1.f};
-                if (gain) {
+            for (int p = 0; p < PQ; ++p) ldsm(fa[p][0], qs + p * CK * KP + (first + m) * 16 * KP + k * 16 + at_a(lane, KP));
+            products<1, 1, PQ, 3>(o[m], fa, fb);
+        }
+    }
+    if (pre) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) gx[e] = gain[m * 16 + 2 * t4 + (e & 1) + (e >> 1) * 8];
-                }
+        for (int m = 0; m < MH; ++m) {
+            const float p0 = pre[(first + m) * 16 + g], p1 = pre[(first + m) * 16 + g + 8];
 #pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    float x[4];
+            for (int n = 0; n < 2; ++n) { o[m][0][n][0] *= p0; o[m][0][n][1] *= p0; o[m][0][n][2] *= p1; o[m][0][n][3] *= p1; }
+        }
+    }
+    int bad[2] = {CK, CK};
 #pragma unroll
-                    for (int e = 3; e >= 0; --e) {
-                        x[e] = gain ? vx[m][n][e] * gx[e] : vx[m][n][e];
-                        if (!(fabsf(x[e]) <= 3.402823466e38f)) { bad[n] = min(bad[n], m * 16 + 2 * t4 + (e & 1) + (e >> 1) * 8); x[e] = 0.f; }
-                    }
+    for (int k = 0; k < QUARTERS; ++k) {                     // from the chunk's own tokens
+        if (k >= first + MH) continue;
+        uint32_t fb[PV][1][4];
+        values.take(k, fb, bad);
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        if constexpr (PV == 1) {
-                            fb[0][0][2 * n + half] = pair_bf16(x[2 * half], x[2 * half + 1]);
-                        } else {
-                            uint32_t p[3];
-                            cut(x[2 * half], x[2 * half + 1], p);
+        for (int m = 0; m < MH; ++m) {
+            if (first + m < k) continue;
+            uint32_t fa[3][1][4];
 #pragma unroll
-                            for (int i = 0; i < 3; ++i) fb[i][0][2 * n + half] = p[i];
-                        }
-                    }
-                }
-                products<1, 1, 3, PV>(o, fa, fb);
-            }
-        const bool any_bad = __any_sync(0xffffffffu, min(bad[0], bad[1]) < CK);
+            for (int p = 0; p < 3; ++p) ldsm(fa[p][0], as + p * CK * AP + (first + m) * 16 * AP + k * 16 + at_a(lane, AP));
+            products<1, 1, 3, PV>(o[m], fa, fb);
+        }
+    }
+    const bool any_bad = __any_sync(0xffffffffu, min(bad[0], bad[1]) < CK);
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int col = wn * 16 + n * 8 + t4 * 2;
-            if (any_bad) {                                   // later outputs of such a column are NaN
-                int b = min(bad[n], __shfl_xor_sync(0xffffffffu, bad[n], 1));
-                b = min(b, __shfl_xor_sync(0xffffffffu, b, 2));
-                const int b0 = __shfl_sync(0xffffffffu, b, 8 * t4), b1 = __shfl_sync(0xffffffffu, b, 8 * t4 + 4);
+    for (int n = 0; n < 2; ++n) {
+        int b0 = CK, b1 = CK;
+        if (any_bad) {                                       // later outputs of such a column are NaN
+            int b = min(bad[n], __shfl_xor_sync(0xffffffffu, bad[n], 1));
+            b = min(b, __shfl_xor_sync(0xffffffffu, b, 2));
+            b0 = __shfl_sync(0xffffffffu, b, 8 * t4);
+            b1 = __shfl_sync(0xffffffffu, b, 8 * t4 + 4);
+        }
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    if (wm * 16 + g + 8 * r >= b0) o[0][n][2 * r] = __int_as_float(0x7fc00000);
-                    if (wm * 16 + g + 8 * r >= b1) o[0][n][2 * r + 1] = __int_as_float(0x7fc00000);
-                }
-            }
+        for (int m = 0; m < MH; ++m)
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-                const int t = wm * 16 + g + 8 * r;
-                if (t < c.n)
-                    *reinterpret_cast<float2*>(out + (size_t)(c.t0 + t) * out_stride + c0 + col) =
-                        make_float2(o[0][n][2 * r] * q_scale, o[0][n][2 * r + 1] * q_scale);
+                const int t = (first + m) * 16 + g + 8 * r;
+                if (t < tokens)
+                    *reinterpret_cast<float2*>(out + (size_t)t * out_stride + n * 8 + t4 * 2) =
+                        make_float2(t >= b0 ? __int_as_float(0x7fc00000) : o[m][0][n][2 * r] * q_scale,
+                                    t >= b1 ? __int_as_float(0x7fc00000) : o[m][0][n][2 * r + 1] * q_scale);
             }
-        }
     }
 }
 
@@ -531,6 +544,8 @@ head_chunk_outputs_kernel(const TA* __restrict__ q, int q_stride, const TA* __re
     float *pre = a + CK, *pre_in = pre + CK, *suf_in = pre_in + CK;      // from the chunk's start; inside a quarter: from its start, to its end
     float* gains = suf_in + CK;
     float* dq = gains + CK;                                  // [4][16][16] decays inside a quarter
+    int* noted = reinterpret_cast<int*>(dq + QUARTERS * 256);            // [64]
+    bf16* vs = sm + OutLayout::v;
     pdl_trigger();
     pdl_wait();
     const Chunk c = find_chunk(cu_q, entries, least, blockIdx.x);
@@ -582,10 +597,35 @@ head_chunk_outputs_kernel(const TA* __restrict__ q, int q_stride, const TA* __re
     for (int hh = 0; hh < heads; ++hh) {
         const int h = h0 + hh;
         const bf16* from = cuts + ((size_t)blockIdx.x * H + h) * 3 * dv * DK;
-        if (tid < CK) { a[tid] = tid < c.n ? next_a : 1.f; }
+        const TA* own = v + (size_t)c.t0 * v_stride + (size_t)h * dv;
+        constexpr int VN = CK * 64 / 4 / OUT_THREADS;        // 64 channels' values: fours a thread
+        float4 x[VN];
+        auto ask_values = [&](int c0) {
+#pragma unroll
+            for (int j = 0; j < VN; ++j) {
+                const int e = tid + j * OUT_THREADS, t = e >> 4;
+                x[j] = t < c.n ? load4(own + (size_t)t * v_stride + c0 + (e & 15) * 4) : zero4();
+            }
+        };
+        auto put_values = [&]() {
+#pragma unroll
+            for (int j = 0; j < VN; ++j) {
+                const int e = tid + j * OUT_THREADS, t = e >> 4, i = (e & 15) * 4;
+                float4 y = gain ? times(x[j], gains[t]) : x[j];
+                const float most = 3.402823466e38f;
+                if (!(fabsf(y.x) <= most) || !(fabsf(y.y) <= most) || !(fabsf(y.z) <= most) || !(fabsf(y.w) <= most)) {
+                    if (!(fabsf(y.x) <= most)) { atomicMin(noted + i, t); y.x = 0.f; }
+                    if (!(fabsf(y.y) <= most)) { atomicMin(noted + i + 1, t); y.y = 0.f; }
+                    if (!(fabsf(y.z) <= most)) { atomicMin(noted + i + 2, t); y.z = 0.f; }
+                    if (!(fabsf(y.w) <= most)) { atomicMin(noted + i + 3, t); y.w = 0.f; }
+                }
+                put4<3>(vs + t * 64 + (((i >> 3) ^ (t & 7)) << 3) + (i & 7), CK * 64, y);
+            }
+        };
+        ask_values(0);
+        if (tid < CK) a[tid] = tid < c.n ? next_a : 1.f;
         __syncthreads();                                     // the last head's (or the keys') readers are done, the decays are there
-        fetch_state(sm + OutLayout::s, from, 0, dv);
-        if (tid < CK) gains[tid] = next_g;
+        if (tid < CK) { gains[tid] = next_g; noted[tid] = CK; }
         if (hh + 1 < heads) ask(h + 1);
         if (warp == 7) chunk_products(a, pre, nullptr);
         if (warp >= 2 && warp < 4) {                         // 64 threads: the column of key j inside its quarter
@@ -634,7 +674,19 @@ head_chunk_outputs_kernel(const TA* __restrict__ q, int q_stride, const TA* __re
                 }
             }
         }
-        value_tiles<TA, PQ, 3>(sm, pre, gain ? gains : nullptr, c, from, v + (size_t)h * dv, v_stride, q_scale, out + (size_t)h * dv, H * dv, dv, 0, dv);
+        for (int c0 = 0; c0 < dv; c0 += 64) {
+            if (c0 > 0) {
+                __syncthreads();                             // the last channels' values are read
+                if (tid < 64) noted[tid] = CK;
+                __syncthreads();
+            }
+            put_values();
+            if (c0 + 64 < dv) ask_values(c0 + 64);
+            __syncthreads();
+            GainedValues values{vs, (warp & 3) * 16, noted};
+            value_columns<PQ, 3, 2>(qs, as, pre, c.n, warp / 4 * 2, from + (c0 / 16 + (warp & 3)) * KS * 256, (size_t)dv * DK, values, q_scale,
+                                    out + (size_t)c.t0 * H * dv + (size_t)h * dv + c0 + (warp & 3) * 16, H * dv);
+        }
     }
 }
 
@@ -822,18 +874,20 @@ gated_chunk_scores_kernel(const bf16* __restrict__ q, int q_stride, const bf16* 
         *reinterpret_cast<uint4*>(to + e * 8) = *reinterpret_cast<const uint4*>(qs + (e / (DK / 8)) * KP + (e % (DK / 8)) * 8);
 }
 
-// dv / gridDim.z value channels of one chunk and head
+// OUT_V (MH 4) or all (MH 2) value channels of one chunk and head
+template <int MH>
 __global__ void __launch_bounds__(OUT_THREADS, 2)
 gated_chunk_outputs_kernel(const bf16* __restrict__ parts, const bf16* __restrict__ v, int v_stride, float q_scale,
                            const bf16* __restrict__ cuts, float* __restrict__ out, const int* __restrict__ cu_q, int entries,
                            int least, int H, int dv) {
     extern __shared__ __align__(16) unsigned char raw[];
     bf16* sm = reinterpret_cast<bf16*>(raw);
+    constexpr int COLS = 64 * (MH / 2);                      // value channels at a time
     pdl_trigger();
     pdl_wait();
     const Chunk c = find_chunk(cu_q, entries, least, blockIdx.x);
     if (c.entry < 0) return;
-    const int h = blockIdx.y, first = (int)blockIdx.z * (dv / (int)gridDim.z), last = first + dv / (int)gridDim.z;
+    const int h = blockIdx.y, warp = threadIdx.x >> 5, col = warp % (COLS / 16) * 16;
     const bf16* from = cuts + ((size_t)blockIdx.x * H + h) * 3 * dv * DK;
     const bf16* own = parts + ((size_t)blockIdx.x * H + h) * GATED_PARTS;
     for (int e = threadIdx.x; e < 3 * CK * CK / 8; e += OUT_THREADS)
@@ -841,8 +895,27 @@ gated_chunk_outputs_kernel(const bf16* __restrict__ parts, const bf16* __restric
     own += 3 * CK * CK;
     for (int e = threadIdx.x; e < 3 * CK * DK / 8; e += OUT_THREADS)
         cp16(sm + OutLayout::q + (e / (DK / 8)) * KP + (e % (DK / 8)) * 8, own + e * 8);
-    fetch_state(sm + OutLayout::s, from, first, dv);
-    value_tiles<bf16, 3, 1>(sm, nullptr, nullptr, c, from, v + (size_t)h * dv, v_stride, q_scale, out + (size_t)h * dv, H * dv, dv, first, last);
+    bf16* vs = sm + OutLayout::v;
+    for (int c0 = blockIdx.z * COLS; c0 < dv; c0 += gridDim.z * COLS) {
+        const bf16* src = v + (size_t)c.t0 * v_stride + (size_t)h * dv + c0;
+        uint2 x[CK * COLS / 4 / OUT_THREADS];
+#pragma unroll
+        for (int j = 0; j < CK * COLS / 4 / OUT_THREADS; ++j) {
+            const int e = threadIdx.x + j * OUT_THREADS, t = e / (COLS / 4), i = (e % (COLS / 4)) * 4;
+            x[j] = t < c.n ? *reinterpret_cast<const uint2*>(src + (size_t)t * v_stride + i) : make_uint2(0u, 0u);
+        }
+        if (c0 != (int)blockIdx.z * COLS) __syncthreads();   // the last channels' values are read
+#pragma unroll
+        for (int j = 0; j < CK * COLS / 4 / OUT_THREADS; ++j) {
+            const int e = threadIdx.x + j * OUT_THREADS, t = e / (COLS / 4), i = (e % (COLS / 4)) * 4;
+            *reinterpret_cast<uint2*>(vs + t * VP + i) = x[j];
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+        StagedValues values{vs + col};
+        value_columns<3, 1, MH>(sm + OutLayout::q, sm + OutLayout::a, nullptr, c.n, MH == 4 ? 0 : warp / 4 * 2, from + (c0 + col) / 16 * KS * 256,
+                                (size_t)dv * DK, values, q_scale, out + (size_t)c.t0 * H * dv + (size_t)h * dv + c0 + col, H * dv);
+    }
 }
 
 inline bool aligned4(const void* p, int esize) { return (reinterpret_cast<uintptr_t>(p) % (4 * (size_t)esize)) == 0; }
@@ -866,10 +939,18 @@ RI_API int ri_head_chunks(const void* q, int q_stride, const void* k, int k_stri
     if (entries <= 0 || chunks <= 0) return 0;
     if (share <= 0 || H % share || !ri_chunks_ok(q, q_stride, k, k_stride, v, v_stride, act_dtype, dv, 0)) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
-    // heads a CTA of the outputs serves: their scores' products are shared; fewer where the CTAs would not fill the SMs twice
-    int heads = share;
-    while (heads % 2 == 0 && (long long)chunks * (H / heads) < 4LL * ri_device_sms()) heads /= 2;
-    const int scan_blocks = (int)(((size_t)H * dv * DK / 4 + 255) / 256);
+    // heads a CTA of the outputs serves: the scores of a key head, as much work as a head's 64 channels, are made once a CTA, and
+    // CTAs go in waves of two an SM.  The layer over 2,048 tokens, heads a CTA 1, 2, 4, 8: 32 heads of 64 in 4 key heads 245, 236, 234,
+    // 277 us (the rule takes 4), 64 in 8 key heads 419, 411, 404, 403 (8).
+    int heads = 1;
+    double best = 0;
+    for (int n = 1; n <= share; ++n) {
+        if (share % n) continue;
+        const long long waves = ((long long)chunks * (H / n) + 2 * ri_device_sms() - 1) / (2 * ri_device_sms());
+        const double cost = (double)waves * (64 + (double)n * dv);
+        if (n == 1 || cost < best) { best = cost; heads = n; }
+    }
+    const int scan_blocks = (int)(((size_t)H * dv * DK / 8 + SCAN_THREADS - 1) / SCAN_THREADS);
 #define RI_STATES(TA, VT) do { \
     static bool allowed = false; \
     if (!allowed) { RI_CHECKED(allow(chunk_states_kernel<TA, VT, false>, states_bytes<TA, VT, false>())); allowed = true; } \
@@ -880,7 +961,7 @@ RI_API int ri_head_chunks(const void* q, int q_stride, const void* k, int k_stri
     static bool allowed = false; \
     if (!allowed) { RI_CHECKED(allow(head_chunk_outputs_kernel<TA>, OutLayout::bytes)); allowed = true; } \
     if (dv % 128 == 0 || (dv == 64 && share % 2 == 0)) RI_STATES(TA, 128); else RI_STATES(TA, 64); \
-    RI_CHECKED(ri_launch(chunk_scan_kernel<false>, dim3(scan_blocks, entries), dim3(256), 0, s, states, totals, (bf16*)cuts, state, cu_q, \
+    RI_CHECKED(ri_launch(chunk_scan_kernel<false>, dim3(scan_blocks, entries), dim3(SCAN_THREADS), 0, s, states, totals, (bf16*)cuts, state, cu_q, \
         state_slots, least, H, dv)); \
     RI_CHECKED(ri_launch(head_chunk_outputs_kernel<TA>, dim3(chunks, H / heads), dim3(OUT_THREADS), OutLayout::bytes, s, (const TA*)q, q_stride, \
         (const TA*)k, k_stride, (const TA*)v, v_stride, decay, a_stride, gain, g_stride, q_scale, (const bf16*)cuts, out, cu_q, entries, least, \
@@ -902,11 +983,12 @@ RI_API int ri_gated_chunks(const void* q, int q_stride, const void* k, int k_str
     if (entries <= 0 || chunks <= 0) return 0;
     if (!ri_chunks_ok(q, q_stride, k, k_stride, v, v_stride, act_dtype, dv, 1)) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
-    const int scan_blocks = (int)(((size_t)H * dv * DK / 4 + 255) / 256);
+    const int scan_blocks = (int)(((size_t)H * dv * DK / 8 + SCAN_THREADS - 1) / SCAN_THREADS);
     static bool allowed = false;
     if (!allowed) {
         RI_CHECKED(allow(gated_chunk_scores_kernel, ScoreLayout::bytes));
-        RI_CHECKED(allow(gated_chunk_outputs_kernel, OutLayout::bytes));
+        RI_CHECKED(allow(gated_chunk_outputs_kernel<4>, OutLayout::gated_bytes));
+        RI_CHECKED(allow(gated_chunk_outputs_kernel<2>, OutLayout::gated_bytes));
         RI_CHECKED(allow(chunk_states_kernel<bf16, 128, true>, states_bytes<bf16, 128, true>()));
         RI_CHECKED(allow(chunk_states_kernel<bf16, 64, true>, states_bytes<bf16, 64, true>()));
         allowed = true;
@@ -917,11 +999,11 @@ RI_API int ri_gated_chunks(const void* q, int q_stride, const void* k, int k_str
     if (dv % 128 == 0) RI_STATES(128);
     else RI_STATES(64);
 #undef RI_STATES
-    RI_CHECKED(ri_launch(chunk_scan_kernel<true>, dim3(scan_blocks, entries), dim3(256), 0, s, states, totals, (bf16*)cuts, state, cu_q, state_slots,
+    RI_CHECKED(ri_launch(chunk_scan_kernel<true>, dim3(scan_blocks, entries), dim3(SCAN_THREADS), 0, s, states, totals, (bf16*)cuts, state, cu_q, state_slots,
                          least, H, dv));
     RI_CHECKED(ri_launch(gated_chunk_scores_kernel, dim3(chunks, H), dim3(OUT_THREADS), ScoreLayout::bytes, s, (const bf16*)q, q_stride,
                          (const bf16*)k, k_stride, alpha, a_stride, (bf16*)parts, cu_q, entries, least, H));
-    RI_CHECKED(ri_launch(gated_chunk_outputs_kernel, dim3(chunks, H, dv % 128 == 0 ? dv / 128 : 1), dim3(OUT_THREADS), OutLayout::bytes, s,
+    RI_CHECKED(ri_launch(dv % OUT_V == 0 ? gated_chunk_outputs_kernel<4> : gated_chunk_outputs_kernel<2>, dim3(chunks, H, dv % OUT_V == 0 ? dv / OUT_V : 1), dim3(OUT_THREADS), OutLayout::gated_bytes, s,
                          (const bf16*)parts, (const bf16*)v, v_stride, q_scale, (const bf16*)cuts, out, cu_q, entries, least, H, dv));
     return ri_launch_status();
 }
