@@ -440,7 +440,7 @@ delta_scan_kernel(const TA* __restrict__ r, int r_stride, const TA* __restrict__
                   const TA* __restrict__ v, int v_stride, const float* __restrict__ w, const float* __restrict__ u,
                   const float* __restrict__ au, int f_stride, float* __restrict__ out,
                   float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
-                  int H, int dv, int vec) {
+                  int H, int dv, int vec, int below) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -451,6 +451,7 @@ delta_scan_kernel(const TA* __restrict__ r, int r_stride, const TA* __restrict__
     const int lt = tid - WORKERS;
     const int cg = tid / R, rg = tid % R;
     const int t_begin = cu_q[b], t_end = cu_q[b + 1];
+    if (below > 0 && t_end - t_begin >= below) return;       // this entry goes in chunks
     const int rounds = (t_end - t_begin + TC - 1) / TC;
     if (DKP != DK) {
         for (int e = tid; e < 2 * HALF; e += THREADS) smem[e] = 0.f;
@@ -1191,7 +1192,7 @@ RI_API int ri_gated_scan(const void* q, int q_stride, const void* k, int k_strid
 RI_API int ri_delta_scan(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride,
                          const float* w, const float* u, const float* au, int f_stride, int act_dtype,
                          float* out, float* state, const int* cu_q, const int* state_slots, int entries, int H,
-                         int dv, int single, void* stream) {
+                         int dv, int single, int below, void* stream) {
     if (entries <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const dim3 grid((dv + COLS - 1) / COLS, H, entries);
@@ -1208,7 +1209,7 @@ RI_API int ri_delta_scan(const void* r, int r_stride, const void* k, int k_strid
     static bool allowed = false; \
     if (!allowed) { RI_CHECKED(allow_shared(delta_scan_kernel<TA>, smem)); allowed = true; } \
     RI_CHECKED(ri_launch(delta_scan_kernel<TA>, grid, dim3(THREADS), smem, s, (const TA*)r, r_stride, \
-        (const TA*)k, k_stride, (const TA*)v, v_stride, w, u, au, f_stride, out, state, cu_q, state_slots, H, dv, vec)); \
+        (const TA*)k, k_stride, (const TA*)v, v_stride, w, u, au, f_stride, out, state, cu_q, state_slots, H, dv, vec, below)); \
     } while (0)
     if (act_dtype == RI_BF16) RI_DS(bf16);
     else RI_DS(float);

@@ -3,6 +3,7 @@
 //
 //   head    S_t = a_t S_{t-1} + k_t (g_t v_t)^T         o_t = S_t^T q_t      a, g one number a head
 //   gated   S_t = diag(alpha_t) S_{t-1} + k_t v_t^T     o_t = S_t^T q_t
+//   delta   further down
 //
 // The walk of recurrent.cu takes a prompt token by token: one request offers heads x value channels of columns, and every
 // column's state waits for the last token's.  With D_ij the product of the decays of the tokens j + 1 .. i, a chunk that starts
@@ -413,7 +414,7 @@ chunk_scan_kernel(const float* __restrict__ states, const float* __restrict__ to
 // The outputs of one chunk for `heads` heads of one key head, two CTAs an SM.  A warp owns a block of 16 value channels for MH
 // quarters of the tokens and works for itself: queries, scores and values, cut up, come from shared memory, the state's pieces
 // straight from memory in the order of the fragments, a step ahead, so that no tile of the state is waited for.
-constexpr int OUT_THREADS = 256, OUT_WARPS = OUT_THREADS / 32;
+constexpr int OUT_THREADS = 256;
 constexpr int AP = CK + 8;
 constexpr int OUT_V = 128, VP = OUT_V + 8;      // value channels of a CTA of the gated form
 struct OutLayout {                              // offsets in bf16, then floats
@@ -426,6 +427,10 @@ struct OutLayout {                              // offsets in bf16, then floats
 
 __device__ __forceinline__ void cp16(bf16* smem, const bf16* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+
+__device__ __forceinline__ void cp8(bf16* smem, const bf16* gmem, bool there) {      // not there: zeros
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem), "r"(there ? 8 : 0));
 }
 
 // The values of a warp's 16 channels as fragments of a quarter of the tokens.  A value that is no number is left out and its
@@ -918,6 +923,703 @@ gated_chunk_outputs_kernel(const bf16* __restrict__ parts, const bf16* __restric
     }
 }
 
+// ------------------------------------------------------------------------------------------------- the delta rule
+// delta   S_t = diag(w_t) S_{t-1} - au_t (u_t^T S_{t-1}) + k_t v_t^T      o_t = S_t^T r_t
+//
+// With d_t = u_t^T S_{t-1} a chunk is the gated form over keys k and values v less keys au and values d, and the d are a
+// triangular system: (I + A) d = U S + B V, A_ij = u_i^T D_{i-1,j} au_j and B_ij = u_i^T D_{i-1,j} k_j for j < i.  With T = (I + A)^-1
+// and P, Q the scores of r against k and au,
+//
+//   d = X S + Y V                     X = T U D, Y = T B
+//   O = (R D - Q T U D) S + (P - Q Y) V                          as the gated form's outputs: queries R', scores P'
+//   S' = D S - (AU D)^T X S + (K D - (AU D)^T Y)^T V
+//
+// so one kernel makes X, R', P' and each chunk's own contribution for all chunks at once (`delta_chunk_parts`), the scan over the
+// chunks takes two products a chunk, d = X S and AU^T d (`delta_chunk_scan`), and the outputs are the gated form's.
+//
+// The decays part at the chunk's middle: a row carries the product from there to its token, a key the product from its token to
+// there, on the other side of the middle the reciprocal.  A term of a score is then a product of two rounded numbers whatever
+// their sizes; the host sends only decays here whose products over half a chunk stay far from the ends of fp32 (DELTA_MOST_DECAY).
+// (The gated form's decays have no such bound, so its scores part at every quarter and multiply their way inside one.)
+//
+// 2,444 tokens in four entries, 16 heads of 128 x 128: parts 140 us, scan 80, outputs 47, where the walk takes 395; one entry of 2,048
+// tokens and 8 heads 166 us with what prepares it, the walk 678.  The parts are bound by what a CTA's phases wait for (products of a
+// few blocks, the inverse: tensor cores 30 % busy, 11 cycles an instruction and warp), the scan by its products (half of the tensor
+// cores' rate, one chunk after the other).  Tried: the parts' next channels asked for ahead (registers; 2 % slower).
+constexpr float DELTA_MOST_DECAY = 1.0f;        // of -log w: factors of a middle lie between e^-32 and e^32
+constexpr int DP_THREADS = 256;
+constexpr int SC = 32, SP = SC + 8;             // channels staged at a time
+constexpr int LOWER = 10;                       // 16 x 16 blocks on and under the diagonal of a chunk
+struct PartsLayout {                            // bytes
+    static constexpr int PF = DK + 4, AF = CK + 4;
+    static constexpr int decay = 0, ends = decay + CK * PF * 4, noted = ends + 2 * DK * 4, work = noted + 128;
+    static constexpr int stage = work, exch = stage + 4 * 3 * CK * SP * 2, one_end = exch + 16 * SC * 8;
+    static constexpr int BLOCKS = LOWER * 3 * 256 * 2;       // three pieces
+    static constexpr int a = work, t = a + CK * AF * 4, b = t + BLOCKS, q = b + BLOCKS, p = q + BLOCKS, two_end = p + LOWER * 256 * 4;
+    static constexpr int y = a, w = b, v = q;                // later tenants
+    static constexpr int bytes = two_end > one_end ? two_end : one_end;
+    static_assert(BLOCKS <= CK * AF * 4 && v + CK * VP * 2 <= bytes, "later tenants fit");
+};
+__device__ __forceinline__ int lower_block(int i, int j) { return i * (i + 1) / 2 + j; }
+// A block's row of 16 is two pieces of 16 bytes that change places every fourth row: ldmatrix meets no conflict.
+__device__ __forceinline__ const bf16* lane_row(const bf16* block, int lane) {
+    const int row = lane & 15;
+    return block + row * 16 + (((lane >> 4) ^ (row >> 2 & 1)) << 3);
+}
+// one block's accumulators into three pieces at `to`
+__device__ __forceinline__ void put_block(bf16* to, const float (&d)[2][4], int lane) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int row = (lane >> 2) + 8 * r;
+            uint32_t x[3];
+            cut(d[n][2 * r], d[n][2 * r + 1], x);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(to + p * 256 + row * 16 + ((n ^ (row >> 2 & 1)) << 3) + (lane & 3) * 2) = x[p];
+        }
+}
+// d += sum over k = j .. i of left(i, k) right(k, j), blocks on and under the diagonal
+__device__ __forceinline__ void block_product(float (&d)[1][2][4], const bf16* left, const bf16* right, int i, int j, int lane) {
+    for (int k = j; k <= i; ++k) {
+        uint32_t fa[3][1][4], fb[3][1][4];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            ldsm(fa[p][0], lane_row(left + (lower_block(i, k) * 3 + p) * 256, lane));
+            ldsm_t(fb[p][0], lane_row(right + (lower_block(k, j) * 3 + p) * 256, lane));
+        }
+        products<1, 1, 3, 3>(d, fa, fb);
+    }
+}
+// a warp's blocks, so that the longest sums (i - j + 1 products) are shared out: at most two
+__device__ __forceinline__ int warp_blocks(int warp, int which) {        // i * 4 + j, -1: none
+    constexpr int first[8] = {12, 8, 13, 4, 9, 14, 15, -1}, second[8] = {-1, -1, -1, 0, 5, 10, -1, -1};
+    return which ? second[warp] : first[warp];
+}
+// 1 / x for x between 2^-60 and 2^60: the special-function unit's and one step of Newton's method, to the last place but one
+__device__ __forceinline__ float reciprocal(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(y, fmaf(-x, y, 1.f), y);
+}
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
+// One chunk and head.  Outputs, all in the order of fragments ([piece][token block][key block][lane][8] for xs and au): xs: X; au: the
+// au with their factor to the middle; ends: the decays' products from the middle to the chunk's end and over the whole chunk;
+// parts: P' and R' as the gated form's; states: the chunk's own contribution.  From the first token on whose k, u, au or w is no number
+// the chunk counts no tokens, and its outputs there and the state behind it are NaN.
+__global__ void __launch_bounds__(DP_THREADS, 2)
+delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* __restrict__ k, int k_stride, const bf16* __restrict__ v, int v_stride,
+                         const float* __restrict__ w, const float* __restrict__ u, const float* __restrict__ au, int f_stride,
+                         bf16* xs, bf16* aus, float* __restrict__ ends, bf16* __restrict__ parts, float* __restrict__ states,
+                         const int* __restrict__ cu_q, int entries, int least, int H, int dv) {
+    using L = PartsLayout;
+    extern __shared__ __align__(16) unsigned char raw[];
+    float* ps = reinterpret_cast<float*>(raw + L::decay);                // [CK][PF]: t < 32: w_{t+1} .. w_31, else w_32 .. w_t
+    float* mid = reinterpret_cast<float*>(raw + L::ends);                // [2][DK]: w_0 .. w_31, w_32 .. w_63
+    int* noted = reinterpret_cast<int*>(raw + L::noted);
+    bf16* stage = reinterpret_cast<bf16*>(raw + L::stage);               // u, r, k, au: [4][3][CK][SP]
+    double* exch = reinterpret_cast<double*>(raw + L::exch);             // [16][SC]
+    float* as = reinterpret_cast<float*>(raw + L::a);                    // [CK][AF]
+    bf16 *ts = reinterpret_cast<bf16*>(raw + L::t), *bs = reinterpret_cast<bf16*>(raw + L::b), *qs = reinterpret_cast<bf16*>(raw + L::q);
+    bf16 *ys = reinterpret_cast<bf16*>(raw + L::y), *ws = reinterpret_cast<bf16*>(raw + L::w), *vs = reinterpret_cast<bf16*>(raw + L::v);
+    float* pf = reinterpret_cast<float*>(raw + L::p);                    // [LOWER][lane][8]
+    pdl_trigger();
+    pdl_wait();
+    const Chunk c = find_chunk(cu_q, entries, least, blockIdx.x);
+    if (c.entry < 0) return;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    const size_t unit = (size_t)blockIdx.x * H + h;
+    xs += unit * 3 * CK * DK;
+    aus += unit * 3 * CK * DK;
+    parts += unit * GATED_PARTS;
+    // ---- scores: rows u and r against k and au.  A warp takes one of each and two rows of blocks, 3 and 0 or 2 and 1.
+    const int rows_of = warp & 1, cols_of = warp >> 1 & 1, long_row = warp < 4 ? 3 : 2, short_row = 3 - long_row;
+    float sl[4][1][2][4], ss[2][1][2][4];
+    if (tid == 0) *noted = CK;
+    __syncthreads();
+    int tokens = c.n;
+    for (bool again = true; again;) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    sl[j][0][n][e] = 0.f;
+                    if (j < 2) ss[j][0][n][e] = 0.f;
+                }
+#pragma unroll 1
+        for (int q0 = 0; q0 < DK; q0 += SC) {
+            const int pair = tid & 15, seg = tid >> 4, ch = q0 + 2 * pair;           // two channels, four tokens a thread
+            float2 ww[4], uu[4], aa[4];
+            uint32_t rr[4], kk[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int t = seg * 4 + i;
+                const size_t at = (size_t)(c.t0 + t), col = (size_t)h * DK + ch;
+                const bool in = t < tokens;
+                ww[i] = in ? *reinterpret_cast<const float2*>(w + at * f_stride + col) : make_float2(1.f, 1.f);
+                uu[i] = in ? *reinterpret_cast<const float2*>(u + at * f_stride + col) : make_float2(0.f, 0.f);
+                aa[i] = in ? *reinterpret_cast<const float2*>(au + at * f_stride + col) : make_float2(0.f, 0.f);
+                rr[i] = in ? *reinterpret_cast<const uint32_t*>(r + at * r_stride + col) : 0u;
+                kk[i] = in ? *reinterpret_cast<const uint32_t*>(k + at * k_stride + col) : 0u;
+            }
+            double px = 1.0, py = 1.0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                px *= ww[i].x;
+                py *= ww[i].y;
+            }
+            float none = 0.f;                                // stays zero while everything is a number
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                none = fmaf(ww[i].x, 0.f, none); none = fmaf(ww[i].y, 0.f, none); none = fmaf(uu[i].x, 0.f, none); none = fmaf(uu[i].y, 0.f, none);
+                none = fmaf(aa[i].x, 0.f, none); none = fmaf(aa[i].y, 0.f, none);
+                none = fmaf(low_of(kk[i]), 0.f, none); none = fmaf(high_of(kk[i]), 0.f, none);
+            }
+            if (!(none == 0.f)) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (!finite(ww[i].x) || !finite(ww[i].y) || !finite(uu[i].x) || !finite(uu[i].y) || !finite(aa[i].x) || !finite(aa[i].y) ||
+                        !finite(low_of(kk[i])) || !finite(high_of(kk[i])))
+                        atomicMin(noted, seg * 4 + i);
+            }
+            *reinterpret_cast<double2*>(exch + seg * SC + 2 * pair) = make_double2(px, py);
+            __syncthreads();
+            // from the middle to this thread's tokens, then token by token away from it (64 bits, rounded once)
+            double fx = 1.0, fy = 1.0;
+            const bool early = seg < 8;
+            for (int m = early ? seg + 1 : 8; m < (early ? 8 : seg); ++m) {
+                const double2 e = *reinterpret_cast<const double2*>(exch + m * SC + 2 * pair);
+                fx *= e.x;
+                fy *= e.y;
+            }
+            if (seg == 0 || seg == 15) {
+                mid[(seg & 1) * DK + ch] = (float)(fx * px);
+                mid[(seg & 1) * DK + ch + 1] = (float)(fy * py);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = early ? 3 - j : j, t = seg * 4 + i;
+                // early: fours from the last to the first
+                const float2 wi = early ? ww[3 - j] : ww[j], ui = early ? uu[3 - j] : uu[j], ai = early ? aa[3 - j] : aa[j];
+                const uint32_t ri = early ? rr[3 - j] : rr[j], ki = early ? kk[3 - j] : kk[j];
+                const double nx = fx * wi.x, ny = fy * wi.y;             // with this token's decay
+                const float bx = (float)fx, by = (float)fy, ax = (float)nx, ay = (float)ny;
+                // the product between the middle and the state behind token t, and that between the middle and the state in front of it
+                const float2 behind = early ? make_float2(bx, by) : make_float2(ax, ay), front = early ? make_float2(ax, ay) : make_float2(bx, by);
+                *reinterpret_cast<float2*>(ps + t * L::PF + ch) = behind;
+                const float2 inv = make_float2(reciprocal(behind.x), reciprocal(behind.y));
+                const float2 row = early ? inv : behind, col = early ? behind : inv;
+                const float2 urow = early ? make_float2(reciprocal(front.x), reciprocal(front.y)) : front;
+                uint32_t x[3];
+                bf16* to = stage + t * SP + 2 * pair;
+                auto put = [&](int which, float p0, float p1) {
+                    cut(p0, p1, x);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(to + (which * 3 + p) * CK * SP) = x[p];
+                };
+                put(0, ui.x * urow.x, ui.y * urow.y);
+                put(1, low_of(ri) * row.x, high_of(ri) * row.y);
+                put(2, low_of(ki) * col.x, high_of(ki) * col.y);
+                put(3, ai.x * col.x, ai.y * col.y);
+                fx = nx;
+                fy = ny;
+            }
+            __syncthreads();
+            // u and au as operands of the later products
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const int id = warp + 8 * j, p = id % 3, blk = id / 3 % 8, which = id / 24;      // 8 blocks of 16 x 16, 3 pieces, 2 arrays
+                uint32_t x[4];
+                ldsm_t(x, stage + ((which ? 9 : 0) + p) * CK * SP + (blk >> 1) * 16 * SP + (blk & 1) * 16 + at_bt(lane, SP));
+                bf16* to = (which ? aus : xs) + p * CK * DK + (((blk >> 1) * KS + q0 / 16 + (blk & 1)) * 32 + lane) * 8;
+                *reinterpret_cast<uint4*>(to) = make_uint4(x[0], x[1], x[2], x[3]);
+            }
+            const bf16 *rows = stage + rows_of * 3 * CK * SP, *cols = stage + (2 + cols_of) * 3 * CK * SP;
+#pragma unroll
+            for (int k0 = 0; k0 < SC; k0 += 16) {
+                uint32_t fl[3][1][4], fs[3][1][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    ldsm(fl[p][0], rows + p * CK * SP + long_row * 16 * SP + k0 + at_a(lane, SP));
+                    ldsm(fs[p][0], rows + p * CK * SP + short_row * 16 * SP + k0 + at_a(lane, SP));
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (j > long_row) continue;
+                    uint32_t fb[3][1][4];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) ldsm(fb[p][0], cols + p * CK * SP + j * 16 * SP + k0 + at_b(lane, SP));
+                    products<1, 1, 3, 3>(sl[j], fl, fb);
+                    if (j < 2 && j <= short_row) products<1, 1, 3, 3>(ss[j], fs, fb);
+                }
+            }
+            __syncthreads();
+        }
+        again = *noted < tokens;
+        if (again) tokens = *noted;                          // once more without the tokens from there on
+    }
+    const int bad = tokens < c.n ? tokens : CK;
+    const float nan = __int_as_float(0x7fc00000);
+    // ---- A in fp32, B and Q in pieces, P in fp32
+    auto put_scores = [&](int i, int j, float (&d)[1][2][4]) {
+        if (rows_of == 0 && cols_of == 1) {
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    *reinterpret_cast<float2*>(as + (i * 16 + g + 8 * e) * L::AF + j * 16 + n * 8 + t4 * 2) = make_float2(d[0][n][2 * e], d[0][n][2 * e + 1]);
+            return;
+        }
+        if (i == j) {                                        // rows u: earlier tokens; rows r: and the token itself
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int row = g + 8 * (e >> 1), col = n * 8 + t4 * 2 + (e & 1);
+                    if (col > row || (rows_of == 0 && col == row)) d[0][n][e] = 0.f;
+                }
+        }
+        const int at = lower_block(i, j);
+        if (rows_of == 1 && cols_of == 0) {
+            float* to = pf + (at * 32 + lane) * 8;
+            *reinterpret_cast<float4*>(to) = make_float4(d[0][0][0], d[0][0][1], d[0][0][2], d[0][0][3]);
+            *reinterpret_cast<float4*>(to + 4) = make_float4(d[0][1][0], d[0][1][1], d[0][1][2], d[0][1][3]);
+        } else {
+            put_block((rows_of ? qs : bs) + at * 3 * 256, d[0], lane);
+        }
+    };
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (j <= long_row) put_scores(long_row, j, sl[j]);
+        if (j < 2 && j <= short_row) put_scores(short_row, j, ss[j]);
+    }
+    __syncthreads();
+    // ---- T = (I + A)^-1 in place: blocks of 16 by substitution, then pairs of blocks, [[T1, 0], [-T2 A T1, T2]]; A T1 lies above the diagonal
+    if (tid < CK) {
+        float x[16];
+        const float* blk = as + (tid >> 4) * 16 * (L::AF + 1);
+        const int col = tid & 15;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float s0 = i == col ? 1.f : 0.f, s1 = 0.f;
+#pragma unroll
+            for (int m = 0; m < 16; ++m) {
+                if (m >= i) continue;
+                if (m & 1) s1 = fmaf(-blk[i * L::AF + m], x[m], s1);
+                else s0 = fmaf(-blk[i * L::AF + m], x[m], s0);
+            }
+            x[i] = s0 + s1;
+        }
+        __syncwarp();
+        float* to = as + (tid >> 4) * 16 * (L::AF + 1) + col;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) to[i * L::AF] = x[i];
+    }
+    __syncthreads();
+    {
+        float* blk = as + (tid >> 7) * 32 * (L::AF + 1);
+        const int i = (tid & 127) >> 3, j = (tid & 7) * 2;
+        float2 m = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int n = 0; n < 16; ++n) {
+            const float x = blk[(16 + i) * L::AF + n];
+            const float2 y = *reinterpret_cast<const float2*>(blk + n * L::AF + j);
+            m = make_float2(fmaf(x, y.x, m.x), fmaf(x, y.y, m.y));
+        }
+        *reinterpret_cast<float2*>(blk + i * L::AF + 16 + j) = m;
+        __syncthreads();
+        m = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int n = 0; n < 16; ++n) {
+            const float x = blk[(16 + i) * L::AF + 16 + n];
+            const float2 y = *reinterpret_cast<const float2*>(blk + n * L::AF + 16 + j);
+            m = make_float2(fmaf(-x, y.x, m.x), fmaf(-x, y.y, m.y));
+        }
+        __syncthreads();
+        *reinterpret_cast<float2*>(blk + (16 + i) * L::AF + j) = m;
+    }
+    __syncthreads();
+    {
+        const int i = tid >> 3, j = (tid & 7) * 4;
+        float4 m = zero4();
+        for (int n = j < 16 ? 0 : 16; n < 32; ++n) {
+            const float x = as[(32 + i) * L::AF + n];
+            const float4 y = load4(as + n * L::AF + j);
+            m = make_float4(fmaf(x, y.x, m.x), fmaf(x, y.y, m.y), fmaf(x, y.z, m.z), fmaf(x, y.w, m.w));
+        }
+        *reinterpret_cast<float4*>(as + i * L::AF + 32 + j) = m;
+        __syncthreads();
+        m = zero4();
+        for (int n = 0; n < (i < 16 ? 16 : 32); ++n) {
+            const float x = as[(32 + i) * L::AF + 32 + n];
+            const float4 y = load4(as + n * L::AF + 32 + j);
+            m = make_float4(fmaf(-x, y.x, m.x), fmaf(-x, y.y, m.y), fmaf(-x, y.z, m.z), fmaf(-x, y.w, m.w));
+        }
+        *reinterpret_cast<float4*>(as + (32 + i) * L::AF + j) = m;
+    }
+    __syncthreads();
+    for (int e = tid; e < LOWER * 128; e += DP_THREADS) {
+        const int at = e >> 7, i = at < 1 ? 0 : at < 3 ? 1 : at < 6 ? 2 : 3, j = at - lower_block(i, 0), row = (e & 127) >> 3, col = (e & 7) * 2;
+        const float2 x = *reinterpret_cast<const float2*>(as + (i * 16 + row) * L::AF + j * 16 + col);
+        uint32_t y[3];
+        cut(x.x, x.y, y);
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+            *reinterpret_cast<uint32_t*>(ts + (at * 3 + p) * 256 + row * 16 + (((col >> 3) ^ (row >> 2 & 1)) << 3) + (col & 7)) = y[p];
+    }
+    __syncthreads();
+    // ---- Y = T B;  then W = Q T and P' = P - Q Y
+    for (int n = 0; n < 2; ++n) {
+        const int at = warp_blocks(warp, n);
+        if (at < 0) continue;
+        float d[1][2][4] = {};
+        block_product(d, ts, bs, at >> 2, at & 3, lane);
+        put_block(ys + lower_block(at >> 2, at & 3) * 3 * 256, d[0], lane);
+    }
+    __syncthreads();
+    for (int n = 0; n < 2; ++n) {
+        const int at = warp_blocks(warp, n), i = at >> 2, j = at & 3;
+        if (at < 0) continue;
+        float d[1][2][4] = {};
+        block_product(d, qs, ts, i, j, lane);
+        put_block(ws + lower_block(i, j) * 3 * 256, d[0], lane);
+        float e[1][2][4] = {};
+        block_product(e, qs, ys, i, j, lane);
+        const float* own = pf + (lower_block(i, j) * 32 + lane) * 8;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int row = i * 16 + g + 8 * x;
+                const float2 was = *reinterpret_cast<const float2*>(own + m * 4 + x * 2);
+                uint32_t y[3];
+                cut(row >= bad ? nan : was.x - e[0][m][2 * x], row >= bad ? nan : was.y - e[0][m][2 * x + 1], y);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(parts + p * CK * CK + row * CK + j * 16 + m * 8 + t4 * 2) = y[p];
+            }
+    }
+    parts += 3 * CK * CK;
+    for (int e = tid; e < DK; e += DP_THREADS) {
+        float* to = ends + unit * 2 * DK + e;
+        to[0] = bad < CK ? nan : mid[DK + e];
+        to[DK] = bad < CK ? nan : mid[e] * mid[DK + e];
+    }
+    auto stage_values = [&](int c0) {
+        for (int e = tid; e < CK * OUT_V / 4; e += DP_THREADS) {
+            const int t = e / (OUT_V / 4), i = (e % (OUT_V / 4)) * 4;
+            if (c0 + i < dv) cp8(vs + t * VP + i, t < tokens ? v + (size_t)(c.t0 + t) * v_stride + (size_t)h * dv + c0 + i : v, t < tokens);
+        }
+    };
+    __syncthreads();
+    stage_values(0);
+    const int kb = warp;                                     // this warp's 16 channels
+    if (kb < KS) {
+        // ---- X = T U D and R' = (R D - W U D), from the middle to the chunk's start by the channel's product
+        uint32_t fu[QUARTERS][3][1][4];
+#pragma unroll
+        for (int t = 0; t < QUARTERS; ++t)
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                const uint4 x = *reinterpret_cast<const uint4*>(xs + p * CK * DK + ((t * KS + kb) * 32 + lane) * 8);
+                fu[t][p][0][0] = x.x; fu[t][p][0][1] = x.y; fu[t][p][0][2] = x.z; fu[t][p][0][3] = x.w;
+            }
+        uint32_t rc[QUARTERS][4];
+#pragma unroll
+        for (int i = 0; i < QUARTERS; ++i)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int t = i * 16 + g + 8 * e;
+                    rc[i][n * 2 + e] = t < tokens ? *reinterpret_cast<const uint32_t*>(r + (size_t)(c.t0 + t) * r_stride + (size_t)h * DK + kb * 16 + n * 8 + t4 * 2) : 0u;
+                }
+#pragma unroll
+        for (int i = 0; i < QUARTERS; ++i) {
+            float dx[1][2][4] = {}, dr[1][2][4] = {};
+#pragma unroll
+            for (int t = 0; t <= i; ++t) {
+                uint32_t ft[3][1][4], fw[3][1][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    ldsm(ft[p][0], lane_row(ts + (lower_block(i, t) * 3 + p) * 256, lane));
+                    ldsm(fw[p][0], lane_row(ws + (lower_block(i, t) * 3 + p) * 256, lane));
+                }
+                products<1, 1, 3, 3>(dx, ft, fu[t]);
+                products<1, 1, 3, 3>(dr, fw, fu[t]);
+            }
+            uint32_t x[4][3];
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int ch = kb * 16 + n * 8 + t4 * 2;
+                const float2 m = *reinterpret_cast<const float2*>(mid + ch);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int t = i * 16 + g + 8 * e;
+                    cut(dx[0][n][2 * e] * m.x, dx[0][n][2 * e + 1] * m.y, x[e * 2 + n]);
+                    float2 f = *reinterpret_cast<const float2*>(ps + t * L::PF + ch);
+                    if (t < 32) f = make_float2(reciprocal(f.x), reciprocal(f.y));
+                    const uint32_t r2 = rc[i][n * 2 + e];
+                    uint32_t y[3];
+                    cut(t >= bad ? nan : (low_of(r2) * f.x - dr[0][n][2 * e]) * m.x, t >= bad ? nan : (high_of(r2) * f.y - dr[0][n][2 * e + 1]) * m.y, y);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(parts + p * CK * DK + t * DK + ch) = y[p];
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+                *reinterpret_cast<uint4*>(xs + p * CK * DK + ((i * KS + kb) * 32 + lane) * 8) = make_uint4(x[0][p], x[1][p], x[2][p], x[3][p]);
+        }
+    }
+    // ---- K D - Y^T AU D, from the middle to the chunk's end by the channel's product
+    uint32_t kp[QUARTERS][3][1][4];                          // as the right operand of the last product
+    if (kb < KS) {
+        uint32_t fa[QUARTERS][3][1][4], kc[QUARTERS][4];
+#pragma unroll
+        for (int t = 0; t < QUARTERS; ++t) {
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                const uint4 x = *reinterpret_cast<const uint4*>(aus + p * CK * DK + ((t * KS + kb) * 32 + lane) * 8);
+                fa[t][p][0][0] = x.x; fa[t][p][0][1] = x.y; fa[t][p][0][2] = x.z; fa[t][p][0][3] = x.w;
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int at = t * 16 + g + 8 * e;
+                    kc[t][n * 2 + e] = at < tokens ? *reinterpret_cast<const uint32_t*>(k + (size_t)(c.t0 + at) * k_stride + (size_t)h * DK + kb * 16 + n * 8 + t4 * 2) : 0u;
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < QUARTERS; ++j) {
+            float d[1][2][4] = {};
+#pragma unroll
+            for (int t = j; t < QUARTERS; ++t) {
+                uint32_t fy[3][1][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {                // the block's transpose as the left operand
+                    const int row = (lane & 7) + (lane >> 4) * 8;
+                    ldsm_t(fy[p][0], ys + (lower_block(t, j) * 3 + p) * 256 + row * 16 + (((lane >> 3 & 1) ^ (row >> 2 & 1)) << 3));
+                }
+                products<1, 1, 3, 3>(d, fy, fa[t]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int ch = kb * 16 + n * 8 + t4 * 2;
+                const float2 m = *reinterpret_cast<const float2*>(mid + DK + ch);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float2 f = *reinterpret_cast<const float2*>(ps + (j * 16 + g + 8 * e) * L::PF + ch);
+                    if (j >= 2) f = make_float2(reciprocal(f.x), reciprocal(f.y));
+                    uint32_t x[3];
+                    cut((low_of(kc[j][n * 2 + e]) * f.x - d[0][n][2 * e]) * m.x, (high_of(kc[j][n * 2 + e]) * f.y - d[0][n][2 * e + 1]) * m.y, x);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p)              // 8 tokens by 8 keys, turned: a lane has two tokens of a key
+                        asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(kp[j][p][0][n * 2 + e]) : "r"(x[p]));
+                }
+            }
+        }
+    }
+    // ---- the chunk's own contribution: values by keys
+    for (int c0 = 0; c0 < dv; c0 += OUT_V) {
+        const int cols = min(OUT_V, dv - c0);
+        if (c0 > 0) {
+            __syncthreads();
+            stage_values(c0);
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+        if (kb < KS) {
+            for (int m = 0; m < cols / 16; ++m) {
+                float d[1][2][4] = {};
+#pragma unroll
+                for (int t = 0; t < QUARTERS; ++t) {
+                    uint32_t fv[1][1][4];
+                    ldsm_t(fv[0][0], vs + t * 16 * VP + m * 16 + at_at(lane, VP));
+                    products<1, 1, 1, 3>(d, fv, kp[t]);
+                }
+                float* to = states + (unit * dv + c0 + m * 16) * DK + (kb * 32 + lane) * 8;
+                *reinterpret_cast<float4*>(to) = make_float4(d[0][0][0], d[0][0][1], d[0][1][0], d[0][1][1]);
+                *reinterpret_cast<float4*>(to + 4) = make_float4(d[0][0][2], d[0][0][3], d[0][1][2], d[0][1][3]);
+            }
+        }
+    }
+}
+
+// The state in front of every chunk: 16 MT value channels x MG of one head of one entry, the chunks in order.  Four warps a group of
+// 16 MT channels: the d of a quarter of the tokens each, then the state of a quarter of the keys; they meet in shared memory
+// twice a chunk.  X and au of the chunks come through a ring of three slots, each asked for a chunk ahead.
+template <int MT, int MG>
+struct ScanLayout {                             // bytes
+    static constexpr int SLOT = 3 * CK * DK * 2;
+    static constexpr int ring = 0, s = 3 * SLOT, d = s + MG * 3 * MT * KS * 512, bytes = d + MG * 3 * MT * QUARTERS * 512;
+};
+template <int MT, int MG>
+__global__ void __launch_bounds__(128 * MG, 1)
+delta_chunk_scan_kernel(const bf16* __restrict__ xs, const bf16* __restrict__ aus, const float* __restrict__ ends, const float* __restrict__ states,
+                        bf16* __restrict__ cuts, float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
+                        int least, int H, int dv) {
+    using L = ScanLayout<MT, MG>;
+    constexpr int KBW = KS / 4;                              // key blocks of a warp
+    extern __shared__ __align__(16) unsigned char raw[];
+    pdl_trigger();
+    pdl_wait();
+    const int b = blockIdx.z, h = blockIdx.y;
+    const int count = chunks_of(cu_q[b + 1] - cu_q[b], least);
+    if (count == 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, group = warp >> 2, wn = warp & 3, g = lane >> 2, t4 = lane & 3;
+    const size_t base = first_chunk(cu_q, b, least), one = (size_t)dv * DK;
+    uint4* sp = reinterpret_cast<uint4*>(raw + L::s) + group * 3 * MT * KS * 32;             // [piece][m][key block][lane]
+    uint4* dp = reinterpret_cast<uint4*>(raw + L::d) + group * 3 * MT * QUARTERS * 32;       // [piece][m][token block][lane]
+    auto ask = [&](int item) {                               // X of chunk item / 2, or its au
+        if (item < 2 * count) {
+            const bf16* from = (item & 1 ? aus : xs) + ((base + (item >> 1)) * H + h) * 3 * CK * DK;
+            bf16* to = reinterpret_cast<bf16*>(raw + L::ring + item % 3 * L::SLOT);
+            for (int e = tid; e < 3 * CK * DK / 8; e += 128 * MG) cp16(to + e * 8, from + e * 8);
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    ask(0);
+    ask(1);
+    const int vb0 = (blockIdx.x * MG + group) * MT;          // the group's first value block
+    float* own = state + ((size_t)state_slots[b] * H + h) * one;
+    float S[MT][KBW][2][4];
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int n = 0; n < KBW; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {                    // rows (value) g, g + 8; keys 2 t4 of the block's halves
+                const float2 x = *reinterpret_cast<const float2*>(own + (size_t)((vb0 + m) * 16 + g + 8 * (e >> 1)) * DK + (wn * KBW + n) * 16 + (e & 1) * 8 + t4 * 2);
+                S[m][n][e & 1][(e >> 1) * 2] = x.x;
+                S[m][n][e & 1][(e >> 1) * 2 + 1] = x.y;
+            }
+    for (int c = 0; c < count; ++c) {
+        const size_t unit = (base + c) * H + h;
+        // the state in front of the chunk: to the outputs' kernel as the right operand, to the other warps as the left one
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < KBW; ++n) {
+                uint32_t x[4][3];                            // value row half, key half
+#pragma unroll
+                for (int e = 0; e < 4; ++e) cut(S[m][n][e & 1][(e >> 1) * 2], S[m][n][e & 1][(e >> 1) * 2 + 1], x[e]);
+                const int kb = wn * KBW + n;
+                bf16* to = cuts + unit * 3 * one + ((size_t)(vb0 + m) * KS + kb) * 256 + lane * 8;
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    *reinterpret_cast<uint4*>(to + p * one) = make_uint4(x[0][p], x[1][p], x[2][p], x[3][p]);
+                    sp[((p * MT + m) * KS + kb) * 32 + lane] = make_uint4(x[0][p], x[2][p], x[1][p], x[3][p]);
+                }
+            }
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncthreads();                                     // X is there, so is the state, and the last chunk's au are read
+        ask(2 * c + 2);
+        // what the chunk itself adds, and its decays, on their way
+        float4 x0[MT][KBW], x1[MT][KBW];
+        float2 f[KBW][2], all[KBW][2];
+#pragma unroll
+        for (int n = 0; n < KBW; ++n) {
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float* from = states + unit * one + ((size_t)(vb0 + m) * KS + wn * KBW + n) * 256 + lane * 8;
+                x0[m][n] = load4(from);
+                x1[m][n] = load4(from + 4);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float* from = ends + unit * 2 * DK + (wn * KBW + n) * 16 + e * 8 + t4 * 2;
+                f[n][e] = *reinterpret_cast<const float2*>(from);
+                all[n][e] = *reinterpret_cast<const float2*>(from + DK);
+            }
+        }
+        const uint4* ring = reinterpret_cast<const uint4*>(raw + L::ring + (2 * c) % 3 * L::SLOT);
+        {
+            float d[MT][1][2][4] = {};
+#pragma unroll 2
+            for (int k = 0; k < KS; ++k) {
+                uint32_t fb[3][1][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const uint4 x = ring[(p * QUARTERS + wn) * KS * 32 + k * 32 + lane];
+                    fb[p][0][0] = x.x; fb[p][0][1] = x.y; fb[p][0][2] = x.z; fb[p][0][3] = x.w;
+                }
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    uint32_t fa[3][1][4];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        const uint4 x = sp[((p * MT + m) * KS + k) * 32 + lane];
+                        fa[p][0][0] = x.x; fa[p][0][1] = x.y; fa[p][0][2] = x.z; fa[p][0][3] = x.w;
+                    }
+                    products<1, 1, 3, 3>(d[m], fa, fb);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                uint32_t x[4][3];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) cut(d[m][0][e >> 1][(e & 1) * 2], d[m][0][e >> 1][(e & 1) * 2 + 1], x[e]);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) dp[((p * MT + m) * QUARTERS + wn) * 32 + lane] = make_uint4(x[0][p], x[1][p], x[2][p], x[3][p]);
+            }
+        }
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncthreads();                                     // the au are there, so are all tokens' d, and X is read
+        ask(2 * c + 3);
+        ring = reinterpret_cast<const uint4*>(raw + L::ring + (2 * c + 1) % 3 * L::SLOT);
+        {
+            float d[MT][KBW][1][2][4] = {};
+#pragma unroll 2
+            for (int t = 0; t < QUARTERS; ++t) {
+                uint32_t fa[MT][3][1][4];
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        const uint4 x = dp[((p * MT + m) * QUARTERS + t) * 32 + lane];
+                        fa[m][p][0][0] = x.x; fa[m][p][0][1] = x.y; fa[m][p][0][2] = x.z; fa[m][p][0][3] = x.w;
+                    }
+#pragma unroll
+                for (int n = 0; n < KBW; ++n) {
+                    uint32_t fb[3][1][4];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        const uint4 x = ring[(p * QUARTERS + t) * KS * 32 + (wn * KBW + n) * 32 + lane];
+                        fb[p][0][0] = x.x; fb[p][0][1] = x.y; fb[p][0][2] = x.z; fb[p][0][3] = x.w;
+                    }
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) products<1, 1, 3, 3>(d[m][n], fa[m], fb);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int n = 0; n < KBW; ++n) {
+                    const float l[2][4] = {{x0[m][n].x, x0[m][n].y, x1[m][n].x, x1[m][n].y}, {x0[m][n].z, x0[m][n].w, x1[m][n].z, x1[m][n].w}};
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+#pragma unroll
+                        for (int z = 0; z < 4; ++z) {
+                            const float ff = z & 1 ? f[n][e].y : f[n][e].x, aa = z & 1 ? all[n][e].y : all[n][e].x;
+                            S[m][n][e][z] = fmaf(aa, S[m][n][e][z], fmaf(-ff, d[m][n][0][e][z], l[e][z]));
+                        }
+                }
+        }
+        // (the state's pieces and the d are written again after the others have read them: the next barriers)
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int n = 0; n < KBW; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                *reinterpret_cast<float2*>(own + (size_t)((vb0 + m) * 16 + g + 8 * (e >> 1)) * DK + (wn * KBW + n) * 16 + (e & 1) * 8 + t4 * 2) =
+                    make_float2(S[m][n][e & 1][(e >> 1) * 2], S[m][n][e & 1][(e >> 1) * 2 + 1]);
+}
+
 inline bool aligned4(const void* p, int esize) { return (reinterpret_cast<uintptr_t>(p) % (4 * (size_t)esize)) == 0; }
 template <typename Kernel>
 int allow(Kernel kernel, int bytes) { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); }
@@ -1007,6 +1709,44 @@ RI_API int ri_gated_chunks(const void* q, int q_stride, const void* k, int k_str
                          (const bf16*)parts, (const bf16*)v, v_stride, q_scale, (const bf16*)cuts, out, cu_q, entries, least, H, dv));
     return ri_launch_status();
 }
+// The delta rule (bf16 r, k, v; w, u, au fp32 [T][f_stride] as the walk's, -log w at most ri_delta_chunk_decay()): xs and aus bf16
+// [chunks][H][3][CK][DK], ends fp32 [chunks][H][2][DK], the rest as the gated form's.
+RI_API float ri_delta_chunk_decay() { return DELTA_MOST_DECAY; }
+RI_API int ri_delta_chunks(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride, const float* w,
+                           const float* u, const float* au, int f_stride, int act_dtype, float* out, float* state, const int* cu_q,
+                           const int* state_slots, int entries, int least, int chunks, int H, int dv, float* states, float* ends, void* cuts,
+                           void* parts, void* xs, void* aus, void* stream) {
+    if (entries <= 0 || chunks <= 0) return 0;
+    if (!ri_chunks_ok(r, r_stride, k, k_stride, v, v_stride, act_dtype, dv, 1) || f_stride % 4 || !aligned4(w, 4) || !aligned4(u, 4) || !aligned4(au, 4))
+        return (int)cudaErrorInvalidValue;
+    cudaStream_t s = (cudaStream_t)stream;
+    static bool allowed = false;
+    if (!allowed) {
+        RI_CHECKED(allow(delta_chunk_parts_kernel, PartsLayout::bytes));
+        RI_CHECKED(allow(delta_chunk_scan_kernel<1, 1>, ScanLayout<1, 1>::bytes));
+        RI_CHECKED(allow(delta_chunk_scan_kernel<2, 1>, ScanLayout<2, 1>::bytes));
+        RI_CHECKED(allow(delta_chunk_scan_kernel<2, 2>, ScanLayout<2, 2>::bytes));
+        RI_CHECKED(allow(gated_chunk_outputs_kernel<4>, OutLayout::gated_bytes));
+        RI_CHECKED(allow(gated_chunk_outputs_kernel<2>, OutLayout::gated_bytes));
+        allowed = true;
+    }
+    RI_CHECKED(ri_launch(delta_chunk_parts_kernel, dim3(chunks, H), dim3(DP_THREADS), PartsLayout::bytes, s, (const bf16*)r, r_stride,
+                         (const bf16*)k, k_stride, (const bf16*)v, v_stride, w, u, au, f_stride, (bf16*)xs, (bf16*)aus, ends, (bf16*)parts,
+                         states, cu_q, entries, least, H, dv));
+    // value channels a CTA of the scan takes, one CTA an SM: the fewest that leave no CTA waiting for an SM
+    const long long blocks = (long long)entries * H * dv / 16;
+#define RI_DSCAN(MT, MG) RI_CHECKED(ri_launch(delta_chunk_scan_kernel<MT, MG>, dim3(dv / (16 * MT * MG), H, entries), dim3(128 * MG), \
+        ScanLayout<MT, MG>::bytes, s, (const bf16*)xs, (const bf16*)aus, (const float*)ends, (const float*)states, (bf16*)cuts, state, cu_q, \
+        state_slots, least, H, dv))
+    if (blocks <= ri_device_sms()) RI_DSCAN(1, 1);
+    else if (blocks <= 2LL * ri_device_sms()) RI_DSCAN(2, 1);
+    else RI_DSCAN(2, 2);
+#undef RI_DSCAN
+    RI_CHECKED(ri_launch(dv % OUT_V == 0 ? gated_chunk_outputs_kernel<4> : gated_chunk_outputs_kernel<2>, dim3(chunks, H, dv % OUT_V == 0 ? dv / OUT_V : 1),
+                         dim3(OUT_THREADS), OutLayout::gated_bytes, s, (const bf16*)parts, (const bf16*)v, v_stride, 1.0f, (const bf16*)cuts, out,
+                         cu_q, entries, least, H, dv));
+    return ri_launch_status();
+}
 #else
 RI_API int ri_chunks_ok(const void*, int, const void*, int, const void*, int, int, int, int) { return 0; }
 RI_API int ri_head_chunks(const void*, int, const void*, int, const void*, int, const float*, int, const float*, int, int, float, float*,
@@ -1018,6 +1758,11 @@ RI_API int ri_gated_chunks(const void*, int, const void*, int, const void*, int,
     return (int)cudaErrorInvalidValue;
 }
 RI_API int ri_gated_chunk_parts() { return 0; }
+RI_API float ri_delta_chunk_decay() { return 0.f; }
+RI_API int ri_delta_chunks(const void*, int, const void*, int, const void*, int, const float*, const float*, const float*, int, int, float*,
+                           float*, const int*, const int*, int, int, int, int, int, float*, float*, void*, void*, void*, void*, void*) {
+    return (int)cudaErrorInvalidValue;
+}
 #endif
 
 RI_API int ri_recurrent_chunk_tokens() { return BUILT ? CK : 0; }

@@ -1289,20 +1289,40 @@ def _scan_chunks(T: int, entries: int, longest: int, heads: int, key_dim: int, v
     """Chunks a call with `longest` tokens in its longest entry is laid out for (an upper bound), 0: every entry walks.  In chunks
     when that is a tenth faster, the other entries taken to be equally long: those too short for chunks walk all the same."""
     least = GATED_CHUNK_MIN_TOKENS if gated else CHUNK_MIN_TOKENS
+    return _chunks_or_walk(T, entries, longest, heads, key_dim, value_dim, num_sms, least, _chunk_sizes(heads, key_dim, value_dim, gated),
+                           _WALK_US[gated], _CHUNK_FIXED_US[gated], _CHUNK_US[gated])
+
+
+def _chunks_or_walk(T: int, entries: int, longest: int, heads: int, key_dim: int, value_dim: int, num_sms: int, least: int,
+                    sizes: Tuple[int, ...], walk_us: float, fixed_us: float, chunk_us: float) -> int:
     if longest < least or entries < 1 or longest > T:
         return 0
     state = heads * key_dim * value_dim
     chunks = T // CHUNK_TOKENS + min(entries, T // least)
-    if chunks * sum(_chunk_sizes(heads, key_dim, value_dim, gated)) > CHUNK_SCRATCH_BYTES:
+    if chunks * sum(sizes) > CHUNK_SCRATCH_BYTES:
         return 0
     filled = heads * value_dim / (16 if key_dim > 64 else 32) / (2 * num_sms)   # of the GPU by one entry's walk: CTAs over places for them
-    walk = lambda most, all_tokens: _WALK_US[gated] * max(most, all_tokens * filled)
+    walk = lambda most, all_tokens: walk_us * max(most, all_tokens * filled)
     rest = T - longest
     short = rest > 0 and rest < least * (entries - 1)
-    cost = _CHUNK_FIXED_US[gated] + _CHUNK_US[gated] * state * (longest if short else T)
+    cost = fixed_us + chunk_us * state * (longest if short else T)
     if short:
         cost += 3.0 + walk(rest / (entries - 1), rest)
     return chunks if cost < 0.9 * walk(longest, T) else 0
+
+
+# the delta rule: 16 heads of 128 x 128 take 90 us in a walk and 86 in chunks at 256 tokens, 175 and 100 at 512, 688 and 246 at 2,048 (8
+# heads: 90 and 79, 171 and 93, 678 and 166); 8 heads of 64 x 64 58 and 48 at 192, 144 and 56 at 512 (fitted to 1 to 5 entries of 128 to
+# 2,048 tokens, 4 to 32 heads)
+DELTA_CHUNK_MIN_TOKENS = 192
+_DELTA_WALK_US, _DELTA_CHUNK_FIXED_US, _DELTA_CHUNK_US = 0.335, 66.0, 3.3e-7
+
+
+def _delta_chunk_sizes(heads: int, key_dim: int, value_dim: int) -> Tuple[int, ...]:
+    """As `_chunk_sizes`, for the delta rule: the chunk's own state, the decays to its end, the state in front of it, scores and queries,
+    and the two operands of its scan."""
+    state, operand = heads * key_dim * value_dim, 6 * heads * CHUNK_TOKENS * key_dim
+    return 4 * state, 8 * heads * key_dim, 6 * state, 6 * heads * CHUNK_TOKENS * CHUNK_TOKENS + operand, operand, operand
 
 
 def _chunk_scratch(chunks: int, device: torch.device, sizes: Tuple[int, ...]):
@@ -1468,11 +1488,12 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
 def delta_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, za: torch.Tensor, za_bias: Optional[torch.Tensor],
                zw: torch.Tensor, zw_bias: Optional[torch.Tensor], decay_rate: float, unit_eps: float,
                out: torch.Tensor, state: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, entries: int,
-               num_heads: int, key_dim: int, value_dim: int) -> None:
+               num_heads: int, key_dim: int, value_dim: int, longest: int = 0) -> None:
     """Delta rule with a decay, over every entry's tokens in order, from and into state[slot]:
     S = diag(w) S - (a * u)(u^T S) + k v^T, out = S^T r, with u = k / sqrt(|k|^2 + unit_eps),
     w = exp(-decay_rate * sigmoid(zw + zw_bias)), a = sigmoid(za + za_bias).  zw is fp32 and is
-    overwritten with the decays.  Two launches: w, u and a * u of all tokens at once, then the walk."""
+    overwritten with the decays.  Two launches: w, u and a * u of all tokens at once, then the walk.  `longest`: as `head_scan`'s (bf16 r,
+    k, v; decay_rate at most 1)."""
     require_cuda(r, k, v, za, za_bias, zw, zw_bias, out, state, cu_q, state_slots)
     T, H, dk, dv = r.shape[0], num_heads, key_dim, value_dim
     _scan_common(state, out, cu_q, state_slots, T, H, dk, dv, "delta_scan")
@@ -1489,10 +1510,23 @@ def delta_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, za: torch.Tens
                                     dtype_code(r.dtype), dtype_code(biases[0].dtype) if biases else 0,
                                     float(decay_rate), float(unit_eps), _p(unit[0]), _p(unit[1]), T, H, dk,
                                     stream_ptr()), "delta_prepare")
-    check(L.recurrent(dk).ri_delta_scan(_p(r), r.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(zw), _p(unit[0]),
-                                        _p(unit[1]), H * dk, dtype_code(r.dtype), _p(out), _p(state), _p(cu_q),
-                                        _p(state_slots), int(entries), H, dv, 1 if T == int(entries) else 0,
-                                        stream_ptr()), "delta_scan")
+    lib = L.recurrent(dk)
+    args = (_p(r), r.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(zw), _p(unit[0]), _p(unit[1]), H * dk, dtype_code(r.dtype), _p(out),
+            _p(state), _p(cu_q), _p(state_slots), int(entries))
+    below = 0
+    if longest >= DELTA_CHUNK_MIN_TOKENS and 0.0 <= decay_rate <= lib.ri_delta_chunk_decay():
+        sizes = _delta_chunk_sizes(H, dk, dv)
+        chunks = _chunks_or_walk(T, int(entries), longest, H, dk, dv, L.num_sms(), DELTA_CHUNK_MIN_TOKENS, sizes, _DELTA_WALK_US,
+                                 _DELTA_CHUNK_FIXED_US, _DELTA_CHUNK_US)
+        held = None
+        if chunks and lib.ri_chunks_ok(*args[:6], dtype_code(r.dtype), dv, 1):
+            held = _chunk_scratch(chunks, r.device, sizes)
+        if held is not None:
+            check(lib.ri_delta_chunks(*args, DELTA_CHUNK_MIN_TOKENS, chunks, H, dv, *held[1], stream_ptr()), "delta_chunks", 3)
+            if T == longest * int(entries):                   # every entry is as long
+                return
+            below = DELTA_CHUNK_MIN_TOKENS
+    check(lib.ri_delta_scan(*args, H, dv, 1 if T == int(entries) else 0, below, stream_ptr()), "delta_scan")
 
 
 # --------------------------------------------- blocks that norm a sublayer's output, and their mixers

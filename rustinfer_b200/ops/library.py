@@ -81,7 +81,8 @@ _SIGNATURES = {
     "ri_gated_chunk_parts": [],
     "ri_recurrent_chunk_tokens": [],
     "ri_gated_scan": [_P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "ri_delta_scan": [_P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _P],
+    "ri_delta_scan": [_P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "ri_delta_chunks": [_P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P],
     "ri_rms_sandwich": [_P, _I, _P, _I, _I, _P, _P, _P, _L, _I, _P, _P, _P, _P, _I, _P, _I, _I, _F, _P, _P, _P, _I, _P],
     "ri_short_conv": [_P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _P, _P, _I, _P],
     "ri_rglru_gates": [_P, _I, _P, _P, _I, _P, _P, _P, _F, _P, _P, _I, _I, _I, _P],
@@ -184,6 +185,7 @@ def recurrent(key_dim: int) -> ctypes.CDLL:
         raise KernelError(f"the recurrence kernels take key sizes up to 512, got {key_dim}")
     lib = _load(f"ri_recurrent_k{key_dim}", ["recurrent.cu", "recurrent_chunks.cu"], [f"RI_KDIM={key_dim}"])
     lib.ri_recurrent_state_rows.restype = _I
+    lib.ri_delta_chunk_decay.restype = _F
     return lib
 
 

@@ -175,7 +175,8 @@ class DeltaRule(_StateMixer):
         zw = self.w2(low, out_dtype=torch.float32)
         o = torch.empty((T, self.H * self.dk), dtype=torch.float32, device=x.device)
         K.delta_scan(p["r"], p["k"], p["v"], p["a"], self.a_bias, zw, self.w_bias, self.decay_rate, self.unit_eps,
-                     o, cache.state, step.cu_q, step.state_slots, step.num_entries, self.H, self.dk, self.dk)
+                     o, cache.state, step.cu_q, step.state_slots, step.num_entries, self.H, self.dk, self.dk,
+                     longest=step.max_q_len if dt == torch.bfloat16 else 0)
         y = torch.empty((T, self.H * self.dk), dtype=dt, device=x.device)
         K.gated_head_norm(o, p["g"], self.norm_w, True, K.GATE_SIGMOID, self.norm_eps, y, self.H, self.dk)
         return self.o(y, out_dtype=dt)
