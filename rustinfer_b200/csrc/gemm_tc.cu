@@ -71,7 +71,7 @@ struct Params {
     int epilogue;
     void* out;                           // bf16 or fp32 [tokens][ld_out]; fp32 residual stream for EPI_RESIDUAL
     int ld_out;
-    int vec;                             // rows of out start on 16-byte boundaries: vector stores allowed
+    int vec;                             // rows of out start on 16-byte boundaries (1) or 32-byte ones (2): vector stores allowed
     int splits;
     float* workspace;                    // [tiles][splits][BN][128] fp32
     int* counters;                       // [tiles], zero between calls
@@ -161,35 +161,63 @@ __device__ __forceinline__ void store_one(const Params& p, int n_tok, int n_feat
 }
 
 
-// 16 consecutive features of one token (activations on the 128-row side)
-__device__ __forceinline__ void store_row16(const Params& p, int tok, int feat0, const float (&v)[16]) {
-    if (tok >= p.a_rows) return;
-    if (!p.vec || feat0 + 16 > p.b_rows) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) store_one(p, p.a_rows, p.b_rows, tok, feat0 + j, v[j], j < 15 ? v[j + 1] : 0.f);
-        return;
+// Eight numbers to 32 bytes that lie on a 32-byte boundary, in one store: a thread owns a row, so a warp's store meets 32 rows, and
+// with 16 bytes each it wrote half of a sector in each (2,048 x 5,120 x 1,024 into fp32 40.3 -> 26.9 us, into
+// bf16 26.7 -> 21.3).
+__device__ __forceinline__ void store8(float* dst, const float* v) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+__device__ __forceinline__ void store8(bf16* dst, uint4 lo, uint4 hi) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(dst), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w) : "memory");
+}
+// 16 numbers rounded to bf16
+__device__ __forceinline__ void store16(bool wide, bf16* dst, const float* v) {
+    const uint4 lo = pack8(v), hi = pack8(v + 8);
+    if (wide) {
+        store8(dst, lo, hi);
+    } else {
+        reinterpret_cast<uint4*>(dst)[0] = lo;
+        reinterpret_cast<uint4*>(dst)[1] = hi;
     }
+}
+
+// N (a multiple of 16) consecutive features of one token (activations on the 128-row side), all inside the matrix and with rows that
+// allow vector stores (the caller has checked both)
+template <int N, bool WIDE = true>
+__device__ __forceinline__ void store_cols(const Params& p, int tok, int feat0, const float (&v)[N]) {
+    static_assert(N % 16 == 0, "whole groups");
+    if (tok >= p.a_rows) return;
+    const bool wide = WIDE && p.vec == 2;                    // (at the edge a few stores: one way is enough)
     const size_t row = (size_t)tok * p.ld_out;
     switch (p.epilogue) {
         case EPI_BF16: {
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.out) + row + feat0);
-            dst[0] = pack8(v);
-            dst[1] = pack8(v + 8);
+            bf16* dst = reinterpret_cast<bf16*>(p.out) + row + feat0;
+#pragma unroll
+            for (int j = 0; j < N; j += 16) store16(wide, dst + j, v + j);
             break;
         }
         case EPI_RELU2: {
-            float m[16];
+            bf16* dst = reinterpret_cast<bf16*>(p.out) + row + feat0;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) m[j] = relu2(v[j]);
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.out) + row + feat0);
-            dst[0] = pack8(m);
-            dst[1] = pack8(m + 8);
+            for (int j = 0; j < N; j += 16) {
+                float m[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) m[i] = relu2(v[j + i]);
+                store16(wide, dst + j, m);
+            }
             break;
         }
         case EPI_F32: {
-            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + row + feat0);
+            float* dst = reinterpret_cast<float*>(p.out) + row + feat0;
+            if (wide) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                for (int j = 0; j < N; j += 8) store8(dst + j, v + j);
+            } else {
+#pragma unroll
+                for (int j = 0; j < N; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            }
             break;
         }
         case EPI_RESIDUAL: {
@@ -198,70 +226,52 @@ __device__ __forceinline__ void store_row16(const Params& p, int tok, int feat0,
             // once, so the result does not depend on any order)
             float* dst = reinterpret_cast<float*>(p.out) + row + feat0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < N; j += 4)
                 asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                             ::"l"(dst + 4 * j), "f"(v[4 * j]), "f"(v[4 * j + 1]), "f"(v[4 * j + 2]), "f"(v[4 * j + 3]) : "memory");
+                             ::"l"(dst + j), "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]) : "memory");
             break;
         }
         case EPI_SILU: {
-            float m[8];
+            bf16* dst = reinterpret_cast<bf16*>(p.out) + row + (feat0 >> 1);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) m[j] = glu_mul(p, v[2 * j], v[2 * j + 1]);
-            *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.out) + row + (feat0 >> 1)) = pack8(m);
+            for (int j = 0; j < N; j += 16) {
+                float m[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) m[i] = glu_mul(p, v[j + 2 * i], v[j + 2 * i + 1]);
+                *reinterpret_cast<uint4*>(dst + (j >> 1)) = pack8(m);
+            }
             break;
         }
     }
 }
 
-
-// 64 consecutive features of one token, all inside the matrix and with rows that allow vector
-// stores (the caller has checked both for the whole warp)
-__device__ __forceinline__ void store_row64(const Params& p, int tok, int feat0, const float (&v)[64]) {
-    if (tok >= p.a_rows) return;
-    const size_t row = (size_t)tok * p.ld_out;
-    switch (p.epilogue) {
-        case EPI_BF16: {
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.out) + row + feat0);
+// The same at the matrix's ragged edge, or where rows allow no vectors: whole groups of 16, then element by element.  In loops, on a
+// copy in local memory: unrolled into a tile's code it was ten thousand instructions that the tile ran through once, each from memory
+// (a last tile of 32 columns in 256: 1,024 x 3,104 x 2,048 32.5 -> 16.4 us; 300 x 5,152 x 1,024 30.3 -> 11.5).
+template <int N>
+__device__ __forceinline__ void store_ragged(const Params& p, int tok, int feat0, const float (&v)[N]) {
+    float kept[N];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) dst[j] = pack8(v + 8 * j);
-            break;
+    for (int j = 0; j < N; ++j) kept[j] = v[j];
+    int at = 0;
+    if (p.vec) {
+#pragma unroll 1
+        for (; at < N && feat0 + at + 16 <= p.b_rows; at += 16) {
+            float w[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) w[j] = kept[at + j];
+            store_cols<16, false>(p, tok, feat0 + at, w);
         }
-        case EPI_RELU2: {
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.out) + row + feat0);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                float m[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) m[j] = relu2(v[8 * q + j]);
-                dst[q] = pack8(m);
-            }
-            break;
-        }
-        case EPI_F32: {
-            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + row + feat0);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            break;
-        }
-        case EPI_RESIDUAL: {
-            float* dst = reinterpret_cast<float*>(p.out) + row + feat0;
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                             ::"l"(dst + 4 * j), "f"(v[4 * j]), "f"(v[4 * j + 1]), "f"(v[4 * j + 2]), "f"(v[4 * j + 3]) : "memory");
-            break;
-        }
-        case EPI_SILU: {
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.out) + row + (feat0 >> 1));
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float m[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) m[j] = glu_mul(p, v[16 * q + 2 * j], v[16 * q + 2 * j + 1]);
-                dst[q] = pack8(m);
-            }
-            break;
-        }
+    }
+#pragma unroll 1
+    for (; at < N && feat0 + at < p.b_rows; ++at) store_one(p, p.a_rows, p.b_rows, tok, feat0 + at, kept[at], kept[at | 1]);
+}
+template <int N>
+__device__ __forceinline__ void store_row(const Params& p, int tok, int feat0, const float (&v)[N]) {
+    if (p.vec && feat0 + N <= p.b_rows) {
+        store_cols<N>(p, tok, feat0, v);
+    } else if (feat0 < p.b_rows) {
+        store_ragged<N>(p, tok, feat0, v);
     }
 }
 
@@ -287,17 +297,12 @@ __device__ __forceinline__ void finish_sums(const Params& p, int tile, int tok, 
 #pragma unroll
             for (int j = 0; j < BN; ++j) sum[j] += __ldcg(base + (size_t)s * (BN * 128) + (size_t)j * 128);
     }
-    if (p.vec && b0 + BN <= p.b_rows) {
 #pragma unroll
-        for (int c0 = 0; c0 < BN; c0 += 64) {
-            float v[64];
+    for (int c0 = 0; c0 < BN; c0 += 64) {
+        float v[64];
 #pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = sum[c0 + j];
-            store_row64(p, tok, b0 + c0, v);
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < BN; ++j) store_one(p, p.a_rows, p.b_rows, tok, b0 + j, sum[j], j + 1 < BN ? sum[j + 1] : 0.f);
+        for (int j = 0; j < 64; ++j) v[j] = sum[c0 + j];
+        store_row<64>(p, tok, b0 + c0, v);
     }
 }
 
@@ -554,7 +559,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         for (int j = 0; j < 16; ++j) v[j] = 0.f;
                     }
                     if (!p.swap) {
-                        store_row16(p, ra, b0 + c0, v);
+                        store_row<16>(p, ra, b0 + c0, v);
                     } else if (p.epilogue == EPI_SILU) {
                         // lanes alternate gate, up: the even lane needs its odd neighbour's value
 #pragma unroll
@@ -746,10 +751,11 @@ __device__ __forceinline__ void rope_rows(const Params& p, unsigned taddr, int t
                         hi[k] = lo[k] * r.s[k] + hi[k] * r.c[k];
                         lo[k] = y1;
                     }
+                    const bool wide = (reinterpret_cast<uintptr_t>(dst) & 31) == 0;
 #pragma unroll
-                    for (int k = 0; k < 32; k += 8) {
-                        *reinterpret_cast<uint4*>(dst + i0 + k) = pack8(lo + k);
-                        *reinterpret_cast<uint4*>(dst + half + i0 + k) = pack8(hi + k);
+                    for (int k = 0; k < 32; k += 16) {
+                        store16(wide, dst + i0 + k, lo + k);
+                        store16(wide, dst + half + i0 + k, hi + k);
                     }
                 }
             } else if (i0 == 0) {
@@ -759,8 +765,9 @@ __device__ __forceinline__ void rope_rows(const Params& p, unsigned taddr, int t
                     float v[32];
                     tmem_ld_row<32>(taddr + c0 + j0, v);
                     if (live && dst) {
+                        const bool wide = (reinterpret_cast<uintptr_t>(dst) & 31) == 0;
 #pragma unroll
-                        for (int k = 0; k < 32; k += 8) *reinterpret_cast<uint4*>(dst + j0 + k) = pack8(v + k);
+                        for (int k = 0; k < 32; k += 16) store16(wide, dst + j0 + k, v + k);
                     }
                 }
             }
@@ -798,6 +805,9 @@ __device__ __forceinline__ bool pair_item(const Params& p, int pair, int pairs, 
     return true;
 }
 
+// EDGE: the features are no whole groups of 64, or rows of the output allow no vectors (a kernel of its own: the code for the edge cost
+// a product of 2,048 x 16,384 x 2,048 without one 2 to 4 %).
+template <bool EDGE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const Params p) {
@@ -954,40 +964,42 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (finish && p.epilogue == EPI_ROPE) {
                 rope_rows(p, taddr, ra, b0, BN, rr);
             } else if (finish) {
-                // 64 columns a round trip to tensor memory where the tile lies inside the matrix:
-                // the epilogue of a pair's last tile has no MMA to hide behind.  At the ragged
-                // edge 16 at a time, element by element.
+                // 64 columns a round trip to tensor memory: the epilogue of a pair's last tile has no MMA to hide
+                // behind.  At the matrix's edge 16 at a time.
+                auto parts_sum = [&](int col, auto& v) {         // the tile's columns from `col` on, part by part
+                    constexpr int Q = sizeof(v) / 16;
+#pragma unroll
+                    for (int j = 0; j < 4 * Q; ++j) v[j] = 0.f;
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 64) {
-                    float v[64];
-                    if (meet) {
+                    for (int pr = first_pair; pr < first_pair + parts; ++pr) {
+                        const int seg = sk_start(p, pr) < sk_tile * n_kb ? 1 : 0;
+                        const float* src = p.sk_acc + (size_t)(pr * 2 + seg) * slot_floats + warp_off;
+                        float4 x[Q];
 #pragma unroll
-                        for (int j = 0; j < 64; ++j) v[j] = 0.f;
-#pragma unroll 1
-                        for (int pr = first_pair; pr < first_pair + parts; ++pr) {
-                            const int seg = sk_start(p, pr) < sk_tile * n_kb ? 1 : 0;
-                            const float* src = p.sk_acc + (size_t)(pr * 2 + seg) * slot_floats + warp_off;
-                            float4 x[16];
+                        for (int j = 0; j < Q; ++j) x[j] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(col / 4 + j) * 128));
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) x[j] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(c0 / 4 + j) * 128));
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                v[4 * j] += x[j].x; v[4 * j + 1] += x[j].y; v[4 * j + 2] += x[j].z; v[4 * j + 3] += x[j].w;
-                            }
+                        for (int j = 0; j < Q; ++j) {
+                            v[4 * j] += x[j].x; v[4 * j + 1] += x[j].y; v[4 * j + 2] += x[j].z; v[4 * j + 3] += x[j].w;
                         }
-                    } else {
-                        tmem_ld_row<64>(taddr + c0, v);
                     }
-                    if (p.vec && b0 + c0 + 64 <= p.b_rows) {
-                        store_row64(p, ra, b0 + c0, v);
-                    } else {
-#pragma unroll
-                        for (int c1 = 0; c1 < 64; c1 += 16) {
-                            float w[16];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) w[j] = v[c1 + j];
-                            store_row16(p, ra, b0 + c0 + c1, w);
-                        }
+                };
+                int c0 = 0;
+                if (!EDGE || p.vec) {
+#pragma unroll 1
+                    for (; c0 < BN && b0 + c0 + 64 <= p.b_rows; c0 += 64) {
+                        float v[64];
+                        if (meet) parts_sum(c0, v);
+                        else tmem_ld_row<64>(taddr + c0, v);
+                        store_cols<64>(p, ra, b0 + c0, v);
+                    }
+                }
+                if constexpr (EDGE) {
+#pragma unroll 1
+                    for (; c0 < BN && b0 + c0 < p.b_rows; c0 += 16) {
+                        float v[16];
+                        if (meet) parts_sum(c0, v);
+                        else tmem_ld16(taddr + c0, v);
+                        store_row<16>(p, ra, b0 + c0, v);
                     }
                 }
             }
@@ -1006,17 +1018,22 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }
 
 int device_sms() { return ri_device_sms(); }
+int vector_rows(const void* out, size_t row_bytes) {
+    const uintptr_t low = reinterpret_cast<uintptr_t>(out) | row_bytes;
+    return low % 32 == 0 ? 2 : low % 16 == 0 ? 1 : 0;
+}
 
+template <bool EDGE>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t s) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TOTAL);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TOTAL);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
     const int sms = device_sms();
     const int pairs = (p.sk_tiles == 0 && p.n_tiles < sms / 2) ? p.n_tiles : sms / 2;
-    RI_CHECKED(ri_launch(gemm_tc_pair_kernel, dim3(2 * pairs), dim3(THREADS), (size_t)p.budget + SMEM_EXTRA, s, ma, mb, p));
+    RI_CHECKED(ri_launch(gemm_tc_pair_kernel<EDGE>, dim3(2 * pairs), dim3(THREADS), (size_t)p.budget + SMEM_EXTRA, s, ma, mb, p));
     return ri_launch_status();
 }
 }  // namespace
@@ -1101,7 +1118,7 @@ int gemm_tc_impl(const void* X, const void* W, int M, int N, int K, void* out, i
     const int tiles_b = (p.b_rows + bn - 1) / bn;
     p.n_tiles = p.tiles_a * tiles_b;
     const int esize = (epilogue == EPI_BF16 || epilogue == EPI_SILU || epilogue == EPI_RELU2) ? 2 : 4;
-    p.vec = ((reinterpret_cast<uintptr_t>(out) & 15) == 0 && ((size_t)ld_out * esize) % 16 == 0) ? 1 : 0;
+    p.vec = vector_rows(out, (size_t)ld_out * esize);
     CUtensorMap ma, mb;
     p.a_box = a_box;
     p.stage_bytes = (a_box + bn) * BK * 2;
@@ -1172,7 +1189,7 @@ int gemm_tc_impl(const void* X, const void* W, int M, int N, int K, void* out, i
         if (stp != 0) return stp;
         stp = make_map(B, p.b_rows, K, p.pair_bn / 2, &mb);
         if (stp != 0) return stp;
-        return launch_pair(ma, mb, p, (cudaStream_t)stream);
+        return p.b_rows % 64 == 0 && p.vec ? launch_pair<false>(ma, mb, p, (cudaStream_t)stream) : launch_pair<true>(ma, mb, p, (cudaStream_t)stream);
     }
     if (rope) return (int)cudaErrorNotSupported;           // only the CTA-pair kernel has that epilogue
     int st = make_map(A, p.a_rows, K, a_box, &ma);
@@ -1230,7 +1247,7 @@ RI_API int ri_gemm_tc_grouped(const void* X, const void* W, int rows, int N, int
     p.tiles_a = (rows + BM - 1) / BM + experts;
     p.n_tiles = p.tiles_a * p.grp_tiles_b;
     const int esize = (epilogue == EPI_BF16 || epilogue == EPI_SILU) ? 2 : 4;
-    p.vec = ((reinterpret_cast<uintptr_t>(out) & 15) == 0 && ((size_t)ld_out * esize) % 16 == 0) ? 1 : 0;
+    p.vec = vector_rows(out, (size_t)ld_out * esize);
     p.a_box = BM;
     p.stage_bytes = (BM + bn) * BK * 2;
     p.budget = SMEM_BUDGET;
