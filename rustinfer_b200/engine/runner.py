@@ -16,6 +16,7 @@ launched with an index the kernels could not follow.
 from __future__ import annotations
 
 import gc
+from array import array
 from dataclasses import dataclass, field
 from typing import Any, Dict, List, Optional, Sequence, Tuple
 
@@ -77,6 +78,17 @@ class _Staging:
         ev = torch.cuda.Event()
         ev.record()
         self.events[i] = ev
+
+
+def _flat_ids(entries: Sequence[StepEntry], vocab: int) -> Optional[np.ndarray]:
+    """The entries' ids one after the other if all are integers inside the vocabulary, else None (they are then looked at one by one)."""
+    try:
+        rows = [np.frombuffer(array("q", e.tokens), dtype=np.int64) if isinstance(e.tokens, (list, tuple))
+                else np.asarray(e.tokens, dtype=np.int64) for e in entries]
+        flat = np.concatenate(rows)
+        return flat if flat.min() >= 0 and flat.max() < vocab else None
+    except (TypeError, ValueError, OverflowError):
+        return None
 
 
 class _DecodeGraph:
@@ -367,7 +379,8 @@ class ModelRunner:
         self.cache.close(request_id)
 
     # --------------------------------------------------------------------------- plan
-    def _validate(self, entries: Sequence[StepEntry]) -> None:
+    def _validate(self, entries: Sequence[StepEntry]) -> Optional[np.ndarray]:
+        """Raises `StepError` for a step that cannot be; returns the ids of a step of many tokens as one array (None: as they are)."""
         if not entries:
             raise StepError("a step needs at least one entry")
         if len(entries) > self.max_batch_seqs:
@@ -375,6 +388,7 @@ class ModelRunner:
         seen = set()
         total = 0
         vocab = self.spec.vocab_size
+        ids = _flat_ids(entries, vocab) if any(len(e.tokens) > 8 for e in entries) else None
         for e in entries:
             if e.request_id in seen:
                 raise StepError(f"request {e.request_id!r} appears twice in one step")
@@ -388,16 +402,18 @@ class ModelRunner:
             if self.cache.length(e.request_id) + q > self.max_model_len:
                 raise StepError(f"request {e.request_id!r} would reach {self.cache.length(e.request_id) + q} "
                                 f"tokens, max_model_len is {self.max_model_len}")
-            for t in e.tokens:
-                if not 0 <= int(t) < vocab:
-                    raise StepError(f"request {e.request_id!r}: token id {t} outside [0, {vocab})")
+            if ids is None:
+                for t in e.tokens:
+                    if not 0 <= int(t) < vocab:
+                        raise StepError(f"request {e.request_id!r}: token id {t} outside [0, {vocab})")
             for w in e.want:
                 if not 0 <= int(w) < q:
                     raise StepError(f"request {e.request_id!r}: wanted place {w} outside its {q} tokens")
         if total > self.max_batch_tokens:
             raise StepError(f"{total} tokens exceed max_batch_tokens {self.max_batch_tokens}")
+        return ids
 
-    def _build(self, entries: Sequence[StepEntry]) -> Tuple[StepContext, Optional[torch.Tensor]]:
+    def _build(self, entries: Sequence[StepEntry], ids: Optional[np.ndarray]) -> Tuple[StepContext, Optional[torch.Tensor]]:
         ps = self.page_size
         B = len(entries)
         q_lens = np.fromiter((len(e.tokens) for e in entries), dtype=np.int64, count=B)
@@ -405,7 +421,7 @@ class ModelRunner:
         cu_q = np.zeros(B + 1, dtype=np.int64)
         np.cumsum(q_lens, out=cu_q[1:])
         T = int(cu_q[-1])
-        token_ids = np.concatenate([np.asarray(e.tokens, dtype=np.int64) for e in entries])
+        token_ids = ids if ids is not None else np.concatenate([np.asarray(e.tokens, dtype=np.int64) for e in entries])
         entry_of_token = np.repeat(np.arange(B), q_lens)
         positions = np.arange(T) - cu_q[entry_of_token] + pos0[entry_of_token]
         kv_len = pos0 + q_lens
@@ -419,16 +435,20 @@ class ModelRunner:
         sections: List[np.ndarray] = [token_ids, positions, cu_q, kv_len, slots,
                                       np.asarray(rows, dtype=np.int64)]
         max_blocks = int(((kv_len + ps - 1) // ps).max())
+        block_of_token = positions // ps
+        offset_in_page = positions - block_of_token * ps
+        at_table = entry_of_token * max_blocks + block_of_token          # a token's place in the tables below, flattened
         for gi in self.layout.paged_groups():
-            table = np.zeros((B, max_blocks), dtype=np.int64)
-            for i, e in enumerate(entries):
+            pages: List[int] = []
+            for e in entries:
                 t = self.cache.block_table(e.request_id, gi)
-                n = min(len(t), max_blocks)
-                table[i, :n] = t[:n]
-            page_of_token = table[entry_of_token, positions // ps]
-            if (page_of_token < 0).any():
+                pages += t[:max_blocks]
+                pages += [0] * (max_blocks - len(t))
+            table = np.array(pages, dtype=np.int64).reshape(B, max_blocks)
+            page_of_token = table.reshape(-1)[at_table]
+            if page_of_token.min() < 0:
                 raise StepError("a token would be written to a page that was given back")
-            slot_of_token = page_of_token * ps + positions % ps
+            slot_of_token = page_of_token * ps + offset_in_page
             np.maximum(table, 0, out=table)
             sections += [table.reshape(-1), slot_of_token]
         sections.append(np.asarray(row_slots, dtype=np.int64))
@@ -449,7 +469,7 @@ class ModelRunner:
         self._staging.upload(idx, at)
         self.h2d_bytes_last = at * 4
         dev = self._staging.dev
-        views = [dev[o: o + n] for o, n in offsets]
+        views = [v if v.numel() == n else v[:n] for v, (_o, n) in zip(dev[:at].split([(n + 3) & ~3 for _o, n in offsets]), offsets)]
         it = iter(views[6:])
         groups = []
         for _ in self.layout.paged_groups():
@@ -477,7 +497,7 @@ class ModelRunner:
         in a step of single tokens: the ids chosen by the last step need not visit the host
         before they are fed back.  With `borrow_logits` the result may be a view of a buffer
         that the next step overwrites (for callers that consume it at once)."""
-        self._validate(entries)
+        ids = self._validate(entries)
         lease = self.cache.lease([(e.request_id, len(e.tokens)) for e in entries])
         try:
             self._zero_new_state()
@@ -487,7 +507,7 @@ class ModelRunner:
                 if logits is not None and not borrow_logits:
                     logits = logits.clone()
             else:
-                step, rows = self._build(entries)
+                step, rows = self._build(entries, ids)
                 if device_tokens is not None:
                     if not step.decode_only:
                         raise StepError("device_tokens only stands for steps of single tokens")
@@ -556,7 +576,14 @@ class ModelRunner:
         new = self.cache.newly_opened_slots
         if not new:
             return
+        slots = sorted(set(new))
+        runs, at = [], 0                                      # neighbouring slots in one go, without an index on the device
+        for i in range(1, len(slots) + 1):
+            if i == len(slots) or slots[i] != slots[i - 1] + 1:
+                runs.append((slots[at], slots[i - 1] + 1))
+                at = i
         for gi, g in enumerate(self.layout.groups):
             if isinstance(g.need, FixedState):
-                self.group_storage[gi][:, new] = 0
+                for a, b in runs:
+                    self.group_storage[gi][:, a:b].zero_()
         new.clear()

@@ -194,7 +194,11 @@ def gemm_tc_plan(M: int, N: int, K: int, num_sms: Optional[int] = None, epilogue
     """(swap, bn, splits, a_box): which operand sits on the 128-row side of the MMA, the
     tile of the other one, how many K slices, and how many rows of the 128 a tile really
     covers, so that about one even wave of CTAs covers the GPU."""
-    num_sms = num_sms or L.num_sms()
+    return _gemm_tc_plan(M, N, K, num_sms or L.num_sms(), epilogue)
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_tc_plan(M: int, N: int, K: int, num_sms: int, epilogue: int):
     if M <= 64:
         swap, bn = 1, (16 if M <= 16 else 32 if M <= 32 else 64)
         tiles = -(-N // 128)
