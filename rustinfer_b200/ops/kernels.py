@@ -199,7 +199,12 @@ def gemm_tc_plan(M: int, N: int, K: int, num_sms: Optional[int] = None, epilogue
 
 @functools.lru_cache(maxsize=4096)
 def _gemm_tc_plan(M: int, N: int, K: int, num_sms: int, epilogue: int):
-    if M <= 64:
+    # Weights on the 128-row side for few tokens.  From 33 on the activations: 33 to 64 tokens in tiles of 64 of them, whose K slices meet
+    # feature by feature, took 17 to 20 us where the tiles of a prompt take 9 to 11 (64 x 2,048 x 2,048 19.9 -> 10.0, 64 x 1,536 x 1,024 with
+    # gates 23.4 -> 8.9, 64 x 16,384 x 2,048 32.0 -> 18.2, 40 x 4,096 x 14,336 38.7 -> 33.1).  Slices that are added into the stream need no
+    # meeting (64 x 2,048 x 2,048 6.4 against 10.3), and a stream of weights that fills the SMs for several waves stays ahead with a
+    # handful of tokens more (36 x 28,672 x 4,096 54.8 against 55.4).
+    if M <= 32 or (M <= 64 and epilogue == EPI_RESIDUAL) or (M <= 36 and N * K >= 1 << 26):
         swap, bn = 1, (16 if M <= 16 else 32 if M <= 32 else 64)
         tiles = -(-N // 128)
     else:

@@ -27,3 +27,17 @@ def test_columns_at_the_edge(plan, N, epilogue):
     K.gemm_tc(x, w[:N].contiguous(), got, epi, plan)
     assert torch.equal(got, want[:, : N // half])
     assert (block[M * (N // half):] == 7.0).all()
+
+
+@pytest.mark.parametrize("M", [33, 36, 37, 64])
+@pytest.mark.parametrize("N,Kd", [(2048, 1024), (72, 2048), (3104, 520), (16, 1024)])
+def test_rows_from_33_on_as_in_a_prompt(M, N, Kd):
+    """33 to 64 rows go the way of 65: their sums have the bits they have there."""
+    from rustinfer_b200.ops import kernels as K
+    torch.manual_seed(Kd)
+    x, w = torch.randn(65, Kd, device=DEV).bfloat16(), torch.randn(N, Kd, device=DEV).bfloat16()
+    for epi, dt in ((K.EPI_F32, torch.float32), (K.EPI_BF16, torch.bfloat16)):
+        few, many = torch.empty(M, N, dtype=dt, device=DEV), torch.empty(65, N, dtype=dt, device=DEV)
+        K.gemm_tc(x[:M], w, few, epi)
+        K.gemm_tc(x, w, many, epi)
+        assert torch.equal(few, many[:M])
