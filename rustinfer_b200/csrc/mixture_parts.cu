@@ -29,9 +29,19 @@ __device__ __forceinline__ void warp_argmax(float& v, int& idx) {
     }
 }
 
-// TT tokens a CTA (a row of the router's matrix is read once for them), each warp a few experts at a time.
-constexpr int ROUTE_CHUNK = 8;
+// The place of lane `lane`'s value among those of the lanes in `live`, the largest first, the lowest lane among equals.
+__device__ __forceinline__ int warp_rank(float v, unsigned live, int lane) {
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        const float o = __shfl_sync(0xffffffffu, v, j);
+        rank += (live >> j & 1u) && (o > v || (o == v && j < lane)) ? 1 : 0;
+    }
+    return rank;
+}
 
+// TT tokens a CTA (a row of the router's matrix is read once for them), each warp a few experts at a time.  8 tokens of 1,024, 33 rows: 15.5 ->
+// 7.5 us; up to 32 experts (and groups) are ranked in registers, all at once, instead of found one after the other.
 template <typename TX, int TT>
 __global__ void __launch_bounds__(512)
 moe_route_kernel(const float* __restrict__ z, const TX* __restrict__ x, const float* __restrict__ router,
@@ -48,8 +58,10 @@ moe_route_kernel(const float* __restrict__ z, const TX* __restrict__ x, const fl
     const int rows = E + (gate && x ? 1 : 0);
     const int per_token = rows + E + n_groups;
     if (x) {
-        // the logits: the warps share the experts, a few (at most eight) at a time; a lane takes every 32nd term of
-        // their sums for every token (x and the matrix are read once for all), then the lanes' parts meet in a butterfly
+        // the logits: the warps share the experts, a few at a time; a lane takes every 32nd term of their sums for every
+        // token (x and the matrix are read once for all), AHEAD of them asked for together (a step's few tokens wait
+        // for nothing but these loads), then the lanes' parts meet in a butterfly
+        constexpr int ROUTE_CHUNK = TT == 1 ? 4 : 8, AHEAD = TT == 1 ? 16 : 4;
         const int ch = min(ROUTE_CHUNK, (rows + warps - 1) / warps);
         for (int e0 = warp * ch; e0 < rows; e0 += warps * ch) {
             const int ne = min(ch, rows - e0);
@@ -58,18 +70,23 @@ moe_route_kernel(const float* __restrict__ z, const TX* __restrict__ x, const fl
             for (int j = 0; j < ROUTE_CHUNK; ++j)
 #pragma unroll
                 for (int k = 0; k < TT; ++k) acc[j][k] = 0.f;
-#pragma unroll 4
-            for (int i = lane; i < d; i += 32) {
-                float xv[TT];
+#pragma unroll 1
+            for (int i0 = lane; i0 < d; i0 += 32 * AHEAD) {
+                float xv[AHEAD][TT], w[ROUTE_CHUNK][AHEAD];
 #pragma unroll
-                for (int k = 0; k < TT; ++k) xv[k] = to_f32<TX>(x[(size_t)min(t0 + k, T - 1) * d + i]);
+                for (int n = 0; n < AHEAD; ++n) {
+                    const int i = i0 + 32 * n;
 #pragma unroll
-                for (int j = 0; j < ROUTE_CHUNK; ++j)
-                    if (j < ne) {
-                        const float w = router[(size_t)(e0 + j) * d + i];
+                    for (int k = 0; k < TT; ++k) xv[n][k] = i < d ? to_f32<TX>(x[(size_t)min(t0 + k, T - 1) * d + i]) : 0.f;
 #pragma unroll
-                        for (int k = 0; k < TT; ++k) acc[j][k] = fmaf(xv[k], w, acc[j][k]);
-                    }
+                    for (int j = 0; j < ROUTE_CHUNK; ++j) w[j][n] = j < ne && i < d ? router[(size_t)(e0 + j) * d + i] : 0.f;
+                }
+#pragma unroll
+                for (int n = 0; n < AHEAD; ++n)
+#pragma unroll
+                    for (int j = 0; j < ROUTE_CHUNK; ++j)
+#pragma unroll
+                        for (int k = 0; k < TT; ++k) acc[j][k] = fmaf(xv[n][k], w[j][n], acc[j][k]);
             }
 #pragma unroll
             for (int j = 0; j < ROUTE_CHUNK; ++j)
@@ -116,6 +133,12 @@ moe_route_kernel(const float* __restrict__ z, const TX* __restrict__ x, const fl
             gs[g] = per > 1 && !group_max ? a + b : a;
         }
         __syncwarp();
+        const float mine = lane < n_groups ? gs[lane] : -INFINITY;
+        if (n_groups <= 32 && __all_sync(0xffffffffu, mine < INFINITY)) {        // (a number that is none, too, goes the other way)
+            const int rank = warp_rank(mine, n_groups < 32 ? (1u << n_groups) - 1u : 0xffffffffu, lane);
+            if (lane < n_groups && rank < keep) gs[lane] = INFINITY;
+            __syncwarp();
+        } else
         // the `keep` best groups get +inf as a mark, one by one
         for (int r = 0; r < keep; ++r) {
             float best = -INFINITY;
@@ -133,6 +156,25 @@ moe_route_kernel(const float* __restrict__ z, const TX* __restrict__ x, const fl
         __syncwarp();
     }
     float wsum = 0.f, zmax = 0.f;
+    if (E <= 32) {
+        const float v = lane < E ? c[lane] : -INFINITY, own = lane < E ? s[lane] : 0.f;
+        const unsigned live = __ballot_sync(0xffffffffu, v > -INFINITY);         // neither cut nor no number
+        if (__popc(live) >= top) {
+            const int place = warp_rank(v, live, lane), rank = live >> lane & 1u ? place : 32;
+            __syncwarp();
+            if (score == 1) zmax = __shfl_sync(0xffffffffu, own, __ffs(__ballot_sync(0xffffffffu, rank == 0)) - 1);
+            const float part = score == 1 ? expf(own - zmax) : own;
+            if (rank < top) c[rank] = part;                // in the order of the choices, as their sum is taken
+            __syncwarp();
+            for (int r = 0; r < top; ++r) wsum += c[r];
+            if (rank < top) {
+                ids[(size_t)t * top + rank] = lane;
+                weights[(size_t)t * top + rank] = score == 1 ? part / wsum : renorm ? own / (wsum + renorm_eps) : own;
+                atomicAdd(counts + lane, 1);
+            }
+            return;
+        }
+    }
     for (int r = 0; r < top; ++r) {
         float best = -INFINITY;
         int bi = 0x7fffffff;
@@ -236,6 +278,34 @@ __device__ __forceinline__ float glu_pair(float g, float u, const GluAct& act) {
     return g / (1.0f + (FAST ? __expf(-g) : expf(-g))) * u;
 }
 
+// {expert, first row, rows} of tile `tile` of BM rows among all experts' (expert E: there is none), by one warp
+template <int BM>
+__device__ __forceinline__ void find_tile(const int* __restrict__ offsets, int E, int tile, int* out) {
+    const int lane = threadIdx.x & 31;
+    int base = 0, e = E, row0 = 0, n_rows = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+        const int i = e0 + lane, lo = i < E ? offsets[i] : 0, cnt = i < E ? offsets[i + 1] - lo : 0;
+        const int tiles = (cnt + BM - 1) / BM;
+        int sum = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += up;
+        }
+        const int at = tile - base - (sum - tiles);          // the tile's number in this lane's expert
+        const unsigned hit = __ballot_sync(0xffffffffu, at >= 0 && at < tiles);
+        if (hit) {
+            const int src = __ffs(hit) - 1, a = __shfl_sync(0xffffffffu, at, src);
+            e = e0 + src;
+            row0 = __shfl_sync(0xffffffffu, lo, src) + a * BM;
+            n_rows = min(BM, __shfl_sync(0xffffffffu, cnt, src) - a * BM);
+            break;
+        }
+        base += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) { out[0] = e; out[1] = row0; out[2] = n_rows; }
+}
+
 template <typename TA, typename TW, typename TO, int BM, bool GATED>
 __global__ void __launch_bounds__(256)
 moe_product_kernel(const TA* __restrict__ a, int a_stride, const TW* __restrict__ w, TO* __restrict__ out,
@@ -249,16 +319,7 @@ moe_product_kernel(const TA* __restrict__ a, int a_stride, const TW* __restrict_
     __shared__ float As[BM][GBK + 1];
     __shared__ float Ws[GBN][GBK + 1];
     __shared__ int s_tile[3];                              // expert, first row, rows
-    if (threadIdx.x == 0) {
-        int tile = blockIdx.x, e = 0, row0 = 0, n_rows = 0;
-        for (; e < E; ++e) {
-            const int lo = offsets[e], cnt = offsets[e + 1] - lo;
-            const int tiles = (cnt + BM - 1) / BM;
-            if (tile < tiles) { row0 = lo + tile * BM; n_rows = min(BM, cnt - tile * BM); break; }
-            tile -= tiles;
-        }
-        s_tile[0] = e; s_tile[1] = row0; s_tile[2] = n_rows;
-    }
+    if (threadIdx.x < 32) find_tile<BM>(offsets, E, blockIdx.x, s_tile);
     __syncthreads();
     const int e = s_tile[0], row0 = s_tile[1], n_rows = s_tile[2];
     if (e >= E || n_rows <= 0) return;
@@ -325,10 +386,10 @@ moe_product_kernel(const TA* __restrict__ a, int a_stride, const TW* __restrict_
 
 // The same products for bf16 rows and matrices on the tensor cores (mma.sync m16n8k16, fp32 accumulation):
 // a CTA of four warps owns BM rows x 64 columns of one expert, a warp 16 of the columns; rows and matrix
-// rows arrive by cp.async in 16-byte pieces through a ring of three stages of 64 k each (the rows gathered
+// rows arrive by cp.async in 16-byte pieces through a ring of three or four stages (STAGES) of 64 k each (the rows gathered
 // through `order`), fragments by ldmatrix from rows padded by 16 bytes.  K must be a multiple of 8 and the
 // rows 16-byte aligned; other shapes take the kernel above.
-constexpr int TBK = 64, TROW = TBK + 8, TSTAGES = 3;
+constexpr int TBK = 64, TROW = TBK + 8;
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -348,11 +409,11 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int BM> constexpr size_t moe_mma_smem() {
-    return (size_t)TSTAGES * (BM + GBN) * TROW * sizeof(bf16);
+template <int BM, int STAGES> constexpr size_t moe_mma_smem() {
+    return (size_t)STAGES * (BM + GBN) * TROW * sizeof(bf16);
 }
 
-template <typename TO, int BM, bool GATED>
+template <typename TO, int BM, bool GATED, int STAGES>
 __global__ void __launch_bounds__(128)
 moe_product_mma_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __restrict__ w, TO* __restrict__ out,
                        int out_stride, const int* __restrict__ offsets, const int* __restrict__ order, int top,
@@ -365,16 +426,7 @@ moe_product_mma_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __r
     bf16* sm = reinterpret_cast<bf16*>(smem_raw);
     __shared__ int s_tile[3];
     __shared__ int s_src[BM];                              // row of `a` behind every row of the tile (-1: none)
-    if (threadIdx.x == 0) {
-        int tile = blockIdx.x, e = 0, row0 = 0, n_rows = 0;
-        for (; e < E; ++e) {
-            const int lo = offsets[e], cnt = offsets[e + 1] - lo;
-            const int tiles = (cnt + BM - 1) / BM;
-            if (tile < tiles) { row0 = lo + tile * BM; n_rows = min(BM, cnt - tile * BM); break; }
-            tile -= tiles;
-        }
-        s_tile[0] = e; s_tile[1] = row0; s_tile[2] = n_rows;
-    }
+    if (threadIdx.x < 32) find_tile<BM>(offsets, E, blockIdx.x, s_tile);
     __syncthreads();
     const int e = s_tile[0], row0 = s_tile[1], n_rows = s_tile[2];
     if (e >= E || n_rows <= 0) return;
@@ -410,16 +462,16 @@ moe_product_mma_kernel(const bf16* __restrict__ a, int a_stride, const bf16* __r
         for (int j = 0; j < 2; ++j) acc[m][j][0] = acc[m][j][1] = acc[m][j][2] = acc[m][j][3] = 0.f;
 
 #pragma unroll
-    for (int st = 0; st < TSTAGES - 1; ++st) {
+    for (int st = 0; st < STAGES - 1; ++st) {
         if (st < kblocks) load_stage(st, st);
         cp_async_commit();
     }
     for (int kb = 0; kb < kblocks; ++kb) {
-        cp_async_wait<TSTAGES - 2>();
+        cp_async_wait<STAGES - 2>();
         __syncthreads();                                   // stage kb has landed; stage kb-1 is free for all
-        if (kb + TSTAGES - 1 < kblocks) load_stage(kb + TSTAGES - 1, (kb + TSTAGES - 1) % TSTAGES);
+        if (kb + STAGES - 1 < kblocks) load_stage(kb + STAGES - 1, (kb + STAGES - 1) % STAGES);
         cp_async_commit();
-        const bf16* As = sm + (size_t)(kb % TSTAGES) * STAGE;
+        const bf16* As = sm + (size_t)(kb % STAGES) * STAGE;
         const bf16* Ws = As + BM * TROW;
 #pragma unroll
         for (int ks = 0; ks < TBK / 16; ++ks) {
@@ -564,17 +616,21 @@ RI_API int ri_moe_product(const void* a, int a_dtype, int a_stride, const void* 
     const bool tensor_cores = a_dtype == RI_BF16 && w_dtype == RI_BF16 && K % 8 == 0 && a_stride % 8 == 0 &&
                               ((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0 && ri_moe_tensor_cores();
     if (tensor_cores && ((gated && out_dtype == RI_BF16) || (!gated && out_dtype == RI_F32))) {
-#define RI_MM(TO, BM, G) do { \
+        // Four stages where few rows leave a CTA waiting for its own matrix (8 tokens, 32 experts of 1,024 x 768, four a token: the layer 46.7
+        // us against 54.5 with three, 52.8 with five) and where K is long (2,048 x 1,536, 64 tokens: 166 against 173); three where CTAs fill the
+        // SMs six times over (1,024 x 768, 64 tokens: 70.8 against 73.9).
+        const bool deep = bm == 16 && (rows <= E || K >= 1536);
+#define RI_MM(TO, BM, G, S) do { \
         static bool configured = false; \
-        const size_t smem = moe_mma_smem<BM>(); \
+        const size_t smem = moe_mma_smem<BM, S>(); \
         if (!configured) { \
-            cudaError_t ce = cudaFuncSetAttribute(moe_product_mma_kernel<TO, BM, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            cudaError_t ce = cudaFuncSetAttribute(moe_product_mma_kernel<TO, BM, G, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             if (ce != cudaSuccess) return (int)ce; \
             configured = true; } \
-        RI_CHECKED(ri_launch(moe_product_mma_kernel<TO, BM, G>, grid, dim3(128), smem, s, (const bf16*)a, a_stride, (const bf16*)w, \
+        RI_CHECKED(ri_launch(moe_product_mma_kernel<TO, BM, G, S>, grid, dim3(128), smem, s, (const bf16*)a, a_stride, (const bf16*)w, \
             (TO*)out, out_stride, offsets, order, top, gather, E, N, K, act)); } while (0)
-        if (gated) { if (bm == 64) RI_MM(bf16, 64, true); else RI_MM(bf16, 16, true); }
-        else { if (bm == 64) RI_MM(float, 64, false); else RI_MM(float, 16, false); }
+        if (gated) { if (bm == 64) RI_MM(bf16, 64, true, 3); else if (deep) RI_MM(bf16, 16, true, 4); else RI_MM(bf16, 16, true, 3); }
+        else { if (bm == 64) RI_MM(float, 64, false, 3); else if (deep) RI_MM(float, 16, false, 4); else RI_MM(float, 16, false, 3); }
 #undef RI_MM
         return ri_launch_status();
     }
