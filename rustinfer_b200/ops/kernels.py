@@ -1276,12 +1276,13 @@ def recurrent_state_rows(key_dim: int) -> int:
 
 
 CHUNK_TOKENS = 64               # tokens of a chunk (recurrent_chunks.cu)
-# tokens from which an entry can go in chunks: 16 heads of 128 x 128 take 38.8 us either way at 256 tokens with one decay a head (270
-# against 107 us at 2,048); 8 heads of 128 x 256 with one a channel 43 against 63 us at 256, 81 against 65 at 512, 312 against 154 at 2,048
+# tokens from which an entry can go in chunks.  Layers in a walk and in chunks: one decay a head, 16 heads of 128 x 128, 256 tokens 76.5 and
+# 78.7 us, 384 99 and 89, 2,048 367 and 199; one a channel, 8 heads of 128 x 256, 384 tokens 107 and 107, 512 128 and 112, 2,048 297 and 197
 CHUNK_MIN_TOKENS, GATED_CHUNK_MIN_TOKENS = 256, 384
 # what the two ways take, in us: a walk so much a token of its longest entry, or of all while its CTAs fill the GPU; chunks a fixed part
-# and so much a token and element of the state (fitted to 1 to 8 entries of 128 to 8,192 tokens, 4 to 64 heads)
-_WALK_US, _CHUNK_FIXED_US, _CHUNK_US = {False: 0.133, True: 0.152}, {False: 25.0, True: 40.0}, {False: 1.7e-7, True: 1.9e-7}
+# and so much a token and element of the state (chosen so that of 112 layers, 1 to 5 entries of 256 to 2,048 tokens, 4 to 64 heads, the
+# fewest go the slower way: three by more than 3 %, at most 9 %)
+_WALK_US, _CHUNK_FIXED_US, _CHUNK_US = {False: 0.133, True: 0.152}, {False: 33.0, True: 38.0}, {False: 9.0e-8, True: 1.5e-7}
 CHUNK_SCRATCH_BYTES = 1288 << 20    # the most scratch a call in chunks takes (1.26 GiB); a call that would take more walks, which takes none
 
 
@@ -1321,10 +1322,9 @@ def _chunks_or_walk(T: int, entries: int, longest: int, heads: int, key_dim: int
 
 
 # the delta rule: 16 heads of 128 x 128 take 90 us in a walk and 86 in chunks at 256 tokens, 175 and 100 at 512, 688 and 246 at 2,048 (8
-# heads: 90 and 79, 171 and 93, 678 and 166); 8 heads of 64 x 64 58 and 48 at 192, 144 and 56 at 512 (fitted to 1 to 5 entries of 128 to
-# 2,048 tokens, 4 to 32 heads)
+# heads: 90 and 79, 171 and 93, 678 and 166); 8 heads of 64 x 64 58 and 48 at 192, 144 and 56 at 512
 DELTA_CHUNK_MIN_TOKENS = 192
-_DELTA_WALK_US, _DELTA_CHUNK_FIXED_US, _DELTA_CHUNK_US = 0.335, 66.0, 3.3e-7
+_DELTA_WALK_US, _DELTA_CHUNK_FIXED_US, _DELTA_CHUNK_US = 0.335, 54.0, 1.9e-7
 
 
 def _delta_chunk_sizes(heads: int, key_dim: int, value_dim: int) -> Tuple[int, ...]:
