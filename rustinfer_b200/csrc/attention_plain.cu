@@ -12,7 +12,7 @@
 // attention on the GPU (crates/infer-backend-cuda/src/kernels/flash_attn_gqa/flash_attn_gqa.h:30).
 //
 // One CTA of 128 threads handles a tile of 16 consecutive query tokens of one request
-// and one q head.  Keys are visited in chunks of KC that start at multiples of KC from
+// and one or two query heads that read the same key head.  Keys are visited in chunks of KC that start at multiples of KC from
 // key 0, with an online softmax; the order of every sum is therefore the same however
 // the tokens were cut into steps or tiles, and so are the bits of the result.
 #include "common.cuh"
@@ -33,9 +33,14 @@ constexpr int QT = 16;                         // query rows per CTA
 constexpr int KC = HD <= 128 ? 64 : 32;        // keys per chunk
 constexpr int THREADS = 128;
 constexpr int NCOL = KC / 8;                   // score columns per thread
-constexpr int NACC = (VD + 7) / 8;             // output dims per thread
-constexpr int QS = HD + 1, KS = HD + 1, PS = KC + 1;
-constexpr size_t SMEM_FLOATS = (size_t)QT * QS + (size_t)KC * KS + (size_t)KC * VD + (size_t)QT * PS;
+constexpr int HP = (HD + 3) / 4 * 4, VP = (VD + 3) / 4 * 4;   // sizes in whole pieces of four
+constexpr int ND4 = (VP / 4 + 7) / 8;          // pieces of an output row per thread: l8, l8 + 8, ...
+// Rows of keys and queries lie an odd number of 16-byte pieces apart: the eight keys that a quarter of a warp reads at once
+// lie in different banks.
+constexpr int QS = 4 * ((HP / 4) | 1), KS = QS, PS = KC + 4;
+constexpr size_t smem_floats(int R) { return (size_t)R * QT * QS + (size_t)KC * KS + (size_t)KC * VP + (size_t)R * QT * PS; }
+// Query heads of one key head a CTA may take, as many as keep a thread's sums in registers (four: the same time or more at every size).
+constexpr int MOST_HEADS = VD <= 256 && HD <= 256 ? 2 : 1;
 
 // What mixers beyond plain grouped-query attention ask for.
 //   softcap > 0      score <- softcap * tanh(score / softcap), after the scale
@@ -67,72 +72,113 @@ __device__ __forceinline__ float gate_of(const Extra& ex, int t, int h) {
     return ex.gate ? ex.gate_scale / (1.0f + expf(-ex.gate[(size_t)t * ex.gate_stride + h])) : 1.f;
 }
 
-// key head and value head of query head h
-__device__ __forceinline__ void heads_of(int h, int Hq, int Hkv, int maps, int& key_head, int& value_head) {
-    const int per = Hq / (Hkv * maps);                   // heads (each of `maps` maps) a kv head
-    value_head = (h / maps) / per;
-    key_head = value_head * maps + h % maps;
+// The keys kb .. kb + KC of one head (keys outside lo .. last as zeros) into dst, rows `stride` apart; N: the elements of a row.
+// Rows of 32-bit values that are whole 16-byte pieces (`pieces`: the cache's pages are aligned too) are copied while the CTA
+// works on; the others, and bf16, pass through registers, eight loads in flight a thread.
+template <int N, typename T>
+__device__ __forceinline__ void stage_keys(float* dst, int stride, const T* cache, const int* bt, size_t page_elems, size_t base,
+                                           int row_elems, int page_size, int kb, int lo, int last, bool pieces) {
+    const int tid = threadIdx.x;
+    if (sizeof(T) == 4 && N % 4 == 0 && pieces) {
+        constexpr int P = N / 4 > 0 ? N / 4 : 1;
+#pragma unroll 4
+        for (int e = tid; e < KC * P; e += THREADS) {
+            const int kk = e / P, d = (e - kk * P) * 4, key = kb + kk;
+            const bool seen = key >= lo && key <= last;
+            const int at = seen ? key : lo;
+            const int blk = at / page_size;
+            const T* src = cache + (size_t)bt[blk] * page_elems + base + (size_t)(at - blk * page_size) * row_elems + d;
+            const unsigned to = (unsigned)__cvta_generic_to_shared(dst + kk * stride + d);
+            const int bytes = seen ? 16 : 0;             // 0: sixteen zeros
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(to), "l"(src), "r"(bytes) : "memory");
+        }
+    } else {
+#pragma unroll 8
+        for (int e = tid; e < KC * N; e += THREADS) {
+            const int kk = e / N, d = e - kk * N, key = kb + kk;
+            const bool seen = key >= lo && key <= last;
+            const int at = seen ? key : lo;
+            const int blk = at / page_size;
+            const T* src = cache + (size_t)bt[blk] * page_elems + base + (size_t)(at - blk * page_size) * row_elems + d;
+            dst[kk * stride + d] = seen ? to_f32<T>(*src) : 0.f;
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-template <typename T, typename TO>
+// Scores of this thread's token for R heads against the keys l8 + 8 c: each one sum over the channels in ascending order.
+template <int R, int N>
+__device__ __forceinline__ void scores_of(float (&s)[R][NCOL], const float* qr, const float* kr) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < N; ++c) s[r][c] = 0.f;
+#pragma unroll (R == 1 ? 2 : 1)
+    for (int d = 0; d < HP; d += 4) {
+        float4 qv[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) qv[r] = *reinterpret_cast<const float4*>(qr + r * QT * QS + d);
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+            const float4 kv = *reinterpret_cast<const float4*>(kr + 8 * c * KS + d);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                s[r][c] = fmaf(qv[r].x, kv.x, s[r][c]);
+                s[r][c] = fmaf(qv[r].y, kv.y, s[r][c]);
+                s[r][c] = fmaf(qv[r].z, kv.z, s[r][c]);
+                s[r][c] = fmaf(qv[r].w, kv.w, s[r][c]);
+            }
+        }
+    }
+}
+
+// A thread has one token, R heads, every eighth key of a chunk and then every eighth piece of four channels of the output.  A piece of
+// a key serves R heads and a piece of a query eight keys, 16 bytes a load from shared memory, which bounds the kernel: with one channel a
+// load it took nine loads for eight multiply-adds.  The page's rows are read once for R heads, the next chunk's keys while the weighted
+// sum runs and its values while the scores do.  Before / now, us, 32-bit, 32 heads of 64 over 8: prompts of 5 tokens 21.5 / 11.6, 300
+// 182 / 54, 2,048 3,207 / 887; a token behind 1,023 keys 632 / 85, of 64 requests 1,830 / 380; heads of 128, 2,048 tokens 10,200 / 1,837.
+template <typename T, typename TO, int R>
 __global__ void __launch_bounds__(THREADS)
 attention_plain_kernel(const T* __restrict__ q, int q_stride, TO* __restrict__ out, int out_stride,
                        const T* __restrict__ cache, const int* __restrict__ block_table,
                        int table_stride, const int* __restrict__ cu_q, const int* __restrict__ kv_len,
                        const int* __restrict__ tile_entry, const int* __restrict__ tile_q0,
-                       int Hq, int Hkv, int page_size, float scale, int window, int block, int sink, Extra ex) {
+                       int Hq, int Hkv, int page_size, float scale, int window, int block, int sink, int pieces, Extra ex) {
     // A successor that is released at once lands on whatever SMs this kernel leaves free, several CTAs to one, and stays there; released
-    // at this kernel's end it spreads out.  At once / at the end, us of a 32-bit layer of 32 heads of 64: a prompt of 300 tokens 567 / 385,
+    // at this kernel's end it spreads out.  At once / at the end, us of a 32-bit layer of 32 heads of 64 (when the kernel took two to four
+    // times as long as it does): a prompt of 300 tokens 567 / 385,
     // three of 80 492 / 288; a token each of 16 requests behind 15 keys 108 / 81 and behind 1,023 706 / 676, of 64 behind 127 439 / 342,
     // of 9 behind 1,023 568 / 555.  Up to eight tiles (a tile is 16 tokens of a prompt, or a request's single token) both take about
     // the same, and eight single tokens behind 1,023 keys 443 / 455.
     const bool late = gridDim.x > 8;
     if (!late) pdl_trigger();
     pdl_wait();
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     float* Qs = smem;
-    float* Ks = Qs + QT * QS;
+    float* Ks = Qs + R * QT * QS;
     float* Vs = Ks + KC * KS;
-    float* Ps = Vs + KC * VD;
+    float* Ps = Vs + KC * VP;
 
-    const int tile = blockIdx.x, h = blockIdx.y;
+    const int tile = blockIdx.x;
     const int b = tile_entry[tile];
     if (b < 0) return;                                   // padding tile
     const int j0 = tile_q0[tile];
     const int q_begin = cu_q[b], q_len = cu_q[b + 1] - q_begin;
     const int kvl = kv_len[b];
     const int pos0 = kvl - q_len;                        // position of the entry's first token
-    int kh, g;                                           // key head, value head
-    heads_of(h, Hq, Hkv, ex.maps, kh, g);
+    // this CTA's heads: h0, h0 + maps, ... of one key head (blockIdx.y: [value head][part of its heads][map])
+    const int per = Hq / (Hkv * ex.maps);
+    const int map = blockIdx.y % ex.maps, first = blockIdx.y / ex.maps * R;
+    const int h0 = first * ex.maps + map;
+    const int g = first / per, kh = g * ex.maps + map;   // value head, key head
     const int tid = threadIdx.x;
     const int row = tid >> 3, l8 = tid & 7;
     const int rows_here = min(QT, q_len - j0);
     if (rows_here <= 0) return;
 
-    for (int e = tid; e < QT * HD; e += THREADS) {
-        const int r = e / HD, d = e - r * HD;
-        Qs[r * QS + d] = r < rows_here
-            ? to_f32<T>(q[(size_t)(q_begin + j0 + r) * q_stride + (size_t)h * HD + d]) : 0.f;
-    }
-
-    const bool row_valid = row < rows_here;
-    const int p_row = pos0 + j0 + row;                   // this row's position
-    int lo_row = window > 0 ? max(0, p_row - window + 1) : 0;
     const int p_last = pos0 + j0 + rows_here - 1;        // last key any row of the tile sees
     int lo_tile = window > 0 ? max(0, pos0 + j0 - window + 1) : 0;   // first key its first row sees
-    if (block > 0) {
-        lo_row = max(lo_row, (p_row / block) * block);
-        lo_tile = max(lo_tile, ((pos0 + j0) / block) * block);
-    }
-
-    // with a sink the sums start from a key of score 0 that has no value: maximum 0, sum exp(0 - 0) = 1
-    // (with sink values: a term exp(sink_h) instead, so the maximum starts at sink_h)
-    float m = sink ? (ex.sink_values ? ex.sink_values[h] : 0.f) : -INFINITY, l = sink ? 1.f : 0.f;
-    const float slope = ex.slopes ? ex.slopes[h] : 0.f;
-    const float* bias = ex.bias ? ex.bias + (size_t)h * ex.bias_len : nullptr;
-    float acc[NACC];
-#pragma unroll
-    for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
+    if (block > 0) lo_tile = max(lo_tile, ((pos0 + j0) / block) * block);
 
     const int* bt = block_table + (size_t)b * table_stride;
     // a page: keys [kv head][slot][HD], then values [kv head][slot][VD]
@@ -141,85 +187,148 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, TO* __restrict__ o
     const size_t k_base = (size_t)kh * page_size * HD;
     const size_t v_base = ex.value_in_key ? k_base : (size_t)Hk * page_size * HD + (size_t)g * page_size * VD;
     const int v_row = ex.value_in_key ? HD : VD;         // elements from one key's value to the next
-    for (int kb = (lo_tile / KC) * KC; kb <= p_last; kb += KC) {
-        __syncthreads();                                 // previous chunk's Vs/Ps reads are done
-        // a warp a key: the page is looked up once per key and the lanes read along the head
-        for (int kk = tid >> 5; kk < KC; kk += THREADS / 32) {
-            const int key = kb + kk;
-            const bool seen = key >= lo_tile && key <= p_last;
-            const T* kp = cache;
-            const T* vp = cache;
-            if (seen) {
-                const int blk = key / page_size;
-                const size_t page = (size_t)bt[blk] * page_elems;
-                const int off = key - blk * page_size;
-                kp = cache + page + k_base + (size_t)off * HD;
-                vp = cache + page + v_base + (size_t)off * v_row;
-            }
-            for (int d = tid & 31; d < HD; d += 32) Ks[kk * KS + d] = seen ? to_f32<T>(kp[d]) : 0.f;
-            for (int d = tid & 31; d < VD; d += 32) Vs[kk * VD + d] = seen ? to_f32<T>(vp[d]) : 0.f;
-        }
+    const int kb0 = (lo_tile / KC) * KC;
+    for (int kk = tid; kk < KC; kk += THREADS) {         // the channels past a row's end
+#pragma unroll
+        for (int d = HD; d < HP; ++d) Ks[kk * KS + d] = 0.f;
+#pragma unroll
+        for (int d = VD; d < VP; ++d) Vs[kk * VP + d] = 0.f;
+    }
+    stage_keys<HD, T>(Ks, KS, cache, bt, page_elems, k_base, HD, page_size, kb0, lo_tile, p_last, pieces);
+    stage_keys<VD, T>(Vs, VP, cache, bt, page_elems, v_base, v_row, page_size, kb0, lo_tile, p_last, pieces);
+
+#pragma unroll 8
+    for (int e = tid; e < R * QT * HP; e += THREADS) {
+        const int rr = e / HP, d = e - rr * HP, r = rr / QT, t = rr % QT;
+        Qs[rr * QS + d] = t < rows_here && d < HD
+            ? to_f32<T>(q[(size_t)(q_begin + j0 + t) * q_stride + (size_t)(h0 + r * ex.maps) * HD + d]) : 0.f;
+    }
+
+    const bool row_valid = row < rows_here;
+    const int p_row = pos0 + j0 + row;                   // this row's position
+    int lo_row = window > 0 ? max(0, p_row - window + 1) : 0;
+    if (block > 0) lo_row = max(lo_row, (p_row / block) * block);
+
+    // with a sink the sums start from a key of score 0 that has no value: maximum 0, sum exp(0 - 0) = 1
+    // (with sink values: a term exp(sink_h) instead, so the maximum starts at sink_h)
+    float m[R], l[R], slope[R];
+    float4 acc[R][ND4];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int h = h0 + r * ex.maps;
+        m[r] = sink ? (ex.sink_values ? ex.sink_values[h] : 0.f) : -INFINITY;
+        l[r] = sink ? 1.f : 0.f;
+        slope[r] = ex.slopes ? ex.slopes[h] : 0.f;
+#pragma unroll
+        for (int i = 0; i < ND4; ++i) acc[r][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+
+    for (int kb = kb0; kb <= p_last; kb += KC) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");   // the keys; the values may still be on their way
         __syncthreads();
 
-        float s[NCOL];
-        float cmax = -INFINITY;
+        float s[R][NCOL];
+        const int here = p_last - kb + 1;                // keys of the chunk that some row may see
+        if (here <= KC / 2) {
+            scores_of<R, NCOL / 2>(s, Qs + row * QS, Ks + l8 * KS);
 #pragma unroll
-        for (int c = 0; c < NCOL; ++c) {
-            const int kk = l8 + 8 * c;
-            const int key = kb + kk;
-            float dot = 0.f;
-            const float* qr = Qs + row * QS;
-            const float* kr = Ks + kk * KS;
-#pragma unroll 8
-            for (int d = 0; d < HD; ++d) dot = fmaf(qr[d], kr[d], dot);
-            const bool seen = row_valid && key <= p_row && key >= lo_row;
-            float sc = dot * scale;
-            if (ex.softcap > 0.f) sc = ex.softcap * tanhf(sc / ex.softcap);
-            if (ex.slopes) sc -= slope * (float)(p_row - key);
-            if (bias && seen) sc += bias[min(p_row - key, ex.bias_len - 1)];
-            s[c] = seen ? sc : -INFINITY;
-            cmax = fmaxf(cmax, s[c]);
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int c = NCOL / 2; c < NCOL; ++c) s[r][c] = 0.f;      // masked below
+        } else {
+            scores_of<R, NCOL>(s, Qs + row * QS, Ks + l8 * KS);
         }
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
-        const float m_new = fmaxf(m, cmax);
-        float alpha = 1.f, psum = 0.f;
-        if (m_new == -INFINITY) {
-#pragma unroll
-            for (int c = 0; c < NCOL; ++c) Ps[row * PS + l8 + 8 * c] = 0.f;
-        } else {
-            alpha = (m == -INFINITY) ? 0.f : expf(m - m_new);
+        for (int r = 0; r < R; ++r) {
+            float* pr = Ps + (r * QT + row) * PS + l8;
+            const float* bias = ex.bias ? ex.bias + (size_t)(h0 + r * ex.maps) * ex.bias_len : nullptr;
+            float cmax = -INFINITY;
 #pragma unroll
             for (int c = 0; c < NCOL; ++c) {
-                const float p = (s[c] == -INFINITY) ? 0.f : expf(s[c] - m_new);
-                Ps[row * PS + l8 + 8 * c] = p;
-                psum += p;
+                const int key = kb + l8 + 8 * c;
+                const bool seen = row_valid && key <= p_row && key >= lo_row;
+                float sc = s[r][c] * scale;
+                if (ex.softcap > 0.f) sc = ex.softcap * tanhf(sc / ex.softcap);
+                if (ex.slopes) sc -= slope[r] * (float)(p_row - key);
+                if (bias && seen) sc += bias[min(p_row - key, ex.bias_len - 1)];
+                s[r][c] = seen ? sc : -INFINITY;
+                cmax = fmaxf(cmax, s[r][c]);
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+            const float m_new = fmaxf(m[r], cmax);
+            float alpha = 1.f, psum = 0.f;
+            if (m_new == -INFINITY) {
+#pragma unroll
+                for (int c = 0; c < NCOL; ++c) pr[8 * c] = 0.f;
+            } else {
+                alpha = (m[r] == -INFINITY) ? 0.f : expf(m[r] - m_new);
+#pragma unroll
+                for (int c = 0; c < NCOL; ++c) {
+                    const float p = (s[r][c] == -INFINITY) ? 0.f : expf(s[r][c] - m_new);
+                    pr[8 * c] = p;
+                    psum += p;
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
+            l[r] = l[r] * alpha + psum;
+            m[r] = m_new;
+#pragma unroll
+            for (int i = 0; i < ND4; ++i) {
+                acc[r][i].x *= alpha; acc[r][i].y *= alpha; acc[r][i].z *= alpha; acc[r][i].w *= alpha;
             }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                 // weights and values are there, the keys have been read
+        const bool more = kb + KC <= p_last;
+        if (more) stage_keys<HD, T>(Ks, KS, cache, bt, page_elems, k_base, HD, page_size, kb + KC, lo_tile, p_last, pieces);
+        // keys past the tile's last have weight 0 in every row
+        const int kend = min(KC, (here + 3) / 4 * 4);
+#pragma unroll (R == 1 ? 2 : 1)
+        for (int kk = 0; kk < kend; kk += 4) {
+            float4 pw[R];
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
-        l = l * alpha + psum;
-        m = m_new;
+            for (int r = 0; r < R; ++r) pw[r] = *reinterpret_cast<const float4*>(Ps + (r * QT + row) * PS + kk);
 #pragma unroll
-        for (int i = 0; i < NACC; ++i) acc[i] *= alpha;
-        __syncthreads();
-        const float* pr = Ps + row * PS;
-        for (int kk = 0; kk < KC; ++kk) {
-            const float p = pr[kk];
-            const float* vr = Vs + kk * VD + l8;
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int i = 0; i < NACC; ++i)
-                if (VD % 8 == 0 || l8 + 8 * i < VD) acc[i] = fmaf(p, vr[8 * i], acc[i]);
+                for (int i = 0; i < ND4; ++i) {
+                    if (VP % 32 != 0 && l8 + 8 * i >= VP / 4) continue;
+                    const float4 v = *reinterpret_cast<const float4*>(Vs + (kk + j) * VP + 4 * (l8 + 8 * i));
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float p = j == 0 ? pw[r].x : j == 1 ? pw[r].y : j == 2 ? pw[r].z : pw[r].w;
+                        acc[r][i].x = fmaf(p, v.x, acc[r][i].x);
+                        acc[r][i].y = fmaf(p, v.y, acc[r][i].y);
+                        acc[r][i].z = fmaf(p, v.z, acc[r][i].z);
+                        acc[r][i].w = fmaf(p, v.w, acc[r][i].w);
+                    }
+                }
+        }
+        if (more) {
+            __syncthreads();                             // the values have been read
+            stage_keys<VD, T>(Vs, VP, cache, bt, page_elems, v_base, v_row, page_size, kb + KC, lo_tile, p_last, pieces);
         }
     }
     if (late) pdl_trigger();
     if (row_valid) {
-        const float inv = l > 0.f ? 1.0f / l : 0.f;
-        const float den = ex.gate ? 1.0f + expf(-ex.gate[(size_t)(q_begin + j0 + row) * ex.gate_stride + h]) : 1.f;
-        TO* o = out + (size_t)(q_begin + j0 + row) * out_stride + (size_t)h * VD + l8;
+        const int t = q_begin + j0 + row;
 #pragma unroll
-        for (int i = 0; i < NACC; ++i)
-            if (VD % 8 == 0 || l8 + 8 * i < VD) o[8 * i] = from_f32<TO>(ex.gate ? ex.gate_scale * (acc[i] * inv) / den : acc[i] * inv);
+        for (int r = 0; r < R; ++r) {
+            const int h = h0 + r * ex.maps;
+            const float inv = l[r] > 0.f ? 1.0f / l[r] : 0.f;
+            const float den = ex.gate ? 1.0f + expf(-ex.gate[(size_t)t * ex.gate_stride + h]) : 1.f;
+            TO* o = out + (size_t)t * out_stride + (size_t)h * VD;
+#pragma unroll
+            for (int i = 0; i < ND4; ++i) {
+                const int d = 4 * (l8 + 8 * i);
+                const float a[4] = {acc[r][i].x, acc[r][i].y, acc[r][i].z, acc[r][i].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (VD % 32 == 0 || d + j < VD) o[d + j] = from_f32<TO>(ex.gate ? ex.gate_scale * (a[j] * inv) / den : a[j] * inv);
+            }
+        }
     }
 }
 
@@ -560,18 +669,24 @@ int launch(const void* q, int q_stride, void* out, int out_stride, const void* c
            const int* block_table, int table_stride, const int* cu_q, const int* kv_len,
            const int* tile_entry, const int* tile_q0, int n_tiles, int Hq, int Hkv, int page_size,
            float scale, int window, int block, int sink, Extra ex, cudaStream_t s) {
-    static bool configured = false;
-    const size_t smem = SMEM_FLOATS * sizeof(float);
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_plain_kernel<T, TO>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
-    dim3 grid(n_tiles, Hq);
-    RI_CHECKED(ri_launch(attention_plain_kernel<T, TO>, dim3(grid), dim3(THREADS), smem, s,
-        (const T*)q, q_stride, (TO*)out, out_stride, (const T*)cache, block_table, table_stride,
-        cu_q, kv_len, tile_entry, tile_q0, Hq, Hkv, page_size, scale, window, block, sink, ex));
+    // 32-bit rows of whole 16-byte pieces, every page and head on a 16-byte boundary
+    const int pieces = HD % 4 == 0 && VD % 4 == 0 && sizeof(T) == 4 && ((uintptr_t)cache & 15) == 0;
+#define RI_PLAIN(R_) do { constexpr int R = R_; static bool configured = false; \
+    const size_t smem = smem_floats(R) * sizeof(float); \
+    if (!configured) { \
+        cudaError_t e = cudaFuncSetAttribute(attention_plain_kernel<T, TO, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (e != cudaSuccess) return (int)e; \
+        configured = true; } \
+    RI_CHECKED(ri_launch(attention_plain_kernel<T, TO, R>, dim3(n_tiles, Hq / R), dim3(THREADS), smem, s, \
+        (const T*)q, q_stride, (TO*)out, out_stride, (const T*)cache, block_table, table_stride, \
+        cu_q, kv_len, tile_entry, tile_q0, Hq, Hkv, page_size, scale, window, block, sink, pieces, ex)); } while (0)
+    const int per = Hq / (Hkv * ex.maps);
+    // Two heads a CTA from 3.5 CTAs an SM on (148), below that they leave SMs idle.  One / two, us, heads of 64, 32 over 8: 200 tokens
+    // (3.0) 37.9 / 39.9, 3 of 80 (3.5) 23.5 / 24.7, 300 (4.3) 55.5 / 54.2, 1,000 362 / 265, 2,048 1,284 / 887; a token of 16 requests
+    // behind 1,023 keys (3.7) 175 / 153, of 64 595 / 380; heads of 128, the same 412 / 244 and 1,419 / 934, 300 tokens 107.6 / 83.0.
+    if (MOST_HEADS == 2 && per % 2 == 0 && (long)n_tiles * Hq * 2 > 7 * 148) RI_PLAIN(MOST_HEADS);
+    else RI_PLAIN(1);
+#undef RI_PLAIN
     return ri_launch_status();
 }
 
