@@ -1,7 +1,8 @@
 """Mixers that keep a matrix per head instead of keys and values: the state S [key channel,
 value channel] of every live request sits in a slot of a fixed-state cache group, in fp32, and a
 step walks each entry's tokens through the recurrence from where the last step left it.  A whole
-prompt, a portion of one and a single decoded token are the same kernel launch.
+prompt, a portion of one and a single decoded token are the same kernel launch; long portions in the bfloat16 engine
+go in chunks of 64 tokens instead (`ops.kernels` chooses by what the two take).
 
     gated_linear_attention   S_t = diag(alpha_t) S_{t-1} + k_t v_t^T,  o_t = S_t^T q_t
                              alpha = sigmoid(W_a2 W_a1 h + b)^(1/tau),  q scaled by key_dim^(-1/2);
