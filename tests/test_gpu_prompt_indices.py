@@ -4,6 +4,17 @@ import pytest
 import torch
 
 from rustinfer_b200.cache.pages import OutOfPages, PagePool
+from rustinfer_b200.engine.runner import StepEntry, _flat_ids
+
+
+def test_every_kind_of_list_is_the_same_array():
+    ids = [int(t) for t in np.random.RandomState(1).randint(0, 50, 20)]
+    for tokens in (ids, tuple(ids), np.array(ids), np.array(ids, dtype=np.int32), [np.int64(t) for t in ids]):
+        flat = _flat_ids([StepEntry(0, tokens, ()), StepEntry(1, [49], ())], 50)
+        assert flat.dtype == np.int64 and flat.tolist() == [*ids, 49]
+    for other in ([*ids, 50], [*ids, -1], [*ids, 1 << 70], [*ids, 50.0], np.array([*ids, 50])):
+        assert _flat_ids([StepEntry(0, other, ())], 50) is None          # looked at one by one, and refused there
+    assert _flat_ids([StepEntry(0, [float(t) for t in ids], ())], 50) is None
 
 
 def test_pages_at_once_are_the_smallest_and_come_back():
@@ -25,10 +36,11 @@ def test_pages_at_once_are_the_smallest_and_come_back():
 
 @pytest.mark.gpu
 def test_ids_are_looked_at_in_long_steps_too(tmp_path):
+    # the 32-bit engine: its logits are the same bits every time (a bfloat16 step of 20 tokens adds its products' slices in the order they arrive)
     from helpers import make_sharp_model
     from rustinfer_b200.engine.runner import ModelRunner, StepEntry, StepError
     folder = make_sharp_model(str(tmp_path / "model"), "D")
-    runner = ModelRunner(folder, dtype="bfloat16", max_model_len=64, max_batch_seqs=2, max_batch_tokens=64, num_pages=8, capture_sizes=[])
+    runner = ModelRunner(folder, dtype="float32", max_model_len=64, max_batch_seqs=2, max_batch_tokens=64, num_pages=8, capture_sizes=[])
     vocab = runner.spec.vocab_size
     ids = [int(t) for t in np.random.RandomState(1).randint(0, vocab, 20)]
     want = None
