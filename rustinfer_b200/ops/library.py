@@ -266,15 +266,23 @@ def num_sms(device=None) -> int:
     """Streaming multiprocessors of a CUDA device (the current one by default), asked of the device."""
     index = torch.cuda.current_device() if device is None else torch.device(device).index
     if index is None:
-        index = _current_device()
+        index = torch.cuda.current_device()
     n = _sms.get(index)
     if n is None:
         n = _sms[index] = int(torch.cuda.get_device_properties(index).multi_processor_count)
     return n
 
 
-# what torch.cuda.current_stream().cuda_stream comes down to, without the objects in between (5 us of a launch's 20)
-_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+def _stream_calls(c):
+    """The current device and its current stream's handle.  `c` (torch._C) has calls for both that make no object (5 us of a launch's 20
+    from Python); they are private to torch and missing from one without CUDA, so the public calls stand in for them."""
+    try:
+        return c._cuda_getDevice, c._cuda_getCurrentRawStream
+    except AttributeError:
+        return torch.cuda.current_device, lambda device: torch.cuda.current_stream(device).cuda_stream
+
+
+_current_device, _raw_stream = _stream_calls(torch._C)
 
 
 def stream_ptr() -> int:
