@@ -1623,9 +1623,11 @@ delta_chunk_scan_kernel(const bf16* __restrict__ xs, const bf16* __restrict__ au
 inline bool aligned4(const void* p, int esize) { return (reinterpret_cast<uintptr_t>(p) % (4 * (size_t)esize)) == 0; }
 template <typename Kernel>
 int allow(Kernel kernel, int bytes) { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); }
+inline bool aligned2(const float* p) { return (reinterpret_cast<uintptr_t>(p) % 8) == 0; }      // outputs leave in pairs
 }  // namespace
 
-// Whether the head form (`gated` 0) or the gated one takes these arrays; what they do not take walks.
+// Whether the head form (`gated` 0) or the gated one takes these arrays; what they do not take walks.  (The outputs' address, and that of
+// the delta rule's decays, the callers look at.)
 RI_API int ri_chunks_ok(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, int act_dtype, int dv, int gated) {
     const int esize = act_dtype == RI_BF16 ? 2 : 4;
     return dv > 0 && dv % 64 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 && aligned4(q, esize) &&
@@ -1639,7 +1641,7 @@ RI_API int ri_head_chunks(const void* q, int q_stride, const void* k, int k_stri
                           float* out, float* state, const int* cu_q, const int* state_slots, int entries, int least, int chunks,
                           int H, int dv, int share, float* states, float* totals, void* cuts, void* stream) {
     if (entries <= 0 || chunks <= 0) return 0;
-    if (share <= 0 || H % share || !ri_chunks_ok(q, q_stride, k, k_stride, v, v_stride, act_dtype, dv, 0)) return (int)cudaErrorInvalidValue;
+    if (share <= 0 || H % share || !aligned2(out) || !ri_chunks_ok(q, q_stride, k, k_stride, v, v_stride, act_dtype, dv, 0)) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
     // heads a CTA of the outputs serves: the scores of a key head, as much work as a head's 64 channels, are made once a CTA, and
     // CTAs go in waves of two an SM.  The layer over 2,048 tokens, heads a CTA 1, 2, 4, 8: 32 heads of 64 in 4 key heads 245, 236, 234,
@@ -1683,7 +1685,7 @@ RI_API int ri_gated_chunks(const void* q, int q_stride, const void* k, int k_str
                            const int* state_slots, int entries, int least, int chunks, int H, int dv, float* states, float* totals,
                            void* cuts, void* parts, void* stream) {
     if (entries <= 0 || chunks <= 0) return 0;
-    if (!ri_chunks_ok(q, q_stride, k, k_stride, v, v_stride, act_dtype, dv, 1)) return (int)cudaErrorInvalidValue;
+    if (!aligned2(out) || !ri_chunks_ok(q, q_stride, k, k_stride, v, v_stride, act_dtype, dv, 1)) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
     const int scan_blocks = (int)(((size_t)H * dv * DK / 8 + SCAN_THREADS - 1) / SCAN_THREADS);
     static bool allowed = false;
@@ -1717,7 +1719,7 @@ RI_API int ri_delta_chunks(const void* r, int r_stride, const void* k, int k_str
                            const int* state_slots, int entries, int least, int chunks, int H, int dv, float* states, float* ends, void* cuts,
                            void* parts, void* xs, void* aus, void* stream) {
     if (entries <= 0 || chunks <= 0) return 0;
-    if (!ri_chunks_ok(r, r_stride, k, k_stride, v, v_stride, act_dtype, dv, 1) || f_stride % 4 || !aligned4(w, 4) || !aligned4(u, 4) || !aligned4(au, 4))
+    if (!aligned2(out) || !ri_chunks_ok(r, r_stride, k, k_stride, v, v_stride, act_dtype, dv, 1) || f_stride % 4 || !aligned4(w, 4) || !aligned4(u, 4) || !aligned4(au, 4))
         return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
     static bool allowed = false;

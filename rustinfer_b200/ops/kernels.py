@@ -1347,6 +1347,14 @@ def _chunk_scratch(chunks: int, device: torch.device, sizes: Tuple[int, ...]):
     return buf, [buf.data_ptr() + a for a in at[:-1]]
 
 
+def _chunks_take(lib, qkv: Tuple[int, ...], dtype: torch.dtype, value_dim: int, gated: bool, out: torch.Tensor,
+                 decays: Optional[torch.Tensor] = None) -> bool:
+    """Whether the kernels in chunks take a call's arrays.  Outputs leave them in pairs and the delta rule's `decays` are read in fours, where
+    the walk stores and reads one number at a time: what is not aligned walks."""
+    return bool(lib.ri_chunks_ok(*qkv, dtype_code(dtype), value_dim, 1 if gated else 0)) and out.data_ptr() % 8 == 0 \
+        and (decays is None or decays.data_ptr() % 16 == 0)
+
+
 def _recurrent_sizes_agree(lib, dk: int, what: str) -> None:
     """The library lays out states and, where it has them, chunks as this module counts them: a shorter chunk there would find no
     place in the scratch and the grids made here."""
@@ -1369,6 +1377,8 @@ def _scan_common(state: torch.Tensor, out: torch.Tensor, cu_q: torch.Tensor, sta
         _rows_checked.add(dk)
     if state.dtype != torch.float32 or state.dim() != 4 or tuple(state.shape[1:]) != (H, dv, rows):
         raise KernelError(f"{what}: state is fp32 [slots, {H}, {dv}, {rows}] (recurrent_state_rows({dk}) rows a column)")
+    if state.data_ptr() % 16:                         # every kernel moves a state in fours
+        raise KernelError(f"{what}: state starts on a 16-byte boundary")
     if out.dtype != torch.float32 or out.shape != (T, H * dv):
         raise KernelError(f"{what}: out is fp32 [T, H*dv]")
 
@@ -1403,7 +1413,7 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tenso
         qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
         chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, True, L.num_sms())
         held = None
-        if chunks and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 1):
+        if chunks and _chunks_take(lib, qkv, q.dtype, dv, True, out):
             held = _chunk_scratch(chunks, q.device, _chunk_sizes(H, dk, dv, True))
         if held is not None:
             scratch = held[1]
@@ -1477,7 +1487,7 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
         qkv = (_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0))
         chunks = _scan_chunks(T, int(entries), longest, H, dk, dv, False, L.num_sms())
         held = None
-        if chunks and lib.ri_chunks_ok(*qkv, dtype_code(q.dtype), dv, 0):
+        if chunks and _chunks_take(lib, qkv, q.dtype, dv, False, out):
             held = _chunk_scratch(chunks, q.device, _chunk_sizes(H, dk, dv, False))
         if held is not None:
             scratch = held[1]
@@ -1528,7 +1538,7 @@ def delta_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, za: torch.Tens
         chunks = _chunks_or_walk(T, int(entries), longest, H, dk, dv, L.num_sms(), DELTA_CHUNK_MIN_TOKENS, sizes, _DELTA_WALK_US,
                                  _DELTA_CHUNK_FIXED_US, _DELTA_CHUNK_US)
         held = None
-        if chunks and lib.ri_chunks_ok(*args[:6], dtype_code(r.dtype), dv, 1):
+        if chunks and _chunks_take(lib, args[:6], r.dtype, dv, True, out, zw):
             held = _chunk_scratch(chunks, r.device, sizes)
         if held is not None:
             check(lib.ri_delta_chunks(*args, DELTA_CHUNK_MIN_TOKENS, chunks, H, dv, *held[1], stream_ptr()), "delta_chunks", 3)

@@ -112,3 +112,19 @@ def test_a_number_that_is_none_spares_earlier_tokens_and_other_heads(where, monk
     assert torch.isnan(out[150:, 1, hit]).all() and torch.isnan(state[1, 1, hit]).all()
     assert off(out[:150, 1], clean[0][:150, 1].double()) <= 1e-6          # the chunk's later tokens are left out of its sums
     assert torch.equal(out[:, 1, rest], clean[0][:, 1, rest]) and torch.equal(state[1, 1, rest], clean[1][1, 1, rest])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("out_at,zw_at", [(1, 0), (0, 1), (0, 2), (3, 3)])
+def test_arrays_off_their_boundaries_walk(out_at, zw_at, monkeypatch):
+    monkeypatch.setattr(K(), "_DELTA_CHUNK_FIXED_US", -1e9)
+    c = make([256], 2, 128, 128)
+    n, got = c["T"] * 2 * 128, []
+    for longest in (0, 256):                                  # the walk, and the call that could go in chunks
+        out, zw = (torch.full((n + 4,), float("nan"), device=c["r"].device)[at: at + n].view(c["T"], -1) for at in (out_at, zw_at))
+        zw.copy_(c["zw"])
+        state = c["state"].clone()
+        K().delta_scan(c["r"], c["k"], c["v"], c["za"], None, zw, c["bias"], 0.6, 1e-6, out, state, c["cu_q"], c["slots"], 1, 2, 128, 128,
+                       longest=longest)
+        got.append((out, state))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and torch.isfinite(got[0][0]).all()

@@ -192,3 +192,24 @@ def test_a_call_without_room_for_scratch_walks(gated, monkeypatch):
     monkeypatch.setattr(torch, "empty", full)
     got = run(T)
     assert all(torch.equal(a, b) for a, b in zip(got, walked)) and not torch.equal(in_chunks[0], walked[0])
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_outputs_off_their_boundary_walk(gated, monkeypatch):
+    monkeypatch.setattr(K(), "_CHUNK_FIXED_US", {False: -1e9, True: -1e9})
+    torch.manual_seed(2)
+    T, H, dk, dv = 450, 2, 64, 64
+    x = torch.randn(T, 2 * H * dk + H * dv, device=DEV).bfloat16()
+    q, k, v = x[:, : H * dk], x[:, H * dk: 2 * H * dk], x[:, 2 * H * dk:]
+    got = {}
+    for at, longest in ((0, 0), (0, T), (1, T)):
+        out = torch.empty(T * H * dv + 1, device=DEV)[at: at + T * H * dv].view(T, H * dv)
+        state = torch.ones(1, H, dv, K().recurrent_state_rows(dk), device=DEV)
+        args = (out, state, i32([0, T]), i32([0]), 1, H, dk, dv)
+        if gated:
+            K().gated_scan(q, k, v, torch.ones(T, H * dk, device=DEV), None, 1.0, 4.0, *args, longest=longest)
+        else:
+            K().head_scan(q, k, v, torch.full((H,), 0.9, device=DEV), 1.0, *args, longest=longest)
+        got[at, longest] = out, state
+    walked, in_chunks, off = got.values()
+    assert all(torch.equal(a, b) for a, b in zip(off, walked)) and not torch.equal(in_chunks[0], walked[0])

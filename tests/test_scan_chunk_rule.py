@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import pytest
+import torch
 
 from rustinfer_b200.ops import kernels as K
 
@@ -31,3 +32,22 @@ def test_a_library_that_counts_otherwise_is_refused(rows, tokens, parts, fits):
     else:
         with pytest.raises(K.KernelError):
             K._recurrent_sizes_agree(lib, 128, "scan")
+
+
+@pytest.mark.parametrize("out_at,zw_at,takes", [(0, 0, True), (1, 0, False), (2, 0, True), (0, 1, False), (0, 2, False), (0, 4, True), (0, None, True),
+                                                (1, None, False)])
+def test_arrays_off_their_boundaries_walk(out_at, zw_at, takes):
+    lib = type("Library", (), dict(ri_chunks_ok=lambda self, *a: a[6:] == (1, 64, 1)))()
+    memory = torch.zeros(64)                                  # (its own address is a multiple of 16)
+    assert memory.data_ptr() % 16 == 0
+    decays = memory[zw_at:] if zw_at is not None else None
+    assert K._chunks_take(lib, (256, 128) * 3, torch.bfloat16, 64, True, memory[out_at:], decays) == takes
+
+
+def test_a_state_off_its_boundary_is_refused(monkeypatch):
+    monkeypatch.setattr(K, "_rows_checked", {64})
+    cu = torch.zeros(2, dtype=torch.int32)
+    state, out = torch.zeros(2 * 64 * 64 + 1), torch.zeros(5, 128)
+    K._scan_common(state[:-1].view(1, 2, 64, 64), out, cu, cu, 5, 2, 64, 64, "scan")
+    with pytest.raises(K.KernelError, match="16-byte"):
+        K._scan_common(state[1:].view(1, 2, 64, 64), out, cu, cu, 5, 2, 64, 64, "scan")
