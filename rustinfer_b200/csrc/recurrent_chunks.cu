@@ -996,12 +996,6 @@ __device__ __forceinline__ int warp_blocks(int warp, int which) {        // i * 
     constexpr int first[8] = {12, 8, 13, 4, 9, 14, 15, -1}, second[8] = {-1, -1, -1, 0, 5, 10, -1, -1};
     return which ? second[warp] : first[warp];
 }
-// 1 / x for x between 2^-60 and 2^60: the special-function unit's and one step of Newton's method, to the last place but one
-__device__ __forceinline__ float reciprocal(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return fmaf(y, fmaf(-x, y, 1.f), y);
-}
 __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
 // One chunk and head.  Outputs, all in the order of fragments ([piece][token block][key block][lane][8] for xs and au): xs: X; au: the
@@ -1110,9 +1104,9 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
                 // the product between the middle and the state behind token t, and that between the middle and the state in front of it
                 const float2 behind = early ? make_float2(bx, by) : make_float2(ax, ay), front = early ? make_float2(ax, ay) : make_float2(bx, by);
                 *reinterpret_cast<float2*>(ps + t * L::PF + ch) = behind;
-                const float2 inv = make_float2(reciprocal(behind.x), reciprocal(behind.y));
+                const float2 inv = make_float2(__frcp_rn(behind.x), __frcp_rn(behind.y));
                 const float2 row = early ? inv : behind, col = early ? behind : inv;
-                const float2 urow = early ? make_float2(reciprocal(front.x), reciprocal(front.y)) : front;
+                const float2 urow = early ? make_float2(__frcp_rn(front.x), __frcp_rn(front.y)) : front;
                 uint32_t x[3];
                 bf16* to = stage + t * SP + 2 * pair;
                 auto put = [&](int which, float p0, float p1) {
@@ -1360,7 +1354,7 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
                     const int t = i * 16 + g + 8 * e;
                     cut(dx[0][n][2 * e] * m.x, dx[0][n][2 * e + 1] * m.y, x[e * 2 + n]);
                     float2 f = *reinterpret_cast<const float2*>(ps + t * L::PF + ch);
-                    if (t < 32) f = make_float2(reciprocal(f.x), reciprocal(f.y));
+                    if (t < 32) f = make_float2(__frcp_rn(f.x), __frcp_rn(f.y));
                     const uint32_t r2 = rc[i][n * 2 + e];
                     uint32_t y[3];
                     cut(t >= bad ? nan : (low_of(r2) * f.x - dr[0][n][2 * e]) * m.x, t >= bad ? nan : (high_of(r2) * f.y - dr[0][n][2 * e + 1]) * m.y, y);
@@ -1412,7 +1406,7 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     float2 f = *reinterpret_cast<const float2*>(ps + (j * 16 + g + 8 * e) * L::PF + ch);
-                    if (j >= 2) f = make_float2(reciprocal(f.x), reciprocal(f.y));
+                    if (j >= 2) f = make_float2(__frcp_rn(f.x), __frcp_rn(f.y));
                     uint32_t x[3];
                     cut((low_of(kc[j][n * 2 + e]) * f.x - d[0][n][2 * e]) * m.x, (high_of(kc[j][n * 2 + e]) * f.y - d[0][n][2 * e + 1]) * m.y, x);
 #pragma unroll
