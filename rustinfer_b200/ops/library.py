@@ -193,10 +193,12 @@ def gemm_tc() -> ctypes.CDLL:
     lib = _loaded.get("ri_gemm_tc")
     if lib is None:
         lib = _load("ri_gemm_tc", ["gemm_tc.cu", "gemm_few.cu", "decode_chain.cu", "decode_chain_wide.cu"])
+    if not getattr(lib, "_budget_set", False):                                   # it may be set at any time ahead of a product
         kb = os.environ.get("RUSTINFER_B200_STREAM_KB")
         if kb:
             lib.ri_gemm_tc_set_stream_budget.argtypes = [_I]
             lib.ri_gemm_tc_set_stream_budget(int(kb) * 1024)
+            lib._budget_set = True
     return lib
 
 
