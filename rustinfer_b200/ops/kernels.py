@@ -199,12 +199,27 @@ def gemm_tc_plan(M: int, N: int, K: int, num_sms: Optional[int] = None, epilogue
 
 @functools.lru_cache(maxsize=4096)
 def _gemm_tc_plan(M: int, N: int, K: int, num_sms: int, epilogue: int):
-    # Weights on the 128-row side for few tokens.  From 33 on the activations: 33 to 64 tokens in tiles of 64 of them, whose K slices meet
-    # feature by feature, took 17 to 20 us where the tiles of a prompt take 9 to 11 (64 x 2,048 x 2,048 19.9 -> 10.0, 64 x 1,536 x 1,024 with
-    # gates 23.4 -> 8.9, 64 x 16,384 x 2,048 32.0 -> 18.2, 40 x 4,096 x 14,336 38.7 -> 33.1).  Slices that are added into the stream need no
-    # meeting (64 x 2,048 x 2,048 6.4 against 10.3), and a stream of weights that fills the SMs for several waves stays ahead with a
-    # handful of tokens more (36 x 28,672 x 4,096 54.8 against 55.4).
-    if M <= 32 or (M <= 64 and epilogue == EPI_RESIDUAL) or (M <= 36 and N * K >= 1 << 26):
+    """Weights on the 128-row side for few tokens.  From 33 on the activations: 33 to 64 tokens in tiles of 64 of them, whose K slices meet
+    feature by feature, took 17 to 20 us where the tiles of a prompt take 9 to 11 (64 x 2,048 x 2,048 19.9 -> 10.0, 64 x 1,536 x 1,024 with
+    gates 23.4 -> 8.9, 64 x 16,384 x 2,048 32.0 -> 18.2, 36 x 28,672 x 4,096 51.1 -> 46.1).  Slices that are added into the stream need no
+    meeting (64 x 2,048 x 2,048 6.4 against 10.3).  Where the tiles of a prompt would be 256 wide and in slices, both are put together from
+    their k-blocks, which take what the CTAs' weights take to arrive, and their meeting: 48 x 16,384 x 8,192 55.0 with the weights on the
+    128-row side against 62.8, 48 x 12,288 x 6,144 45.8 and 48.6, 48 x 10,240 x 14,336 76.9 and 71.6.  Of 546 products of 33 to 64 rows
+    (2,048 to 128,256 features, K of 2,048 to 28,672) five go the way that is slower by more than 3 %, at most 5 %."""
+    few = M <= 32 or (M <= 64 and epilogue == EPI_RESIDUAL)
+    plan = _plan_of_side(M, N, K, num_sms, epilogue, few)
+    if few or M > 64 or plan[1] != 256 or plan[2] == 1:
+        return plan
+    swapped, kblocks = _plan_of_side(M, N, K, num_sms, epilogue, True), -(-K // 64)
+    rows_us = 12.0 + 3.6 * plan[2] + max(0.5, 0.005 * -(-N // 256) * plan[2]) * kblocks / plan[2]
+    slices = swapped[2]
+    us = 6.0 + max(0.295, 0.0026 * -(-N // 128) * slices) * kblocks / slices + (1.5 * slices if slices > 1 else 0.0)
+    return swapped if us < rows_us else plan
+
+
+def _plan_of_side(M: int, N: int, K: int, num_sms: int, epilogue: int, weights: bool):
+    """The plan with the weights, or the activations, on the 128-row side."""
+    if weights:
         swap, bn = 1, (16 if M <= 16 else 32 if M <= 32 else 64)
         tiles = -(-N // 128)
     else:
