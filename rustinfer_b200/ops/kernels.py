@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import math
 from typing import Dict, Optional, Sequence, Tuple
 
 import torch
@@ -1294,10 +1295,15 @@ CHUNK_TOKENS = 64               # tokens of a chunk (recurrent_chunks.cu)
 # tokens from which an entry can go in chunks.  Layers in a walk and in chunks: one decay a head, 16 heads of 128 x 128, 256 tokens 76.5 and
 # 78.7 us, 384 99 and 89, 2,048 367 and 199; one a channel, 8 heads of 128 x 256, 384 tokens 107 and 107, 512 128 and 112, 2,048 297 and 197
 CHUNK_MIN_TOKENS, GATED_CHUNK_MIN_TOKENS = 256, 384
-# what the two ways take, in us: a walk so much a token of its longest entry, or of all while its CTAs fill the GPU; chunks a fixed part
-# and so much a token and element of the state (chosen so that of 112 layers, 1 to 5 entries of 256 to 2,048 tokens, 4 to 64 heads, the
-# fewest go the slower way: three by more than 3 %, at most 9 %)
-_WALK_US, _CHUNK_FIXED_US, _CHUNK_US = {False: 0.133, True: 0.152}, {False: 33.0, True: 38.0}, {False: 9.0e-8, True: 1.5e-7}
+# What the two ways take, in us, by size of the keys.  A walk: so much a token of its longest entry with two CTAs an SM, and the part of it with
+# one.  Chunks: a fixed part; a set of CTAs, two an SM, for all chunks and heads (and the share of it that each 64 value channels add: the
+# head form's CTAs take them in turn); a chunk's and head's element of the state; a chunk of the longest entry, whose states follow one
+# another; and what entries of 32 tokens and more that walk beside them add to their walk (shorter ones in proportion).
+_WALK_US = {False: {64: (0.140, 0.80), 128: (0.179, 0.643)}, True: {64: (0.163, 0.947), 128: (0.171, 0.984)}}
+_CHUNK_FIXED_US = {False: 7.0, True: 4.5}
+_CHUNK_US = {False: {64: (3.36, 1.0, 5.26e-6, 0.41, 4.9), 128: (5.78, 1.0, 3.81e-6, 0.204, 3.5)},
+             True: {64: (19.4, 0.0, 7.06e-6, 0.31, 4.7), 128: (42.3, 0.0, 6.07e-6, 0.335, 7.1)}}
+CHUNK_TIMED_TOKENS = 4096       # of an entry, at most, where the above was measured
 CHUNK_SCRATCH_BYTES = 1288 << 20    # the most scratch a call in chunks takes (1.26 GiB); a call that would take more walks, which takes none
 
 
@@ -1319,27 +1325,42 @@ def _scan_chunks(T: int, entries: int, longest: int, heads: int, key_dim: int, v
 
 
 def _chunks_or_walk(T: int, entries: int, longest: int, heads: int, key_dim: int, value_dim: int, num_sms: int, least: int,
-                    sizes: Tuple[int, ...], walk_us: float, fixed_us: float, chunk_us: float) -> int:
-    if longest < least or entries < 1 or longest > T:
+                    sizes: Tuple[int, ...], walk_us: Dict[int, Tuple[float, ...]], fixed_us: float, chunk_us: Dict[int, Tuple[float, ...]]) -> int:
+    """Fitted to calls that were timed both ways (1 to 16 entries of 192 to 4,096 tokens, short ones beside them, 2 to 128 heads, keys of 64
+    and 128, values of 64 to 256): of 3,325, 121 go the way that is slower by more than 3 %, 18 by more than 15 %, most of those because
+    the lengths between the longest entry's and the shortest's are not known here."""
+    if longest < least or entries < 1 or longest > T or key_dim not in chunk_us:
         return 0
-    state = heads * key_dim * value_dim
     chunks = T // CHUNK_TOKENS + min(entries, T // least)
     if chunks * sum(sizes) > CHUNK_SCRATCH_BYTES:
         return 0
-    filled = heads * value_dim / (16 if key_dim > 64 else 32) / (2 * num_sms)   # of the GPU by one entry's walk: CTAs over places for them
-    walk = lambda most, all_tokens: walk_us * max(most, all_tokens * filled)
+    places = 2 * num_sms
+    filled = heads * value_dim / (16 if key_dim > 64 else 32) / places          # of the GPU by one entry's walk: CTAs over places for them
+    a_token, alone = walk_us[key_dim]
+    a_set, a_column, an_element, a_link, beside = chunk_us[key_dim]
+
+    def walk(most: float, tokens: float) -> float:
+        full = filled * tokens / most                         # the shorter ones' CTAs leave their places early
+        return a_token * most * (alone if full <= 0.45 else max(1.0, (full + math.ceil(full)) / 2))
+
+    def in_chunks(most: int, tokens: int, n: int) -> float:
+        units = (tokens // CHUNK_TOKENS + (n if tokens % (CHUNK_TOKENS * n) else 0)) * heads
+        return (fixed_us + a_set * -(-units // places) * (1 + a_column * value_dim / 64) + an_element * units * key_dim * value_dim
+                + a_link * -(-most // CHUNK_TOKENS))
     rest = T - longest
-    short = rest > 0 and rest < least * (entries - 1)
-    cost = fixed_us + chunk_us * state * (longest if short else T)
-    if short:
-        cost += 3.0 + walk(rest / (entries - 1), rest)
-    return chunks if cost < 0.9 * walk(longest, T) else 0
+    if rest > 0 and rest < least * (entries - 1):
+        mean = rest / (entries - 1)
+        cost = in_chunks(longest, longest, 1) + 3.0 + beside * min(1.0, mean / 32) + walk(mean, rest)
+    else:
+        cost = in_chunks(longest, T, entries)
+    return chunks if longest > CHUNK_TIMED_TOKENS or cost < 0.9 * walk(longest, T) else 0
 
 
 # the delta rule: 16 heads of 128 x 128 take 90 us in a walk and 86 in chunks at 256 tokens, 175 and 100 at 512, 688 and 246 at 2,048 (8
 # heads: 90 and 79, 171 and 93, 678 and 166); 8 heads of 64 x 64 58 and 48 at 192, 144 and 56 at 512
 DELTA_CHUNK_MIN_TOKENS = 192
-_DELTA_WALK_US, _DELTA_CHUNK_FIXED_US, _DELTA_CHUNK_US = 0.335, 54.0, 1.9e-7
+_DELTA_WALK_US, _DELTA_CHUNK_FIXED_US = {64: (0.339, 0.92), 128: (0.380, 1.011)}, 9.0
+_DELTA_CHUNK_US = {64: (31.0, 0.0, 2.11e-5, 1.59, 6.3), 128: (61.3, 0.0, 8.29e-6, 1.54, 5.3)}
 
 
 def _delta_chunk_sizes(heads: int, key_dim: int, value_dim: int) -> Tuple[int, ...]:
