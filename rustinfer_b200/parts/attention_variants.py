@@ -28,6 +28,31 @@ from .short_conv import ConvState
 from .spec import PartSpec
 
 
+# us of the two kernels for prompt portions, by size of the heads: CTAs an SM holds, a CTA, a tile of 64 keys, and what more CTAs than places
+# cost as a part of the first set and a part of every set's worth; the tcgen05 kernel also: a table of biases; the other one: the part of
+# a tile's time that rows of queries add where all 64 are there
+_EXACT_US = {64: (2, 4.5, 1.59, 0.64, 0.93, 0.66), 128: (1, 4.9, 1.37, 0.69, 0.97, 0.54)}
+_ROWS_US = {64: (3, 4.2, 2.31, 1.27, 0.62, 0.48), 128: (2, 4.2, 4.92, 0.76, 0.82, 0.42)}
+
+
+def rows_are_sooner(tiles: int, kv_heads: int, group: int, head_dim: int, tokens: int, keys: int, bias: bool, num_sms: int) -> bool:
+    """Whether `attention_rows` takes `tiles` short portions (at most 64 / group tokens: one tile in either kernel) sooner than
+    `attention_prefill_exact`, whose CTAs take twice the rows and find fewer places.  That is for many portions over few keys: 16 portions of 2
+    tokens, 16 heads of 128 with a key head each 9.3 us against 14.5, behind 64 keys 14.1 against 17.7, behind 200 25.0 against 22.3; 24 of 16
+    heads of 64 6.4 against 12.9.  Of 2,958 calls timed both ways (1 to 64 portions of 2 to 64 tokens behind 0
+    to 1,000 keys, 2 to 32 key heads) 124 go the way that is slower by more than 3 %, 28 by more than 10 %, none by 24 (617 and 2,189
+    were it always the one or the other)."""
+    ctas, key_tiles = tiles * kv_heads, -(-keys // 64)
+
+    def us(a_sm, a_cta, a_tile, first, every):
+        sets = ctas / (a_sm * num_sms)
+        return (a_cta + a_tile * key_tiles) * (1.0 if sets <= 1 else first + every * sets)
+    a_sm, a_cta, a_tile, first, every, table = _EXACT_US[head_dim]
+    exact = us(a_sm, a_cta + (table if bias else 0.0), a_tile, first, every)
+    a_sm, a_cta, a_tile, first, every, filled = _ROWS_US[head_dim]
+    return us(a_sm, a_cta, a_tile * (1 + filled * tokens * group / 64), first, every) < exact
+
+
 class PlainAttend:
     """How a mixer sends its queries to the attention kernels with fp32 scores and softmax weights.  The bfloat16
     engine, where the sizes are multiples of 16: prompt portions go to the tensor-core kernel in tiles of 64 (token, head)
@@ -73,8 +98,8 @@ class PlainAttend:
             if "zero_tok0" not in ctx.shared:
                 ctx.shared["zero_tok0"] = torch.zeros(ctx.max_batch_seqs + 4, dtype=torch.int32, device=ctx.device)
             self.zero_tok0 = ctx.shared["zero_tok0"]
-        self.exact = False
-        self._tiles = token_tiles(rows, skip_single_token=self._single is not None)
+        self.exact, self._row_tokens = False, rows
+        self._tiles = self._row_tiles = token_tiles(rows, skip_single_token=self._single is not None)
 
     def take_exact(self, bias: Optional[torch.Tensor]) -> None:
         """From here on prompt portions go to the tcgen05 kernel with unrounded weights where it takes the geometry and the
@@ -83,8 +108,14 @@ class PlainAttend:
         226 -> 66; heads of 128, 8 over 2, 2 tokens 8.5 -> 6.7, 2,048 tokens 200 -> 51."""
         self.exact = (self.rows and self.maps == 1 and not self.value_in_key and self.vd == self.hd and not self.block
                       and K.tc_exact_supports(self.Hq, self.Hkv, self.hd, self.ctx.page_size, bias.shape[1] if bias is not None else 0))
-        if self.exact:
-            self._tiles = token_tiles(K.tc_tokens_per_tile(self.Hq, self.Hkv), skip_single_token=True)
+        self._tiles = token_tiles(K.tc_tokens_per_tile(self.Hq, self.Hkv), skip_single_token=True) if self.exact else self._row_tiles
+
+    def _rows_sooner(self, tiles: int, step: StepContext, bias: Optional[torch.Tensor]) -> bool:
+        tokens = step.max_q_len
+        if tokens > self._row_tokens:                         # the two kernels cut such portions differently
+            return False
+        keys = min([step.max_kv_len] + [w + tokens for w in (self.window,) if w])
+        return rows_are_sooner(tiles, self.Hkv, self.Hq // self.Hkv, self.hd, tokens, keys, bias is not None, self.ctx.num_sms)
 
     def step_indices(self):
         return [self._tiles] if self._single is None else [self._single, self._tiles]
@@ -127,7 +158,7 @@ class PlainAttend:
         opts.update(value_dim=self.vd, maps=self.maps, value_in_key=self.value_in_key)
         tile_entry, tile_tok0 = step.index(self._tiles)
         if tile_entry.numel():
-            if self.exact:
+            if self.exact and not self._rows_sooner(tile_entry.numel(), step, bias):
                 K.attention_prefill_exact(q, out, cache.kv, g.block_table, step.cu_q, step.kv_len, tile_entry, tile_tok0, self.Hq, self.Hkv,
                                           self.hd, scale, self.window, sink_values, bias, gate, gate_scale)
             elif self.rows:

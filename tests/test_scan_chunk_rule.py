@@ -51,3 +51,18 @@ def test_a_state_off_its_boundary_is_refused(monkeypatch):
     K._scan_common(state[:-1].view(1, 2, 64, 64), out, cu, cu, 5, 2, 64, 64, "scan")
     with pytest.raises(K.KernelError, match="16-byte"):
         K._scan_common(state[1:].view(1, 2, 64, 64), out, cu, cu, 5, 2, 64, 64, "scan")
+
+
+@pytest.mark.parametrize("form,H,dk,dv,T,entries,longest,chunks", [
+    ("delta", 8, 64, 64, 6400, 16, 400, False), ("delta", 8, 64, 64, 512, 1, 512, True), ("delta", 4, 128, 128, 192, 1, 192, False),
+    ("delta", 16, 128, 128, 2444, 4, 761, True), ("gated", 32, 64, 64, 6400, 16, 400, False), ("gated", 8, 128, 256, 507, 8, 500, True),
+    ("gated", 64, 128, 64, 2048, 1, 2048, False), ("gated", 64, 128, 64, 5000, 1, 5000, True), ("head", 32, 64, 64, 300, 1, 300, True),
+    ("head", 64, 128, 64, 1138, 5, 272, False), ("head", 16, 128, 128, 900, 3, 300, True), ("head", 16, 100, 128, 2048, 1, 2048, False),
+])
+def test_the_sooner_way(form, H, dk, dv, T, entries, longest, chunks):
+    if form == "delta":
+        got = K._chunks_or_walk(T, entries, longest, H, dk, dv, 148, K.DELTA_CHUNK_MIN_TOKENS, K._delta_chunk_sizes(H, dk, dv), K._DELTA_WALK_US,
+                                K._DELTA_CHUNK_FIXED_US, K._DELTA_CHUNK_US)
+    else:
+        got = K._scan_chunks(T, entries, longest, H, dk, dv, form == "gated", 148)
+    assert (got > 0) == chunks
