@@ -144,14 +144,10 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, TO* __restrict__ o
                        int table_stride, const int* __restrict__ cu_q, const int* __restrict__ kv_len,
                        const int* __restrict__ tile_entry, const int* __restrict__ tile_q0,
                        int Hq, int Hkv, int page_size, float scale, int window, int block, int sink, int pieces, Extra ex) {
-    // A successor that is released at once lands on whatever SMs this kernel leaves free, several CTAs to one, and stays there; released
-    // at this kernel's end it spreads out.  At once / at the end, us of a 32-bit layer of 32 heads of 64 (when the kernel took two to four
-    // times as long as it does): a prompt of 300 tokens 567 / 385,
-    // three of 80 492 / 288; a token each of 16 requests behind 15 keys 108 / 81 and behind 1,023 706 / 676, of 64 behind 127 439 / 342,
-    // of 9 behind 1,023 568 / 555.  Up to eight tiles (a tile is 16 tokens of a prompt, or a request's single token) both take about
-    // the same, and eight single tokens behind 1,023 keys 443 / 455.
-    const bool late = gridDim.x > 8;
-    if (!late) pdl_trigger();
+    // The successor is released at this kernel's end, where it spreads out: released at once it lands on whatever SMs this kernel leaves
+    // free, several CTAs to one, and stays there.  At once / at the end, us of a 32-bit layer of 32 heads of 64: a prompt of 16 tokens 71 / 64,
+    // 128 225 / 196, 300 406 / 315, 1,000 907 / 803, three of 80 513 / 258; a token each of 4 requests behind 1,023 keys 138 / 126, of
+    // 16 behind 15 148 / 67 and behind 1,023 345 / 232, of 64 behind 127 253 / 189.
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
     float* Qs = smem;
@@ -311,7 +307,7 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, TO* __restrict__ o
             stage_keys<VD, T>(Vs, VP, cache, bt, page_elems, v_base, v_row, page_size, kb + KC, lo_tile, p_last, pieces);
         }
     }
-    if (late) pdl_trigger();
+    pdl_trigger();
     if (row_valid) {
         const int t = q_begin + j0 + row;
 #pragma unroll
@@ -681,10 +677,10 @@ int launch(const void* q, int q_stride, void* out, int out_stride, const void* c
         (const T*)q, q_stride, (TO*)out, out_stride, (const T*)cache, block_table, table_stride, \
         cu_q, kv_len, tile_entry, tile_q0, Hq, Hkv, page_size, scale, window, block, sink, pieces, ex)); } while (0)
     const int per = Hq / (Hkv * ex.maps);
-    // Two heads a CTA from 3.5 CTAs an SM on (148), below that they leave SMs idle.  One / two, us, heads of 64, 32 over 8: 200 tokens
+    // Two heads a CTA from 3.5 CTAs an SM on, below that they leave SMs idle.  One / two, us, heads of 64, 32 over 8: 200 tokens
     // (3.0) 37.9 / 39.9, 3 of 80 (3.5) 23.5 / 24.7, 300 (4.3) 55.5 / 54.2, 1,000 362 / 265, 2,048 1,284 / 887; a token of 16 requests
     // behind 1,023 keys (3.7) 175 / 153, of 64 595 / 380; heads of 128, the same 412 / 244 and 1,419 / 934, 300 tokens 107.6 / 83.0.
-    if (MOST_HEADS == 2 && per % 2 == 0 && (long)n_tiles * Hq * 2 > 7 * 148) RI_PLAIN(MOST_HEADS);
+    if (MOST_HEADS == 2 && per % 2 == 0 && (long)n_tiles * Hq * 2 > 7L * ri_device_sms()) RI_PLAIN(MOST_HEADS);
     else RI_PLAIN(1);
 #undef RI_PLAIN
     return ri_launch_status();
