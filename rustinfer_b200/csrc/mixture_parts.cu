@@ -41,7 +41,9 @@ __device__ __forceinline__ int warp_rank(float v, unsigned live, int lane) {
 }
 
 // TT tokens a CTA (a row of the router's matrix is read once for them), each warp a few experts at a time.  8 tokens of 1,024, 33 rows: 15.5 ->
-// 7.5 us; up to 32 experts (and groups) are ranked in registers, all at once, instead of found one after the other.
+// 7.5 us.  Up to 32 experts (and groups) are ranked in registers, all at once, where that takes no longer than finding the chosen ones one
+// after the other: a rank of 32 costs two rounds, of 32 groups four (one of 32 experts found and ranked 1.6 and 2.2 us, three 2.35 and
+// 2.27, eight 4.0 and 2.25; one of 8 groups 3.8 and 4.1, two 4.2 and 4.1; two of 32 groups 4.7 and 5.1, four 5.3 and 5.1).
 // EARLY: the terms of a lane are asked for together, for calls whose CTAs all fit at once and wait for nothing but those loads; its registers
 // leave an SM one CTA of 16 warps, and it multiplies for absent experts too (300 tokens of 512, 64 experts, without and with: 9.3 and 17.2 us).
 template <typename TX, int TT, bool EARLY>
@@ -152,7 +154,7 @@ moe_route_kernel(const float* __restrict__ z, const TX* __restrict__ x, const fl
         }
         __syncwarp();
         const float mine = lane < n_groups ? gs[lane] : -INFINITY;
-        if (n_groups <= 32 && __all_sync(0xffffffffu, mine < INFINITY)) {        // (a number that is none, too, goes the other way)
+        if (n_groups <= 32 && keep > 1 + n_groups / 16 && __all_sync(0xffffffffu, mine < INFINITY)) {        // (a number that is none, too, goes the other way)
             const int rank = warp_rank(mine, n_groups < 32 ? (1u << n_groups) - 1u : 0xffffffffu, lane);
             if (lane < n_groups && rank < keep) gs[lane] = INFINITY;
             __syncwarp();
@@ -174,7 +176,7 @@ moe_route_kernel(const float* __restrict__ z, const TX* __restrict__ x, const fl
         __syncwarp();
     }
     float wsum = 0.f, zmax = 0.f;
-    if (E <= 32) {
+    if (E <= 32 && top > (E > 16 ? 2 : 1)) {
         const float v = lane < E ? c[lane] : -INFINITY, own = lane < E ? s[lane] : 0.f;
         const unsigned live = __ballot_sync(0xffffffffu, v > -INFINITY);         // neither cut nor no number
         if (__popc(live) >= top) {
