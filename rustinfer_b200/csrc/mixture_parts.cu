@@ -637,10 +637,13 @@ RI_API int ri_moe_product(const void* a, int a_dtype, int a_stride, const void* 
     const bool tensor_cores = a_dtype == RI_BF16 && w_dtype == RI_BF16 && K % 8 == 0 && a_stride % 8 == 0 &&
                               ((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0 && ri_moe_tensor_cores();
     if (tensor_cores && ((gated && out_dtype == RI_BF16) || (!gated && out_dtype == RI_F32))) {
-        // Four stages where few rows leave a CTA waiting for its own matrix (8 tokens, 32 experts of 1,024 x 768, four a token: the layer 46.7
-        // us against 54.5 with three, 52.8 with five) and where K is long (2,048 x 1,536, 64 tokens: 166 against 173); three where CTAs fill the
-        // SMs six times over (1,024 x 768, 64 tokens: 70.8 against 73.9).
-        const bool deep = bm == 16 && (rows <= E || K >= 1536);
+        // A fourth stage where it costs no wave of CTAs: an SM holds six of them with three stages and four with four.  How many find rows is
+        // the router's choice; an even one is taken, with a tenth to spare.  Three / four, us, 32 experts, four a token: 8 tokens of 1,024,
+        // gated 768 (one wave either way) 19.1 / 14.9, 64 tokens (one / two) 23.8 / 28.1; 64 of 1,408, gated 1,024 (two) 44.0 / 38.5; 4 of
+        // 2,880, 2,880 (one / two) 50.7 / 63.3.
+        const double used = E * (1.0 - pow(1.0 - 1.0 / E, rows)), tiles = used * fmax(1.0, rows / (16.0 * E) + 0.5);
+        const double resident = tiles * grid.y / ri_device_sms();
+        const bool deep = bm == 16 && ceil(1.1 * resident / 4) == ceil(resident / 6);
 #define RI_MM(TO, BM, G, S) do { \
         static bool configured = false; \
         const size_t smem = moe_mma_smem<BM, S>(); \
