@@ -247,20 +247,24 @@ __device__ __forceinline__ void store_cols(const Params& p, int tok, int feat0, 
 
 // The same at the matrix's ragged edge, or where rows allow no vectors: whole groups of 16, then element by element.  In loops, on a
 // copy in local memory: unrolled into a tile's code it was ten thousand instructions that the tile ran through once, each from memory
-// (a last tile of 32 columns in 256: 1,024 x 3,104 x 2,048 32.5 -> 16.4 us; 300 x 5,152 x 1,024 30.3 -> 11.5).
+// (a last tile of 32 columns in 256: 1,024 x 3,104 x 2,048 32.5 -> 16.4 us; 300 x 5,152 x 1,024 30.3 -> 11.5).  A group of a row without
+// vectors is unrolled too (element by element / now: 65 x 2,052 x 2,048 into bf16 22.9 / 16.9, 300 x 1,000 x 1,024 with gates 22.7 / 17.1).
 template <int N>
 __device__ __forceinline__ void store_ragged(const Params& p, int tok, int feat0, const float (&v)[N]) {
     float kept[N];
 #pragma unroll
     for (int j = 0; j < N; ++j) kept[j] = v[j];
     int at = 0;
-    if (p.vec) {
 #pragma unroll 1
-        for (; at < N && feat0 + at + 16 <= p.b_rows; at += 16) {
-            float w[16];
+    for (; at < N && feat0 + at + 16 <= p.b_rows; at += 16) {
+        float w[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) w[j] = kept[at + j];
+        for (int j = 0; j < 16; ++j) w[j] = kept[at + j];
+        if (p.vec) {
             store_cols<16, false>(p, tok, feat0 + at, w);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) store_one(p, p.a_rows, p.b_rows, tok, feat0 + at + j, w[j], w[j | 1]);
         }
     }
 #pragma unroll 1
@@ -296,6 +300,17 @@ __device__ __forceinline__ void finish_sums(const Params& p, int tile, int tok, 
         for (int s = 0; s < p.splits; ++s)
 #pragma unroll
             for (int j = 0; j < BN; ++j) sum[j] += __ldcg(base + (size_t)s * (BN * 128) + (size_t)j * 128);
+    }
+    const bool whole = p.vec && b0 + BN <= p.b_rows;         // (asked once: with the edge's code between a tile's stores SiLU's were 3 % slower)
+    if (whole) {
+#pragma unroll
+        for (int c0 = 0; c0 < BN; c0 += 64) {
+            float v[64];
+#pragma unroll
+            for (int j = 0; j < 64; ++j) v[j] = sum[c0 + j];
+            store_cols<64>(p, tok, b0 + c0, v);
+        }
+        return;
     }
 #pragma unroll
     for (int c0 = 0; c0 < BN; c0 += 64) {
