@@ -27,6 +27,7 @@ from ..cache.manager import CacheLayout, CacheManager
 from ..cache.pages import OutOfPages
 from ..config.registry import load_model_description
 from ..models.decoder import Decoder
+from ..ops.library import read_stream_budget
 from ..parts.base import (BuildContext, FixedState, GroupStep, HostEntry, PagedKV, PagedLayerCache,
                           StateLayerCache, StepContext, StepShape)
 from ..weights.loader import load_weights
@@ -256,6 +257,7 @@ class ModelRunner:
             raise RuntimeError("rustinfer_b200 runs on a CUDA device (sm_100a) only; there is no CPU path")
         self.device = torch.device(device)
         torch.cuda.set_device(self.device)
+        read_stream_budget()
         self.dtype = parse_dtype(dtype)
         # the 32-bit path is true fp32 everywhere: no TF32 in any library product either
         torch.backends.cuda.matmul.allow_tf32 = False

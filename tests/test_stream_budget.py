@@ -1,4 +1,4 @@
-"""The ring of the products' operand stages takes its size from the environment whenever that is set, once."""
+"""The ring of the products' operand stages takes its size from the environment when the library is loaded and when a runner is made."""
 from types import SimpleNamespace
 
 from rustinfer_b200.ops import library as L
@@ -12,4 +12,7 @@ def test_a_size_set_after_the_first_product_counts(monkeypatch):
     monkeypatch.delenv("RUSTINFER_B200_STREAM_KB", raising=False)
     assert L.gemm_tc() is lib and sizes == []
     monkeypatch.setenv("RUSTINFER_B200_STREAM_KB", "96")
-    assert L.gemm_tc() is lib and L.gemm_tc() is lib and sizes == [96 * 1024]
+    L.read_stream_budget()
+    assert L.gemm_tc() is lib and sizes == [96 * 1024]
+    monkeypatch.setattr(L, "_loaded", {})
+    assert L.gemm_tc() is lib and sizes == [96 * 1024] * 2
