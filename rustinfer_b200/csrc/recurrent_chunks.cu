@@ -942,9 +942,9 @@ gated_chunk_outputs_kernel(const bf16* __restrict__ parts, const bf16* __restric
 // their sizes; the host sends only decays here whose products over half a chunk stay far from the ends of fp32 (DELTA_MOST_DECAY).
 // (The gated form's decays have no such bound, so its scores part at every quarter and multiply their way inside one.)
 //
-// 2,444 tokens in four entries, 16 heads of 128 x 128: parts 140 us, scan 80, outputs 47, where the walk takes 395; one entry of 2,048
-// tokens and 8 heads 166 us with what prepares it, the walk 678.  The parts are bound by what a CTA's phases wait for (products of a
-// few blocks, the inverse: tensor cores 30 % busy, 11 cycles an instruction and warp), the scan by its products (half of the tensor
+// 2,444 tokens in four entries, 16 heads of 128 x 128: 296 us with what prepares it (parts some 145, scan 80, outputs 47), where the walk
+// takes 395; one entry of 2,048 tokens and 8 heads 163, the walk 678.  The parts are bound by what a CTA's phases wait for (products of a
+// few blocks, the inverse: tensor cores a third busy, 10 cycles an instruction and warp), the scan by its products (half of the tensor
 // cores' rate, one chunk after the other).  Tried: the parts' next channels asked for ahead (registers; 2 % slower).
 constexpr float DELTA_MOST_DECAY = 1.0f;        // of -log w: factors of a middle lie between e^-32 and e^32
 constexpr int DP_THREADS = 256;
@@ -1093,6 +1093,7 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
                 mid[(seg & 1) * DK + ch] = (float)(fx * px);
                 mid[(seg & 1) * DK + ch + 1] = (float)(fy * py);
             }
+            float2 beyond = make_float2(1.f, 1.f);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int i = early ? 3 - j : j, t = seg * 4 + i;
@@ -1104,9 +1105,11 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
                 // the product between the middle and the state behind token t, and that between the middle and the state in front of it
                 const float2 behind = early ? make_float2(bx, by) : make_float2(ax, ay), front = early ? make_float2(ax, ay) : make_float2(bx, by);
                 *reinterpret_cast<float2*>(ps + t * L::PF + ch) = behind;
-                const float2 inv = make_float2(__frcp_rn(behind.x), __frcp_rn(behind.y));
+                // (early: what lies in front of a token lies behind the next)
+                const float2 inv = early && j > 0 ? beyond : make_float2(__frcp_rn(behind.x), __frcp_rn(behind.y));
+                if (early) beyond = make_float2(__frcp_rn(front.x), __frcp_rn(front.y));
                 const float2 row = early ? inv : behind, col = early ? behind : inv;
-                const float2 urow = early ? make_float2(__frcp_rn(front.x), __frcp_rn(front.y)) : front;
+                const float2 urow = early ? beyond : front;
                 uint32_t x[3];
                 bf16* to = stage + t * SP + 2 * pair;
                 auto put = [&](int which, float p0, float p1) {
@@ -1191,7 +1194,12 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
         if (j < 2 && j <= short_row) put_scores(short_row, j, ss[j]);
     }
     __syncthreads();
-    // ---- T = (I + A)^-1 in place: blocks of 16 by substitution, then pairs of blocks, [[T1, 0], [-T2 A T1, T2]]; A T1 lies above the diagonal
+    // ---- T = (I + A)^-1: blocks of 16 on the diagonal by substitution, then the ones one, two and three blocks below it,
+    // T_ij = -T_ii sum of A_ik T_kj over k = j .. i - 1, a warp a block.  Where keys resemble one another the terms of these sums cancel, and
+    // sixteen at a time from the tensor cores they lose less than one after another in 32 bits, in less time (304 us a call for 312).
+    // Repeated keys of 64 and 128 that hardly decay: the outputs 2.0e-6 and 1.8e-6 from 64 bits where they were 3.5e-6 and 3.4e-6 (the walk
+    // 1.0e-6 and 1.1e-6); that decay by 2 % a token 0.8e-6 and 1.0e-6, were 3.4e-6 and 3.5e-6 (0.35e-6); a twentieth of noise in the keys and
+    // hardly any decay 1.6e-6, were 1.7e-6 and 1.8e-6 (1.4e-6 and 1.5e-6).  What is left is the scores' own rounding: sums in 64 bits give no less.
     if (tid < CK) {
         float x[16];
         const float* blk = as + (tid >> 4) * 16 * (L::AF + 1);
@@ -1210,61 +1218,58 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
         __syncwarp();
         float* to = as + (tid >> 4) * 16 * (L::AF + 1) + col;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) to[i * L::AF] = x[i];
+        for (int i = 0; i < 16; ++i) to[i * L::AF] = (float)x[i];
     }
     __syncthreads();
-    {
-        float* blk = as + (tid >> 7) * 32 * (L::AF + 1);
-        const int i = (tid & 127) >> 3, j = (tid & 7) * 2;
-        float2 m = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int n = 0; n < 16; ++n) {
-            const float x = blk[(16 + i) * L::AF + n];
-            const float2 y = *reinterpret_cast<const float2*>(blk + n * L::AF + j);
-            m = make_float2(fmaf(x, y.x, m.x), fmaf(x, y.y, m.y));
-        }
-        *reinterpret_cast<float2*>(blk + i * L::AF + 16 + j) = m;
-        __syncthreads();
-        m = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int n = 0; n < 16; ++n) {
-            const float x = blk[(16 + i) * L::AF + 16 + n];
-            const float2 y = *reinterpret_cast<const float2*>(blk + n * L::AF + 16 + j);
-            m = make_float2(fmaf(-x, y.x, m.x), fmaf(-x, y.y, m.y));
-        }
-        __syncthreads();
-        *reinterpret_cast<float2*>(blk + (16 + i) * L::AF + j) = m;
-    }
-    __syncthreads();
-    {
-        const int i = tid >> 3, j = (tid & 7) * 4;
-        float4 m = zero4();
-        for (int n = j < 16 ? 0 : 16; n < 32; ++n) {
-            const float x = as[(32 + i) * L::AF + n];
-            const float4 y = load4(as + n * L::AF + j);
-            m = make_float4(fmaf(x, y.x, m.x), fmaf(x, y.y, m.y), fmaf(x, y.z, m.z), fmaf(x, y.w, m.w));
-        }
-        *reinterpret_cast<float4*>(as + i * L::AF + 32 + j) = m;
-        __syncthreads();
-        m = zero4();
-        for (int n = 0; n < (i < 16 ? 16 : 32); ++n) {
-            const float x = as[(32 + i) * L::AF + 32 + n];
-            const float4 y = load4(as + n * L::AF + 32 + j);
-            m = make_float4(fmaf(-x, y.x, m.x), fmaf(-x, y.y, m.y), fmaf(-x, y.z, m.z), fmaf(-x, y.w, m.w));
-        }
-        *reinterpret_cast<float4*>(as + (32 + i) * L::AF + j) = m;
-    }
-    __syncthreads();
-    for (int e = tid; e < LOWER * 128; e += DP_THREADS) {
-        const int at = e >> 7, i = at < 1 ? 0 : at < 3 ? 1 : at < 6 ? 2 : 3, j = at - lower_block(i, 0), row = (e & 127) >> 3, col = (e & 7) * 2;
-        const float2 x = *reinterpret_cast<const float2*>(as + (i * 16 + row) * L::AF + j * 16 + col);
+    for (int e = tid; e < QUARTERS * 128; e += DP_THREADS) {
+        const int i = e >> 7, row = (e & 127) >> 3, col = (e & 7) * 2;
+        const float2 x = *reinterpret_cast<const float2*>(as + (i * 16 + row) * L::AF + i * 16 + col);
         uint32_t y[3];
         cut(x.x, x.y, y);
 #pragma unroll
         for (int p = 0; p < 3; ++p)
-            *reinterpret_cast<uint32_t*>(ts + (at * 3 + p) * 256 + row * 16 + (((col >> 3) ^ (row >> 2 & 1)) << 3) + (col & 7)) = y[p];
+            *reinterpret_cast<uint32_t*>(ts + (lower_block(i, i) * 3 + p) * 256 + row * 16 + (((col >> 3) ^ (row >> 2 & 1)) << 3) + (col & 7)) = y[p];
     }
     __syncthreads();
+#pragma unroll 1
+    for (int below = 1; below < QUARTERS; ++below) {
+        const int j = warp, i = warp + below;
+        if (i < QUARTERS) {
+            uint32_t fa[3][1][4], fb[3][1][4];
+            float d[1][2][4] = {}, z[1][2][4] = {};
+#pragma unroll 1
+            for (int k = j; k < i; ++k) {
+                const float* from = as + (i * 16 + g) * L::AF + k * 16 + t4 * 2;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 x = *reinterpret_cast<const float2*>(from + (e & 1) * 8 * L::AF + (e >> 1) * 8);
+                    uint32_t y[3];
+                    cut(x.x, x.y, y);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) fa[p][0][e] = y[p];
+                }
+#pragma unroll
+                for (int p = 0; p < 3; ++p) ldsm_t(fb[p][0], lane_row(ts + (lower_block(k, j) * 3 + p) * 256, lane));
+                products<1, 1, 3, 3>(d, fa, fb);
+            }
+            bf16* to = ts + lower_block(i, j) * 3 * 256;     // the sum, then the block itself
+            put_block(to, d[0], lane);
+            __syncwarp();
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                ldsm(fa[p][0], lane_row(ts + (lower_block(i, i) * 3 + p) * 256, lane));
+                ldsm_t(fb[p][0], lane_row(to + p * 256, lane));
+            }
+            products<1, 1, 3, 3>(z, fa, fb);
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) z[0][n][e] = -z[0][n][e];
+            __syncwarp();
+            put_block(to, z[0], lane);
+        }
+        __syncthreads();
+    }
     // ---- Y = T B;  then W = Q T and P' = P - Q Y
     for (int n = 0; n < 2; ++n) {
         const int at = warp_blocks(warp, n);

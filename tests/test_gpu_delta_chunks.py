@@ -128,3 +128,22 @@ def test_arrays_off_their_boundaries_walk(out_at, zw_at, monkeypatch):
                        longest=longest)
         got.append((out, state))
     assert all(torch.equal(a, b) for a, b in zip(*got)) and torch.isfinite(got[0][0]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("noise", [0.0, 0.05, 0.5])
+@pytest.mark.parametrize("dk", [64, 128])
+def test_keys_that_resemble_one_another(noise, dk, monkeypatch):
+    """Where the triangular system is far from the identity: keys around a common vector, hardly any decay, nearly all of u^T S taken away."""
+    monkeypatch.setattr(K(), "_DELTA_CHUNK_FIXED_US", -1e9)
+    c = make([320], 2, dk, dk, -9.0, -8.0)
+    gen = torch.Generator().manual_seed(3)
+    common = torch.randn((1, 2 * dk), generator=gen).to(c["k"].device)
+    c["k"] = (common + noise * torch.randn((c["T"], 2 * dk), generator=gen).to(common.device)).to(BF)
+    c["za"] = torch.full_like(c["k"], 6.0)
+    rate = math.exp(-0.5)
+    want, walked, got = exact(c, rate), scan(c, 0, rate), scan(c, 320, rate)
+    assert not torch.equal(walked[0], got[0])
+    for a, b, x in zip(got, walked, want):
+        # repeated keys: earlier values are erased by differences of scores that are equal but for their roundings (2^-23 each), 64 in a chunk
+        assert off(a, x) <= 1.25 * off(b, x) + (2.0 ** -23 if noise else 64 ** 0.5 * 2 * 2.0 ** -23)
