@@ -996,6 +996,19 @@ __device__ __forceinline__ int warp_blocks(int warp, int which) {        // i * 
     constexpr int first[8] = {12, 8, 13, 4, 9, 14, 15, -1}, second[8] = {-1, -1, -1, 0, 5, 10, -1, -1};
     return which ? second[warp] : first[warp];
 }
+// 1 / x for x between 2^-60 and 2^60: one step of Newton's method, y + y (1 - x y), from the special-function unit's approximation.  That is off
+// by a unit of the last place at the most, so the step leaves its square, 2^-46, and one rounding: half a unit, as the correctly rounded
+// __frcp_rn, whose way costs 3 % of a call with keys of 128 and up to 10 % with keys of 64 (16 heads, 2,444 tokens in four entries: 304 us
+// against 296, and 180 against 166).
+__device__ __forceinline__ float reciprocal(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(y, fmaf(-x, y, 1.f), y);
+}
+__global__ void reciprocal_kernel(const float* x, float* y, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[i] = reciprocal(x[i]);
+}
 __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
 // One chunk and head.  Outputs, all in the order of fragments ([piece][token block][key block][lane][8] for xs and au): xs: X; au: the
@@ -1106,8 +1119,8 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
                 const float2 behind = early ? make_float2(bx, by) : make_float2(ax, ay), front = early ? make_float2(ax, ay) : make_float2(bx, by);
                 *reinterpret_cast<float2*>(ps + t * L::PF + ch) = behind;
                 // (early: what lies in front of a token lies behind the next)
-                const float2 inv = early && j > 0 ? beyond : make_float2(__frcp_rn(behind.x), __frcp_rn(behind.y));
-                if (early) beyond = make_float2(__frcp_rn(front.x), __frcp_rn(front.y));
+                const float2 inv = early && j > 0 ? beyond : make_float2(reciprocal(behind.x), reciprocal(behind.y));
+                if (early) beyond = make_float2(reciprocal(front.x), reciprocal(front.y));
                 const float2 row = early ? inv : behind, col = early ? behind : inv;
                 const float2 urow = early ? beyond : front;
                 uint32_t x[3];
@@ -1359,7 +1372,7 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
                     const int t = i * 16 + g + 8 * e;
                     cut(dx[0][n][2 * e] * m.x, dx[0][n][2 * e + 1] * m.y, x[e * 2 + n]);
                     float2 f = *reinterpret_cast<const float2*>(ps + t * L::PF + ch);
-                    if (t < 32) f = make_float2(__frcp_rn(f.x), __frcp_rn(f.y));
+                    if (t < 32) f = make_float2(reciprocal(f.x), reciprocal(f.y));
                     const uint32_t r2 = rc[i][n * 2 + e];
                     uint32_t y[3];
                     cut(t >= bad ? nan : (low_of(r2) * f.x - dr[0][n][2 * e]) * m.x, t >= bad ? nan : (high_of(r2) * f.y - dr[0][n][2 * e + 1]) * m.y, y);
@@ -1411,7 +1424,7 @@ delta_chunk_parts_kernel(const bf16* __restrict__ r, int r_stride, const bf16* _
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     float2 f = *reinterpret_cast<const float2*>(ps + (j * 16 + g + 8 * e) * L::PF + ch);
-                    if (j >= 2) f = make_float2(__frcp_rn(f.x), __frcp_rn(f.y));
+                    if (j >= 2) f = make_float2(reciprocal(f.x), reciprocal(f.y));
                     uint32_t x[3];
                     cut((low_of(kc[j][n * 2 + e]) * f.x - d[0][n][2 * e]) * m.x, (high_of(kc[j][n * 2 + e]) * f.y - d[0][n][2 * e + 1]) * m.y, x);
 #pragma unroll
@@ -1713,6 +1726,12 @@ RI_API int ri_gated_chunks(const void* q, int q_stride, const void* k, int k_str
 // The delta rule (bf16 r, k, v; w, u, au fp32 [T][f_stride] as the walk's, -log w at most ri_delta_chunk_decay()): xs and aus bf16
 // [chunks][H][3][CK][DK], ends fp32 [chunks][H][2][DK], the rest as the gated form's.
 RI_API float ri_delta_chunk_decay() { return DELTA_MOST_DECAY; }
+// The reciprocals that the decays' products take (n floats), for their test.
+RI_API int ri_delta_chunk_reciprocals(const float* x, float* y, int n, void* stream) {
+    if (n <= 0) return 0;
+    reciprocal_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(x, y, n);
+    return ri_launch_status();
+}
 RI_API int ri_delta_chunks(const void* r, int r_stride, const void* k, int k_stride, const void* v, int v_stride, const float* w,
                            const float* u, const float* au, int f_stride, int act_dtype, float* out, float* state, const int* cu_q,
                            const int* state_slots, int entries, int least, int chunks, int H, int dv, float* states, float* ends, void* cuts,
@@ -1760,6 +1779,7 @@ RI_API int ri_gated_chunks(const void*, int, const void*, int, const void*, int,
 }
 RI_API int ri_gated_chunk_parts() { return 0; }
 RI_API float ri_delta_chunk_decay() { return 0.f; }
+RI_API int ri_delta_chunk_reciprocals(const float*, float*, int, void*) { return (int)cudaErrorInvalidValue; }
 RI_API int ri_delta_chunks(const void*, int, const void*, int, const void*, int, const float*, const float*, const float*, int, int, float*,
                            float*, const int*, const int*, int, int, int, int, int, float*, float*, void*, void*, void*, void*, void*) {
     return (int)cudaErrorInvalidValue;

@@ -147,3 +147,18 @@ def test_keys_that_resemble_one_another(noise, dk, monkeypatch):
     for a, b, x in zip(got, walked, want):
         # repeated keys: earlier values are erased by differences of scores that are equal but for their roundings (2^-23 each), 64 in a chunk
         assert off(a, x) <= 1.25 * off(b, x) + (2.0 ** -23 if noise else 64 ** 0.5 * 2 * 2.0 ** -23)
+
+
+@pytest.mark.gpu
+def test_reciprocals():
+    """Every significand of one power of two, and the range that products of 32 decays of at least e^-1 have."""
+    from rustinfer_b200.ops import library as L
+    lib = L.recurrent(128)
+    for bits in (torch.arange(0x3f800000, 0x40000000, dtype=torch.int32, device="cuda:0"),
+                 torch.arange(0x28000000, 0x57800000, 251, dtype=torch.int32, device="cuda:0")):          # 2^-47 .. 2^48
+        x = bits.view(torch.float32)
+        y = torch.empty_like(x)
+        L.check(lib.ri_delta_chunk_reciprocals(x.data_ptr(), y.data_ptr(), x.numel(), L.stream_ptr()), "reciprocals")
+        # a rounding, and the square of the approximation's error (2^-46): half a unit of the last place, as CUDA's own is
+        assert float((y.double() * x.double() - 1).abs().max()) <= 2.0 ** -24 * (1 + 2.0 ** -10)
+        assert int((y.view(torch.int32) - torch.reciprocal(x).view(torch.int32)).abs().max()) <= 1
