@@ -13,7 +13,7 @@
 //
 // One CTA = 128 rows x one kv head; a row is (query token, q head of the kv head's group),
 // so the group's heads share every K/V tile.  192 threads:
-//   warp 0      TMA producer (one thread): K and V boxes of each 64-key tile, 3 stages each
+//   warp 0      TMA producer (a lane a box): K and V boxes of each 64-key tile, 2 stages each
 //   warp 1      tensor memory allocation; one thread issues the MMAs, S of tile j+1 before
 //               P V of tile j, so the tensor core computes scores while the softmax of the
 //               tile before is still running
@@ -26,8 +26,10 @@
 // (their sum is the weight), P V runs once a piece into the same accumulator, the small pieces first; scores may carry a bias by
 // distance, the denominator a sink, the output a gate, each a head.  The biases of the group's heads lie in shared memory; a
 // warp whose rows see a whole tile from the table's last distance on (most tiles of a long prompt) adds one number a row, the
-// others read one a score.  What bounds it is the softmax warps' issue rate (about ten instructions a score, half of them
-// the pieces) before the tensor core (16 MMAs a tile, 2/3 of the cycles reading operands).  Against the mma.sync kernel
+// others read one a score.  Values of keys that no row of a tile sees are cleared; one that a row does see and that is no number
+// reaches every row of the tile, 128 / (heads a key head) tokens, since a weight of zero times NaN is NaN.
+// What bounds it is the softmax warps' chain a tile (about ten instructions a score, half of them the pieces): 43 % of the issue slots
+// go, the tensor pipe is a quarter busy (16 MMAs a tile), and two CTAs an SM take turns.  Against the mma.sync kernel
 // (attention_rows.cu), 32 heads of 64 over 8, bias of 128 distances: 2 tokens 6.7 -> 6.6 us, 300 tokens 20.8 -> 14.1,
 // 2,048 tokens 226 -> 66, 16 x 300 101 -> 62; 8 heads of 128 over 2: 2 tokens 8.5 -> 6.7, 2,048 tokens 200 -> 51.
 // Every wait on an mbarrier is bounded; a time-out leaves a code in *error and the kernel

@@ -1496,7 +1496,8 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
     keys and queries are rotated on the way in; only for a step in which every entry brings one token (T == entries).
     `longest`: the most tokens an entry brings, from a caller that does not need a token's sums to be the same however its
     prompt was cut and whichever entries share the call: entries of CHUNK_MIN_TOKENS or more may then go in chunks
-    (recurrent_chunks.cu), which differ from the walk in rounding, and make NaN of an infinity that the walk carries on."""
+    (recurrent_chunks.cu), which differ from the walk in rounding, and make NaN of an infinity that the walk carries on.  (out on an 8-byte
+    boundary; one that is not walks.)"""
     require_cuda(q, k, v, decay, out, state, cu_q, state_slots, gain, *(rotation[:3] if rotation else ()))
     T, H, dk, dv = q.shape[0], num_heads, key_dim, value_dim
     G = key_heads or H
@@ -1547,8 +1548,8 @@ def delta_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, za: torch.Tens
     """Delta rule with a decay, over every entry's tokens in order, from and into state[slot]:
     S = diag(w) S - (a * u)(u^T S) + k v^T, out = S^T r, with u = k / sqrt(|k|^2 + unit_eps),
     w = exp(-decay_rate * sigmoid(zw + zw_bias)), a = sigmoid(za + za_bias).  zw is fp32 and is
-    overwritten with the decays.  Two launches: w, u and a * u of all tokens at once, then the walk.  `longest`: as `head_scan`'s (bf16 r,
-    k, v; decay_rate at most 1)."""
+    overwritten with the decays.  One launch makes w, u and a * u of all tokens; then the walk, or the entries that go in chunks (three
+    launches) and a walk for the others.  `longest`: as `head_scan`'s (bf16 r, k, v; decay_rate at most 1; zw on a 16-byte boundary)."""
     require_cuda(r, k, v, za, za_bias, zw, zw_bias, out, state, cu_q, state_slots)
     T, H, dk, dv = r.shape[0], num_heads, key_dim, value_dim
     _scan_common(state, out, cu_q, state_slots, T, H, dk, dv, "delta_scan")
@@ -1900,7 +1901,8 @@ def attention_prefill_exact(q, out, cache, block_table, cu_q, kv_len, tile_entry
                             head_dim: int, scale: float, window: Optional[int], sink_values: Optional[torch.Tensor] = None,
                             bias: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, gate_scale: float = 1.0) -> None:
     """`attention_prefill_tc` with the softmax weights unrounded (three bf16 pieces a weight) and `attention_plain`'s bias by
-    distance, sinks and gate a head.  bf16 out; tiles as `attention_prefill_tc`'s."""
+    distance, sinks and gate a head.  bf16 out; tiles as `attention_prefill_tc`'s.  A value that is no number makes NaN of every token
+    that sees it and of those ahead of it in its own tile, up to 128 / (heads a key head) - 1 of them (`attention_rows`: 64)."""
     _attention_args(q, out, cache, block_table, cu_q, kv_len, num_heads, num_kv_heads, head_dim)
     require_cuda(tile_entry, tile_tok0, sink_values, bias, gate)
     _i32(tile_entry, "tile_entry"); _i32(tile_tok0, "tile_tok0")

@@ -7,8 +7,8 @@
     distance_bias_attention  (also `gated_attention`) grouped-query attention with the parts such layers share: a bias by
                              distance or a rotation, a query temperature, a sink, a gate a head
 
-All run on the fp32-arithmetic attention kernels in both engine precisions: scores, softmax weights and
-the weighted sum of values are 32-bit there.  The reference engine has one attention
+Scores, softmax weights and the weighted sum of values are 32-bit in both engine precisions: on the fp32-arithmetic kernels, or in the
+bfloat16 engine on the tensor cores with the weights unrounded.  The reference engine has one attention
 (crates/infer-worker/src/components/attention.rs:21-37); these are parts of the same kind with caches of
 their own shapes.
 """
@@ -56,7 +56,9 @@ def rows_are_sooner(tiles: int, kv_heads: int, group: int, head_dim: int, tokens
 class PlainAttend:
     """How a mixer sends its queries to the attention kernels with fp32 scores and softmax weights.  The bfloat16
     engine, where the sizes are multiples of 16: prompt portions go to the tensor-core kernel in tiles of 64 (token, head)
-    rows (heads of 64 and 128 whose scores have no cap and no slopes: to the tcgen05 kernel in tiles of 128, `take_exact`), entries of one token to its sister for single tokens, whose warps walk the keys of a key head side by side for up to
+    rows, or, for heads of 64 and 128 whose scores have no cap and no slopes, to the tcgen05 kernel in tiles of 128 (`take_exact`;
+    not many short portions over few keys, `rows_are_sooner`).  Entries of one token go to the former's sister for single tokens, whose
+    warps walk the keys of a key head side by side for up to
     16 of its query heads.  Other sizes: entries of one token go to the fp32-arithmetic kernel that reads a key head once for
     all its query heads (where it takes the geometry).  All of them cut the keys of single tokens into ranges when few CTAs
     would walk many keys.  What none of them takes runs on the fp32-arithmetic kernel in tiles of 16 query rows.  The 32-bit
