@@ -40,7 +40,7 @@ def rows_are_sooner(tiles: int, kv_heads: int, group: int, head_dim: int, tokens
     `attention_prefill_exact`, whose CTAs take twice the rows and find fewer places.  That is for many portions over few keys: 16 portions of 2
     tokens, 16 heads of 128 with a key head each 9.3 us against 14.5, behind 64 keys 14.1 against 17.7, behind 200 25.0 against 22.3; 24 of 16
     heads of 64 6.4 against 12.9.  Of 2,958 calls timed both ways (1 to 64 portions of 2 to 64 tokens behind 0
-    to 1,000 keys, 2 to 32 key heads) 124 go the way that is slower by more than 3 %, 28 by more than 10 %, none by 24 (617 and 2,189
+    to 1,000 keys, 2 to 32 key heads) 124 go the way that is slower by more than 3 %, 28 by more than 10 %, at most 24 % (617 and 2,189
     were it always the one or the other)."""
     ctas, key_tiles = tiles * kv_heads, -(-keys // 64)
 
