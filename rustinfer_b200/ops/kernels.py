@@ -1327,7 +1327,7 @@ def _scan_chunks(T: int, entries: int, longest: int, heads: int, key_dim: int, v
 def _chunks_or_walk(T: int, entries: int, longest: int, heads: int, key_dim: int, value_dim: int, num_sms: int, least: int,
                     sizes: Tuple[int, ...], walk_us: Dict[int, Tuple[float, ...]], fixed_us: float, chunk_us: Dict[int, Tuple[float, ...]]) -> int:
     """Fitted to calls that were timed both ways (1 to 16 entries of 192 to 4,096 tokens, short ones beside them, 2 to 128 heads, keys of 64
-    and 128, values of 64 to 256): of 3,325, 122 go the way that is slower by more than 3 %, 18 by more than 15 %, most of those because
+    and 128, values of 64 to 256): of 3,325, 90 go the way that is slower by more than 3 %, 13 by more than 15 %, most of those because
     the lengths between the longest entry's and the shortest's are not known here."""
     if longest < least or entries < 1 or longest > T or key_dim not in chunk_us:
         return 0
@@ -1344,7 +1344,7 @@ def _chunks_or_walk(T: int, entries: int, longest: int, heads: int, key_dim: int
         return a_token * most * (alone if full <= 0.45 else max(1.0, (full + math.ceil(full)) / 2))
 
     def in_chunks(most: int, tokens: int, n: int) -> float:
-        units = (tokens // CHUNK_TOKENS + (n if tokens % (CHUNK_TOKENS * n) else 0)) * heads
+        units = n * -(-tokens // (CHUNK_TOKENS * n)) * heads
         return (fixed_us + a_set * -(-units // places) * (1 + a_column * value_dim / 64) + an_element * units * key_dim * value_dim
                 + a_link * -(-most // CHUNK_TOKENS))
     rest = T - longest
@@ -1359,8 +1359,8 @@ def _chunks_or_walk(T: int, entries: int, longest: int, heads: int, key_dim: int
 # the delta rule: 16 heads of 128 x 128 take 91 us in a walk and 85 in chunks at 256 tokens, 175 and 98 at 512, 680 and 241 at 2,048 (8
 # heads: 89 and 81, 171 and 93, 677 and 162); 8 heads of 64 x 64 58 and 41 at 192, 144 and 54 at 512
 DELTA_CHUNK_MIN_TOKENS = 192
-_DELTA_WALK_US, _DELTA_CHUNK_FIXED_US = {64: (0.335, 0.977), 128: (0.375, 0.931)}, 9.0
-_DELTA_CHUNK_US = {64: (30.2, 0.0, 1.30e-5, 1.40, 6.4), 128: (50.3, 0.0, 1.08e-5, 1.95, 4.9)}
+_DELTA_WALK_US, _DELTA_CHUNK_FIXED_US = {64: (0.313, 1.053), 128: (0.384, 0.937)}, 9.0
+_DELTA_CHUNK_US = {64: (29.9, 0.0, 1.35e-5, 1.54, 8.2), 128: (53.6, 0.0, 1.046e-5, 1.91, 4.9)}
 
 
 def _delta_chunk_sizes(heads: int, key_dim: int, value_dim: int) -> Tuple[int, ...]:
