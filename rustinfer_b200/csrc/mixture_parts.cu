@@ -595,7 +595,10 @@ RI_API int ri_moe_route(const float* z, const void* x, int x_dtype, const float*
     if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
     if ((z == nullptr) == (x == nullptr) || (x && !router)) return (int)cudaErrorInvalidValue;
     const dim3 grid((T + tt - 1) / tt);
-    const bool early = x && T <= ri_device_sms() * (16 / warps);             // all CTAs at once, with the registers that takes
+    // early: all CTAs at once, with the registers that takes; or up to three times as many where the rows are one round of a CTA's warps and
+    // long (300 tokens of 4,096, 8 and 32 experts: 28.9 and 31.2 us against 32.8 and 33.8; of 2,048, 32: 20.7 against 18.8)
+    const int places = ri_device_sms() * (16 / warps);
+    const bool early = !x || T <= places || (T <= 3 * places && rows <= 33 && d >= 4096);
 #define RI_MR(TX, TT, EARLY) RI_CHECKED(ri_launch(moe_route_kernel<TX, TT, EARLY>, grid, dim3(32 * warps), smem, (cudaStream_t)stream, z, (const TX*)x, router, d, \
                                            correction, T, E, top, n_groups > 0 ? n_groups : 0, keep, renorm, ids, weights, counts, score, \
                                            group_max, renorm_eps, gate))
@@ -638,12 +641,12 @@ RI_API int ri_moe_product(const void* a, int a_dtype, int a_stride, const void* 
                               ((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0 && ri_moe_tensor_cores();
     if (tensor_cores && ((gated && out_dtype == RI_BF16) || (!gated && out_dtype == RI_F32))) {
         // A fourth stage where it costs no wave of CTAs: an SM holds six of them with three stages and four with four.  How many find rows is
-        // the router's choice; an even one is taken, with a tenth to spare.  Three / four, us, 32 experts, four a token: 8 tokens of 1,024,
-        // gated 768 (one wave either way) 19.1 / 14.9, 64 tokens (one / two) 23.8 / 28.1; 64 of 1,408, gated 1,024 (two) 44.0 / 38.5; 4 of
-        // 2,880, 2,880 (one / two) 50.7 / 63.3.
+        // the router's choice; what an even one would give is taken.  Three / four, us, 32 experts, four a token: 8 tokens of 1,024, gated 768
+        // (one wave either way) 19.1 / 14.9, 64 tokens (one / two) 23.8 / 28.1; 64 of 1,408, gated 1,024 (two) 44.0 / 38.5; 12 of 2,880,
+        // 2,880 (two) 88.5 / 71.0.
         const double used = E * (1.0 - pow(1.0 - 1.0 / E, rows)), tiles = used * fmax(1.0, rows / (16.0 * E) + 0.5);
         const double resident = tiles * grid.y / ri_device_sms();
-        const bool deep = bm == 16 && ceil(1.1 * resident / 4) == ceil(resident / 6);
+        const bool deep = bm == 16 && ceil(resident / 4) == ceil(resident / 6);
 #define RI_MM(TO, BM, G, S) do { \
         static bool configured = false; \
         const size_t smem = moe_mma_smem<BM, S>(); \
