@@ -640,13 +640,14 @@ RI_API int ri_moe_product(const void* a, int a_dtype, int a_stride, const void* 
     const bool tensor_cores = a_dtype == RI_BF16 && w_dtype == RI_BF16 && K % 8 == 0 && a_stride % 8 == 0 &&
                               ((uintptr_t)a & 15) == 0 && ((uintptr_t)w & 15) == 0 && ri_moe_tensor_cores();
     if (tensor_cores && ((gated && out_dtype == RI_BF16) || (!gated && out_dtype == RI_F32))) {
-        // A fourth stage where it costs no wave of CTAs: an SM holds six of them with three stages and four with four.  How many find rows is
+        // A fourth stage where it costs no wave of CTAs, or one of many: an SM holds six of them with three stages and four with four.  How many find rows is
         // the router's choice; what an even one would give is taken.  Three / four, us, 32 experts, four a token: 8 tokens of 1,024, gated 768
         // (one wave either way) 19.1 / 14.9, 64 tokens (one / two) 23.8 / 28.1; 64 of 1,408, gated 1,024 (two) 44.0 / 38.5; 12 of 2,880,
-        // 2,880 (two) 88.5 / 71.0.
+        // 2,880 (two) 88.5 / 71.0; 32 of 2,880, gated 2,880 (four / five: one more of many is less than the stage brings) 193 / 182.
         const double used = E * (1.0 - pow(1.0 - 1.0 / E, rows)), tiles = used * fmax(1.0, rows / (16.0 * E) + 0.5);
         const double resident = tiles * grid.y / ri_device_sms();
-        const bool deep = bm == 16 && ceil(resident / 4) == ceil(resident / 6);
+        const double threes = ceil(resident / 6);
+        const bool deep = bm == 16 && ceil(resident / 4) <= threes + (threes >= 3 ? 1 : 0);
 #define RI_MM(TO, BM, G, S) do { \
         static bool configured = false; \
         const size_t smem = moe_mma_smem<BM, S>(); \
